@@ -702,6 +702,20 @@ def _attention_cost(q, rows: int, H: int, K: int, d: int, which: str) -> None:
         _pending_cost["rows"] = which
 
 
+#: 32-bit prompt portions go to the tile kernel (False: the plain kernel takes every row)
+use_attention_tiles = True
+#: ... when the step's longest portion has at least this many tokens (a tile's 32 rows are then at least a quarter full for two heads a kv head)
+ATTENTION_TILES_FROM = 4
+
+
+def _attention_tiles(q, k_cache, v_cache, out, H: int, K: int, d: int, window: int, ctx) -> bool:
+    """Whether the tile kernel takes the step's portions: float32, heads of up to 128 in whole 16-byte steps at 16-byte addresses, no window (its
+    chunks start at position 0, a window's at the window's first key)."""
+    return (use_attention_tiles and q.dtype == torch.float32 and d <= 128 and d % 4 == 0 and H // K <= 32 and window <= 0
+            and ctx.num_requests > ctx.num_decode and ctx.max_query_len >= ATTENTION_TILES_FROM
+            and all(t.data_ptr() % 16 == 0 for t in (q, k_cache, v_cache, out)))
+
+
 def attention(q, k_cache, v_cache, out, ctx, block_table, H, K, d, scale, window=0, plan: Optional[DecodePlan] = None) -> None:
     """Causal attention of the step's tokens over the paged cache (their own keys included).  The first
     ``ctx.num_decode`` requests bring one token each (rows 0..num_decode-1); the rest bring portions.  ``plan``
@@ -744,10 +758,22 @@ def attention(q, k_cache, v_cache, out, ctx, block_table, H, K, d, scale, window
                                        _c_int(ctx.max_query_len), _c_int(K), _c_int(page_size), _c_float(scale),
                                        _c_int(window), _stream()), "attention (prefill)")
         return
-    _attention_cost(q, T, H, K, d, "all")
+    rows = T
+    if _attention_tiles(q, k_cache, v_cache, out, H, K, d, window, ctx):
+        nd = ctx.num_decode
+        # 32-bit prompt portions by tiles of 32 rows: the same bits as the plain kernel's, which then takes the single tokens alone
+        _attention_cost(q, T - nd, H, K, d, "prefill" if nd else "all")
+        _check(_lib("mb_attention_simple").mb_attention_tile(
+            _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), _c_int(block_table.shape[1]), _ptr(ctx.cu_tokens), _ptr(ctx.seq_lens),
+            _c_int(nd), _c_int(ctx.num_requests - nd), _c_int(ctx.max_query_len), _c_int(H), _c_int(K), _c_int(d), _c_int(page_size),
+            _c_float(scale), _stream()), "attention (tiles)")
+        rows = nd
+    if rows == 0:
+        return
+    _attention_cost(q, rows, H, K, d, "all" if rows == T else "decode")
     _check(_lib("mb_attention_simple").mb_attention_simple(
         _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _code(q), _ptr(block_table), _c_int(block_table.shape[1]),
-        _ptr(ctx.req_index), _ptr(ctx.positions), _c_int(T), _c_int(H), _c_int(K), _c_int(d), _c_int(page_size),
+        _ptr(ctx.req_index), _ptr(ctx.positions), _c_int(rows), _c_int(H), _c_int(K), _c_int(d), _c_int(page_size),
         _c_float(scale), _c_int(window), _stream()), "attention")
 
 

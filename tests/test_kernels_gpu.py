@@ -810,3 +810,42 @@ def test_sampling_kernels_mark_rows_that_are_not_finite(ops):
     got = ids.tolist()
     assert [got[i] for i in (1, 3, 4)] == [-1, -1, -1] and got[0] == want[0] and all(0 <= got[i] < 50000 for i in (2, 5, 6))
     ops.check_device_errors()
+
+
+@pytest.mark.parametrize("H,K,d,page", [(16, 8, 128, 16), (10, 2, 64, 4), (6, 1, 36, 8), (33, 1, 16, 16), (4, 4, 100, 32)])
+def test_float32_attention_tiles_give_the_plain_kernels_bits(ops, H, K, d, page):
+    """Portions at the edges of tiles (32 rows), half chunks (64 keys) and chunks (128), behind cached positions and beside single tokens, with a
+    value that is not finite behind some queries' positions (33 heads a kv head and portions below four tokens stay with the plain kernel)."""
+    g = torch.Generator(device=DEV).manual_seed(7)
+    lens_new = [(200, 1), (64, 1), (1, 1), (2, 2), (128, 128), (129, 129), (300, 47), (333, 333), (16, 5), (500, 64)]
+    q, kc, vc, table, ctx = paged_case(g, torch.float32, lens_new, H, K, d, page, 700)
+    far = 583                                                          # of the request with 333 tokens behind 333: its last 83 see it
+    vc[int(table[7, far // page]), :, far % page] = math.nan
+    vc[int(table[7, far // page]), :, far % page, 0] = math.inf
+    got, want = torch.full_like(q, 7.0), torch.full_like(q, 9.0)
+    ops.attention(q, kc, vc, got, ctx, table, H, K, d, 1.0 / math.sqrt(d), 0)
+    ops.use_attention_tiles = False
+    try:
+        ops.attention(q, kc, vc, want, ctx, table, H, K, d, 1.0 / math.sqrt(d), 0)
+    finally:
+        ops.use_attention_tiles = True
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    assert int(torch.isfinite(got).all(dim=1).sum()) == got.shape[0] - 83
+
+
+@pytest.mark.parametrize("T,N,K", [(1, 32, 16), (33, 31, 15), (65, 3072, 17), (64, 3073, 64), (7, 65, 1023), (333, 1024, 3072), (100, 3200, 130)])
+def test_float32_product_at_tile_edges(ops, T, N, K):
+    """Sums of K products of numbers near 1 differ from 64 bits by at most about K roundings of partial sums of size sqrt(K); rows do not depend on
+    the batch, whatever the tile."""
+    g = torch.Generator().manual_seed(T + N + K)
+    x, w = torch.randn(T, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    out = torch.full((T, N), math.nan, device="cuda")
+    ops.gemm(x, w, out)
+    want = x.double() @ w.double().t()
+    assert float((out - want).abs().max()) <= 6e-8 * K * math.sqrt(K) + 1e-5
+    one = torch.empty(1, N, device="cuda")
+    ops.gemm(x[T - 1:].contiguous(), w, one)
+    assert torch.equal(one[0], out[T - 1])
+    added = out.clone()
+    ops.gemm(x, w, added, accumulate=True)
+    assert torch.equal(added, out + out)
