@@ -29,60 +29,15 @@ __host__ __device__ __forceinline__ int gate_up_row(int c, int which, int ff, in
     return interleaved ? (c / 16) * 32 + which * 16 + c % 16 : which * ff + c;
 }
 
-// ---- router and top-k: a token per block -------------------------------------------------------------------------------
+// ---- router and top-k: a token (or a few) per block -------------------------------------------------------------------------------
 // expert_out int32 [tokens][top], weight_out float32 [tokens][top], choices in order of decreasing score (the lower expert
 // among equals).  score_mode 0: sigmoid, 1: softmax over all experts.  A warp takes every eighth expert; its lanes walk the
 // row in a fixed order, so a token's logits do not depend on the batch.
-template <typename T>
-__global__ void __launch_bounds__(MR_THREADS) moe_route_kernel(const T* __restrict__ h_rows, const float* __restrict__ router,
-                                                               const float* __restrict__ router_bias, int* __restrict__ expert_out, float* __restrict__ weight_out,
-                                                               int tokens, int h, int E, int top, int score_mode, int renorm,
-                                                               const float* __restrict__ correction, int groups, int keep, float factor) {
-    PDL_ENTER();
-    h_rows = pdl_fresh(h_rows);
-    extern __shared__ float smem[];
-    float* xrow = smem;                        // [h] (first: 16-byte aligned)
-    float* z = smem + h;                       // [E]: logits, and what the choice goes by
-    float* score_of = z + E;                   // [E] (with a correction)
-    float* group_top = score_of + E;           // [groups]
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = blockIdx.x;
-    const T* x = h_rows + (size_t)t * h;
-    for (int i = threadIdx.x; i < h; i += MR_THREADS) xrow[i] = to_f32(x[i]);
-    __syncthreads();
-    for (int e = warp; e < E; e += MR_THREADS / 32) {
-        const float* w = router + (size_t)e * h;
-        float d0 = 0.0f, d1 = 0.0f, d2 = 0.0f, d3 = 0.0f;
-        int i = lane;
-        if ((h & 3) == 0 && (((uintptr_t)w) & 15) == 0) {         // 16-byte loads, four of them in flight
-            const float4* w4 = reinterpret_cast<const float4*>(w);
-            const float4* x4 = reinterpret_cast<const float4*>(xrow);
-            const int n4 = h >> 2;
-            int j = lane;
-            for (; j + 96 < n4; j += 128) {
-                const float4 a0 = w4[j], a1 = w4[j + 32], a2 = w4[j + 64], a3 = w4[j + 96];
-                const float4 b0 = x4[j], b1 = x4[j + 32], b2 = x4[j + 64], b3 = x4[j + 96];
-                d0 = fmaf(b0.x, a0.x, fmaf(b0.y, a0.y, fmaf(b0.z, a0.z, fmaf(b0.w, a0.w, d0))));
-                d1 = fmaf(b1.x, a1.x, fmaf(b1.y, a1.y, fmaf(b1.z, a1.z, fmaf(b1.w, a1.w, d1))));
-                d2 = fmaf(b2.x, a2.x, fmaf(b2.y, a2.y, fmaf(b2.z, a2.z, fmaf(b2.w, a2.w, d2))));
-                d3 = fmaf(b3.x, a3.x, fmaf(b3.y, a3.y, fmaf(b3.z, a3.z, fmaf(b3.w, a3.w, d3))));
-            }
-            for (; j < n4; j += 32) {
-                const float4 a0 = w4[j], b0 = x4[j];
-                d0 = fmaf(b0.x, a0.x, fmaf(b0.y, a0.y, fmaf(b0.z, a0.z, fmaf(b0.w, a0.w, d0))));
-            }
-            i = h;
-        }
-        for (; i + 96 < h; i += 128) {
-            d0 = fmaf(xrow[i], w[i], d0); d1 = fmaf(xrow[i + 32], w[i + 32], d1);
-            d2 = fmaf(xrow[i + 64], w[i + 64], d2); d3 = fmaf(xrow[i + 96], w[i + 96], d3);
-        }
-        for (; i < h; i += 32) d0 = fmaf(xrow[i], w[i], d0);
-        const float dot = warp_sum((d0 + d1) + (d2 + d3));
-        if (lane == 0) z[e] = router_bias != nullptr ? dot + router_bias[e] : dot;
-    }
-    __syncthreads();
-    if (warp != 0) return;
+
+// What a warp does with a token's logits z[E] (shared memory, left changed): the choice and the weights.  score_of: [E] (with a correction), group_top: [groups].
+__device__ __forceinline__ void moe_choose(float* z, float* score_of, float* group_top, int t, int* __restrict__ expert_out, float* __restrict__ weight_out, int E,
+                                           int top, int score_mode, int renorm, const float* __restrict__ correction, int groups, int keep, float factor) {
+    const int lane = threadIdx.x & 31;
     float denom = 1.0f, zmax = 0.0f;
     if (score_mode == 1) {
         float mx = -INFINITY;
@@ -147,6 +102,101 @@ __global__ void __launch_bounds__(MR_THREADS) moe_route_kernel(const T* __restri
         }
 }
 
+template <typename T>
+__global__ void __launch_bounds__(MR_THREADS) moe_route_kernel(const T* __restrict__ h_rows, const float* __restrict__ router,
+                                                               const float* __restrict__ router_bias, int* __restrict__ expert_out, float* __restrict__ weight_out,
+                                                               int tokens, int h, int E, int top, int score_mode, int renorm,
+                                                               const float* __restrict__ correction, int groups, int keep, float factor) {
+    PDL_ENTER();
+    h_rows = pdl_fresh(h_rows);
+    extern __shared__ float smem[];
+    float* xrow = smem;                        // [h] (first: 16-byte aligned)
+    float* z = smem + h;                       // [E]: logits, and what the choice goes by
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t = blockIdx.x;
+    const T* x = h_rows + (size_t)t * h;
+    for (int i = threadIdx.x; i < h; i += MR_THREADS) xrow[i] = to_f32(x[i]);
+    __syncthreads();
+    for (int e = warp; e < E; e += MR_THREADS / 32) {
+        const float* w = router + (size_t)e * h;
+        float d0 = 0.0f, d1 = 0.0f, d2 = 0.0f, d3 = 0.0f;
+        int i = lane;
+        if ((h & 3) == 0 && (((uintptr_t)w) & 15) == 0) {         // 16-byte loads, four of them in flight
+            const float4* w4 = reinterpret_cast<const float4*>(w);
+            const float4* x4 = reinterpret_cast<const float4*>(xrow);
+            const int n4 = h >> 2;
+            int j = lane;
+            for (; j + 96 < n4; j += 128) {
+                const float4 a0 = w4[j], a1 = w4[j + 32], a2 = w4[j + 64], a3 = w4[j + 96];
+                const float4 b0 = x4[j], b1 = x4[j + 32], b2 = x4[j + 64], b3 = x4[j + 96];
+                d0 = fmaf(b0.x, a0.x, fmaf(b0.y, a0.y, fmaf(b0.z, a0.z, fmaf(b0.w, a0.w, d0))));
+                d1 = fmaf(b1.x, a1.x, fmaf(b1.y, a1.y, fmaf(b1.z, a1.z, fmaf(b1.w, a1.w, d1))));
+                d2 = fmaf(b2.x, a2.x, fmaf(b2.y, a2.y, fmaf(b2.z, a2.z, fmaf(b2.w, a2.w, d2))));
+                d3 = fmaf(b3.x, a3.x, fmaf(b3.y, a3.y, fmaf(b3.z, a3.z, fmaf(b3.w, a3.w, d3))));
+            }
+            for (; j < n4; j += 32) {
+                const float4 a0 = w4[j], b0 = x4[j];
+                d0 = fmaf(b0.x, a0.x, fmaf(b0.y, a0.y, fmaf(b0.z, a0.z, fmaf(b0.w, a0.w, d0))));
+            }
+            i = h;
+        }
+        for (; i + 96 < h; i += 128) {
+            d0 = fmaf(xrow[i], w[i], d0); d1 = fmaf(xrow[i + 32], w[i + 32], d1);
+            d2 = fmaf(xrow[i + 64], w[i + 64], d2); d3 = fmaf(xrow[i + 96], w[i + 96], d3);
+        }
+        for (; i < h; i += 32) d0 = fmaf(xrow[i], w[i], d0);
+        const float dot = warp_sum((d0 + d1) + (d2 + d3));
+        if (lane == 0) z[e] = router_bias != nullptr ? dot + router_bias[e] : dot;
+    }
+    __syncthreads();
+    if (warp == 0) moe_choose(z, z + E, z + 2 * E, t, expert_out, weight_out, E, top, score_mode, renorm, correction, groups, keep, factor);
+}
+
+// The same sums (the same chains, the same bits) straight from memory in bf16, a warp a token and expert, no row staged ahead: the kernel above is a
+// chain of waits, the row's numbers two bytes at a time, then the experts (10 us for 48 tokens, 31 us for 2,048 of 2,560 and 8 experts).
+// MANY: a block takes eight tokens, a warp each, whose loads of a router row meet in L1; else a block takes one token, its warps the experts in turn.
+__device__ __forceinline__ float route_dot(const bf16* __restrict__ x, const float* __restrict__ w, int h) {
+    const float4* w4 = reinterpret_cast<const float4*>(w);
+    const uint2* x4 = reinterpret_cast<const uint2*>(x);
+    const int n4 = h >> 2;
+    float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    auto add = [](float& s, const uint2& u, const float4& a) {
+        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+        s = fmaf(lo.x, a.x, fmaf(lo.y, a.y, fmaf(hi.x, a.z, fmaf(hi.y, a.w, s))));
+    };
+    int j = threadIdx.x & 31;
+#pragma unroll 2
+    for (; j + 96 < n4; j += 128) {
+        const float4 a[4] = {w4[j], w4[j + 32], w4[j + 64], w4[j + 96]};
+        const uint2 b[4] = {x4[j], x4[j + 32], x4[j + 64], x4[j + 96]};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) add(d[c], b[c], a[c]);
+    }
+    for (; j < n4; j += 32) add(d[0], x4[j], w4[j]);
+    return warp_sum((d[0] + d[1]) + (d[2] + d[3]));
+}
+
+template <bool MANY>
+__global__ void __launch_bounds__(MR_THREADS) moe_route_direct_kernel(const bf16* __restrict__ h_rows, const float* __restrict__ router,
+                                                                      const float* __restrict__ router_bias, int* __restrict__ expert_out,
+                                                                      float* __restrict__ weight_out, int tokens, int h, int E, int top, int score_mode, int renorm,
+                                                                      const float* __restrict__ correction, int groups, int keep, float factor) {
+    PDL_ENTER();
+    h_rows = pdl_fresh(h_rows);
+    extern __shared__ float smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per = 2 * E + groups;
+    const int t = MANY ? blockIdx.x * (MR_THREADS / 32) + warp : blockIdx.x;
+    if (t >= tokens) return;                                   // (many: nobody waits for this warp)
+    float* z = smem + (MANY ? warp * per : 0);
+    for (int e = MANY ? 0 : warp; e < E; e += MANY ? 1 : MR_THREADS / 32) {
+        const float dot = route_dot(h_rows + (size_t)t * h, router + (size_t)e * h, h);
+        if (lane == 0) z[e] = router_bias != nullptr ? dot + router_bias[e] : dot;
+    }
+    if (MANY) __syncwarp();
+    else __syncthreads();
+    if (MANY || warp == 0) moe_choose(z, z + E, z + 2 * E, t, expert_out, weight_out, E, top, score_mode, renorm, correction, groups, keep, factor);
+}
+
 // E: all outputs of the router (identity outputs included).  groups 1: no groups; correction null: none; factor: on the weights.
 MB_API int mb_moe_route(const void* h_rows, int dtype, const float* router, const float* router_bias, int* expert_out, float* weight_out, int tokens, int h,
                         int E, int top, int score_mode, int renorm, const float* correction, int groups, int keep, float factor, cudaStream_t s) {
@@ -155,6 +205,15 @@ MB_API int mb_moe_route(const void* h_rows, int dtype, const float* router, cons
     if (groups <= 0 || E % groups != 0 || keep <= 0 || keep > groups || (keep < groups && top > E / groups * keep)) return MB_ERR_BAD_SIZE;
     const size_t smem = (size_t)(2 * E + groups + h) * sizeof(float);
     if (smem > 48 * 1024) return MB_ERR_BAD_SIZE;
+    const size_t per = (size_t)(2 * E + groups) * sizeof(float), few = MR_THREADS / 32;
+    if (dtype == MB_BF16 && h % 4 == 0 && (((uintptr_t)h_rows) & 7) == 0 && (((uintptr_t)router) & 15) == 0) {
+        // a warp a token once that puts a block on every SM (148 blocks of eight tokens)
+        if (tokens >= 148 * (int)few && few * per <= 48 * 1024)
+            return launch_kernel(moe_route_direct_kernel<true>, (tokens + (int)few - 1) / (int)few, MR_THREADS, few * per, s, 0, (const bf16*)h_rows, router, router_bias,
+                                 expert_out, weight_out, tokens, h, E, top, score_mode, renorm, correction, groups, keep, factor);
+        return launch_kernel(moe_route_direct_kernel<false>, tokens, MR_THREADS, per, s, 0, (const bf16*)h_rows, router, router_bias, expert_out, weight_out, tokens,
+                             h, E, top, score_mode, renorm, correction, groups, keep, factor);
+    }
     if (dtype == MB_F32)
         return launch_kernel(moe_route_kernel<float>, tokens, MR_THREADS, smem, s, 0, (const float*)h_rows, router, router_bias, expert_out,
                              weight_out, tokens, h, E, top, score_mode, renorm, correction, groups, keep, factor);
@@ -352,6 +411,13 @@ __global__ void moe_gather_kernel(const T* __restrict__ h_rows, const int* __res
     const int token = p / top;
     const float w = weight_of[p];
     if (threadIdx.x == 0 && blockIdx.y == 0) { token_sorted[i] = token; weight_sorted[i] = w; inv[p] = i; }
+    if (!weight_on_input && ((h * sizeof(T)) & 15) == 0 && (((uintptr_t)h_rows | (uintptr_t)xs) & 15) == 0) {      // rows as they are: 16 bytes at a time
+        const uint4* src = reinterpret_cast<const uint4*>(h_rows + (size_t)token * h);
+        uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)i * h);
+        const int n = (int)(h * sizeof(T) / 16);
+        for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < n; c += gridDim.y * blockDim.x) dst[c] = src[c];
+        return;
+    }
     const float f = weight_on_input ? w : 1.0f;
     for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < h; c += gridDim.y * blockDim.x)
         xs[(size_t)i * h + c] = from_f32<T>(to_f32(h_rows[(size_t)token * h + c]) * f);
@@ -503,25 +569,45 @@ __global__ void __launch_bounds__(128) moe_grouped_kernel(const bf16* __restrict
 }
 
 // y[t][c] += sum over the token's choices, in choice order, of rows[inv[t top + choice]][c] (times the choice's weight, if given);
-// a choice numbered E or above is the identity: its row is h_rows[t] times identity_weight
+// a choice numbered E or above is the identity: its row is h_rows[t] times identity_weight.  more (null: none): rows [tokens][h] added last.
+// rows and more may come in `parts` parts, rows_part and more_part numbers apart: a row is their sum, in order.
+// Bound by the bytes: four columns a thread by 16-byte accesses (h a multiple of 4).
 __global__ void moe_combine_kernel(const float* __restrict__ rows, const int* __restrict__ inv, const float* __restrict__ weight_of,
                                    float* __restrict__ y, int h, int top, const int* __restrict__ expert_of, const bf16* __restrict__ h_rows,
-                                   const float* __restrict__ identity_weight, int E) {
+                                   const float* __restrict__ identity_weight, int E, const float* __restrict__ more, int parts,
+                                   long long rows_part, long long more_part) {
     PDL_ENTER();
     rows = pdl_fresh(rows); inv = pdl_fresh(inv); y = pdl_fresh(y); weight_of = pdl_fresh(weight_of);
-    expert_of = pdl_fresh(expert_of); h_rows = pdl_fresh(h_rows); identity_weight = pdl_fresh(identity_weight);
+    expert_of = pdl_fresh(expert_of); h_rows = pdl_fresh(h_rows); identity_weight = pdl_fresh(identity_weight); more = pdl_fresh(more);
     const int t = blockIdx.x;
-    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < h; c += gridDim.y * blockDim.x) {
-        float a = y[(size_t)t * h + c];
+    for (int c = 4 * (blockIdx.y * blockDim.x + threadIdx.x); c < h; c += 4 * gridDim.y * blockDim.x) {
+        float4 a = *reinterpret_cast<const float4*>(y + (size_t)t * h + c);
         for (int k = 0; k < top; ++k) {
             if (h_rows != nullptr && expert_of[t * top + k] >= E) {
-                a += identity_weight[t * top + k] * __bfloat162float(h_rows[(size_t)t * h + c]);
+                const float w = identity_weight[t * top + k];
+                const bf16* x = h_rows + (size_t)t * h + c;
+                a.x += w * __bfloat162float(x[0]); a.y += w * __bfloat162float(x[1]);
+                a.z += w * __bfloat162float(x[2]); a.w += w * __bfloat162float(x[3]);
                 continue;
             }
-            const float v = rows[(size_t)inv[t * top + k] * h + c];
-            a += weight_of != nullptr ? v * weight_of[t * top + k] : v;
+            const float* src = rows + (size_t)inv[t * top + k] * h + c;
+            float4 v = *reinterpret_cast<const float4*>(src);
+            for (int z = 1; z < parts; ++z) {
+                const float4 p = *reinterpret_cast<const float4*>(src + z * rows_part);
+                v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+            }
+            const float w = weight_of != nullptr ? weight_of[t * top + k] : 1.0f;
+            a.x += v.x * w; a.y += v.y * w; a.z += v.z * w; a.w += v.w * w;
         }
-        y[(size_t)t * h + c] = a;
+        if (more != nullptr) {
+            float4 v = *reinterpret_cast<const float4*>(more + (size_t)t * h + c);
+            for (int z = 1; z < parts; ++z) {
+                const float4 p = *reinterpret_cast<const float4*>(more + z * more_part + (size_t)t * h + c);
+                v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+            }
+            a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+        }
+        *reinterpret_cast<float4*>(y + (size_t)t * h + c) = a;
     }
 }
 
@@ -583,9 +669,11 @@ MB_API int mb_moe_grouped_down(const void* act, const void* w_down, const int* o
     return grouped_by_rows<1>((const bf16*)act, (const bf16*)w_down, offsets, E, h, ff, nullptr, out, dst_rows, row_scale, accumulate, 0, pairs, s);
 }
 
-// h_rows null: no identity choices (expert_of, identity_weight and E are not read).
+// h_rows null: no identity choices (expert_of, identity_weight and E are not read); more null: no further rows.
 MB_API int mb_moe_combine(const float* rows, const int* inv, const float* weight_of, float* y, int tokens, int h, int top, const int* expert_of,
-                          const void* h_rows, const float* identity_weight, int E, cudaStream_t s) {
+                          const void* h_rows, const float* identity_weight, int E, const float* more, int parts, cudaStream_t s) {
     if (tokens <= 0) return 0;
-    return launch_kernel(moe_combine_kernel, spread(tokens, h, 256), 256, 0, s, 0, rows, inv, weight_of, y, h, top, expert_of, (const bf16*)h_rows, identity_weight, E);
+    if (parts < 1 || h % 4 != 0 || (((uintptr_t)rows | (uintptr_t)y | (uintptr_t)more) & 15) != 0) return MB_ERR_BAD_SIZE;
+    return launch_kernel(moe_combine_kernel, dim3(tokens, tokens >= 512 ? 1 : (h / 4 + 127) / 128), tokens >= 512 ? 256 : 128, 0, s, 0, rows, inv, weight_of, y, h, top,
+                         expert_of, (const bf16*)h_rows, identity_weight, E, more, parts, (long long)tokens * top * h, (long long)tokens * h);
 }

@@ -159,6 +159,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "mb_attention_sink": ["attention_sink.cu"],
     "mb_attention_latent": ["attention_latent.cu"],
     "mb_moe": ["moe.cu"],
+    "mb_moe_tc": ["moe_tc.cu"],
     "mb_attention_pooled": ["attention_pooled.cu"],
     "mb_ssm": ["ssm.cu"],
     "mb_layer_norm": ["layer_norm.cu"],

@@ -1756,34 +1756,60 @@ def fast_experts_supported(h: int, ff: int) -> bool:
 
 
 def moe_jobs(dtype, h: int, ff: int) -> dict:
-    return library_jobs("mb_moe")
+    return library_jobs("mb_moe", "mb_moe_tc") if dtype == torch.bfloat16 and fast_experts_supported(h, ff) else library_jobs("mb_moe")
 
 
-#: from this many (token, choice) pairs per expert on, a step that is not being captured in a graph reads the experts'
-#: counts back to the host and gives every expert's rows to the dense tcgen05 products (``gemm_swiglu``, ``gemm``) instead
-#: of the grouped mma.sync kernel
-EXPERTS_DENSE_FROM = 96
-#: streams the experts' dense products are dealt over: one expert's products fill the device only partly (a quarter of the
-#: step's rows, tiles that do not make whole rounds over the SMs), several at a time fill the gaps.  1: one after the other.
-EXPERT_STREAMS = 4
-_side_streams = {}
+#: from this many (token, choice) pairs on, the experts' products go to the persistent tcgen05 kernel; below, to the grouped mma.sync kernel,
+#: whose smaller tiles put more CTAs on the few experts that are read
+EXPERTS_TC_FROM = 1
 
 
-def _expert_streams(device, n: int):
-    key = (device.index, n)
-    if key not in _side_streams:
-        _side_streams[key] = [torch.cuda.Stream(device=device) for _ in range(n)]
-    return _side_streams[key]
+#: the capped form runs behind the plain product, whose rows are bf16: only with many pairs an expert (the mma.sync kernel applies it to its float32 sums)
+EXPERTS_CAPPED_TC_FROM = 96
+
+
+def _experts_on_tcgen05(E: int, pairs: int, interleaved: bool, activation: str) -> bool:
+    """Whether the grouped tcgen05 products take these experts (up to 512; a gated form that its epilogue applies needs gate and up rows in alternating
+    blocks)."""
+    if activation == "glu_capped" and (pairs < EXPERTS_CAPPED_TC_FROM * E or torch.cuda.is_current_stream_capturing()):
+        return False
+    return use_tensor_cores and E <= 512 and pairs >= EXPERTS_TC_FROM and (interleaved or activation != "swiglu")
+
+
+def _expert_tile(pairs: int, E: int) -> int:
+    """The widest tile of rows, from the experts' average share: one tile holds an ordinary expert's rows while the rows are few (its weights are then
+    read once, and a small tile leaves room for a deep ring); equal tiles of at most 256 beyond."""
+    average = pairs / E
+    return 32 if average <= 20 else 64 if average <= 44 else 128 if average <= 100 else 256
+
+
+def _down_parts(touched: int, shared_rows: int, average: float, tile: int, h: int, ff: int, shared_ff: int) -> int:
+    """Parts of K the experts' last products are cut into: with few rows there are few tiles (8 experts of width 2,560: 160 for 148 SMs, two rounds), and the parts
+    make the rounds finer.  A part keeps at least eight k-blocks; beyond a hundred rows an expert the tensor pipe, not the rounds, sets the time."""
+    if average > 100:
+        return 1
+    tiles = -(-h // 128) * (touched + -(-shared_rows // tile))
+    kbs = [k // 64 for k in (ff, shared_ff) if k]
+    fits = [p for p in (1, 2, 3, 4) if all(-(-n // p) >= 8 and (p - 1) * -(-n // p) < n for n in kbs)] or [1]
+    return min(fits, key=lambda p: (-(-tiles * p // SM_COUNT) / p + 0.02 * p, p))
+
+
+def moe_joins_shared(x: torch.Tensor, h: int, ff: int, shared_ff: int, E: int, top: int, interleaved: bool, activation: str) -> bool:
+    """Whether ``moe_experts`` takes a shared expert of this width into its launches (``shared``): the tcgen05 products, sizes in steps of 64."""
+    return (use_fast_experts and x.dtype == torch.bfloat16 and fast_experts_supported(h, ff) and shared_ff % 64 == 0 and activation != "glu_capped"
+            and _experts_on_tcgen05(E, x.shape[0] * top, interleaved, activation) and x.data_ptr() % 16 == 0 and x.shape[0] > 0)
 
 
 def moe_experts(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, experts: torch.Tensor, weights: torch.Tensor,
                 y: torch.Tensor, weight_on_input: bool, workspace, interleaved: bool = False, activation: str = "swiglu", form=None,
-                identity: int = 0) -> None:
+                identity: int = 0, shared=None) -> None:
     """The chosen experts' outputs added into ``y`` (float32 ``[T, h]``); see ``moe_experts_plain``.  Choices may also name ``identity``
     numbers behind the experts': the grouped products never see their pairs, the sum over a token's choices adds them.  bf16 with sizes in steps
-    of 64: the pairs are sorted by expert on the device and their inputs gathered in that order; then either two grouped
-    products over all experts (few pairs: single-token steps, captured or not: nothing is read back), or, with many pairs
-    per expert, the dense tensor-core products expert by expert over the sorted rows (the counts are read back once)."""
+    of 64: the pairs are sorted by expert on the device and their inputs gathered in that order; then two grouped products over all experts, on the
+    tensor cores, which read the experts' shares on the device (nothing is read back: a step may be captured).
+
+    ``shared`` (``(first, down)``, where ``moe_joins_shared`` says so): the matrices of one more expert of the same form that every token goes through with
+    weight 1; its products ride in the same two launches and its result is added last."""
     T, top = experts.shape
     E, h, ff = w_down.shape
     pairs = T * top
@@ -1811,54 +1837,10 @@ def moe_experts(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, 
     _cost(2 * pairs * h * size)
     _check(lib.mb_moe_gather(_ptr(x), _ptr(order), _ptr(weights), _ptr(xs), _ptr(token_sorted), _ptr(weight_sorted), _ptr(inv), _c_int(pairs),
                              _c_int(h), _c_int(top), _c_int(int(weight_on_input)), _stream()), "experts' inputs gathered")
-    dense = ((interleaved or not gated or activation == "glu_capped") and pairs >= EXPERTS_DENSE_FROM * E and use_tensor_cores and not torch.cuda.is_current_stream_capturing())
-    if dense:
-        rows = workspace.get("moe_rows", (pairs, h), torch.float32)
-        bounds = offsets.tolist()                       # the one wait on the host: how many pairs each expert got
-        active = [e for e in range(E) if bounds[e + 1] > bounds[e]]
-        # (while the stages of a step are being recorded everything stays on one stream, in launch order)
-        lanes = min(EXPERT_STREAMS, len(active)) if launch_log is None else 1
-        gate_up = workspace.get("moe_gate_up", (pairs, 2 * ff), x.dtype) if activation == "glu_capped" else None
-
-        def first_product(lo, hi, e):
-            if activation == "glu_capped":        # the dense product, then the capped form over its rows (gate rows first)
-                gemm(xs[lo:hi], w_gate_up[e], gate_up[lo:hi])
-                glu_capped(gate_up[lo:hi], ff, act[lo:hi], limit, alpha, shift)
-            elif gated:
-                gemm_swiglu(xs[lo:hi], w_gate_up[e], act[lo:hi], workspace)
-            else:
-                gemm_act(xs[lo:hi], w_gate_up[e], act[lo:hi], "relu2")
-
-        if lanes <= 1:
-            for e in active:
-                lo, hi = bounds[e], bounds[e + 1]
-                first_product(lo, hi, e)
-                gemm(act[lo:hi], w_down[e], rows[lo:hi])
-        else:
-            global stream_k
-            current = torch.cuda.current_stream(x.device)
-            side = _expert_streams(x.device, lanes)
-            ready = torch.cuda.Event()
-            ready.record(current)
-            keep, stream_k = stream_k, False            # stream-K parks tiles in scratch memory that one stream of work owns
-            try:
-                for i, e in enumerate(active):
-                    lo, hi = bounds[e], bounds[e + 1]
-                    if i < lanes:
-                        side[i].wait_event(ready)
-                    with torch.cuda.stream(side[i % lanes]):
-                        first_product(lo, hi, e)
-                        gemm(act[lo:hi], w_down[e], rows[lo:hi])
-            finally:
-                stream_k = keep
-            for st in side:
-                done = torch.cuda.Event()
-                done.record(st)
-                current.wait_event(done)
-        _cost(_size(rows) + 2 * _size(y))
-        _check(lib.mb_moe_combine(_ptr(rows), _ptr(inv), _ptr(None if weight_on_input else weights), _ptr(y), _c_int(T), _c_int(h),
-                                  _c_int(top), *same, _stream()), "experts' outputs added")
+    if _experts_on_tcgen05(E, pairs, interleaved, activation) and w_gate_up.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0:
+        _experts_tc(x, xs, w_gate_up, w_down, offsets, act, inv, weights, y, weight_on_input, workspace, activation, (limit, alpha, shift), same, shared)
         return
+    assert shared is None
     _cost(touched * (2 if gated else 1) * ff * h * size + pairs * (h + ff) * size, (4.0 if gated else 2.0) * pairs * ff * h)
     _check(lib.mb_moe_grouped_gate_up(_ptr(xs), _ptr(w_gate_up), _ptr(offsets), _ptr(act), _c_int(pairs), _c_int(h), _c_int(ff), _c_int(E),
                                       _c_int(int(interleaved)), _c_int(EXPERT_ACTIVATIONS[activation]), _c_float(limit), _c_float(alpha),
@@ -1874,7 +1856,47 @@ def moe_experts(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, 
     _check(lib.mb_moe_grouped_down(_ptr(act), _ptr(w_down), _ptr(offsets), _ptr(rows), _ptr(None), _ptr(scale), _c_int(0),
                                    _c_int(pairs), _c_int(h), _c_int(ff), _c_int(E), _stream()), "experts, down (grouped, tensor cores)")
     _cost(_size(rows) + 2 * _size(y))
-    _check(lib.mb_moe_combine(_ptr(rows), _ptr(inv), _ptr(None), _ptr(y), _c_int(T), _c_int(h), _c_int(top), *same, _stream()), "experts' outputs added")
+    _check(lib.mb_moe_combine(_ptr(rows), _ptr(inv), _ptr(None), _ptr(y), _c_int(T), _c_int(h), _c_int(top), *same, _ptr(None), _c_int(1),
+                              _stream()), "experts' outputs added")
+
+
+def _experts_tc(x, xs, w_gate_up, w_down, offsets, act, inv, weights, y, weight_on_input: bool, workspace, activation: str, form, same, shared) -> None:
+    """The products of ``moe_experts`` by the persistent tcgen05 kernel, a shared expert's in the same launches, and the sum over a token's choices."""
+    T, top = weights.shape
+    E, h, ff = w_down.shape
+    pairs, size, touched = xs.shape[0], x.element_size(), min(xs.shape[0], w_down.shape[0])
+    gated = activation != "relu2"
+    lib, s, tile = _lib("mb_moe_tc"), _scratch_for(x.device), _expert_tile(pairs, E)
+    first2 = down2 = act2 = rows2 = None
+    ff2 = 0
+    if shared is not None:
+        first2, down2 = shared
+        ff2 = down2.shape[1]
+    n2 = T if shared is not None else 0
+    parts = _down_parts(touched, T if n2 else 0, pairs / E, tile, h, ff, ff2)
+    if n2:
+        act2, rows2 = workspace.get("moe_shared_act", (T, ff2), x.dtype), workspace.get("moe_shared_rows", (parts, T, h), torch.float32)
+    capped = activation == "glu_capped"
+    mode = 0 if capped else _GLU_MODES["silu"] if gated else 4
+    first = workspace.get("moe_gate_up", (pairs, 2 * ff), x.dtype) if capped else act
+    N = w_gate_up.shape[1]
+    _cost(touched * N * h * size + pairs * (h + ff) * size + (_size(first2) + _size(x) + _size(act2) if n2 else 0),
+          2.0 * pairs * N * h + (2.0 * T * first2.numel() if n2 else 0.0))
+    _check(lib.mb_moe_grouped_tc(_ptr(xs), _ptr(w_gate_up), _ptr(offsets), _c_int(E), _c_int(pairs), _c_int(N), _c_int(h), _ptr(first), _ptr(x if n2 else None),
+                                 _ptr(first2), _c_int(n2), _c_int(first2.shape[0] if n2 else 0), _c_int(h), _ptr(act2), _c_int(mode), _c_int(tile),
+                                 _c_int(1), _c_int(SM_COUNT), _ptr(s.error), _stream()),
+           "experts, gate|up (grouped, tcgen05)" if gated else "experts, up, relu squared (grouped, tcgen05)")
+    if capped:
+        glu_capped(first, ff, act, *form)
+    rows = workspace.get("moe_rows", (parts, pairs, h), torch.float32)
+    _cost(touched * ff * h * size + pairs * ff * size + _size(rows) + (_size(down2) + _size(act2) + _size(rows2) if n2 else 0),
+          2.0 * pairs * ff * h + (2.0 * T * down2.numel() if n2 else 0.0))
+    _check(lib.mb_moe_grouped_tc(_ptr(act), _ptr(w_down), _ptr(offsets), _c_int(E), _c_int(pairs), _c_int(h), _c_int(ff), _ptr(rows), _ptr(act2), _ptr(down2),
+                                 _c_int(n2), _c_int(h if n2 else 0), _c_int(ff2), _ptr(rows2), _c_int(1), _c_int(tile), _c_int(parts), _c_int(SM_COUNT),
+                                 _ptr(s.error), _stream()), "experts, down (grouped, tcgen05)")
+    _cost(_size(rows) + 2 * _size(y) + (_size(rows2) if n2 else 0))
+    _check(_lib("mb_moe").mb_moe_combine(_ptr(rows), _ptr(inv), _ptr(None if weight_on_input else weights), _ptr(y), _c_int(T), _c_int(h), _c_int(top), *same,
+                                         _ptr(rows2), _c_int(parts), _stream()), "experts' outputs added")
 
 
 # ---- attention over a window and pooled blocks before it (csrc/attention_pooled.cu) ------------------------------------------------

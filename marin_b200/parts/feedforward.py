@@ -365,8 +365,15 @@ class RoutedExperts(FeedForward):
             ops.moe_route(x, self.router, chosen, weights, self.score, self.renormalize, self.router_b, self.correction_b, self.groups,
                           self.keep_groups, self.weight_scale)
         ops.stage_name = "experts"
+        # (a shared expert's two products ride in the experts' launches where those are the tcgen05 ones)
+        joined = None
+        if self.shared is not None and self.form is None:
+            first, down = (self.shared.w_gate_up, self.shared.w_down) if self.gated else (self.shared.w_up, self.shared.w_down)
+            if (getattr(self.shared, "fused", True) and down.dtype == x.dtype
+                    and ops.moe_joins_shared(x, self.hidden, self.intermediate, down.shape[1], self.experts, self.top, self.interleaved, self.activation)):
+                joined = (first, down)
         ops.moe_experts(x, self.w_gate_up, self.w_down, chosen, weights, residual, self.weight_on == "input", ws, self.interleaved,
-                        self.activation, self.form, self.identity)
-        if self.shared is not None:
+                        self.activation, self.form, self.identity, joined)
+        if self.shared is not None and joined is None:
             self.shared.forward(x, ctx, residual)
         return None

@@ -849,3 +849,58 @@ def test_float32_product_at_tile_edges(ops, T, N, K):
     added = out.clone()
     ops.gemm(x, w, added, accumulate=True)
     assert torch.equal(added, out + out)
+
+
+@pytest.mark.parametrize("activation,form", [("swiglu", None), ("relu2", None), ("glu_capped", (2.0, 1.5, 1.0))])
+@pytest.mark.parametrize("counts,h,ff,shared_ff", [((1,), 64, 64, 0), ((0, 16, 17, 0, 33, 1), 128, 192, 64), ((300, 0, 257, 256, 40), 192, 320, 128),
+                                                   ((64, 65, 31, 60), 320, 64, 192), ((2,) * 100, 64, 128, 0), ((540, 3), 128, 128, 64)])
+def test_grouped_expert_products_on_tcgen05_match_the_plain_twin(ops, request, activation, form, counts, h, ff, shared_ff):
+    """Experts whose rows fill no tile, one, or several (their widths follow the count), experts without rows, odd tiles of weight rows, the shared expert's
+    rows in the same launches, identity choices.  The twin rounds the activation to bf16 as well, so results differ where a sum in another order moves a
+    rounding: one bf16 step (2^-8) of some of ff terms.  The capped form runs over rows of gate and up numbers that are bf16 (the twin's are float32):
+    a rounding of 2^-9 / sqrt(3) = 1.1e-3 root mean square each, which the gate's slope of up to 1 + alpha |g| can double."""
+    from marin_b200.engine.context import Workspace
+
+    ops.EXPERTS_CAPPED_TC_FROM, keep = 0, ops.EXPERTS_CAPPED_TC_FROM
+    request.addfinalizer(lambda: setattr(ops, "EXPERTS_CAPPED_TC_FROM", keep))
+    E, T, identity = len(counts), sum(counts), 2 if activation == "swiglu" else 0
+    g = torch.Generator(device=DEV).manual_seed(T + h)
+    first = torch.tensor([e for e, n in enumerate(counts) for _ in range(n)], dtype=torch.int32, device=DEV)[torch.randperm(T, generator=g, device=DEV)]
+    other = torch.randint(0, E + identity, (T,), generator=g, device=DEV, dtype=torch.int32)
+    experts = torch.stack([first, other], dim=1).contiguous()
+    weights = torch.rand(T, 2, generator=g, device=DEV)
+    rnd = lambda *shape: (torch.randn(*shape, generator=g, device=DEV) * shape[-1] ** -0.5).to(torch.bfloat16)
+    x = torch.randn(T, h, generator=g, device=DEV).to(torch.bfloat16)
+    gated, interleaved = activation != "relu2", activation == "swiglu"
+    w1 = rnd(E, (2 if gated else 1) * ff, h)
+    w2 = rnd(E, h, ff)
+    shared = None
+    y0 = torch.randn(T, h, generator=g, device=DEV)
+    want, got = y0.clone(), y0.clone()
+    ops.moe_experts_plain(x, w1, w2, experts, weights, torch.empty(T * 2, ff, device=DEV, dtype=torch.bfloat16), want, False, interleaved, activation, form)
+    if shared_ff and activation != "glu_capped":
+        assert ops.moe_joins_shared(x, h, ff, shared_ff, E, 2, interleaved, activation)
+        shared = (rnd((2 if gated else 1) * shared_ff, h), rnd(h, shared_ff))
+        none = torch.zeros(T, 1, dtype=torch.int32, device=DEV)
+        ops.moe_experts_plain(x, shared[0][None], shared[1][None], none, torch.ones(T, 1, device=DEV), torch.empty(T, shared_ff, device=DEV, dtype=torch.bfloat16),
+                              want, False, interleaved, activation, form)
+    ops.moe_experts(x, w1, w2, experts, weights, got, False, Workspace(DEV), interleaved, activation, form, identity, shared)
+    ops.check_device_errors()
+    off = (got - want).abs()
+    assert float(off.pow(2).mean().sqrt()) <= (4e-3 if activation == "glu_capped" else 2e-3) * float((want - y0).pow(2).mean().sqrt())
+    assert float(off.max()) <= 0.05 * float((want - y0).abs().max())
+
+
+@pytest.mark.parametrize("T,h,E", [(1183, 96, 3), (1184, 96, 8), (1187, 2560, 9), (2049, 52, 20), (5, 2560, 64), (3, 132, 7)])
+def test_router_straight_from_memory_has_the_staged_kernels_bits(ops, T, h, E):
+    """A warp a token (from 1,184 on), a block a token below, and the kernel that stages the row (taken for rows that are not at 8-byte addresses)."""
+    g = torch.Generator(device=DEV).manual_seed(T)
+    flat = torch.zeros(T * h + 1, device=DEV, dtype=torch.bfloat16)
+    x = torch.randn(T, h, generator=g, device=DEV).to(torch.bfloat16)
+    odd = flat[1:].view(T, h)
+    odd.copy_(x)
+    router, corr = torch.randn(E, h, generator=g, device=DEV), torch.randn(E, generator=g, device=DEV)
+    out = [(torch.empty(T, 2, dtype=torch.int32, device=DEV), torch.empty(T, 2, device=DEV)) for _ in range(2)]
+    ops.moe_route(x, router, *out[0], "softmax", True, None, corr)
+    ops.moe_route(odd, router, *out[1], "softmax", True, None, corr)
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
