@@ -14,6 +14,12 @@
 // middle, and the 8 x 8 squares left on the diagonal pair by pair.  Decays, sums and the state are float32; where a float32 number has to be
 // an operand of a product it is split into two bf16 numbers (value = hi + lo) and the larger products are taken, so that about 16
 // bits of it enter.  k and v are bf16 as the projection left them.
+//
+// -DTIME_MIXING: time mixing (recurrent.cu) instead, whose output is read before the token's own decay, with a bonus for the token itself:
+//     o_i = (r_i exp(G_(i-1))) S0 + sum_(j < i) P_ij v_j + (sum_c r_i[c] u[c] k_i[c]) v_i,   P_ij = sum_c r_i[c] k_j[c] exp(G_(i-1)[c] - G_j[c]):
+// the same products with the queries' sums a row earlier, nothing under a root, and log-decays -exp(wraw + w0) that come as float32 rows.
+// Measured on B200, one prompt of 2,048 tokens, 40 heads of 64: the walks over blocks of 128 tokens (recurrent.cu, twice the arithmetic a token
+// at a time), their combination and the heads' norm 598 us.
 #define MB_LIB "gated_linear_chunked"
 #define MB_LIB_ID 23
 #include "common.cuh"
@@ -62,6 +68,19 @@ __device__ __forceinline__ void mma3(float* c, const uint32_t* ah, const uint32_
     mma_bf16_16816(c, ah, bl0, bl1);
 }
 
+// A token's log2-decay in one channel from its number z (rate: -LOG2E / tau).
+#ifdef TIME_MIXING
+#define EARLIER 1                     // a query's sum ends a token before it
+#define LEAST -150.0f                 // log2 of a decay that leaves nothing (anything below adds only rounding to the sums)
+__device__ __forceinline__ float log_decay(float z, float) {
+    const float x = -LOG2E * expf(z);
+    return x < LEAST ? LEAST : x;
+}
+#else
+#define EARLIER 0
+__device__ __forceinline__ float log_decay(float z, float rate) { return rate * softplus_f(-z); }
+#endif
+
 // What a chunk and head keeps between the kernels, float32: G in log2 units [64][DQ], then what it adds to the state, replaced by the state before it, [DQ][dv].
 #define CHUNK_F32(dv) (CH * DQ + DQ * (dv))
 
@@ -80,12 +99,14 @@ __device__ __forceinline__ void take_rows(bf16* dst, int ld, const bf16* src, si
 
 #define ADD_SMEM(rank) (CH * LDR * 2 + CH * LDV * 2 + CH * LDG * 4 + (CH + DQ) * ((rank) + 8) * 2)
 
+// (time mixing: `bias` is w0, inv_tau is not used; where wraw is given its float32 rows, H DQ numbers apart, stand for l W_2^T and rank is 0)
+
 __global__ void __launch_bounds__(THREADS, 2) add_kernel(
     const bf16* __restrict__ k, const bf16* __restrict__ v, const bf16* __restrict__ l, int in_stride, const bf16* __restrict__ w2,
     const float* __restrict__ bias, int rank, float inv_tau, const int* __restrict__ cu_tokens, int first_req, float* __restrict__ floats, int H, int dv,
-    int slices) {
+    int slices, int l_stride, const float* __restrict__ wraw) {
     PDL_ENTER();
-    k = pdl_fresh(k); v = pdl_fresh(v); l = pdl_fresh(l);
+    k = pdl_fresh(k); v = pdl_fresh(v); l = pdl_fresh(l); wraw = pdl_fresh(wraw);
     extern __shared__ __align__(16) uint8_t smem_raw[];
     float* sG = reinterpret_cast<float*>(smem_raw);            // [CH][LDG], log2 units
     bf16* sk = reinterpret_cast<bf16*>(sG + CH * LDG);         // [CH][LDR]
@@ -99,7 +120,7 @@ __global__ void __launch_bounds__(THREADS, 2) add_kernel(
     if (rows <= 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t2 = 2 * (lane & 3);
     float* out = floats + ((size_t)(first_chunk(cu_tokens, first_req, req) + blockIdx.x) * H + head) * CHUNK_F32(dv);
-    take_rows(sl, LDL, l + (size_t)tok0 * in_stride, in_stride, rows, rank, rank);
+    if (rank > 0) take_rows(sl, LDL, l + (size_t)tok0 * l_stride, l_stride, rows, rank, rank);
     {
         const int per = rank / 8;
         for (int idx = tid; idx < DQ * per; idx += THREADS) {
@@ -113,6 +134,18 @@ __global__ void __launch_bounds__(THREADS, 2) add_kernel(
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();
+    if (wraw != nullptr) {
+        const float* src = wraw + (size_t)tok0 * H * DQ + (size_t)head * DQ;
+        for (int idx = tid; idx < CH * DQ / 4; idx += THREADS) {
+            const int row = idx / (DQ / 4), c = idx % (DQ / 4) * 4;
+            float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (row < rows) {
+                const float4 z = *reinterpret_cast<const float4*>(src + (size_t)row * H * DQ + c), b = *reinterpret_cast<const float4*>(bias + head * DQ + c);
+                x = make_float4(log_decay(z.x + b.x, 1.0f), log_decay(z.y + b.y, 1.0f), log_decay(z.z + b.z, 1.0f), log_decay(z.w + b.w, 1.0f));
+            }
+            *reinterpret_cast<float4*>(sG + row * LDG + c) = x;
+        }
+    } else
     // ---- log-decays: z = l W_2^T, 16 tokens and half of the channels per warp
     {
         const int i0 = (warp & 3) * 16 + g, i1 = i0 + 8, n_first = (warp >> 2) * (DQ / 16);
@@ -129,10 +162,10 @@ __global__ void __launch_bounds__(THREADS, 2) add_kernel(
             }
             const float2 b = *reinterpret_cast<const float2*>(bias + head * DQ + c + t2);
             float2 x, y;
-            x.x = i0 < rows ? rate * softplus_f(-(z[0] + b.x)) : 0.0f;
-            x.y = i0 < rows ? rate * softplus_f(-(z[1] + b.y)) : 0.0f;
-            y.x = i1 < rows ? rate * softplus_f(-(z[2] + b.x)) : 0.0f;
-            y.y = i1 < rows ? rate * softplus_f(-(z[3] + b.y)) : 0.0f;
+            x.x = i0 < rows ? log_decay(z[0] + b.x, rate) : 0.0f;
+            x.y = i0 < rows ? log_decay(z[1] + b.y, rate) : 0.0f;
+            y.x = i1 < rows ? log_decay(z[2] + b.x, rate) : 0.0f;
+            y.y = i1 < rows ? log_decay(z[3] + b.y, rate) : 0.0f;
             *reinterpret_cast<float2*>(sG + i0 * LDG + c + t2) = x;
             *reinterpret_cast<float2*>(sG + i1 * LDG + c + t2) = y;
         }
@@ -211,18 +244,24 @@ __global__ void __launch_bounds__(THREADS, 2) add_kernel(
 
 // ---- the states before every chunk, and the one behind the last -----------------------------------------------------------------
 #define CARRY_AHEAD 4
-__global__ void __launch_bounds__(256) carry_kernel(float* floats, float* __restrict__ state, const int* __restrict__ cu_tokens, const int* __restrict__ slots,
-                                                    int first_req, int H, int dv) {
+// (time mixing: a request's last row of the mixer's input goes to `last` of its slot too, for the next step's token shift)
+__global__ void __launch_bounds__(256) carry_kernel(float* floats, float* __restrict__ state, long long state_stride, const int* __restrict__ cu_tokens,
+                                                    const int* __restrict__ slots, int first_req, int H, int dv, const bf16* __restrict__ h, int width,
+                                                    float* __restrict__ last) {
     PDL_ENTER();
-    floats = pdl_fresh(floats);
+    floats = pdl_fresh(floats); h = pdl_fresh(h);
     const int req = first_req + blockIdx.z, head = blockIdx.y;
     const int count = cu_tokens[req + 1] - cu_tokens[req];
+#ifdef TIME_MIXING
+    if (blockIdx.x == 0 && head == 0 && count > 0)
+        for (int i = threadIdx.x; i < width; i += 256) last[(size_t)slots[req] * state_stride + i] = to_f32(h[(size_t)(cu_tokens[req + 1] - 1) * width + i]);
+#endif
     const int at = (blockIdx.x * 256 + threadIdx.x) * 4;       // four numbers of one row (dv is a multiple of 4)
     if (count <= 0 || at >= DQ * dv) return;
     const int chunks = (count + CH - 1) / CH, n = at / dv;
     const size_t step = (size_t)H * CHUNK_F32(dv);
     float* base = floats + ((size_t)first_chunk(cu_tokens, first_req, req) * H + head) * CHUNK_F32(dv);
-    float4* kept = reinterpret_cast<float4*>(state + ((size_t)slots[req] * H + head) * DQ * dv + at);
+    float4* kept = reinterpret_cast<float4*>(state + (size_t)slots[req] * state_stride + (size_t)head * DQ * dv + at);
     float4 s = *kept;
     float4 add[CARRY_AHEAD];
     float decay[CARRY_AHEAD];
@@ -248,24 +287,26 @@ __global__ void __launch_bounds__(256) carry_kernel(float* floats, float* __rest
 // ---- the outputs -------------------------------------------------------------------------------------------------------------------
 #define QK_BYTES (2 * CH * LDR * 2)
 #define S_BYTES (2 * 2 * ST * LDV * 2)
-#define READ_SMEM (CH * LDG * 4 + (QK_BYTES > S_BYTES ? QK_BYTES : S_BYTES) + CH * LDV * 2 + 2 * CH * LDP * 2)
+#define G_BYTES ((CH + EARLIER) * LDG * 4)
+#define READ_SMEM (G_BYTES + (QK_BYTES > S_BYTES ? QK_BYTES : S_BYTES) + CH * LDV * 2 + 2 * CH * LDP * 2)
 static_assert(CH * LDG * 4 == 2 * CH * LDR * 2, "the weighted queries take the sums' place");
 
 template <bool WHOLE>
 __global__ void __launch_bounds__(THREADS, 2) read_kernel(
     const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v, int in_stride, const float* __restrict__ floats,
     const int* __restrict__ cu_tokens, int first_req, int H, int dv, int slices, float* __restrict__ o, const bf16* __restrict__ gate_rows, int gate_stride,
-    int gate, const float* __restrict__ norm_w, float eps, float factor, bf16* __restrict__ out, int out_stride) {
+    int gate, const float* __restrict__ norm_w, float eps, float factor, bf16* __restrict__ out, int out_stride, const float* __restrict__ bonus) {
     PDL_ENTER();
     q = pdl_fresh(q); k = pdl_fresh(k); v = pdl_fresh(v); floats = pdl_fresh(floats); gate_rows = pdl_fresh(gate_rows);
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ float s_qk[CH], s_ss[2][CH];
-    float* sG = reinterpret_cast<float*>(smem_raw);            // [CH][LDG]; later q exp(G), hi and lo: [2][CH][LDR] bf16
-    bf16* sQ = reinterpret_cast<bf16*>(sG);
-    bf16* sq = reinterpret_cast<bf16*>(sG + CH * LDG);         // [CH][LDR] q, then k; later two tiles of the state, hi and lo: [2][2][ST][LDV]
+    float* sG = reinterpret_cast<float*>(smem_raw) + EARLIER * LDG;     // [CH][LDG]; later q exp(G), hi and lo: [2][CH][LDR] bf16
+    const float* sGq = sG - EARLIER * LDG;                     // the queries' rows of it (time mixing: a row of zeros first)
+    bf16* sQ = reinterpret_cast<bf16*>(smem_raw);
+    bf16* sq = reinterpret_cast<bf16*>(smem_raw + G_BYTES);    // [CH][LDR] q, then k; later two tiles of the state, hi and lo: [2][2][ST][LDV]
     bf16* sk = sq + CH * LDR;
     bf16* sS = sq;
-    bf16* sv = reinterpret_cast<bf16*>(smem_raw + CH * LDG * 4 + (QK_BYTES > S_BYTES ? QK_BYTES : S_BYTES));
+    bf16* sv = reinterpret_cast<bf16*>(smem_raw + G_BYTES + (QK_BYTES > S_BYTES ? QK_BYTES : S_BYTES));
     bf16* sP = sv + CH * LDV;                                  // [2][CH][LDP] hi, lo
     const int req = first_req + blockIdx.z / slices, head = blockIdx.y, vs0 = (blockIdx.z % slices) * VS;
     const int tok0 = cu_tokens[req] + blockIdx.x * CH;
@@ -307,12 +348,21 @@ __global__ void __launch_bounds__(THREADS, 2) read_kernel(
         }
     };
     ask(0);
+#ifdef TIME_MIXING
+    const float scale = 1.0f;
+    for (int c = tid; c < DQ; c += THREADS) sG[c - LDG] = 0.0f;
+#else
     const float scale = 1.0f / sqrtf((float)DQ);
+#endif
     cp_async_wait<0>();
     __syncthreads();
     for (int row = warp; row < CH; row += THREADS / 32) {
         float qk = 0.0f;
+#ifdef TIME_MIXING
+        for (int c = lane; c < DQ; c += 32) qk = fmaf(__bfloat162float(sq[row * LDR + c]) * bonus[head * DQ + c], __bfloat162float(sk[row * LDR + c]), qk);
+#else
         for (int c = lane; c < DQ; c += 32) qk = fmaf(__bfloat162float(sq[row * LDR + c]), __bfloat162float(sk[row * LDR + c]), qk);
+#endif
         qk = warp_sum(qk);
         if (lane == 0) s_qk[row] = qk;
     }
@@ -346,7 +396,7 @@ __global__ void __launch_bounds__(THREADS, 2) read_kernel(
                 const float r[4] = {ra.x, ra.y, rb.x, rb.y};
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const float2 gi = *reinterpret_cast<const float2*>(sG + ((u & 1) ? i1 : i0) * LDG + c + (u >> 1) * 8), q2 = bf2(rq[u]);
+                    const float2 gi = *reinterpret_cast<const float2*>(sGq + ((u & 1) ? i1 : i0) * LDG + c + (u >> 1) * 8), q2 = bf2(rq[u]);
                     split_bf16(q2.x * ex2_approx(gi.x - r[(u >> 1) * 2]), q2.y * ex2_approx(gi.y - r[(u >> 1) * 2 + 1]), qh[u], ql[u]);
                 }
 #pragma unroll
@@ -367,7 +417,7 @@ __global__ void __launch_bounds__(THREADS, 2) read_kernel(
                 qh[0] = qh[2] = ql[0] = ql[2] = 0u;
 #pragma unroll
                 for (int u = 1; u < 4; u += 2) {
-                    const float2 gi = *reinterpret_cast<const float2*>(sG + i1 * LDG + c + (u >> 1) * 8), q2 = bf2(rq[u]);
+                    const float2 gi = *reinterpret_cast<const float2*>(sGq + i1 * LDG + c + (u >> 1) * 8), q2 = bf2(rq[u]);
                     split_bf16(q2.x * ex2_approx(gi.x - r[(u >> 1) * 2]), q2.y * ex2_approx(gi.y - r[(u >> 1) * 2 + 1]), qh[u], ql[u]);
                 }
                 // (token g of the block: the same index as row i0)
@@ -401,7 +451,7 @@ __global__ void __launch_bounds__(THREADS, 2) read_kernel(
 #pragma unroll 4
             for (int c = 0; c < DQ; c += 2) {
                 const float2 qi = bf2(word(sq + i * LDR + c)), kj = bf2(word(sk + j * LDR + c));
-                const float2 gi = *reinterpret_cast<const float2*>(sG + i * LDG + c), gj = *reinterpret_cast<const float2*>(sG + j * LDG + c);
+                const float2 gi = *reinterpret_cast<const float2*>(sGq + i * LDG + c), gj = *reinterpret_cast<const float2*>(sG + j * LDG + c);
                 b = fmaf(qi.x * kj.x, ex2_approx(gi.x - gj.x), b);
                 b2 = fmaf(qi.y * kj.y, ex2_approx(gi.y - gj.y), b2);
             }
@@ -424,7 +474,7 @@ __global__ void __launch_bounds__(THREADS, 2) read_kernel(
 #pragma unroll
         for (int u = 0; u < ITEMS; ++u) {
             const int idx = tid + u * THREADS, row = idx / (DQ / 2), c = idx % (DQ / 2) * 2;
-            const float2 g2 = *reinterpret_cast<const float2*>(sG + row * LDG + c), q2 = bf2(word(sq + row * LDR + c));
+            const float2 g2 = *reinterpret_cast<const float2*>(sGq + row * LDG + c), q2 = bf2(word(sq + row * LDR + c));
             split_bf16(q2.x * scale * ex2_approx(g2.x), q2.y * scale * ex2_approx(g2.y), hi[u], lo[u]);
         }
         __syncthreads();                                       // everyone has left G, q and k
@@ -524,7 +574,11 @@ __global__ void __launch_bounds__(THREADS, 2) read_kernel(
         for (int h = 0; h < 2; ++h) {
             const int col = wc * (VP / 2) + n * 16 + h * 8 + t2;
             if (col >= VS) continue;
+#ifdef TIME_MIXING
+            const float2 w = *reinterpret_cast<const float2*>(norm_w + (size_t)head * dv + col);      // (a weight per head and channel)
+#else
             const float2 w = *reinterpret_cast<const float2*>(norm_w + col);
+#endif
 #pragma unroll
             for (int rr = 0; rr < 2; ++rr) {
                 const int i = rr ? i1 : i0;
@@ -542,6 +596,7 @@ __global__ void __launch_bounds__(THREADS, 2) read_kernel(
 // How many float32 numbers a chunk and head needs between the kernels.
 MB_API int mb_gla_chunked_scratch(int dv) { return CHUNK_F32(dv); }
 
+#ifndef TIME_MIXING
 // Requests first_req .. requests - 1; which: 0 adds, 1 carries, 2 reads (in this order).  q, k, v, l, w2, bias, state as mb_gla_scan takes them (bf16, 16-byte
 // aligned, in_stride a multiple of 8, rank a multiple of 16 up to 128); dv a multiple of V_SLICE.  floats holds (tokens / 64 + requests) * H
 // pieces of mb_gla_chunked_scratch.  A whole head in one slice (dv == V_SLICE): normed and gated rows go to `out`; else the sums to `o`.
@@ -558,17 +613,50 @@ MB_API int mb_gla_chunked(int which, const void* q, const void* k, const void* v
     if (which == 0) {
         cudaFuncSetAttribute(add_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ADD_SMEM(rank));
         return launch_kernel(add_kernel, grid, THREADS, ADD_SMEM(rank), s, 0, (const bf16*)k, (const bf16*)v, (const bf16*)l, in_stride, (const bf16*)w2, bias, rank,
-                             inv_tau, cu_tokens, first_req, floats, H, dv, slices);
+                             inv_tau, cu_tokens, first_req, floats, H, dv, slices, in_stride, (const float*)nullptr);
     }
     if (which == 1)
-        return launch_kernel(carry_kernel, dim3((DQ * dv / 4 + 255) / 256, H, count), 256, 0, s, 0, floats, state, cu_tokens, slots, first_req, H, dv);
+        return launch_kernel(carry_kernel, dim3((DQ * dv / 4 + 255) / 256, H, count), 256, 0, s, 0, floats, state, (long long)H * DQ * dv, cu_tokens,
+                             slots, first_req, H, dv, (const bf16*)nullptr, 0, (float*)nullptr);
     if (slices == 1) {
         if ((((uintptr_t)gate_rows | (uintptr_t)out) & 3) != 0 || gate_stride % 2 != 0 || out_stride % 2 != 0 || out_stride < H * dv || ((uintptr_t)norm_w & 7) != 0) return MB_ERR_BAD_SIZE;
         cudaFuncSetAttribute(read_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, READ_SMEM);
         return launch_kernel(read_kernel<true>, grid, THREADS, READ_SMEM, s, 0, (const bf16*)q, (const bf16*)k, (const bf16*)v, in_stride, (const float*)floats, cu_tokens,
-                             first_req, H, dv, slices, o, (const bf16*)gate_rows, gate_stride, gate, norm_w, eps, factor, (bf16*)out, out_stride);
+                             first_req, H, dv, slices, o, (const bf16*)gate_rows, gate_stride, gate, norm_w, eps, factor, (bf16*)out, out_stride, (const float*)nullptr);
     }
     cudaFuncSetAttribute(read_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, READ_SMEM);
     return launch_kernel(read_kernel<false>, grid, THREADS, READ_SMEM, s, 0, (const bf16*)q, (const bf16*)k, (const bf16*)v, in_stride, (const float*)floats, cu_tokens,
-                         first_req, H, dv, slices, o, (const bf16*)gate_rows, gate_stride, gate, norm_w, eps, factor, (bf16*)out, out_stride);
+                         first_req, H, dv, slices, o, (const bf16*)gate_rows, gate_stride, gate, norm_w, eps, factor, (bf16*)out, out_stride, (const float*)nullptr);
 }
+#else
+// Time mixing over requests first_req .. requests - 1; which: 0 adds, 1 carries, 2 reads (in this order).  r, k, v, gate_rows, out bf16 [tokens][H * QK_DIM]; the
+// decays' numbers either as float32 rows wraw likewise, or (wraw null) as l W_2^T of l bf16 [tokens][rank] and w2 bf16 [H * QK_DIM][rank], rank a multiple of 16
+// up to 128; w0, u and norm_w float32 [H * QK_DIM]; all 16-byte aligned.  A slot's row of `state_stride` floats (a multiple of 4) has the heads'
+// matrices at `state` and the last row of h ([tokens][width]) at `last`.  floats holds (tokens / 64 + requests) * H pieces of mb_gla_chunked_scratch.
+MB_API int mb_wkv_chunked(int which, const void* r, const void* k, const void* v, const float* wraw, const void* l, const void* w2, int rank, const float* w0,
+                          const float* u, float* state,
+                          long long state_stride, const void* h, int width, float* last, const int* cu_tokens, const int* slots, float* floats,
+                          const void* gate_rows, const float* norm_w, float eps, void* out, int first_req, int requests, int max_query_len, int H, cudaStream_t s) {
+    static_assert(VS == DQ, "time mixing: values as wide as keys, a whole head a CTA");
+    if (requests <= first_req || max_query_len <= 0) return 0;
+    if (H <= 0 || first_req < 0 || width <= 0 || state_stride % 4 != 0) return MB_ERR_BAD_SIZE;
+    if (wraw != nullptr) rank = 0;
+    else if (l == nullptr || w2 == nullptr || rank <= 0 || rank % 16 != 0 || rank > 128) return MB_ERR_BAD_SIZE;
+    if ((((uintptr_t)r | (uintptr_t)k | (uintptr_t)v | (uintptr_t)wraw | (uintptr_t)l | (uintptr_t)w2 | (uintptr_t)w0 | (uintptr_t)u | (uintptr_t)floats | (uintptr_t)state | (uintptr_t)gate_rows |
+          (uintptr_t)norm_w | (uintptr_t)out) & 15) != 0)
+        return MB_ERR_BAD_SIZE;
+    const int count = requests - first_req, stride = H * DQ;
+    dim3 grid((max_query_len + CH - 1) / CH, H, count);
+    if (which == 0) {
+        cudaFuncSetAttribute(add_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ADD_SMEM(rank));
+        return launch_kernel(add_kernel, grid, THREADS, ADD_SMEM(rank), s, 0, (const bf16*)k, (const bf16*)v, (const bf16*)l, stride, (const bf16*)w2, w0,
+                             rank, 1.0f, cu_tokens, first_req, floats, H, DQ, 1, rank, wraw);
+    }
+    if (which == 1)
+        return launch_kernel(carry_kernel, dim3((DQ * DQ / 4 + 255) / 256, H, count), 256, 0, s, 0, floats, state, state_stride, cu_tokens, slots, first_req, H, DQ,
+                             (const bf16*)h, width, last);
+    cudaFuncSetAttribute(read_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, READ_SMEM);
+    return launch_kernel(read_kernel<true>, grid, THREADS, READ_SMEM, s, 0, (const bf16*)r, (const bf16*)k, (const bf16*)v, stride, (const float*)floats, cu_tokens,
+                         first_req, H, DQ, 1, (float*)nullptr, (const bf16*)gate_rows, stride, 1, norm_w, eps, 1.0f, (bf16*)out, stride, u);
+}
+#endif

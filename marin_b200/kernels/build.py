@@ -219,7 +219,7 @@ def attention_tc_name(d: int, group: int, dv: int = 0, values_in_keys: bool = Fa
 #: One or two layouts of every source that is otherwise compiled for a model's own sizes when it first runs (the names and
 #: defines are those the wrappers in ``ops`` use): sink attention with keys and values of their own and over a shared latent
 #: with sixteen heads a CTA, sigmoid attention, chunked linear attention, attention over a window and pooled blocks, the chunked
-#: delta rule, chunked gated linear attention, two maps per head.
+#: delta rule, chunked gated linear attention and time mixing, two maps per head.
 PER_LAYOUT_SAMPLES = {
     "mb_attention_sink_fast_d128_v128_g4": (["attention_sink_fast.cu"], ["HEAD_DIM=128", "V_DIM=128", "GROUP=4"]),
     "mb_attention_sink_fast_d160_v128_g16_vk": (["attention_sink_fast.cu"], ["HEAD_DIM=160", "V_DIM=128", "GROUP=16", "V_IN_K"]),

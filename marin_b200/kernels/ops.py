@@ -508,6 +508,31 @@ def gemm(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, then_n
     return None
 
 
+#: several products of as many inputs and matrices of the same sizes run as one launch where there are many tokens (False: one after the other)
+use_side_by_side = True
+
+
+def gemm_side_by_side(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+    """``out[g] = x[g] w[g]^T`` for every ``g`` (``x`` ``[G, T, K]``, ``w`` ``[G, N, K]``, ``out`` ``[G, T, N]``).  bf16 with more than 128 tokens: one persistent
+    launch over all tiles, whose rounds over the SMs waste less than each product's own (2,048 tokens, four of 2,560 x 2,560: 880 tiles in 6 rounds
+    instead of four times 260 in 2); else product by product."""
+    _need_cuda(x, w, out)
+    G, T, K = x.shape
+    N = w.shape[1]
+    assert tuple(w.shape) == (G, N, K) and tuple(out.shape) == (G, T, N)
+    if not (use_side_by_side and use_tensor_cores and G > 1 and T > 128 and K % 64 == 0 and x.dtype == w.dtype == out.dtype == torch.bfloat16
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and G <= 512):
+        for g in range(G):
+            gemm(x[g], w[g], out[g])
+        return
+    rows = G * -(-N // 128)
+    tile = min(PERSISTENT_TILES, key=lambda bn: (-(-(rows * -(-T // bn)) // SM_COUNT) * (bn + 24), bn))
+    _cost(_size(x) + _size(w) + _size(out), 2.0 * G * T * N * K)
+    _check(_lib("mb_moe_tc").mb_moe_grouped_tc(
+        _ptr(x), _ptr(w), _ptr(None), _c_int(G), _c_int(G * T), _c_int(N), _c_int(K), _ptr(out), _ptr(None), _ptr(None), _c_int(0), _c_int(0), _c_int(0),
+        _ptr(None), _c_int(0), _c_int(tile), _c_int(1), _c_int(SM_COUNT), _ptr(_scratch_for(x.device).error), _stream()), "gemm (side by side, tcgen05)")
+
+
 #: with few tokens the q|k|v product finishes its heads itself (norm, rotation, cache write) where the layout allows
 fuse_heads = True
 FUSED_HEADS_MAX_TOKENS = 128
@@ -1096,8 +1121,74 @@ WKV_BLOCK_TOKENS = 128
 WKV_BLOCKS_FROM = 256
 
 
+#: bf16 prompt portions of time mixing go 64 tokens at a time through the tensor-core kernels (False: the walks over blocks)
+use_chunked_wkv = True
+#: ... when the step's longest portion has more tokens than this (a walk takes about 1.3 us a token, the three kernels some 20 us however few there are)
+WKV_CHUNKED_FROM = 16
+
+
+def wkv_chunked_supported(dtype, dim: int) -> bool:
+    return dtype == torch.bfloat16 and dim % 16 == 0 and 16 <= dim <= 128
+
+
+def _wkv_chunked_job(dim: int) -> tuple:
+    return f"mb_wkv_chunked_d{dim}", (["gated_linear_chunked.cu"], [f"QK_DIM={dim}", f"V_SLICE={dim}", "TIME_MIXING"])
+
+
+def wkv_jobs(dtype, dim: int) -> dict:
+    jobs = library_jobs("mb_activations", "mb_recurrent")
+    if use_chunked_wkv and wkv_chunked_supported(dtype, dim):
+        name, job = _wkv_chunked_job(dim)
+        jobs[name] = job
+        jobs.update(library_jobs("mb_moe_tc"))
+    return jobs
+
+
+def wkv_goes_chunked(ctx, dtype, dim: int, state: torch.Tensor, *rows: torch.Tensor) -> bool:
+    """Whether ``wkv_chunked`` takes the step's portions: bf16 heads in whole 16s, a portion long enough, every row and the state at 16-byte addresses."""
+    return (use_chunked_wkv and wkv_chunked_supported(dtype, dim) and ctx.max_query_len > WKV_CHUNKED_FROM and state.stride(0) % 4 == 0
+            and all(t.data_ptr() % 16 == 0 for t in (state,) + rows))
+
+
+def wkv_chunked(r, k, v, gate, low, w2, w0, u, norm_w, eps: float, state: torch.Tensor, carry: torch.Tensor, h: torch.Tensor, ctx, slots: torch.Tensor,
+                out: torch.Tensor, heads: int, dim: int, wraw: Optional[torch.Tensor] = None) -> None:
+    """``wkv_scan`` and ``head_norm_gate`` over requests ``ctx.num_decode`` on (those before bring a token each), 64 tokens at a time on the tensor cores, from the
+    projections' rows to the gated heads in ``out``.  The decays' numbers are ``low w2^T`` (``low`` bf16 ``[T, rank]``, rank a multiple of 16 up to 128) or the
+    rows of ``wraw``."""
+    _need_cuda(r, k, v, gate, low, w2, w0, u, norm_w, h, out, slots, wraw)
+    T, n = r.shape
+    assert n == heads * dim and all(tuple(x.shape) == (T, n) and x.dtype == torch.bfloat16 for x in (r, k, v, gate, out))
+    assert all(x.dtype == torch.float32 and x.numel() == n for x in (w0, u, norm_w)) and h.dtype == torch.bfloat16 and h.shape[0] == T
+    assert state.dtype == torch.float32 and carry.dtype == torch.float32 and state.stride(0) == carry.stride(0)
+    assert state.shape[1] == heads * dim * dim and carry.shape[1] == h.shape[1]
+    rank = 0
+    if wraw is not None:
+        assert wraw.dtype == torch.float32 and tuple(wraw.shape) == (T, n)
+    else:
+        rank = low.shape[1]
+        assert low.dtype == w2.dtype == torch.bfloat16 and tuple(w2.shape) == (n, rank) and low.shape[0] == T
+    first = ctx.num_decode
+    tokens = T - first
+    chunks = tokens // 64 + ctx.num_requests - first
+    floats = ctx.workspace.get("wkv_chunks", (chunks * heads * gla_chunk_bytes(dim, dim) // 4,), torch.float32)
+    name, job = _wkv_chunked_job(dim)
+    lib = build.load(name, *job)
+    args = (_ptr(r), _ptr(k), _ptr(v), _ptr(wraw), _ptr(low if wraw is None else None), _ptr(w2 if wraw is None else None), _c_int(rank), _ptr(w0), _ptr(u),
+            _c_void_p(state.data_ptr()), ctypes.c_longlong(state.stride(0)), _ptr(h), _c_int(h.shape[1]), _c_void_p(carry.data_ptr()), _ptr(ctx.cu_tokens),
+            _ptr(slots), _ptr(floats), _ptr(gate), _ptr(norm_w), _c_float(eps), _ptr(out), _c_int(first), _c_int(ctx.num_requests), _c_int(ctx.max_query_len),
+            _c_int(heads), _stream())
+    rows = 2 * tokens * n
+    # what the algorithm needs is shared out over the three: its inputs once, the state once, the outputs once
+    _cost(2 * rows + (_size(wraw) if wraw is not None else _size(low) + _size(w2)), 2.0 * tokens * n * (dim + rank))
+    _check(lib.mb_wkv_chunked(_c_int(0), *args), "time mixing (chunks' parts)")
+    _cost((ctx.num_requests - first) * n * dim * 8, 0.0)
+    _check(lib.mb_wkv_chunked(_c_int(1), *args), "time mixing (states carried)")
+    _cost(3 * rows, 2.0 * tokens * n * dim)
+    _check(lib.mb_wkv_chunked(_c_int(2), *args), "time mixing (outputs)")
+
+
 def wkv_scan(r, k, v, wraw, w0, u, state: torch.Tensor, carry: torch.Tensor, h: torch.Tensor, ctx, slots: torch.Tensor,
-             o: torch.Tensor, heads: int, dim: int) -> None:
+             o: torch.Tensor, heads: int, dim: int, requests: Optional[int] = None) -> None:
     """``o_t = (S_(t-1) + diag(u) k_t v_t^T)^T r_t; S_t = diag(w_t) S_(t-1) + k_t v_t^T`` with ``w = exp(-exp(wraw + w0))``; ``o``
     float32 ``[T, heads * dim]`` before its norm (``head_norm_gate``).  ``state`` and ``carry`` are column slices of one float32
     state tensor (``[slots, heads * dim * dim]`` and ``[slots, width]``); the last row of ``h`` of every request goes to ``carry``.
@@ -1106,7 +1197,9 @@ def wkv_scan(r, k, v, wraw, w0, u, state: torch.Tensor, carry: torch.Tensor, h: 
     are walked side by side: each from a zero state for its end state and the product of its decays; a short pass turns these
     into the states the blocks start from (``S <- W_b S + S_b``, block after block); each block again from its true start, for
     the outputs.  Twice the arithmetic, on all of the device instead of one CTA per head.  The result differs from the single
-    walk by rounding (the sums are associated differently), which is why the 32-bit path never does it."""
+    walk by rounding (the sums are associated differently), which is why the 32-bit path never does it.
+
+    ``requests``: only the step's first so many, which bring a token each (None: all of them)."""
     _need_cuda(r, k, v, wraw, w0, u, h, o, slots)
     T, n = r.shape
     assert n == heads * dim and all(tuple(x.shape) == (T, n) and x.dtype == r.dtype for x in (k, v))
@@ -1114,9 +1207,9 @@ def wkv_scan(r, k, v, wraw, w0, u, state: torch.Tensor, carry: torch.Tensor, h: 
     assert o.dtype == torch.float32 and tuple(o.shape) == (T, n)
     assert state.dtype == torch.float32 and carry.dtype == torch.float32 and state.stride(0) == carry.stride(0)
     assert state.shape[1] == heads * dim * dim and carry.shape[1] == h.shape[1] and h.dtype == r.dtype and h.shape[0] == T
-    R = ctx.num_requests
+    R = ctx.num_requests if requests is None else int(requests)
     nblocks, block_state, block_decay = 1, None, None
-    if (WKV_BLOCK_TOKENS and r.dtype == torch.bfloat16 and dim in (16, 32, 64, 128) and ctx.max_query_len >= WKV_BLOCKS_FROM):
+    if (WKV_BLOCK_TOKENS and r.dtype == torch.bfloat16 and dim in (16, 32, 64, 128) and requests is None and ctx.max_query_len >= WKV_BLOCKS_FROM):
         nblocks = -(-ctx.max_query_len // WKV_BLOCK_TOKENS)
         block_state = ctx.workspace.get("wkv_block_state", (R * nblocks, heads, dim, dim), torch.float32)
         block_decay = ctx.workspace.get("wkv_block_decay", (R * nblocks, heads, dim), torch.float32)

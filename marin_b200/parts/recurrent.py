@@ -131,8 +131,13 @@ class WKV(Mixer):
 
     def load(self, tensors: Dict[str, torch.Tensor], rt: Runtime) -> None:
         self.mu = rt.f32(torch.stack([tensors.pop(f"{self._n('mu')}.{s}").to(torch.float32) for s in self.MIXES]))
-        self.w_r, self.w_k, self.w_v, self.w_g = (rt.matrix(tensors.pop(self._n(p))) for p in "rkvg")
-        self.w_1, self.w_2 = rt.matrix(tensors.pop(self._n("w1"))), rt.matrix(tensors.pop(self._n("w2")))
+        self.w_rkvg = torch.stack([rt.matrix(tensors.pop(self._n(p))) for p in "rkvg"])       # [4, heads * dim, hidden]: products side by side
+        first, second = tensors.pop(self._n("w1")), tensors.pop(self._n("w2"))
+        # (the decays' numbers between the matrices padded with zeros to whole 16s: the chunked kernels apply the second matrix themselves)
+        self.low_dim = self.rank + (-self.rank % 16 if rt.dtype == torch.bfloat16 else 0)
+        pad = self.low_dim - self.rank
+        self.w_1 = rt.matrix(torch.cat([first, first.new_zeros(pad, first.shape[1])], dim=0) if pad else first)
+        self.w_2 = rt.matrix(torch.cat([second, second.new_zeros(second.shape[0], pad)], dim=1) if pad else second)
         self.w0 = rt.f32(tensors.pop(self._n("w0")))
         self.u = rt.f32(tensors.pop(self._n("u"))).reshape(-1)
         self.norm_w = rt.f32(tensors.pop(self._n("norm")))
@@ -143,7 +148,13 @@ class WKV(Mixer):
         return super().flops(tokens, pairs) + 6.0 * tokens * self.heads * self.dim * self.dim
 
     def kernel_jobs(self, dtype) -> Dict[str, tuple]:
-        return ops.library_jobs("mb_activations", "mb_recurrent")
+        return ops.wkv_jobs(dtype, self.dim)
+
+    def workspace_per_token(self, dtype) -> int:
+        """Bytes a step keeps per token beside the products' rows: the five mixes, and what the chunked kernels hand over (or, walked, the decays' and
+        the heads' float32 rows)."""
+        chunked = self.heads * ops.gla_chunk_bytes(self.dim, self.dim) // 64 if ops.wkv_chunked_supported(dtype, self.dim) else 0
+        return len(self.MIXES) * self.hidden * element_size(dtype) + max(chunked, 8 * self.n)
 
     def forward(self, x, ctx, cache, residual: torch.Tensor):
         T = x.shape[0]
@@ -156,20 +167,31 @@ class WKV(Mixer):
         ops.shift_mix(x, carry, ctx, cache.slots, self.mu, mixes)
         ops.stage_name = "r, k, v, g"
         rkvg = ws.get("wkv_rkvg", (4, T, n), x.dtype)
-        for i, w in enumerate((self.w_r, self.w_k, self.w_v, self.w_g)):
-            ops.gemm(mixes[i], w, rkvg[i])
+        ops.gemm_side_by_side(mixes[:4], self.w_rkvg, rkvg)
         ops.stage_name = "decay"
-        low = ws.get("wkv_low", (T, self.rank), x.dtype)
+        low = ws.get("wkv_low", (T, self.low_dim), x.dtype)
         ops.gemm(mixes[4], self.w_1, low)
         ops.tanh_cap(low, 1.0)
-        wraw = ws.get("wkv_wraw", (T, n), torch.float32)
-        ops.gemm(low, self.w_2, wraw)
-        ops.stage_name = "recurrence"
-        o = ws.get("wkv_o", (T, n), torch.float32)
-        ops.wkv_scan(rkvg[0], rkvg[1], rkvg[2], wraw, self.w0, self.u, state, carry, x, ctx, cache.slots, o, self.heads, self.dim)
-        ops.stage_name = "norm, gate"
         out = ws.get("wkv_out", (T, n), x.dtype)
-        ops.head_norm_gate(o, self.norm_w, rkvg[3], self.norm_eps, out, self.heads, self.dim)
+        # prompt portions 64 tokens at a time on the tensor cores; single tokens (and sizes those kernels are not made for, and the 32-bit path) token by token
+        chunked = ops.wkv_goes_chunked(ctx, x.dtype, self.dim, state, rkvg[0], rkvg[1], rkvg[2], rkvg[3], low)
+        inside = chunked and self.low_dim <= 128                # the chunked kernels apply the decays' second matrix themselves
+        walked = ctx.num_decode if chunked else None            # the requests that are walked: all, or those with a single token
+        wraw = None
+        if not inside or walked:
+            wraw = ws.get("wkv_wraw", (T, n), torch.float32)
+            ops.gemm(low, self.w_2, wraw)
+        if chunked:
+            ops.stage_name = "recurrence, norm, gate"
+            ops.wkv_chunked(rkvg[0], rkvg[1], rkvg[2], rkvg[3], low, self.w_2, self.w0, self.u, self.norm_w, self.norm_eps, state, carry, x, ctx, cache.slots,
+                            out, self.heads, self.dim, None if inside else wraw)
+        if walked != 0:
+            ops.stage_name = "recurrence"
+            o = ws.get("wkv_o", (T, n), torch.float32)
+            ops.wkv_scan(rkvg[0], rkvg[1], rkvg[2], wraw, self.w0, self.u, state, carry, x, ctx, cache.slots, o, self.heads, self.dim, walked)
+            ops.stage_name = "norm, gate"
+            rows = T if walked is None else walked
+            ops.head_norm_gate(o[:rows], self.norm_w, rkvg[3][:rows], self.norm_eps, out[:rows], self.heads, self.dim)
         ops.stage_name = "o"
         ops.gemm(out, self.w_o, residual, accumulate=True)
         return None
