@@ -227,8 +227,10 @@ PER_LAYOUT_SAMPLES = {
     "mb_linear_attention_chunked_d128_v32": (["linear_attention_chunked.cu"], ["QK_DIM=128", "V_SLICE=32"]),
     "mb_delta_rule_chunked_d128_v32": (["delta_rule_chunked.cu"], ["QK_DIM=128", "V_SLICE=32"]),
     "mb_gated_linear_chunked_d128_v128": (["gated_linear_chunked.cu"], ["QK_DIM=128", "V_SLICE=128"]),
+    "mb_wkv_chunked_d64": (["gated_linear_chunked.cu"], ["QK_DIM=64", "V_SLICE=64", "TIME_MIXING"]),
     "mb_attention_sink_fast_d128_v128_g8": (["attention_sink_fast.cu"], ["HEAD_DIM=128", "V_DIM=128", "GROUP=8"]),
     "mb_attention_tc_d128_g8_pair": (["attention_tc.cu"], ["HEAD_DIM=128", "GROUP=8", "PAIR"]),
+    "mb_attention_pooled_mix_d128_v128_g4_k8": (["attention_pooled_mix.cu"], ["HEAD_DIM=128", "V_DIM=128", "GROUP=4", "KV_HEADS=8"]),
     "mb_attention_pooled_fast_d128_v128_g4_c2": (["attention_pooled_fast.cu"], ["HEAD_DIM=128", "V_DIM=128", "GROUP=4", "VALUE_HEADS=2"]),
 }
 

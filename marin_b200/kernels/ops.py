@@ -2023,8 +2023,16 @@ def attention_pooled(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table,
     if T == 0:
         return
     size = q.element_size()
-    parts = ctx.workspace.get("pooled_parts", (T, H, K, dv), torch.float32) if talk is not None else None
     rows = -(-page_size // pool) if pool else 0
+    if talk is not None and ctx.num_requests > ctx.num_decode:
+        blocks = _pooled_mix_blocks(ctx, window, pool)
+        if (use_pooled_mix and pooled_mix_supported(q.dtype, H, K, d, dv) and page_size & (page_size - 1) == 0 and blocks * 32 <= 2 * K * dv
+                and ctx.max_query_len >= POOLED_MIX_FROM and all(t is None or t.data_ptr() % 16 == 0 for t in (q, k_cache, v_cache, k_pool, v_pool, out))):
+            _pooled_mix(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table, H, K, d, dv, scale, softcap or 0.0, window, pool, rows, talk, blocks)
+            if ctx.num_decode == 0:
+                return
+            ctx, T = _first_requests(ctx, ctx.num_decode), ctx.num_decode      # the requests with one token each go on alone
+    parts = ctx.workspace.get("pooled_parts", (T, H, K, dv), torch.float32) if talk is not None else None
     pair_flops = 2.0 * H * (d + (K if talk is not None else 1) * dv)
     plain_tokens = T
     if use_fast_pooled_attention and fast_pooled_attention_supported(q.dtype, H, K, d, dv) and page_size & (page_size - 1) == 0:
@@ -2054,6 +2062,71 @@ def attention_pooled(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table,
         _cost(_size(parts) + _size(out), 2.0 * T * H * H * dv)
         _check(_lib("mb_attention_pooled").mb_talk_mix(_ptr(parts), _ptr(talk), _ptr(out), _code(out), _c_int(T), _c_int(H), _c_int(K), _c_int(dv),
                                                       _stream()), "heads' weights mixed")
+
+
+#: prompt portions with mixed head weights go to the kernels that mix the weights ahead of the values (False: every head's sums over every kv head's values,
+#: mixed afterwards)
+use_pooled_mix = True
+#: ... when the step's longest portion fills at least one tile of queries
+POOLED_MIX_FROM = 16
+
+
+def pooled_mix_supported(dtype, H: int, K: int, d: int, dv: int) -> bool:
+    """16 or 32 heads, two or four of them a kv head: the heads are an operand's rows in whole 16s, a warp takes a kv head's."""
+    return fast_pooled_attention_supported(dtype, H, K, d, dv) and H in (16, 32) and H // K in (2, 4) and _pooled_mix_smem(H, K, d) <= 227 * 1024
+
+
+def _pooled_mix_smem(H: int, K: int, d: int) -> int:
+    """Bytes of shared memory the mixing kernel needs (its keys, the weights of 512 pairs in two parts, the mixed rows, the mixing matrix)."""
+    return K * 32 * (d + 8) * 2 + 2 * 16 * (32 * (2 * H + 16) + 16) + H * (16 * 80 + 16) + 2 * (H // 16) ** 2 * 512
+
+
+def _pooled_mix_blocks(ctx, window: int, pool: int) -> int:
+    """The most blocks of 32 rows that a tile of 16 queries of the step meets: pooled rows, then positions."""
+    longest = ctx.max_seq_len
+    pooled = -(-max(0, (longest - window) // pool) // 32) if pool and window else 0
+    seen = min(longest, window + 15) if window else longest
+    return pooled + (seen + 30) // 32 + 1
+
+
+def _pooled_mix_name(d: int, dv: int, H: int, K: int) -> str:
+    return f"mb_attention_pooled_mix_d{d}_v{dv}_g{H // K}_k{K}"
+
+
+def _pooled_mix_job(d: int, dv: int, H: int, K: int) -> tuple:
+    return (["attention_pooled_mix.cu"], [f"HEAD_DIM={d}", f"V_DIM={dv}", f"GROUP={H // K}", f"KV_HEADS={K}"])
+
+
+def _first_requests(ctx, n: int):
+    """The step as its first ``n`` requests see it, which bring one token each."""
+    import copy
+
+    first = copy.copy(ctx)
+    first.num_requests = first.num_tokens = n
+    first.max_query_len = 1
+    return first
+
+
+def _pooled_mix(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table, H: int, K: int, d: int, dv: int, scale: float, softcap: float, window: int,
+                pool: int, rows: int, talk, blocks: int) -> None:
+    """The step's portions (requests ``num_decode`` on) through the three kernels that mix the heads' weights ahead of the values."""
+    nd, T, ws = ctx.num_decode, q.shape[0], ctx.workspace
+    count = ctx.num_requests - nd
+    lse = ws.get("pooled_lse", (T, H), torch.float32)
+    mixed = ws.get("pooled_mixed", (((T - nd) // 16 + count) * blocks * H * 512,), q.dtype)
+    lib = build.load(_pooled_mix_name(d, dv, H, K), *_pooled_mix_job(d, dv, H, K))
+    args = (_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(k_pool), _ptr(v_pool), _ptr(lse), _ptr(talk), _ptr(mixed), _ptr(out), _ptr(block_table),
+            _c_int(block_table.shape[1]), _ptr(ctx.cu_tokens), _ptr(ctx.seq_lens), _c_int(nd), _c_int(count), _c_int(ctx.max_query_len),
+            _c_int(k_cache.shape[2]), _c_float(scale), _c_float(softcap), _c_int(window), _c_int(pool), _c_int(rows), _c_int(blocks), _stream())
+    size = q.element_size()
+    # what the algorithm needs is shared out: the queries and keys with the sums, the mixing of a pair's weights, the values and results with the last
+    for which, what, nbytes, per_key, per_pair in (
+            (0, "attention (sums of weights)", (T - nd) * H * d * size, K * d * size, 2.0 * H * d), (1, "attention (weights mixed)", 0, 0, 2.0 * H * H),
+            (2, "attention (mixed weights, values)", (T - nd) * H * dv * size, K * dv * size, 2.0 * H * dv)):
+        if launch_log is not None:
+            _cost(nbytes, 0.0, per_key, per_pair)
+            _pending_cost["rows"], _pending_cost["window"] = ("prefill" if nd else "all"), window
+        _check(lib.mb_attn_pooled_mix(_c_int(which), *args), what)
 
 
 #: bf16 attention over a window and pooled blocks goes to the tensor-core kernel where the head layout allows
@@ -2094,6 +2167,8 @@ def pooled_attention_jobs(dtype, H: int, K: int, d: int, dv: int) -> dict:
     if use_fast_pooled_attention and fast_pooled_attention_supported(dtype, H, K, d, dv):
         vh = pooled_value_heads(K, dv)
         jobs[_pooled_name(d, dv, H // K, vh)] = _pooled_job(d, dv, H // K, vh)
+        if use_pooled_mix and pooled_mix_supported(dtype, H, K, d, dv):
+            jobs[_pooled_mix_name(d, dv, H, K)] = _pooled_mix_job(d, dv, H, K)
     return jobs
 
 
