@@ -89,30 +89,29 @@ __global__ void __launch_bounds__(AS_THREADS) attention_simple_kernel(
 // 32 rows instead of once for each.  A row's numbers are made in attention_simple_kernel's order (a score summed over d from 0 up, a chunk's
 // sum as its warps' butterflies, values added key by key, chunks from position 0 on; a chunk behind a row's position changes nothing),
 // so a token's result is the same bits whichever kernel it went through and however the prompt was cut.
-// Bound by the multiply-adds: a lane is a row, its query lies in registers, and a warp's lanes read the same key or value, which is
-// one cycle of shared memory for 16 bytes (two rows x four keys a thread took three times the multiply-adds' cycles).  The keys' and values' half
-// chunks arrive by cp.async one ahead of the arithmetic.  Measured on B200 (333 tokens, 16 heads of 128 over 8 kv heads):
-// attention_simple_kernel 605 us.
+// Bound by shared memory and the multiply-adds: a 16-byte load takes four cycles of a warp whatever it reads, so scores are made 4 rows x 4 keys a thread
+// and values added 4 rows x 8 columns (1.5 to 2 cycles of loads for one of multiply-adds).  The keys' and values' half chunks arrive by cp.async one
+// ahead of the arithmetic.  Measured on B200 (333 tokens, 16 heads of 128 over 8 kv heads): attention_simple_kernel 605 us, this
+// one 88 us; with 2 x 4 and 2 x 8 a thread, or a lane a row with its query in registers and every key read by the whole warp, 115 us.
 #define AT_ROWS 32
 #define AT_THREADS 128
 #define AT_WARPS (AT_THREADS / 32)
 #define AT_CHUNK AS_THREADS
 #define AT_HALF 64
 #define AT_LD 132                     // floats a row of 128 takes in shared memory
-#define AT_PLD 33                     // floats a key's 32 scores take
-#define AT_SMEM ((2 * AT_HALF * AT_LD + AT_CHUNK * AT_PLD + AT_ROWS) * 4)
+#define AT_SMEM ((2 * AT_ROWS * AT_LD + 2 * AT_HALF * AT_LD + AT_ROWS) * 4)
 
-template <int DM>                     // the most numbers of a head: 64 or 128
-__global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(
+__global__ void __launch_bounds__(AT_THREADS, 2) attention_tile_kernel(
     const float* __restrict__ q, const float* __restrict__ k_cache, const float* __restrict__ v_cache, float* __restrict__ out,
     const int* __restrict__ block_table, int max_pages, const int* __restrict__ cu_tokens, const int* __restrict__ seq_lens,
     int first_req, int H, int K, int d, int page_size, float scale) {
     PDL_ENTER();
     q = pdl_fresh(q); k_cache = pdl_fresh(k_cache); v_cache = pdl_fresh(v_cache);
     extern __shared__ __align__(16) float at_smem[];
-    float* sKV = at_smem;                                  // two half chunks of keys or values in turn, rows of AT_LD
-    float* sP = sKV + 2 * AT_HALF * AT_LD;                 // [128 keys][33]: scores of the 32 rows, then weights
-    float* sCorr = sP + AT_CHUNK * AT_PLD;                 // [rows]
+    float* sQ = at_smem;                                   // [rows][d]
+    float* sP = sQ + AT_ROWS * AT_LD;                      // [rows][128]: scores, then weights
+    float* sKV = sP + AT_ROWS * AT_LD;                     // two half chunks of keys or values in turn
+    float* sCorr = sKV + 2 * AT_HALF * AT_LD;              // [rows]
     const int G = H / K, per_tile = AT_ROWS / G;
     const int r = first_req + blockIdx.z, kh = blockIdx.y;
     const int tok0 = cu_tokens[r], n = cu_tokens[r + 1] - tok0;
@@ -122,13 +121,7 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(
     const int pos0 = seq_lens[r] - n + q0, last = pos0 + queries - 1;         // positions of the tile's first and last query
     const int* table = block_table + (size_t)r * max_pages;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, d4 = d >> 2;
-    const bool mine = lane < rows;                         // this lane's row: query lane / G, head lane % G of the group
-    const int my_pos = pos0 + lane / G;
-    const size_t my_row = ((size_t)(tok0 + q0 + lane / G) * H + kh * G + lane % G) * d;
 
-    float4 qr[DM / 4];
-#pragma unroll
-    for (int c = 0; c < DM / 4; ++c) qr[c] = mine && c < d4 ? *reinterpret_cast<const float4*>(q + my_row + 4 * c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     // stage: chunk * 4 + {0, 1: its keys' halves; 2, 3: its values' halves}
     auto fetch = [&](int stage) {
         const float* src = (stage & 2) ? v_cache : k_cache;
@@ -145,13 +138,25 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(
     };
     const int chunks = last / AT_CHUNK + 1, stages = chunks * 4;
     fetch(0);
-    constexpr int KEYS = 8, COLS = DM / AT_WARPS;          // keys whose sums run side by side; columns of the values a warp has
-    constexpr int OWN = AT_ROWS / AT_WARPS;                // rows whose softmax a warp does
-    float m[OWN], l[OWN], acc[COLS];
+    for (int row = warp; row < AT_ROWS; row += AT_WARPS) {
+        if (lane >= d4) continue;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (row < rows) v = *reinterpret_cast<const float4*>(q + ((size_t)(tok0 + q0 + row / G) * H + kh * G + row % G) * d + 4 * lane);
+        *reinterpret_cast<float4*>(sQ + row * AT_LD + 4 * lane) = v;
+    }
+    // scores: rows ty + 8 i x keys tx + 16 j; values: rows 4 ty + i x columns 4 tx.. and 64 + 4 tx..; softmax: rows 8 warp ..
+    const int tx = tid & 15, ty = tid >> 4;
+    constexpr int OWN = AT_ROWS / AT_WARPS;
+    float m[OWN], l[OWN], acc[4][8];
+    int row_pos[4];                                        // (of rows that are not there: nobody reads their results)
 #pragma unroll
     for (int i = 0; i < OWN; ++i) { m[i] = -INFINITY; l[i] = 0.0f; }
 #pragma unroll
-    for (int j = 0; j < COLS; ++j) acc[j] = 0.0f;
+    for (int i = 0; i < 4; ++i) {
+        row_pos[i] = pos0 + (4 * ty + i) / G;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+    }
     for (int stage = 0; stage < stages; ++stage) {
         const int base = (stage >> 2) * AT_CHUNK, off = (stage & 1) * AT_HALF;
         cp_async_wait<0>();
@@ -159,22 +164,32 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(
         if (stage + 1 < stages) fetch(stage + 1);
         const float* kv = sKV + (stage & 1) * AT_HALF * AT_LD;
         if (!(stage & 2)) {
-#pragma unroll 1
-            for (int k0 = warp * KEYS; k0 < AT_HALF; k0 += AT_WARPS * KEYS) {
-                float s[KEYS];
+            float s[4][4];
 #pragma unroll
-                for (int j = 0; j < KEYS; ++j) s[j] = 0.0f;
+            for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int c = 0; c < DM / 4; ++c) {
-                    if (c >= d4) break;
+                for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
+#pragma unroll 2
+            for (int c = 0; c < d4; ++c) {
+                float4 a[4];
 #pragma unroll
-                    for (int j = 0; j < KEYS; ++j) {
-                        const float4 k = *reinterpret_cast<const float4*>(kv + (k0 + j) * AT_LD + 4 * c);
-                        s[j] = fmaf(qr[c].w, k.w, fmaf(qr[c].z, k.z, fmaf(qr[c].y, k.y, fmaf(qr[c].x, k.x, s[j]))));
-                    }
+                for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(sQ + (ty + 8 * i) * AT_LD + 4 * c);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 k = *reinterpret_cast<const float4*>(kv + (tx + 16 * j) * AT_LD + 4 * c);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        s[i][j] = fmaf(a[i].w, k.w, fmaf(a[i].z, k.z, fmaf(a[i].y, k.y, fmaf(a[i].x, k.x, s[i][j]))));
                 }
+            }
 #pragma unroll
-                for (int j = 0; j < KEYS; ++j) sP[(off + k0 + j) * AT_PLD + lane] = base + off + k0 + j <= my_pos ? s[j] * scale : -INFINITY;
+            for (int i = 0; i < 4; ++i) {
+                const int row = ty + 8 * i, pos = pos0 + row / G;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int key = off + tx + 16 * j;
+                    sP[row * AT_LD + key] = base + key <= pos ? s[i][j] * scale : -INFINITY;
+                }
             }
             if (!(stage & 1)) continue;
             __syncthreads();                               // the chunk's scores are all there
@@ -182,14 +197,14 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(
             for (int i = 0; i < OWN; ++i) {
                 const int row = OWN * warp + i, pos = pos0 + row / G;
                 if (row >= rows) continue;
-                float* p = sP + lane * AT_PLD + row;       // a lane a key
-                const float s0 = p[0], s1 = p[32 * AT_PLD], s2 = p[64 * AT_PLD], s3 = p[96 * AT_PLD];
+                float* p = sP + row * AT_LD + lane;        // a lane a key
+                const float s0 = p[0], s1 = p[32], s2 = p[64], s3 = p[96];
                 const float m_new = fmaxf(m[i], warp_max(fmaxf(fmaxf(s0, s1), fmaxf(s2, s3))));
                 const float corr = expf(m[i] - m_new);
                 const int key = base + lane;
                 const float p0 = key <= pos ? expf(s0 - m_new) : 0.0f, p1 = key + 32 <= pos ? expf(s1 - m_new) : 0.0f;
                 const float p2 = key + 64 <= pos ? expf(s2 - m_new) : 0.0f, p3 = key + 96 <= pos ? expf(s3 - m_new) : 0.0f;
-                p[0] = p0; p[32 * AT_PLD] = p1; p[64 * AT_PLD] = p2; p[96 * AT_PLD] = p3;
+                p[0] = p0; p[32] = p1; p[64] = p2; p[96] = p3;
                 const float sum = (warp_sum(p0) + warp_sum(p2)) + (warp_sum(p1) + warp_sum(p3));      // block_sum's order
                 l[i] = fmaf(l[i], corr, sum);
                 m[i] = m_new;
@@ -198,39 +213,57 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(
             continue;                                      // (the barrier at the top of the next stage publishes the weights)
         }
         if (!(stage & 1)) {
-            const float corr = mine ? sCorr[lane] : 1.0f;
 #pragma unroll
-            for (int j = 0; j < COLS; ++j) acc[j] *= corr;
+            for (int i = 0; i < 4; ++i) {
+                const float corr = 4 * ty + i < rows ? sCorr[4 * ty + i] : 1.0f;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] *= corr;
+            }
         }
-        if (warp * COLS >= d) continue;
-        const float* p = sP + off * AT_PLD + lane;
-        const int seen = mine ? my_pos - base - off + 1 : 0;                 // keys of this half the row sees (may be beyond it)
-        const int whole = min(AT_HALF, max(0, pos0 - base - off + 1));       // keys that every row of the tile sees
+        const float* p = sP + 4 * ty * AT_LD + off;
+        const int first = base + off;
+        // four keys at a time; `all`: every row of the tile sees them
         auto add = [&](int j, bool all) {
-            const float w = p[j * AT_PLD];
-            if (!all && j >= seen) return;
+            float w[4][4];
 #pragma unroll
-            for (int c = 0; c < COLS; c += 4) {
-                const float4 v = *reinterpret_cast<const float4*>(kv + j * AT_LD + warp * COLS + c);
-                acc[c] = fmaf(w, v.x, acc[c]); acc[c + 1] = fmaf(w, v.y, acc[c + 1]); acc[c + 2] = fmaf(w, v.z, acc[c + 2]); acc[c + 3] = fmaf(w, v.w, acc[c + 3]);
+            for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(w[i]) = *reinterpret_cast<const float4*>(p + i * AT_LD + j);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float* row = kv + (j + e) * AT_LD + 4 * tx;
+                const float4 lo = *reinterpret_cast<const float4*>(row), hi = *reinterpret_cast<const float4*>(row + 64);
+                const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (!all && first + j + e > row_pos[i]) continue;
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) acc[i][c] = fmaf(w[i][e], v[c], acc[i][c]);
+                }
             }
         };
+        const int whole = min(AT_HALF, max(0, pos0 - first + 1)) & ~3, most = min(AT_HALF, last - first + 1);
         int j = 0;
-#pragma unroll 4
-        for (; j < whole; ++j) add(j, true);
-        for (; j < min(AT_HALF, last - base - off + 1); ++j) add(j, false);
+#pragma unroll 1
+        for (; j < whole; j += 4) add(j, true);
+#pragma unroll 1
+        for (; j < most; j += 4) add(j, false);
     }
     __syncthreads();                                       // (sCorr takes the sums now)
 #pragma unroll
     for (int i = 0; i < OWN; ++i)
         if (lane == 0) sCorr[OWN * warp + i] = l[i];
     __syncthreads();
-    if (!mine) return;
-    const float sum = sCorr[lane];
 #pragma unroll
-    for (int c = 0; c < COLS; c += 4)
-        if (warp * COLS + c < d)
-            *reinterpret_cast<float4*>(out + my_row + warp * COLS + c) = make_float4(acc[c] / sum, acc[c + 1] / sum, acc[c + 2] / sum, acc[c + 3] / sum);
+    for (int i = 0; i < 4; ++i) {
+        const int row = 4 * ty + i;
+        if (row >= rows) continue;
+        float* o = out + ((size_t)(tok0 + q0 + row / G) * H + kh * G + row % G) * d;
+        const float sum = sCorr[row];
+#pragma unroll
+        for (int c = 0; c < 8; c += 4) {
+            const int col = c * 16 + 4 * tx;
+            if (col < d) *reinterpret_cast<float4*>(o + col) = make_float4(acc[i][c] / sum, acc[i][c + 1] / sum, acc[i][c + 2] / sum, acc[i][c + 3] / sum);
+        }
+    }
 }
 
 // Float32 prompt portions: requests first_req .. first_req + count - 1, every earlier key visible; heads of up to 128 in whole 16-byte
@@ -242,10 +275,9 @@ MB_API int mb_attention_tile(const void* q, const void* k_cache, const void* v_c
     if (d <= 0 || d > 128 || d % 4 != 0 || K <= 0 || H % K != 0 || H / K > AT_ROWS || page_size <= 0) return MB_ERR_BAD_SIZE;
     const int per_tile = AT_ROWS / (H / K);
     if ((((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) & 15) != 0) return MB_ERR_BAD_SIZE;
-    auto kernel = d <= 64 ? attention_tile_kernel<64> : attention_tile_kernel<128>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM);
+    cudaFuncSetAttribute(attention_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM);
     dim3 grid((max_query_len + per_tile - 1) / per_tile, K, count);
-    return launch_kernel(kernel, grid, AT_THREADS, AT_SMEM, s, 0, (const float*)q, (const float*)k_cache, (const float*)v_cache,
+    return launch_kernel(attention_tile_kernel, grid, AT_THREADS, AT_SMEM, s, 0, (const float*)q, (const float*)k_cache, (const float*)v_cache,
                          (float*)out, block_table, max_pages, cu_tokens, seq_lens, first_req, H, K, d, page_size, scale);
 }
 

@@ -162,14 +162,15 @@ static int launch_tile(const void* x, const void* w, void* out, int T, int N, in
     return launch_kernel(kernel, grid, S::THREADS, smem, s, 0, (const TX*)x, (const TW*)w, (TO*)out, T, N, K, vec);
 }
 
-// Few weight rows: tiles of 32 x 32 whose block cuts k over eight half warps, so that N = 1,024 and a few hundred tokens still put some eight
-// warps on every SM.  The border lies in N alone (the order of a row's sums must not follow the batch).
+// A block's tile is worked on by groups that cut k, so that a few hundred tokens put enough warps on every SM: two groups of two warps on 64 x 64, and
+// with few weight rows eight half warps on 32 x 32 (333 tokens by 4,096 + 6,144 weight rows of 1,024: 190 us with two groups, 346 us with one; by 1,024
+// rows of 2,048 and 3,072: 206 us).  The border lies in N alone (the order of a row's sums must not follow the batch).
 #define GS_FEW_ROWS 3072
 
 template <typename TX, typename TW, typename TO, bool ACC>
 static int launch(const void* x, const void* w, void* out, int T, int N, int K, int vec, cudaStream_t s) {
     if (N <= GS_FEW_ROWS) return launch_tile<TX, TW, TO, ACC, 32, 32, 8, 8>(x, w, out, T, N, K, vec, s);
-    return launch_tile<TX, TW, TO, ACC, 64, 64, 8, 1>(x, w, out, T, N, K, vec, s);
+    return launch_tile<TX, TW, TO, ACC, 64, 64, 8, 2>(x, w, out, T, N, K, vec, s);
 }
 
 template <typename TX, typename TW, typename TO>
