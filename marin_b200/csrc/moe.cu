@@ -71,7 +71,7 @@ __device__ __forceinline__ void moe_choose(float* z, float* score_of, float* gro
         }
         __syncwarp();
     }
-    float chosen_sum = 0.0f;
+    float chosen_sum = 0.0f, kept = 0.0f;                      // (lane c keeps choice c's score; more than 32 choices are read back)
     for (int c = 0; c < top; ++c) {
         float best = -INFINITY;
         int at = 0x7fffffff;
@@ -88,18 +88,20 @@ __device__ __forceinline__ void moe_choose(float* z, float* score_of, float* gro
         if (at >= E) at = c;                                   // logits that are not numbers order nothing: stay inside the table
         const float score = correction != nullptr ? score_of[at] : score_mode == 1 ? expf(best - zmax) / denom : 1.0f / (1.0f + expf(-best));
         chosen_sum += score;
+        if (lane == c) kept = score;
         if (lane == 0) {
             expert_out[(size_t)t * top + c] = at;
-            weight_out[(size_t)t * top + c] = score;
+            if (top > 32) weight_out[(size_t)t * top + c] = score;
             z[at] = -INFINITY;
         }
         __syncwarp();
     }
-    if ((renorm || factor != 1.0f) && lane == 0)
-        for (int c = 0; c < top; ++c) {
-            const float w = weight_out[(size_t)t * top + c];
-            weight_out[(size_t)t * top + c] = (renorm ? w / (chosen_sum + 1e-20f) : w) * factor;
-        }
+    const auto final_of = [&](float w) { return renorm || factor != 1.0f ? (renorm ? w / (chosen_sum + 1e-20f) : w) * factor : w; };
+    if (top <= 32) {
+        if (lane < top) weight_out[(size_t)t * top + lane] = final_of(kept);
+    } else if (lane == 0) {
+        for (int c = 0; c < top; ++c) weight_out[(size_t)t * top + c] = final_of(weight_out[(size_t)t * top + c]);
+    }
 }
 
 template <typename T>
@@ -152,49 +154,64 @@ __global__ void __launch_bounds__(MR_THREADS) moe_route_kernel(const T* __restri
     if (warp == 0) moe_choose(z, z + E, z + 2 * E, t, expert_out, weight_out, E, top, score_mode, renorm, correction, groups, keep, factor);
 }
 
-// The same sums (the same chains, the same bits) straight from memory in bf16, a warp a token and expert, no row staged ahead: the kernel above is a
-// chain of waits, the row's numbers two bytes at a time, then the experts (10 us for 48 tokens, 31 us for 2,048 of 2,560 and 8 experts).
-// MANY: a block takes eight tokens, a warp each, whose loads of a router row meet in L1; else a block takes one token, its warps the experts in turn.
-__device__ __forceinline__ float route_dot(const bf16* __restrict__ x, const float* __restrict__ w, int h) {
-    const float4* w4 = reinterpret_cast<const float4*>(w);
-    const uint2* x4 = reinterpret_cast<const uint2*>(x);
-    const int n4 = h >> 2;
-    float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+// The same sums (the same chains, the same bits) for PER tokens a block in bf16: a warp takes an expert, whose row it loads once for all of them, while the
+// tokens' rows lie in shared memory as they came (PER 1: are read where they are).  Bound by the router's rows through L2 (a block a token: 168 MB for 2,048
+// tokens of 2,560 and 8 experts, 31 us; L1 keeps nothing of them beside a neighbour's 200 KB of shared memory) and, with few tokens, by the chain of waits.  Measured (2,560 numbers,
+// 8 experts): 2,048 tokens 20 us where the kernel above takes 31, 48 tokens 8.4 us for 10.3.
+template <int PER>
+__global__ void __launch_bounds__(MR_THREADS) moe_route_rows_kernel(const bf16* __restrict__ h_rows, const float* __restrict__ router,
+                                                                    const float* __restrict__ router_bias, int* __restrict__ expert_out,
+                                                                    float* __restrict__ weight_out, int tokens, int h, int E, int top, int score_mode, int renorm,
+                                                                    const float* __restrict__ correction, int groups, int keep, float factor) {
+    PDL_ENTER();
+    h_rows = pdl_fresh(h_rows);
+    extern __shared__ __align__(16) float smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per = 2 * E + groups;
+    const int t0 = blockIdx.x * PER, here = min(PER, tokens - t0), n4 = h >> 2;
+    float* z = smem;                                           // [PER][per]: a token's logits, scores and groups
+    const uint2* x = reinterpret_cast<const uint2*>(h_rows + (size_t)t0 * h);
+    if (PER > 1) {
+        uint2* rows = reinterpret_cast<uint2*>(smem + (PER * per + 3) / 4 * 4);
+        const int total = here * n4;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < PER * n4; i += MR_THREADS) rows[i] = i < total ? x[i] : make_uint2(0u, 0u);
+        x = rows;
+        __syncthreads();
+    }
     auto add = [](float& s, const uint2& u, const float4& a) {
         const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
         s = fmaf(lo.x, a.x, fmaf(lo.y, a.y, fmaf(hi.x, a.z, fmaf(hi.y, a.w, s))));
     };
-    int j = threadIdx.x & 31;
-#pragma unroll 2
-    for (; j + 96 < n4; j += 128) {
-        const float4 a[4] = {w4[j], w4[j + 32], w4[j + 64], w4[j + 96]};
-        const uint2 b[4] = {x4[j], x4[j + 32], x4[j + 64], x4[j + 96]};
+    for (int e = warp; e < E; e += MR_THREADS / 32) {
+        const float4* w4 = reinterpret_cast<const float4*>(router + (size_t)e * h);
+        float d[PER][4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) add(d[c], b[c], a[c]);
+        for (int p = 0; p < PER; ++p) d[p][0] = d[p][1] = d[p][2] = d[p][3] = 0.0f;
+        int j = lane;
+#pragma unroll 2
+        for (; j + 96 < n4; j += 128) {
+            const float4 a[4] = {w4[j], w4[j + 32], w4[j + 64], w4[j + 96]};
+#pragma unroll
+            for (int p = 0; p < PER; ++p)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) add(d[p][c], x[p * n4 + j + 32 * c], a[c]);
+        }
+        for (; j < n4; j += 32) {
+            const float4 a = w4[j];
+#pragma unroll
+            for (int p = 0; p < PER; ++p) add(d[p][0], x[p * n4 + j], a);
+        }
+#pragma unroll
+        for (int p = 0; p < PER; ++p) {
+            const float dot = warp_sum((d[p][0] + d[p][1]) + (d[p][2] + d[p][3]));
+            if (lane == 0) z[p * per + e] = router_bias != nullptr ? dot + router_bias[e] : dot;
+        }
     }
-    for (; j < n4; j += 32) add(d[0], x4[j], w4[j]);
-    return warp_sum((d[0] + d[1]) + (d[2] + d[3]));
-}
-
-template <bool MANY>
-__global__ void __launch_bounds__(MR_THREADS) moe_route_direct_kernel(const bf16* __restrict__ h_rows, const float* __restrict__ router,
-                                                                      const float* __restrict__ router_bias, int* __restrict__ expert_out,
-                                                                      float* __restrict__ weight_out, int tokens, int h, int E, int top, int score_mode, int renorm,
-                                                                      const float* __restrict__ correction, int groups, int keep, float factor) {
-    PDL_ENTER();
-    h_rows = pdl_fresh(h_rows);
-    extern __shared__ float smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per = 2 * E + groups;
-    const int t = MANY ? blockIdx.x * (MR_THREADS / 32) + warp : blockIdx.x;
-    if (t >= tokens) return;                                   // (many: nobody waits for this warp)
-    float* z = smem + (MANY ? warp * per : 0);
-    for (int e = MANY ? 0 : warp; e < E; e += MANY ? 1 : MR_THREADS / 32) {
-        const float dot = route_dot(h_rows + (size_t)t * h, router + (size_t)e * h, h);
-        if (lane == 0) z[e] = router_bias != nullptr ? dot + router_bias[e] : dot;
+    __syncthreads();
+    if (warp < here) {
+        z += warp * per;
+        moe_choose(z, z + E, z + 2 * E, t0 + warp, expert_out, weight_out, E, top, score_mode, renorm, correction, groups, keep, factor);
     }
-    if (MANY) __syncwarp();
-    else __syncthreads();
-    if (MANY || warp == 0) moe_choose(z, z + E, z + 2 * E, t, expert_out, weight_out, E, top, score_mode, renorm, correction, groups, keep, factor);
 }
 
 // E: all outputs of the router (identity outputs included).  groups 1: no groups; correction null: none; factor: on the weights.
@@ -205,14 +222,12 @@ MB_API int mb_moe_route(const void* h_rows, int dtype, const float* router, cons
     if (groups <= 0 || E % groups != 0 || keep <= 0 || keep > groups || (keep < groups && top > E / groups * keep)) return MB_ERR_BAD_SIZE;
     const size_t smem = (size_t)(2 * E + groups + h) * sizeof(float);
     if (smem > 48 * 1024) return MB_ERR_BAD_SIZE;
-    const size_t per = (size_t)(2 * E + groups) * sizeof(float), few = MR_THREADS / 32;
     if (dtype == MB_BF16 && h % 4 == 0 && (((uintptr_t)h_rows) & 7) == 0 && (((uintptr_t)router) & 15) == 0) {
-        // a warp a token once that puts a block on every SM (148 blocks of eight tokens)
-        if (tokens >= 148 * (int)few && few * per <= 48 * 1024)
-            return launch_kernel(moe_route_direct_kernel<true>, (tokens + (int)few - 1) / (int)few, MR_THREADS, few * per, s, 0, (const bf16*)h_rows, router, router_bias,
-                                 expert_out, weight_out, tokens, h, E, top, score_mode, renorm, correction, groups, keep, factor);
-        return launch_kernel(moe_route_direct_kernel<false>, tokens, MR_THREADS, per, s, 0, (const bf16*)h_rows, router, router_bias, expert_out, weight_out, tokens,
-                             h, E, top, score_mode, renorm, correction, groups, keep, factor);
+        // as many tokens a block as still give every SM a block or two (148 SMs), if their rows fit
+        const size_t per = (size_t)(2 * E + groups) * sizeof(float);
+#define MR_CASE(PER, FROM)                                                                                                                                        if (tokens >= FROM && (PER == 1 || PER * (per + (size_t)h * 2) + 16 <= 48 * 1024))                                                                                return launch_kernel(moe_route_rows_kernel<PER>, (tokens + PER - 1) / PER, MR_THREADS, PER * per + (PER > 1 ? (size_t)PER * h * 2 + 16 : 0), s, 0,                                 (const bf16*)h_rows, router, router_bias, expert_out, weight_out, tokens, h, E, top, score_mode, renorm, correction, groups, keep, factor);
+        MR_CASE(8, 8 * 148) MR_CASE(4, 4 * 148) MR_CASE(2, 2 * 148) MR_CASE(1, 1)
+#undef MR_CASE
     }
     if (dtype == MB_F32)
         return launch_kernel(moe_route_kernel<float>, tokens, MR_THREADS, smem, s, 0, (const float*)h_rows, router, router_bias, expert_out,

@@ -891,9 +891,9 @@ def test_grouped_expert_products_on_tcgen05_match_the_plain_twin(ops, request, a
     assert float(off.max()) <= 0.05 * float((want - y0).abs().max())
 
 
-@pytest.mark.parametrize("T,h,E", [(1183, 96, 3), (1184, 96, 8), (1187, 2560, 9), (2049, 52, 20), (5, 2560, 64), (3, 132, 7)])
+@pytest.mark.parametrize("T,h,E", [(1183, 96, 3), (1184, 96, 8), (1187, 2560, 9), (2049, 52, 20), (5, 2560, 64), (3, 132, 7), (301, 96, 8), (603, 132, 5)])
 def test_router_straight_from_memory_has_the_staged_kernels_bits(ops, T, h, E):
-    """A warp a token (from 1,184 on), a block a token below, and the kernel that stages the row (taken for rows that are not at 8-byte addresses)."""
+    """Eight, four, two tokens a block (from 1,184, 592, 296 on) and one, and the kernel that stages the row (taken for rows that are not at 8-byte addresses)."""
     g = torch.Generator(device=DEV).manual_seed(T)
     flat = torch.zeros(T * h + 1, device=DEV, dtype=torch.bfloat16)
     x = torch.randn(T, h, generator=g, device=DEV).to(torch.bfloat16)
