@@ -19,36 +19,40 @@
 #include "common.cuh"
 #include "launch.cuh"
 
-#define PB_THREADS 128
+// ---- pooled rows: a block per run of tokens and kv head; only tokens that end a block of `pool` positions do anything --------
+// A thread sums one column over the block's rows, page by page, so that many rows are in flight (a block per token whose threads looked every
+// row's page up in turn: 40 us for 2,048 tokens, 8 heads of 128 + 128 and pools of 64, of which 8.5 MB are read; 8 us this way).
+#define PB_TOKENS 32
+#define PB_BLOCK 256
 
-// ---- pooled rows: a block per (token, kv head); only a token that ends a block of `pool` positions does anything ---------
 template <typename T>
-__global__ void __launch_bounds__(PB_THREADS) pool_blocks_kernel(
+__global__ void __launch_bounds__(PB_BLOCK) pool_blocks_kernel(
     const T* __restrict__ k_cache, const T* __restrict__ v_cache, T* __restrict__ k_pool, T* __restrict__ v_pool,
     const int* __restrict__ block_table, int max_pages, const int* __restrict__ req_index, const int* __restrict__ positions,
-    const int* __restrict__ slot_mapping, int K, int d, int dv, int page_size, int pool, int pool_rows) {
+    const int* __restrict__ slot_mapping, int K, int d, int dv, int page_size, int pool, int pool_rows, int tokens) {
     PDL_ENTER();
     k_cache = pdl_fresh(k_cache); v_cache = pdl_fresh(v_cache);
-    const int t = blockIdx.x, kh = blockIdx.y;
-    const int pos = positions[t];
-    if (slot_mapping[t] < 0 || (pos + 1) % pool != 0) return;
-    const int* table = block_table + (size_t)req_index[t] * max_pages;
-    const int first = pos + 1 - pool;
-    const size_t dst_page = (size_t)table[pos / page_size];
-    const size_t dst_row = (dst_page * K + kh) * pool_rows + (size_t)((pos % page_size) / pool);
-    const float inv = 1.0f / (float)pool;
-    for (int i = threadIdx.x; i < d + dv; i += PB_THREADS) {
-        const bool key = i < d;
-        const int e = key ? i : i - d;
-        const int width = key ? d : dv;
-        const T* src = key ? k_cache : v_cache;
-        float sum = 0.0f;
-        for (int j = 0; j < pool; ++j) {
-            const int p = first + j;
-            const size_t page = (size_t)table[p / page_size];
-            sum += to_f32(src[((page * K + kh) * page_size + (size_t)(p % page_size)) * width + e]);
+    const int t0 = blockIdx.x * PB_TOKENS, kh = blockIdx.y, mine = t0 + (threadIdx.x & 31);
+    unsigned ends = __ballot_sync(0xffffffffu, mine < tokens && slot_mapping[min(mine, tokens - 1)] >= 0 && (positions[min(mine, tokens - 1)] + 1) % pool == 0);
+    for (; ends != 0; ends &= ends - 1) {                      // (every warp finds the same tokens)
+        const int t = t0 + __ffs(ends) - 1, pos = positions[t];
+        const int* table = block_table + (size_t)req_index[t] * max_pages;
+        const size_t dst_row = ((size_t)table[pos / page_size] * K + kh) * pool_rows + (size_t)((pos % page_size) / pool);
+        const float inv = 1.0f / (float)pool;
+        for (int i = threadIdx.x; i < d + dv; i += PB_BLOCK) {
+            const bool key = i < d;
+            const int e = key ? i : i - d, width = key ? d : dv;
+            const T* src = (key ? k_cache : v_cache) + e;
+            float sum = 0.0f;
+            for (int p = pos + 1 - pool; p <= pos;) {          // in the order of the positions
+                const int at = p % page_size, run = min(page_size - at, pos + 1 - p);
+                const T* rows = src + (((size_t)table[p / page_size] * K + kh) * page_size + at) * width;
+#pragma unroll 16
+                for (int j = 0; j < run; ++j) sum += to_f32(rows[(size_t)j * width]);
+                p += run;
+            }
+            (key ? k_pool : v_pool)[dst_row * width + e] = from_f32<T>(sum * inv);
         }
-        (key ? k_pool : v_pool)[dst_row * width + e] = from_f32<T>(sum * inv);
     }
 }
 
@@ -57,15 +61,15 @@ MB_API int mb_pool_blocks(const void* k_cache, const void* v_cache, void* k_pool
                           int dv, int page_size, int pool, int pool_rows, cudaStream_t s) {
     if (tokens <= 0) return 0;
     if (K <= 0 || d <= 0 || dv <= 0 || pool <= 0 || pool_rows != (page_size + pool - 1) / pool) return MB_ERR_BAD_SIZE;
-    dim3 grid(tokens, K);
+    dim3 grid((tokens + PB_TOKENS - 1) / PB_TOKENS, K);
     if (dtype == MB_F32)
-        return launch_kernel(pool_blocks_kernel<float>, grid, PB_THREADS, 0, s, 0, (const float*)k_cache, (const float*)v_cache,
+        return launch_kernel(pool_blocks_kernel<float>, grid, PB_BLOCK, 0, s, 0, (const float*)k_cache, (const float*)v_cache,
                              (float*)k_pool, (float*)v_pool, block_table, max_pages, req_index, positions, slot_mapping, K, d, dv, page_size,
-                             pool, pool_rows);
+                             pool, pool_rows, tokens);
     if (dtype == MB_BF16)
-        return launch_kernel(pool_blocks_kernel<bf16>, grid, PB_THREADS, 0, s, 0, (const bf16*)k_cache, (const bf16*)v_cache,
+        return launch_kernel(pool_blocks_kernel<bf16>, grid, PB_BLOCK, 0, s, 0, (const bf16*)k_cache, (const bf16*)v_cache,
                              (bf16*)k_pool, (bf16*)v_pool, block_table, max_pages, req_index, positions, slot_mapping, K, d, dv, page_size,
-                             pool, pool_rows);
+                             pool, pool_rows, tokens);
     return MB_ERR_BAD_DTYPE;
 }
 

@@ -7,12 +7,13 @@
 // times the products with V, and a float32 [tokens][H][KV_HEADS][V_DIM] that a second kernel reads.)  Mixing needs the weights already
 // divided by their sums, so three kernels:
 //   stats_kernel  (a CTA per kv head and 128 rows = queries x its heads): the logarithm of every row's sum of weights;
-//   mix_kernel    (a CTA per 16 queries, a warp per kv head, 32 keys at a time): the weights of all heads, mixed, to scratch memory as bf16;
-//   value_kernel  (a CTA per 16 queries and kv head, a warp per head): mixed weights x values.
+//   mix_kernel    (a CTA per 16 queries, two heads a warp, 32 keys at a time): the weights of all heads, mixed, to scratch memory as bf16;
+//   value_kernel  (a CTA per 32 queries and kv head, a warp per head and 16 queries): mixed weights x values.
 // Exactness: the weights p are float32 and enter the mixing product as pairs of bf16 numbers (p = hi + lo), as does talk; the three larger of the four
 // products are taken, so about 16 bits of each enter, and the mixed weights are rounded to bf16 once, where the other kernel rounds every head's.
 // Scratch: [tile][block][H][16][32] bf16, a tile of 16 queries of one request, its blocks of 32 pooled rows, then of 32 positions.
-// Measured on B200, 2,048 tokens, 32 heads of 128 over 8, window 1,024, pools of 64: the other kernel and its mixing 1,189 us.
+// Measured on B200, 2,048 tokens, 32 heads of 128 over 8, window 1,024, pools of 64: the other kernel and its mixing 1,189 us;
+// these 95 + 216 + 100 us.  mix_kernel is bound by the instructions that make a weight (about fourteen a score, with the cap) and its two mixing products.
 #define MB_LIB "attention_pooled_mix"
 #define MB_LIB_ID 25
 #include "common.cuh"
@@ -53,9 +54,39 @@ __device__ __forceinline__ float ex2_approx(float x) {
 }
 // tanh(x) = 1 - 2 / (1 + e^(2x)) from the fast exponential: its absolute error is a few 1e-7 (see attention_pooled_fast.cu)
 __device__ __forceinline__ float tanh_approx(float x) { return 1.0f - __fdividef(2.0f, 1.0f + ex2_approx(x * (2.0f * LOG2E))); }
-// A score in the exp2 domain, capped where there is a cap.
-struct Cap { float scaled, cap_l2, sl2; bool on; };
-__device__ __forceinline__ float score_of(float s, const Cap& c) { return c.on ? c.cap_l2 * tanh_approx(s * c.scaled) : s * c.sl2; }
+// Scores in the exp2 domain, capped where there is a cap: cap tanh(x) with x = s scale / cap.  Where every |x| of a warp's block is at most 0.5, tanh(x) = x P(x^2)
+// with the cubic fitted there by least squares that attention_tc.cu uses (relative error 6e-7), which leaves the one exponential of the weight to the unit for
+// functions; else from the fast exponential.
+struct Cap {
+    float to_cap, sl2, p0, p1, p2, p3;
+    bool on;
+    __device__ Cap(float scale, float cap) {
+        on = cap > 0.0f;
+        to_cap = on ? scale / cap : 0.0f;
+        sl2 = (on ? cap : scale) * LOG2E;
+        const float c2 = to_cap * to_cap;
+        p0 = 0.999999464f * to_cap; p1 = -0.333264679f * to_cap * c2; p2 = 0.131918818f * to_cap * c2 * c2; p3 = -0.0444444381f * to_cap * c2 * c2 * c2;
+    }
+    // what sl2 multiplies
+    __device__ float small(float s) const { const float t = s * s; return s * fmaf(t, fmaf(t, fmaf(t, p3, p2), p1), p0); }
+    template <int N> __device__ void apply(float (*s)[4]) const {
+        if (!on) return;
+        float top = 0.0f;
+#pragma unroll
+        for (int j = 0; j < N; ++j) top = fmaxf(top, fmaxf(fmaxf(fabsf(s[j][0]), fabsf(s[j][1])), fmaxf(fabsf(s[j][2]), fabsf(s[j][3]))));
+        if (__all_sync(0xffffffffu, top * fabsf(to_cap) <= 0.5f)) {
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[j][e] = small(s[j][e]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[j][e] = tanh_approx(s[j][e] * to_cap);
+        }
+    }
+};
 
 // What a query at position p sees: pooled rows below nb, positions from lo on.
 __device__ __forceinline__ int first_seen(int p, int window) { return window > 0 ? max(0, p - window + 1) : 0; }
@@ -147,7 +178,7 @@ __global__ void __launch_bounds__(256, 2) stats_kernel(
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) q_fragment(qa[kk], rows[0], rows[1], kk * 16 + 2 * (lane & 3));
     }
-    const Cap c = {cap > 0.0f ? scale / cap : 0.0f, cap * LOG2E, scale * LOG2E, cap > 0.0f};
+    const Cap c(scale, cap);
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};
     for (int b = 0; b < blocks.count; ++b) {
         const bool pooled = blocks.is_pooled(b);
@@ -168,24 +199,32 @@ __global__ void __launch_bounds__(256, 2) stats_kernel(
                 mma_bf16_16816(s[j], qa[kk], b0, b1);
                 mma_bf16_16816(s[j + 1], qa[kk], b2, b3);
             }
+        c.apply<SN / 8>(s);
         float mx[2] = {-INFINITY, -INFINITY};
+        const bool inside = pooled ? key0 + SN <= nb[0] : key0 + SN - 1 <= qp[0] && key0 >= lo[1];      // (rows that are not there: positions beyond)
+        if (!inside) {
+#pragma unroll
+            for (int j = 0; j < SN / 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int rr = e >> 1, kj = key0 + j * 8 + 2 * (lane & 3) + (e & 1);
+                    if (!(pooled ? kj < nb[rr] : (kj <= qp[rr] && kj >= lo[rr]))) s[j][e] = -INFINITY;
+                }
+        }
 #pragma unroll
         for (int j = 0; j < SN / 8; ++j)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int rr = e >> 1, kj = key0 + j * 8 + 2 * (lane & 3) + (e & 1);
-                const bool seen = pooled ? kj < nb[rr] : (kj <= qp[rr] && kj >= lo[rr]);
-                s[j][e] = seen ? score_of(s[j][e], c) : -INFINITY;
-                mx[rr] = fmaxf(mx[rr], s[j][e]);
+                mx[e >> 1] = fmaxf(mx[e >> 1], s[j][e]);
             }
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
             mx[rr] = fmaxf(mx[rr], __shfl_xor_sync(0xffffffffu, mx[rr], 1));
             mx[rr] = fmaxf(mx[rr], __shfl_xor_sync(0xffffffffu, mx[rr], 2));
-            const float m_new = fmaxf(m_run[rr], mx[rr]), base = m_new == -INFINITY ? 0.0f : m_new;
+            const float m_new = fmaxf(m_run[rr], mx[rr] * c.sl2), base = m_new == -INFINITY ? 0.0f : m_new;
             float sum = 0.0f;
 #pragma unroll
-            for (int j = 0; j < SN / 8; ++j) sum += ex2_approx(s[j][2 * rr] - base) + ex2_approx(s[j][2 * rr + 1] - base);
+            for (int j = 0; j < SN / 8; ++j) sum += ex2_approx(fmaf(s[j][2 * rr], c.sl2, -base)) + ex2_approx(fmaf(s[j][2 * rr + 1], c.sl2, -base));
             l_run[rr] = l_run[rr] * ex2_approx(m_run[rr] - base) + sum;
             m_run[rr] = m_new;
         }
@@ -200,7 +239,10 @@ __global__ void __launch_bounds__(256, 2) stats_kernel(
 }
 
 // ---- the weights of all heads, mixed -----------------------------------------------------------------------------------------------------
-#define MIX_THREADS (32 * KH)
+#define HW 2                          // heads a warp: their queries and scores then fit 128 registers, and 16 warps hide one another's waits
+#define WK (G / HW)                   // warps a kv head
+#define MIX_WARPS (KH * WK)
+#define MIX_THREADS (32 * MIX_WARPS)
 #define P_PITCH (2 * NH + 16)         // bytes of a pair's row of H weights
 #define P_QUERY (NK * P_PITCH + 16)   // bytes between queries (ldmatrix over a query's keys and the stores over queries both spread over the banks)
 #define P_BYTES (NQ * P_QUERY)
@@ -224,7 +266,7 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
     PDL_ENTER();
     q = pdl_fresh(q); k_cache = pdl_fresh(k_cache); k_pool = pdl_fresh(k_pool); lse = pdl_fresh(lse);
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    bf16* sK = reinterpret_cast<bf16*>(smem_raw);              // [KH][NK][LDK]: a kv head's block belongs to its warp alone
+    bf16* sK = reinterpret_cast<bf16*>(smem_raw);              // [KH][NK][LDK]: a kv head's block is fetched and read by its own warps
     uint8_t* sPh = smem_raw + KH * NK * LDK * 2;               // [NQ][NK] rows of H weights: the larger part ...
     uint8_t* sPl = sPh + P_BYTES;                              // ... and what it leaves
     uint8_t* sW = sPl + P_BYTES;                               // [H][NQ] rows of NK mixed weights
@@ -237,16 +279,17 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
     const Blocks blocks(pos0, pos0 + here - 1, window, pool, NK);
     bf16* dst = mixed + (size_t)(first_tile(cu_tokens, first_req, r) + qt) * most_blocks * (NH * NQ * NK);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t2 = 2 * (lane & 3);
-    bf16* myK = sK + warp * NK * LDK;
-    auto fetch = [&](int b) {                                  // this warp's kv head's keys: 16 bytes a lane
+    const int kv = warp / WK;
+    bf16* myK = sK + kv * NK * LDK;
+    auto fetch = [&](int b) {                                  // this warp's part of its kv head's keys: 16 bytes a lane
         const bool pooled = blocks.is_pooled(b);
         const int key0 = blocks.key0(b, NK), last = pooled ? blocks.nb_most - 1 : pos0 + here - 1;
         const bf16* src = pooled ? k_pool : k_cache;
         constexpr int PER = D / 8;
 #pragma unroll 4
-        for (int idx = lane; idx < NK * PER; idx += 32) {
+        for (int idx = warp % WK * 32 + lane; idx < NK * PER; idx += 32 * WK) {
             const int row = idx / PER, c = idx % PER, key = key0 + row;
-            if (key <= last) cp_async16(myK + row * LDK + c * 8, src + row_at(table, key, pooled, warp, page_shift, pool, pool_rows) * D + c * 8);
+            if (key <= last) cp_async16(myK + row * LDK + c * 8, src + row_at(table, key, pooled, kv, page_shift, pool, pool_rows) * D + c * 8);
             else *reinterpret_cast<uint4*>(myK + row * LDK + c * 8) = make_uint4(0, 0, 0, 0);
         }
         cp_async_commit();
@@ -263,8 +306,8 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
         sT[TALK_FRAGS * 32 + idx] = lo;
     }
     // the queries of this warp's heads stay in registers; a thread's rows are queries g8 and g8 + 8
-    uint32_t qa[G][D / 16][4];
-    float base[G][2];
+    uint32_t qa[HW][D / 16][4];
+    float base[HW][2];
     int qp[2], lo[2], nb[2];
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
@@ -273,26 +316,28 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
         nb[rr] = qp[rr] >= 0 ? pools_seen(qp[rr], window, pool) : 0;
     }
 #pragma unroll
-    for (int h = 0; h < G; ++h) {
-        const size_t a0 = (size_t)(tok0 + qt * NQ + g8) * NH + warp * G + h, a1 = a0 + (size_t)8 * NH;
+    for (int h = 0; h < HW; ++h) {
+        const size_t a0 = (size_t)(tok0 + qt * NQ + g8) * NH + warp * HW + h, a1 = a0 + (size_t)8 * NH;
         const bf16 *r0 = qp[0] >= 0 ? q + a0 * D : nullptr, *r1 = qp[1] >= 0 ? q + a1 * D : nullptr;
         base[h][0] = qp[0] >= 0 ? lse[a0] : 0.0f;
         base[h][1] = qp[1] >= 0 ? lse[a1] : 0.0f;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) q_fragment(qa[h][kk], r0, r1, kk * 16 + t2);
     }
-    const Cap c = {cap > 0.0f ? scale / cap : 0.0f, cap * LOG2E, scale * LOG2E, cap > 0.0f};
+    const Cap c(scale, cap);
     const uint32_t k_addr = (uint32_t)__cvta_generic_to_shared(myK + ((lane & 7) + (lane >> 4) * 8) * LDK + ((lane >> 3) & 1) * 8);
     // a pair's row read as a B operand: eight keys of one query, 8 weights a matrix, up to 32 weights at a time
     const uint32_t p_addr = (uint32_t)__cvta_generic_to_shared(sPh + (lane & 7) * P_PITCH + (lane >> 3) * 16);
+    constexpr int MT = NH / 16;                                // 16 mixed heads at a time: a warp keeps to one of the MT, whose operands it loads once a block
+    const int mt = warp % MT;
+    cp_async_wait<0>();
+    __syncthreads();                                           // the first block's keys and talk are there
     for (int b = 0; b < blocks.count; ++b) {
         const bool pooled = blocks.is_pooled(b);
         const int key0 = blocks.key0(b, NK);
-        cp_async_wait<0>();
-        __syncwarp();                                          // this warp's keys are there
-        float s[G][NK / 8][4];
+        float s[HW][NK / 8][4];
 #pragma unroll
-        for (int h = 0; h < G; ++h)
+        for (int h = 0; h < HW; ++h)
 #pragma unroll
             for (int j = 0; j < NK / 8; ++j) s[h][j][0] = s[h][j][1] = s[h][j][2] = s[h][j][3] = 0.0f;
 #pragma unroll
@@ -302,38 +347,35 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
                 uint32_t b0, b1, b2, b3;
                 ldsm_x4(k_addr + (uint32_t)(j * 8 * LDK * 2 + kk * 32), b0, b1, b2, b3);
 #pragma unroll
-                for (int h = 0; h < G; ++h) {
+                for (int h = 0; h < HW; ++h) {
                     mma_bf16_16816(s[h][j], qa[h][kk], b0, b1);
                     mma_bf16_16816(s[h][j + 1], qa[h][kk], b2, b3);
                 }
             }
-        __syncwarp();
-        if (b + 1 < blocks.count) fetch(b + 1);
+        c.apply<HW * NK / 8>(&s[0][0]);
+        const bool inside = pooled ? key0 + NK <= nb[0] && qp[1] >= 0 : key0 + NK - 1 <= qp[0] && key0 >= lo[1] && qp[1] >= 0;
         // the weights, in two parts, to the pairs' rows
 #pragma unroll
         for (int j = 0; j < NK / 8; ++j)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int rr = e >> 1, in = j * 8 + t2 + (e & 1), kj = key0 + in;
-                const bool seen = pooled ? kj < nb[rr] : (kj <= qp[rr] && kj >= lo[rr]);
-                uint32_t hi[G / 2], low[G / 2];
-#pragma unroll
-                for (int h = 0; h < G; h += 2)
-                    split_bf16(seen ? ex2_approx(score_of(s[h][j][e], c) - base[h][rr]) : 0.0f,
-                               seen ? ex2_approx(score_of(s[h + 1][j][e], c) - base[h + 1][rr]) : 0.0f, hi[h / 2], low[h / 2]);
-                const int at = (g8 + 8 * rr) * P_QUERY + in * P_PITCH + warp * G * 2;
-                if (G == 4) {
-                    *reinterpret_cast<uint2*>(sPh + at) = make_uint2(hi[0], hi[G / 2 - 1]);
-                    *reinterpret_cast<uint2*>(sPl + at) = make_uint2(low[0], low[G / 2 - 1]);
-                } else {
-                    *reinterpret_cast<uint32_t*>(sPh + at) = hi[0];
-                    *reinterpret_cast<uint32_t*>(sPl + at) = low[0];
-                }
+                float w0 = ex2_approx(fmaf(s[0][j][e], c.sl2, -base[0][rr])), w1 = ex2_approx(fmaf(s[1][j][e], c.sl2, -base[1][rr]));
+                if (!inside && !(pooled ? kj < nb[rr] : (kj <= qp[rr] && kj >= lo[rr]))) w0 = w1 = 0.0f;
+                uint32_t hi, low;
+                split_bf16(w0, w1, hi, low);
+                const int at = (g8 + 8 * rr) * P_QUERY + in * P_PITCH + warp * HW * 2;
+                *reinterpret_cast<uint32_t*>(sPh + at) = hi;
+                *reinterpret_cast<uint32_t*>(sPl + at) = low;
             }
-        __syncthreads();                                       // every head's weights of the block are there; the mixed rows of the last one have left
+        __syncthreads();                                       // every head's weights of the block are there; its keys and the last mixed rows are done with
+        if (b + 1 < blocks.count) fetch(b + 1);
         // talk x weights: eight pairs (one query, eight keys) at a time
-#pragma unroll 2
-        for (int job = warp; job < NQ * (NK / 8); job += KH) {
+        uint4 th[MT], tl[MT];
+#pragma unroll
+        for (int ks = 0; ks < MT; ++ks) { th[ks] = sT[(mt * MT + ks) * 32 + lane]; tl[ks] = sT[(TALK_FRAGS + mt * MT + ks) * 32 + lane]; }
+#pragma unroll 4
+        for (int job = warp / MT; job < NQ * (NK / 8); job += MIX_WARPS / MT) {
             const int query = job / (NK / 8), k8 = job % (NK / 8) * 8;
             uint32_t ph[4], pl[4];
             const uint32_t row = p_addr + (uint32_t)(query * P_QUERY + k8 * P_PITCH);
@@ -345,23 +387,20 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
                 asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(ph[0]), "=r"(ph[1]) : "r"(row));
                 asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(pl[0]), "=r"(pl[1]) : "r"(row + P_BYTES));
             }
+            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-            for (int mt = 0; mt < NH / 16; ++mt) {
-                float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                for (int ks = 0; ks < NH / 16; ++ks) {
-                    const uint4 th = sT[(mt * (NH / 16) + ks) * 32 + lane], tl = sT[(TALK_FRAGS + mt * (NH / 16) + ks) * 32 + lane];
-                    const uint32_t ah[4] = {th.x, th.y, th.z, th.w}, al[4] = {tl.x, tl.y, tl.z, tl.w};
-                    mma_bf16_16816(acc, ah, ph[2 * ks], ph[2 * ks + 1]);
-                    mma_bf16_16816(acc, al, ph[2 * ks], ph[2 * ks + 1]);
-                    mma_bf16_16816(acc, ah, pl[2 * ks], pl[2 * ks + 1]);
-                }
-                uint8_t* w = sW + (mt * 16 + g8) * W_HEAD + query * W_PITCH + (k8 + t2) * 2;
-                *reinterpret_cast<uint32_t*>(w) = pack_bf16(acc[0], acc[1]);
-                *reinterpret_cast<uint32_t*>(w + 8 * W_HEAD) = pack_bf16(acc[2], acc[3]);
+            for (int ks = 0; ks < MT; ++ks) {
+                const uint32_t ah[4] = {th[ks].x, th[ks].y, th[ks].z, th[ks].w}, al[4] = {tl[ks].x, tl[ks].y, tl[ks].z, tl[ks].w};
+                mma_bf16_16816(acc, ah, ph[2 * ks], ph[2 * ks + 1]);
+                mma_bf16_16816(acc, al, ph[2 * ks], ph[2 * ks + 1]);
+                mma_bf16_16816(acc, ah, pl[2 * ks], pl[2 * ks + 1]);
             }
+            uint8_t* w = sW + (mt * 16 + g8) * W_HEAD + query * W_PITCH + (k8 + t2) * 2;
+            *reinterpret_cast<uint32_t*>(w) = pack_bf16(acc[0], acc[1]);
+            *reinterpret_cast<uint32_t*>(w + 8 * W_HEAD) = pack_bf16(acc[2], acc[3]);
         }
-        __syncthreads();                                       // the mixed rows are there; the pairs' rows may be written again
+        cp_async_wait<0>();
+        __syncthreads();                                       // the mixed rows and the next block's keys are there; the pairs' rows may be written again
         for (int idx = tid; idx < NH * NQ * (NK / 8); idx += MIX_THREADS) {
             const int row = idx / (NK / 8), c8 = idx % (NK / 8);
             *reinterpret_cast<uint4*>(dst + (size_t)b * (NH * NQ * NK) + row * NK + c8 * 8) =
@@ -371,39 +410,59 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
 }
 
 // ---- mixed weights x values -----------------------------------------------------------------------------------------------------------------
+// Bound by what a CTA fetches through L2: two neighbouring tiles share every block of values (their ranges of blocks differ by one at most at either end).
 #define V_STAGES 4
+#define VT 2                          // tiles of 16 queries a CTA
 #define A_PITCH (NK + 8)              // elements of a row of mixed weights in shared memory
-#define V_STAGE_BYTES (G * NQ * A_PITCH * 2 + NK * LDV * 2)
+#define A_TILE (G * NQ * A_PITCH)
+#define V_STAGE_BYTES (VT * A_TILE * 2 + NK * LDV * 2)
 #define VALUE_SMEM (V_STAGES * V_STAGE_BYTES)
+#define VALUE_THREADS (32 * G * VT)
 
-__global__ void __launch_bounds__(32 * G) value_kernel(
+__global__ void __launch_bounds__(VALUE_THREADS) value_kernel(
     const bf16* __restrict__ mixed, const bf16* __restrict__ v_cache, const bf16* __restrict__ v_pool, bf16* __restrict__ out,
     const int* __restrict__ block_table, int max_pages, const int* __restrict__ cu_tokens, const int* __restrict__ seq_lens, int first_req, int page_shift,
     int window, int pool, int pool_rows, int most_blocks) {
     PDL_ENTER();
     mixed = pdl_fresh(mixed); v_cache = pdl_fresh(v_cache); v_pool = pdl_fresh(v_pool);
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    const int r = first_req + blockIdx.z, kh = blockIdx.y, qt = gridDim.x - 1 - blockIdx.x;
+    const int r = first_req + blockIdx.z, kh = blockIdx.y, qt = (gridDim.x - 1 - blockIdx.x) * VT;
     const int tok0 = cu_tokens[r], n = cu_tokens[r + 1] - tok0;
     if (qt * NQ >= n) return;
-    const int here = min(NQ, n - qt * NQ), pos0 = seq_lens[r] - n + qt * NQ;
+    const int here = min(VT * NQ, n - qt * NQ), pos0 = seq_lens[r] - n + qt * NQ;
     const int* table = block_table + (size_t)r * max_pages;
-    const Blocks blocks(pos0, pos0 + here - 1, window, pool, NK);
+    const Blocks all(pos0, pos0 + here - 1, window, pool, NK);
+    const Blocks own[VT] = {Blocks(pos0, pos0 + min(here, NQ) - 1, window, pool, NK), Blocks(pos0 + min(here - 1, NQ), pos0 + here - 1, window, pool, NK)};
+    // block b of the CTA as a tile's own block (negative: the tile has no such block)
+    auto block_of = [&](int b, int tile) {
+        if (tile * NQ >= here) return -1;
+        const Blocks& o = own[tile];
+        if (all.is_pooled(b)) return b < o.pooled ? b : -1;
+        const int at = all.first + b - all.pooled - o.first;
+        return at >= 0 && at < o.count - o.pooled ? o.pooled + at : -1;
+    };
     const bf16* src = mixed + (size_t)(first_tile(cu_tokens, first_req, r) + qt) * most_blocks * (NH * NQ * NK) + (size_t)kh * G * NQ * NK;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const size_t per_tile = (size_t)most_blocks * (NH * NQ * NK);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tile = warp / G;
     auto fetch = [&](int b) {
-        if (b < blocks.count) {
+        if (b < all.count) {
             bf16* sA = reinterpret_cast<bf16*>(smem_raw + (b % V_STAGES) * V_STAGE_BYTES);
-            bf16* sV = sA + G * NQ * A_PITCH;
-            for (int idx = tid; idx < G * NQ * (NK / 8); idx += 32 * G) {
-                const int row = idx / (NK / 8), c8 = idx % (NK / 8) * 8;
-                cp_async16(sA + row * A_PITCH + c8, src + (size_t)b * (NH * NQ * NK) + row * NK + c8);
+            bf16* sV = sA + VT * A_TILE;
+            constexpr int PER_TILE = G * NQ * (NK / 8);
+#pragma unroll
+            for (int t = 0; t < VT; ++t) {
+                const int mine = block_of(b, t);
+                if (mine < 0) continue;
+                for (int idx = tid; idx < PER_TILE; idx += VALUE_THREADS) {
+                    const int row = idx / (NK / 8), c8 = idx % (NK / 8) * 8;
+                    cp_async16(sA + t * A_TILE + row * A_PITCH + c8, src + t * per_tile + (size_t)mine * (NH * NQ * NK) + row * NK + c8);
+                }
             }
-            const bool pooled = blocks.is_pooled(b);
-            const int key0 = blocks.key0(b, NK), last = pooled ? blocks.nb_most - 1 : pos0 + here - 1;
+            const bool pooled = all.is_pooled(b);
+            const int key0 = all.key0(b, NK), last = pooled ? all.nb_most - 1 : pos0 + here - 1;
             const bf16* from = pooled ? v_pool : v_cache;
             constexpr int PER = DV / 8;
-            for (int idx = tid; idx < NK * PER; idx += 32 * G) {
+            for (int idx = tid; idx < NK * PER; idx += VALUE_THREADS) {
                 const int row = idx / PER, c = idx % PER, key = key0 + row;
                 if (key <= last) cp_async16(sV + row * LDV + c * 8, from + row_at(table, key, pooled, kh, page_shift, pool, pool_rows) * DV + c * 8);
                 else *reinterpret_cast<uint4*>(sV + row * LDV + c * 8) = make_uint4(0, 0, 0, 0);
@@ -416,13 +475,14 @@ __global__ void __launch_bounds__(32 * G) value_kernel(
     float o[DV / 8][4];
 #pragma unroll
     for (int i = 0; i < DV / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
-    for (int b = 0; b < blocks.count; ++b) {
+    for (int b = 0; b < all.count; ++b) {
         cp_async_wait<V_STAGES - 2>();
         __syncthreads();                                       // block b is there, and everyone is done with the stage that is filled next
         fetch(b + V_STAGES - 1);
+        if (block_of(b, tile) < 0) continue;
         const bf16* sA = reinterpret_cast<const bf16*>(smem_raw + (b % V_STAGES) * V_STAGE_BYTES);
         const uint32_t a_addr = (uint32_t)__cvta_generic_to_shared(sA + (warp * NQ + (lane & 7) + ((lane >> 3) & 1) * 8) * A_PITCH + (lane >> 4) * 8);
-        const uint32_t v_addr = (uint32_t)__cvta_generic_to_shared(sA + G * NQ * A_PITCH + ((lane & 7) + ((lane >> 3) & 1) * 8) * LDV + (lane >> 4) * 8);
+        const uint32_t v_addr = (uint32_t)__cvta_generic_to_shared(sA + VT * A_TILE + ((lane & 7) + ((lane >> 3) & 1) * 8) * LDV + (lane >> 4) * 8);
 #pragma unroll
         for (int ks = 0; ks < NK / 16; ++ks) {
             uint32_t a[4];
@@ -439,9 +499,9 @@ __global__ void __launch_bounds__(32 * G) value_kernel(
     cp_async_wait<0>();
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
-        const int row = (lane >> 2) + 8 * rr;
+        const int row = tile * NQ + (lane >> 2) + 8 * rr;
         if (row >= here) continue;
-        bf16* to = out + ((size_t)(tok0 + qt * NQ + row) * NH + kh * G + warp) * DV + 2 * (lane & 3);
+        bf16* to = out + ((size_t)(tok0 + qt * NQ + row) * NH + kh * G + warp % G) * DV + 2 * (lane & 3);
 #pragma unroll
         for (int i = 0; i < DV / 8; ++i) *reinterpret_cast<uint32_t*>(to + i * 8) = pack_bf16(o[i][2 * rr], o[i][2 * rr + 1]);
     }
@@ -470,13 +530,13 @@ MB_API int mb_attn_pooled_mix(int which, const void* q, const void* k_cache, con
         return launch_kernel(stats_kernel, dim3((max_query_len + SQ - 1) / SQ, KH, count), 256, STATS_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache,
                              (const bf16*)k_pool, lse, block_table, max_pages, cu_tokens, seq_lens, first_req, shift, scale, cap, window, pool, pool_rows);
     }
-    dim3 tiles((max_query_len + NQ - 1) / NQ, which == 1 ? 1 : KH, count);
+    const int tiles_of = (max_query_len + NQ - 1) / NQ;
     if (which == 1) {
         cudaFuncSetAttribute(mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MIX_SMEM);
-        return launch_kernel(mix_kernel, tiles, MIX_THREADS, MIX_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache, (const bf16*)k_pool, (const float*)lse, talk,
+        return launch_kernel(mix_kernel, dim3(tiles_of, 1, count), MIX_THREADS, MIX_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache, (const bf16*)k_pool, (const float*)lse, talk,
                              (bf16*)mixed, block_table, max_pages, cu_tokens, seq_lens, first_req, shift, scale, cap, window, pool, pool_rows, most_blocks);
     }
     cudaFuncSetAttribute(value_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VALUE_SMEM);
-    return launch_kernel(value_kernel, tiles, 32 * G, VALUE_SMEM, s, 0, (const bf16*)mixed, (const bf16*)v_cache, (const bf16*)v_pool, (bf16*)out, block_table,
+    return launch_kernel(value_kernel, dim3((tiles_of + VT - 1) / VT, KH, count), VALUE_THREADS, VALUE_SMEM, s, 0, (const bf16*)mixed, (const bf16*)v_cache, (const bf16*)v_pool, (bf16*)out, block_table,
                          max_pages, cu_tokens, seq_lens, first_req, shift, window, pool, pool_rows, most_blocks);
 }

@@ -2027,7 +2027,7 @@ def attention_pooled(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table,
     if talk is not None and ctx.num_requests > ctx.num_decode:
         blocks = _pooled_mix_blocks(ctx, window, pool)
         if (use_pooled_mix and pooled_mix_supported(q.dtype, H, K, d, dv) and page_size & (page_size - 1) == 0 and blocks * 32 <= 2 * K * dv
-                and ctx.max_query_len >= POOLED_MIX_FROM and all(t is None or t.data_ptr() % 16 == 0 for t in (q, k_cache, v_cache, k_pool, v_pool, out))):
+                and ctx.max_query_len >= POOLED_MIX_FROM and scale > 0 and all(t is None or t.data_ptr() % 16 == 0 for t in (q, k_cache, v_cache, k_pool, v_pool, out))):
             _pooled_mix(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table, H, K, d, dv, scale, softcap or 0.0, window, pool, rows, talk, blocks)
             if ctx.num_decode == 0:
                 return

@@ -828,7 +828,7 @@ class PooledAttention(Mixer):
         pos = self.position
         ops.qkv_finish(rows, q, self.q_b, self.k_b, self.v_b, "head" if self.qk_norm else None, self.ones, self.ones, self.norm_eps,
                        ctx.positions, pos.inv_freq, pos.rotary_dim, pos.magnitude, cache.slot_mapping, cache.k, cache.v, None, None, None,
-                       self.heads, self.kv_heads, self.head_dim, self.v_head_dim, writes, pos.interleaved)
+                       self.heads, self.kv_heads, self.head_dim, self.v_head_dim, writes, pos.interleaved, ctx=ctx)
         if self.pool and writes:
             ops.stage_name = "pooled blocks"
             ops.pool_blocks(cache.k, cache.v, cache.k_pool, cache.v_pool, ctx, cache.block_table, cache.slot_mapping, self.pool)
