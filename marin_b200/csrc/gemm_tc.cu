@@ -603,6 +603,10 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
 // TMA and runs ahead into the next tile; warp 1 issues the MMAs into one of two accumulators in tensor memory;
 // warps 2..9 drain the other accumulator (tcgen05.ld, convert, store; two warps per 32-lane quarter) meanwhile, so the tensor cores do not wait
 // for the epilogue.
+// PAIR: two CTAs of a cluster work on 256 weight rows x BN tokens (cta_group::2): each loads its own 128 weight rows and half of the tokens, the
+// first one's MMA thread issues for both, each drains its own 128 rows.  A tile's tokens then lie in shared memory once for two SMs instead of twice: a third
+// less to fetch, write and read at 256 tokens, which is power, and power is the clock (2,048 tokens,
+// 24,576 weight rows of 4,096, back to back: 362 us alone, 349 in pairs; 19,456 of 2,560: 223 and 218; K in the same order, the same bits).
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -636,7 +640,7 @@ struct TcStreamK {
 struct TcWalk {
     int nkb, limit, step, at, token_tile, tiles_t;
     bool streamk;
-    __device__ TcWalk(const TcStreamK& sk, bool streamk_, int tiles_n, int tiles_t_, int nkb_) : nkb(nkb_), tiles_t(tiles_t_), streamk(streamk_) {
+    __device__ TcWalk(const TcStreamK& sk, bool streamk_, int tiles_n, int tiles_t_, int nkb_, int ctas) : nkb(nkb_), tiles_t(tiles_t_), streamk(streamk_) {
         if (streamk) {
             const int group = blockIdx.x / tiles_t_;
             token_tile = blockIdx.x - group * tiles_t_;
@@ -646,7 +650,7 @@ struct TcWalk {
             limit = (int)(to < total ? to : total);
             step = 0;
         } else {
-            at = blockIdx.x; limit = tiles_n * tiles_t_; step = gridDim.x; token_tile = 0;
+            at = blockIdx.x / ctas; limit = tiles_n * tiles_t_; step = gridDim.x / ctas; token_tile = 0;     // (ctas: CTAs a tile)
         }
     }
     // the next piece: k-blocks [kb0, kb1) of `tile` (numbered with the token tiles fastest)
@@ -679,7 +683,12 @@ MB_API int mb_gemm_tc_probe_read(long long* host) { return (int)cudaMemcpyFromSy
 #define PROBE_OUT(slot, name)
 #endif
 
-template <int BN, int STAGES, bool SK>
+template <int BN, bool PAIR>
+struct TcRing {
+    static constexpr int A_BYTES = TC_BM * TC_BK * 2, B_ROWS = PAIR ? BN / 2 : BN, STAGE_BYTES = A_BYTES + B_ROWS * TC_BK * 2;
+};
+
+template <int BN, int STAGES, bool SK, bool PAIR>
 __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                  const __grid_constant__ CUtensorMap map_x,
                                                                  void* __restrict__ out, int mode, int T, int N, int K,
@@ -692,7 +701,10 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
     // heads finished in the epilogue: per half of the columns (its four warps), two staging buffers of sixteen tokens
     __shared__ __align__(128) bf16 s_hx[2][2][16 * TC_BM];     // (also, as floats, the staging of a "+=" by TMA reduction: 8 KB per half)
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    using L = TcSmem<BN>;
+    using L = TcRing<BN, PAIR>;
+    static_assert(!SK || !PAIR, "stream-K deals k-blocks to single CTAs");
+    constexpr int CTAS = PAIR ? 2 : 1;
+    const int rank = PAIR ? (int)cluster_rank() : 0;
     uint64_t* full = (uint64_t*)(smem + STAGES * L::STAGE_BYTES);
     uint64_t* empty = full + STAGES;
     uint64_t* acc_full = empty + STAGES;       // [2]
@@ -700,22 +712,22 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
     uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles_n = (N + TC_BM - 1) / TC_BM, tiles_t = (T + BN - 1) / BN;
+    const int tiles_n = (N + CTAS * TC_BM - 1) / (CTAS * TC_BM), tiles_t = (T + BN - 1) / BN;
     const int nkb = (K + TC_BK - 1) / TC_BK;
     constexpr uint32_t TMEM_COLS = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8 * CTAS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
         __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        tmem_alloc<PAIR>(tmem_slot, TMEM_COLS);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    if (PAIR) cluster_sync();                  // (the other CTA's barriers are set up before anything is counted there)
+    else __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     PDL_ENTER_EARLY();
@@ -724,9 +736,9 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
         int it = 0;                                                   // k-blocks issued so far, over all tiles
         bool ok = true;
         PROBE_DECL(p_wait); PROBE_DECL(p_issue);
-        TcWalk walk(sk, SK, tiles_n, tiles_t, nkb);
+        TcWalk walk(sk, SK, tiles_n, tiles_t, nkb, CTAS);
         for (int tile, kb0, kb1; ok && walk.next(tile, kb0, kb1);) {
-            const int n0 = tile_rows(tile, tiles_n, tiles_t) * TC_BM, t0 = tile_tokens(tile, tiles_n, tiles_t) * BN;
+            const int n0 = (tile_rows(tile, tiles_n, tiles_t) * CTAS + rank) * TC_BM, t0 = tile_tokens(tile, tiles_n, tiles_t) * BN + rank * L::B_ROWS;
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
                 const int s = it % STAGES;
                 const uint32_t phase = (it / STAGES) & 1;
@@ -734,21 +746,28 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
                 if (!mbar_wait(&empty[s], phase ^ 1)) { atomicExch(error_flag, 11); ok = false; break; }
                 PROBE_ADD(p_wait, pt0);
                 const long long pt1 = PROBE_T();
-                mbar_expect_tx(&full[s], L::STAGE_BYTES);
                 uint8_t* a = smem + s * L::STAGE_BYTES;
-                tma_load_2d(a, &map_w, kb * TC_BK, n0, &full[s]);
-                tma_load_2d(a + L::A_BYTES, &map_x, kb * TC_BK, t0, &full[s]);
+                if (PAIR) {
+                    if (rank == 0) mbar_expect_tx(&full[s], 2 * L::STAGE_BYTES);
+                    const uint32_t bar = leader_addr(&full[s]);
+                    tma_load_2d_pair(a, &map_w, kb * TC_BK, n0, bar);
+                    tma_load_2d_pair(a + L::A_BYTES, &map_x, kb * TC_BK, t0, bar);
+                } else {
+                    mbar_expect_tx(&full[s], L::STAGE_BYTES);
+                    tma_load_2d(a, &map_w, kb * TC_BK, n0, &full[s]);
+                    tma_load_2d(a + L::A_BYTES, &map_x, kb * TC_BK, t0, &full[s]);
+                }
                 PROBE_ADD(p_issue, pt1);
             }
         }
         PROBE_OUT(0, p_wait); PROBE_OUT(1, p_issue);
-    } else if (warp == 1 && lane == 0) {
-        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+    } else if (warp == 1 && lane == 0 && rank == 0) {
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(CTAS * TC_BM >> 4) << 24);
         int it = 0, local = 0;
         bool ok = true;
         PROBE_DECL(m_full); PROBE_DECL(m_acc); PROBE_DECL(m_all);
         const long long mt_start = PROBE_T();
-        TcWalk walk(sk, SK, tiles_n, tiles_t, nkb);
+        TcWalk walk(sk, SK, tiles_n, tiles_t, nkb, CTAS);
         for (int tile, kb0, kb1; ok && walk.next(tile, kb0, kb1); ++local) {
             const int buf = local & 1;
             const uint32_t acc_phase = (local >> 1) & 1;
@@ -767,11 +786,15 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
                 const uint32_t a = smem_u32(smem + s * L::STAGE_BYTES);
                 const uint64_t adesc = umma_desc(a), bdesc = umma_desc(a + L::A_BYTES);
 #pragma unroll
-                for (int kk = 0; kk < TC_BK / 16; ++kk)
-                    umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
-                umma_commit(&empty[s]);
+                for (int kk = 0; kk < TC_BK / 16; ++kk) {
+                    if (PAIR) umma_bf16_pair(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
+                    else umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
+                }
+                if (PAIR) umma_commit_pair(&empty[s]);
+                else umma_commit(&empty[s]);
             }
-            umma_commit(&acc_full[buf]);
+            if (PAIR) umma_commit_pair(&acc_full[buf]);
+            else umma_commit(&acc_full[buf]);
         }
         PROBE_ADD(m_all, mt_start);
         PROBE_OUT(2, m_full); PROBE_OUT(3, m_acc); PROBE_OUT(4, m_all);
@@ -782,11 +805,11 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
         int local = 0;
         int heads_chunk = 0;                                          // chunks this warp has staged (TcHeadsOut): picks the buffer
         bool ok = true;
-        TcWalk walk(sk, SK, tiles_n, tiles_t, nkb);
+        TcWalk walk(sk, SK, tiles_n, tiles_t, nkb, CTAS);
         for (int tile, kb0, kb1; walk.next(tile, kb0, kb1); ++local) {
             const bool is_tail = SK && kb0 > 0;    // the tile's last k-blocks: parked for the CTA that has its first ones
             const bool is_head = SK && kb1 < nkb;  // the tile's first k-blocks: the next CTA's parked piece is added
-            const int tile_row = tile_rows(tile, tiles_n, tiles_t);
+            const int tile_row = tile_rows(tile, tiles_n, tiles_t) * CTAS + rank;
             const int n0 = tile_row * TC_BM, t0 = tile_tokens(tile, tiles_n, tiles_t) * BN;
             const int buf = local & 1;
             const uint32_t acc_phase = (local >> 1) & 1;
@@ -828,7 +851,8 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
                     kv_slot[r] = (there && !is_q) ? __ldg(heads.slot_mapping + t) : -1;
                 }
             };
-            if (!SK && heads.q_out != nullptr) heads_fetch(c_begin);
+            const bool beyond = PAIR && n0 >= N;       // (a pair's second 128 rows may lie past the last)
+            if (!SK && heads.q_out != nullptr && !beyond) heads_fetch(c_begin);
             // the four warps that share a half of the columns meet at barriers inside some epilogues' chunks (ids 2 and
             // 3): there they go on together or not at all
             auto half_agrees = [&](bool mine) {
@@ -1015,7 +1039,7 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
                 if (!ok) continue;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-                for (int c0 = c_begin; c0 < c_end; c0 += 16) {
+                for (int c0 = c_begin; c0 < c_end && !beyond; c0 += 16) {
                     float v[16];
                     tmem_ld16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c0), v);
                     if (SK && is_tail) {
@@ -1030,7 +1054,8 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
             if (is_tail) __threadfence();
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive(&acc_empty[buf]);
+                if (PAIR) mbar_arrive_leader(&acc_empty[buf]);
+                else mbar_arrive(&acc_empty[buf]);
                 if (is_tail) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(parked_flag), "r"(1) : "memory");
                 if (is_head) asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(parked_flag), "r"(0) : "memory");   // for the next launch
             }
@@ -1039,10 +1064,12 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
         if (reduce_out && quarter == 0 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    __syncwarp();
+    if (PAIR) cluster_sync();                  // nothing of the other CTA's is counted here any more, and its MMAs have left this one's memory
+    else __syncthreads();
     if (warp == 0) {
         __syncwarp();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+        tmem_free<PAIR>(tmem_base, TMEM_COLS);
     }
 }
 
@@ -1090,7 +1117,7 @@ static bool tc_reduce_out() {
     return state == 1;
 }
 
-template <int BN, int STAGES, bool SK>
+template <int BN, int STAGES, bool SK, bool PAIR = false>
 static int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, void* out, int mode, int T, int N, int K, int ctas,
                              int* error_flag, const TcNormOut& norm, const TcRowScale& scale, TcStreamK sk, cudaStream_t s,
                              const TcGlu& glu, const TcHeadsOut& heads = TcHeadsOut{}, const float* rope = nullptr) {
@@ -1107,16 +1134,17 @@ static int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, void*
                                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
             reduce_out = 1;
     }
-    constexpr int smem = STAGES * TcSmem<BN>::STAGE_BYTES + 1024 + 256;
-    static_assert(smem <= 227 * 1024, "the ring does not fit shared memory");
+    constexpr int smem = STAGES * TcRing<BN, PAIR>::STAGE_BYTES + 1024 + 256;
+    static_assert(smem + 16384 + 8 * BN <= 227 * 1024, "the ring does not fit shared memory");
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN, STAGES, SK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN, STAGES, SK, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    const int tiles_n = (N + TC_BM - 1) / TC_BM, tiles_t = (T + BN - 1) / BN, tiles = tiles_n * tiles_t;
-    int grid = tiles < ctas ? tiles : ctas;
+    constexpr int CTAS = PAIR ? 2 : 1;
+    const int tiles_n = (N + CTAS * TC_BM - 1) / (CTAS * TC_BM), tiles_t = (T + BN - 1) / BN, tiles = tiles_n * tiles_t;
+    int grid = CTAS * (tiles < ctas / CTAS ? tiles : ctas / CTAS);
     if (SK) {
         // every group the same number of k-blocks; at least a tile's worth each, so that a tile has two owners at most
         const int groups = ctas / tiles_t;
@@ -1124,7 +1152,7 @@ static int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, void*
         sk.units_per_group = (int)((units + groups - 1) / groups);
         grid = groups * tiles_t;
     }
-    return launch_kernel(gemm_tc_persistent_kernel<BN, STAGES, SK>, dim3(grid), dim3(320), smem, s, 0, mw, mx, out, mode, T, N, K,
+    return launch_kernel(gemm_tc_persistent_kernel<BN, STAGES, SK, PAIR>, dim3(grid), dim3(320), smem, s, PAIR ? -2 : 0, mw, mx, out, mode, T, N, K,
                          error_flag, norm, scale, sk, heads, rope, mo, reduce_out, glu);
 }
 
@@ -1136,10 +1164,12 @@ static int persistent_dispatch(const void* x, const void* w, void* out, int mode
     if (mode < 0 || mode >= TC_OUT_MODES || (tc_gated(mode) && N % 32 != 0) || !glu_fits(glu, mode, N)) return MB_ERR_BAD_DTYPE;
     if (norm.weight != nullptr && (mode != TC_OUT_F32_ACC || norm.scaled == nullptr || norm.sumsq == nullptr)) return MB_ERR_BAD_DTYPE;
     if (scale.sumsq != nullptr && (scale.slots <= 0 || scale.dim <= 0)) return MB_ERR_BAD_SIZE;
+    const bool pair = bn < 0;                           // CTAs in pairs, -bn tokens a tile: nothing coupled, no stream-K
+    if (pair && (norm.weight != nullptr || scale.sumsq != nullptr || sk.partials != nullptr || ctas < 2)) return MB_ERR_BAD_SIZE;
     CUtensorMap mw, mx;
     int rc = make_map(&mw, w, N, K, TC_BM);
     if (rc) return rc;
-    rc = make_map(&mx, x, T, K, bn);
+    rc = make_map(&mx, x, T, K, pair ? -bn / 2 : bn);
     if (rc) return rc;
     if (sk.partials != nullptr) {
         switch (bn) {                                   // stream-K: three widths
@@ -1149,7 +1179,18 @@ static int persistent_dispatch(const void* x, const void* w, void* out, int mode
             default: return MB_ERR_BAD_SIZE;
         }
     }
+#define PAIR_CASE(BN, STAGES) \
+    case -BN: return launch_persistent<BN, STAGES, false, true>(mw, mx, out, mode, T, N, K, ctas, error_flag, norm, scale, sk, s, glu, heads, rope)
     switch (bn) {
+        PAIR_CASE(128, 8);
+        PAIR_CASE(144, 8);
+        PAIR_CASE(160, 7);
+        PAIR_CASE(176, 7);
+        PAIR_CASE(192, 7);
+        PAIR_CASE(208, 7);
+        PAIR_CASE(224, 6);
+        PAIR_CASE(240, 6);
+        PAIR_CASE(256, 6);
         case 128: return launch_persistent<128, 6, false>(mw, mx, out, mode, T, N, K, ctas, error_flag, norm, scale, sk, s, glu, heads, rope);
         case 144: return launch_persistent<144, 6, false>(mw, mx, out, mode, T, N, K, ctas, error_flag, norm, scale, sk, s, glu, heads, rope);
         case 160: return launch_persistent<160, 5, false>(mw, mx, out, mode, T, N, K, ctas, error_flag, norm, scale, sk, s, glu, heads, rope);
@@ -1176,7 +1217,7 @@ static int sm_count_of_current_device() {
     return known[device];
 }
 
-// The persistent kernel: bn tokens per tile (a multiple of 16 from 128 to 256), `ctas` CTAs (one per SM).
+// The persistent kernel: bn tokens per tile (a multiple of 16 from 128 to 256; negative: -bn, by CTAs in pairs), `ctas` CTAs (one per SM).
 MB_API int mb_gemm_tc_persistent(const void* x, const void* w, void* out, int mode, int T, int N, int K, int bn, int ctas,
                                  int* error_flag, cudaStream_t s) {
     return persistent_dispatch(x, w, out, mode, T, N, K, bn, ctas, error_flag, TcNormOut{}, TcRowScale{}, TcStreamK{}, s);

@@ -332,6 +332,25 @@ def persistent_plan(T: int, N: int) -> int:
     return _tile_by_tile(T, N)[1]
 
 
+#: two SMs on one tile of 256 weight rows in the persistent kernel
+pair_tiles = True
+#: from this many multiply-adds on: what pairs save is a share of the time (a third less operand traffic, so less power and a higher clock), what they cost
+#: is about 2 us a launch (clusters to place, two SMs' ends to wait for).  Measured on B200 back to back, one and two SMs a tile of the same width: 2,048 tokens,
+#: 24,576 rows of 4,096 362 and 349 us; 6,144 of 2,560 63.7 and 62.0; 2,560 of 4,096 (2.1e10) 54.0 and 53.1; 2,560 of 2,560 (1.2e10) 35.8 and
+#: 35.3, but 2,560 of 1,024 16.7 and 17.5; 10,240 of 256 25.0 and 28.8; 1,900 tokens, 5,120 rows of 128 12.1 and 14.5.
+PAIRS_FROM = 1 << 34
+
+
+def paired_plan(T: int, N: int, K: int) -> int:
+    """``persistent_plan``'s width, negative where CTAs work in pairs on 256 weight rows of it: from ``PAIRS_FROM`` multiply-adds on, wherever that
+    takes no more rounds (each pair is two SMs; an odd last row tile leaves one idle)."""
+    bn = persistent_plan(T, N)
+    if not pair_tiles or T * N * K < PAIRS_FROM:
+        return bn
+    rows, across = -(-N // 128), -(-T // bn)
+    return -bn if -(-(-(-rows // 2) * across) // (SM_COUNT // 2)) <= -(-(rows * across) // SM_COUNT) else bn
+
+
 def _tile_by_tile(T: int, N: int):
     best = None
     for bn in PERSISTENT_TILES:
@@ -398,7 +417,7 @@ def _persistent_product(x, w, out, mode: int, T: int, N: int, K: int, s, what: s
             what + ", stream-K")
         return
     _check(lib.mb_gemm_tc_persistent(_ptr(x), _ptr(w), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K),
-                                     _c_int(persistent_plan(T, N)), _c_int(SM_COUNT), _ptr(s.error), _stream()), what)
+                                     _c_int(paired_plan(T, N, K)), _c_int(SM_COUNT), _ptr(s.error), _stream()), what)
 
 
 class NormOut:
@@ -586,7 +605,7 @@ def gemm_qkv_heads(x, w: torch.Tensor, q_out: torch.Tensor, q_weight, k_weight, 
         _cost(_size(w) + _size(rows) + T * N * 2 + (_size(table) if table is not None else 0), 2.0 * T * N * Kdim)
         s = _scratch_for(rows.device)
         _check(_lib("mb_gemm_tc").mb_gemm_tc_persistent_heads(
-            _ptr(rows), _ptr(w), _c_int(T), _c_int(N), _c_int(Kdim), _c_int(persistent_plan(T, N)), _c_int(SM_COUNT), _ptr(q_out),
+            _ptr(rows), _ptr(w), _c_int(T), _c_int(N), _c_int(Kdim), _c_int(paired_plan(T, N, Kdim)), _c_int(SM_COUNT), _ptr(q_out),
             _ptr(k_cache) if write_kv else None, _ptr(v_cache) if write_kv else None, _ptr(q_weight), _ptr(k_weight), _c_float(eps),
             _ptr(table), _ptr(slot_mapping) if write_kv else None, _c_int(H), _c_int(K), _c_int(page_size), _ptr(s.error), _stream()),
             "gemm (persistent) with heads finished in the epilogue")
@@ -854,7 +873,7 @@ def gemm_glu_rows(x: torch.Tensor, w: torch.Tensor, rows: Optional[torch.Tensor]
             parked, flags, floats = s.parked, s.parked_flags, s.parked.numel()
             what += ", stream-K"
         else:
-            bn = persistent_plan(T, N)
+            bn = paired_plan(T, N, K)
     else:
         bn, _ = gemm_plan(T, N, K)
     _check(_lib("mb_gemm_tc").mb_gemm_tc_glu(

@@ -114,6 +114,34 @@ def test_gemm_of_many_tokens_adds_into_float32(ops, T, N, K):
     ops.check_device_errors()
 
 
+@pytest.mark.parametrize("T,N,K", [(1025, 4990, 320), (1500, 1981, 72), (129, 19000, 64), (1171, 6144, 1000), (2000, 25 * 128, 512)])
+def test_products_by_pairs_of_sms_have_the_same_bits(ops, monkeypatch, T, N, K):
+    """Two SMs on a tile of 256 weight rows add up k in the same order as one on 128: the same bits for odd row tiles, ragged rows, few and ragged
+    k-blocks, in every epilogue (bfloat16, float32, added to float32, gated)."""
+    g = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randn(T, K, device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(N, K, device=DEV, generator=g) / math.sqrt(K)).to(torch.bfloat16)
+    base = torch.randn(T, N, device=DEV, generator=g)
+    gated = torch.cat([w, w])[:N // 32 * 32]
+    monkeypatch.setattr(ops, "stream_k", False)
+    monkeypatch.setattr(ops, "PAIRS_FROM", 0)
+    results = []
+    for pairs in (True, False):
+        monkeypatch.setattr(ops, "pair_tiles", pairs)
+        assert (ops.paired_plan(T, N, K) < 0) == pairs and (ops.paired_plan(T, len(gated), K) < 0) == pairs
+        outs = [torch.zeros(T, N, device=DEV, dtype=torch.bfloat16), torch.zeros(T, N, device=DEV), base.clone(),
+                torch.zeros(T, len(gated) // 2, device=DEV, dtype=torch.bfloat16)]
+        ops.gemm(x, w, outs[0])
+        ops.gemm(x, w, outs[1])
+        ops.gemm(x, w, outs[2], accumulate=True)
+        ops.gemm_swiglu(x, gated, outs[3])
+        ops.check_device_errors()
+        results.append(outs)
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    torch.testing.assert_close(results[0][1].double(), x.double() @ w.double().t(), rtol=1e-5, atol=2e-5)
+
+
 def test_gemm_rows_do_not_depend_on_the_batch(ops):
     """A row's result is the same alone and among 200 other rows (float32 path: bit for bit)."""
     g = torch.Generator(device=DEV).manual_seed(4)
