@@ -1,5 +1,5 @@
 // The gated delta rule over prompt portions, 64 tokens at a time on the tensor cores (mma.sync), compiled for one head layout:
-// -DQK_DIM (key channels, a multiple of 16 up to 128), -DV_SLICE (value channels a CTA takes: 16 or 32).
+// -DQK_DIM (key channels, a multiple of 16 up to 128), -DV_SLICE (value channels a CTA of the walk takes: 16, 32 or 64).
 //
 // The recurrence (delta_rule.cu) per head:  S <- g S,  u = beta (v - S^T k),  S <- S + k u^T,  o = S^T q.  With S0 the state before
 // a chunk of 64 tokens, G_i the sum of the log-decays of its tokens 0 .. i (per key channel), and the weighted products
@@ -7,29 +7,35 @@
 // unrolling it gives (Yang, Wang, Zhang, Shen, Kim, "Parallelizing Linear Transformers with the Delta Rule over Sequence Length")
 //     (I + diag(beta) A) U = diag(beta) (V - K+ S0),   K+_i = exp(G_i) k_i,
 //     O = Q+ S0 + P U,   Q+_i = exp(G_i) q_i,          S = exp(G_63) S0 + sum_j (exp(G_63 - G_j) k_j) u_j^T.
-// prepare_kernel (a CTA per chunk and head, all of them side by side) makes what does not need the state: P, and by forward
-// substitution W = (I + diag(beta) A)^-1 diag(beta) K+ and U0 = (I + diag(beta) A)^-1 diag(beta) V.  walk_kernel (a CTA per request, head
-// and slice of value channels) then walks the chunks in order: U = U0 - W S0, O, S.
+// prepare_kernel (a CTA per chunk and head, all of them side by side) makes what does not need the state: P, W = (I + diag(beta) A)^-1
+// diag(beta) K+ and U0 = (I + diag(beta) A)^-1 diag(beta) V, by forward substitution over blocks of 16 tokens.  walk_kernel (a CTA per request,
+// head and slice of value channels) walks the chunks in order and does only what the next chunk waits for: U = U0 - W S0 and S; it leaves U and
+// each chunk's S0.  read_kernel (a CTA per chunk and head, side by side again) makes O and, where it has a whole head, its norm, weight and gate.
 //
 // Exactness.  Every exponent that is taken is of a non-positive number: with one decay per channel a block of 16 rows is worked out
 // against a reference between it and the earlier rows (exp(G_i - R) exp(R - G_j), both at most 1), the lower half of a block's diagonal
-// square against one in its middle, and the 8 x 8 squares left on the diagonal pair by pair.  Decays, sums, unit vectors, A, the substitution and the state are float32; where a float32 number has to be an
-// operand of a product it is split into two bf16 numbers (value = hi + lo) and the three larger products are taken, so that about 16
-// bits of it enter.
+// square against one in its middle, and the 8 x 8 squares left on the diagonal pair by pair.  Decays, sums, unit vectors, A, the inverses of the diagonal blocks, what
+// the substitution adds up and the state are float32; where a float32 number has to be an operand of a product it is split into two bf16
+// numbers (value = hi + lo) and the three larger products are taken, so that about 16 bits of it enter (of a block's inverse only what lies
+// below its unit diagonal).
+// Measured on B200, two prompts of 712 and 1,188 tokens, 20 heads of 128 x 128, a decay per channel: prepare 101 us (141 with a column of the substitution a
+// thread), walk 65 (124 with the outputs made in it, 32 value channels a CTA and operands from shared memory on both sides), read 39 (with the norm, 12 us as a
+// kernel of its own).
 #define MB_LIB "delta_rule_chunked"
 #define MB_LIB_ID 21
 #include "common.cuh"
 #include "launch.cuh"
 #include "mma_helpers.cuh"
+#include "tc_common.cuh"
 
 #ifndef QK_DIM
 #define QK_DIM 128
 #endif
 #ifndef V_SLICE
-#define V_SLICE 32
+#define V_SLICE 64
 #endif
 static_assert(QK_DIM % 16 == 0 && QK_DIM >= 16 && QK_DIM <= 128, "key channels: a multiple of 16 up to 128");
-static_assert(V_SLICE == 16 || V_SLICE == 32, "a CTA takes 16 or 32 value channels");
+static_assert(V_SLICE == 16 || V_SLICE == 32 || V_SLICE == 64, "a CTA takes 16, 32 or 64 value channels");
 
 #define DQ QK_DIM
 #define VS V_SLICE
@@ -77,20 +83,32 @@ struct Sums3 {
     __device__ __forceinline__ float at(int n, int e) const { return hh[n][e] + (lh[n][e] + hl[n][e]); }
 };
 
-// What a chunk and head leaves for the walk, in bf16 planes of [64][DQ] (W, Q+, K exp(G_63 - G), each hi then lo), [64][64] (P hi, lo),
-// then float32 U0 [64][dv] and exp(G_63) [DQ].
-#define PLANE (CH * DQ)
-#define PPLANE (CH * CH)
-#define CHUNK_BF16 (6 * PLANE + 2 * PPLANE)
+// What a chunk and head hands over, every piece laid out as its reader holds it, so that one bulk copy (or a warp's 16-byte loads) brings it.  bf16
+// planes, hi then lo: W transposed [DQ][LDW], K exp(G_63 - G) and Q+ [64][LDQ], P [64][LDW], rows padded against bank conflicts; S0 as row operands of
+// (value channels x key channels): [dv / 16][DQ / 16][hi, lo][lane][8].  float32: U0 transposed [dv][64], its runs of eight tokens swapped by TURN0, 16 columns
+// of it replaced by the walk with U as row operands (value channels x tokens): [dv / 16][4][hi, lo][lane][8] bf16; exp(G_63) [DQ].
+#define LDQ (DQ + 8)
+#define LDW (CH + 8)
+#define WPLANE (DQ * LDW)
+#define KPLANE (CH * LDQ)
+#define PPLANE (CH * LDW)
+#define AT_K (2 * WPLANE)
+#define AT_Q (AT_K + 2 * KPLANE)
+#define AT_P (AT_Q + 2 * KPLANE)
+#define AT_S (AT_P + 2 * PPLANE)
+#define CHUNK_BF16(dv) (AT_S + 2 * DQ * (dv))
 #define CHUNK_F32(dv) (CH * (dv) + DQ)
+#define TURN0(column) (8 * ((column) & 3))
+#define KT (DQ / 16)                  // blocks of 16 key channels
 
 // Where request r's chunks start among all chunks of the step (room is left for a partial chunk per request).
 __device__ __forceinline__ int first_chunk(const int* cu_tokens, int first_req, int r) { return (cu_tokens[r] - cu_tokens[first_req]) / CH + (r - first_req); }
 
 #define LDR (DQ + 8)                  // raw q and k rows in shared memory (bf16) and sums (float32): eight rows of four lanes meet all banks
 #define LDG (DQ + 8)
-#define LDL (CH + 4)
-#define PREP_SMEM(CHANNEL, dv) (2 * CH * LDR * 2 + ((CHANNEL) ? CH * LDG : CH) * 4 + CH * LDL * 4 + 4 * CH * 4 + CH * ((dv) + 8) * 2 + 16)
+#define LDL (CH + 8)                  // the matrix of the substitution, bf16 planes
+#define LDD 20                        // its diagonal blocks, float32
+#define PREP_SMEM(CHANNEL, dv) (2 * CH * LDR * 2 + ((CHANNEL) ? CH * LDG : CH) * 4 + 2 * CH * LDL * 2 + 4 * 16 * LDD * 4 + 4 * CH * 4 + CH * ((dv) + 8) * 2 + 16)
 #define PREP_THREADS 256
 
 template <bool CHANNEL>
@@ -100,11 +118,12 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(
     bf16* __restrict__ planes, float* __restrict__ floats, int H, int G, int dv, int a_vec) {
     PDL_ENTER();
     qkv = pdl_fresh(qkv); b_rows = pdl_fresh(b_rows); a_rows = pdl_fresh(a_rows);
-    extern __shared__ __align__(16) uint8_t smem_raw[];
+    extern __shared__ __align__(128) uint8_t smem_raw[];
     bf16* sq = reinterpret_cast<bf16*>(smem_raw);              // [CH][LDR]
     bf16* sk = sq + CH * LDR;
-    float* sL = reinterpret_cast<float*>(sk + CH * LDR);       // [CH][LDL] beta_i A_ij
-    float* sG = sL + CH * LDL;                                 // [CH][LDG], or [CH] with one decay per head (log2 units)
+    bf16* sL = sk + CH * LDR;                                  // [2][CH][LDL] hi, lo: -beta_i A_ij of earlier blocks; in a diagonal block its inverse less 1
+    float* sD = reinterpret_cast<float*>(sL + 2 * CH * LDL);   // [4][16][LDD] beta_i A_ij of the diagonal blocks
+    float* sG = sD + 4 * 16 * LDD;                             // [CH][LDG], or [CH] with one decay per head (log2 units)
     float* s_beta = sG + (CHANNEL ? CH * LDG : CH);
     float* s_fq = s_beta + CH;
     float* s_fk = s_fq + CH;
@@ -116,7 +135,7 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(
     const int kh = head / (H / G), channels = 2 * G * DQ + H * dv;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t2 = 2 * (lane & 3);
     const size_t slot = (size_t)(first_chunk(cu_tokens, first_req, req) + blockIdx.x) * H + head;
-    bf16* out = planes + slot * CHUNK_BF16;
+    bf16* out = planes + slot * CHUNK_BF16(dv);
     float* fout = floats + slot * CHUNK_F32(dv);
     // ---- q, k and v as the convolution left them; rows past the request's tokens are zero
     bf16* sv = reinterpret_cast<bf16*>(s_qk + CH);             // [CH][dv + 8]
@@ -204,12 +223,12 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(
         }
     }
     // (the upper triangles stay zero; of P's only what lies in a diagonal block is ever read)
-    for (int idx = tid; idx < CH * LDL; idx += PREP_THREADS) sL[idx] = 0.0f;
-    bf16* ph = out + 6 * PLANE;
-    for (int idx = tid; idx < 4 * 16 * 8; idx += PREP_THREADS) {
-        const int row = (idx >> 3), at = row * CH + (row & ~15) + (idx & 7) * 2;
-        *reinterpret_cast<uint32_t*>(ph + at) = 0u;
-        *reinterpret_cast<uint32_t*>(ph + PPLANE + at) = 0u;
+    for (int idx = tid; idx < 4 * 16 * LDD; idx += PREP_THREADS) sD[idx] = 0.0f;
+    bf16* ph = out + AT_P;
+    for (int idx = tid; idx < 4 * 16 * 2; idx += PREP_THREADS) {
+        const int row = (idx >> 1), at = row * LDW + (row & ~15) + (idx & 1) * 8;
+        *reinterpret_cast<uint4*>(ph + at) = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4*>(ph + PPLANE + at) = make_uint4(0, 0, 0, 0);
     }
     __syncthreads();
     // ---- A and P: two warps make the rows 16 I .. 16 I + 15, each eight columns of every block of sixteen
@@ -308,12 +327,18 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(
                     const float w = CHANNEL ? 1.0f : j + e <= i ? ex2_approx(sG[i] - sG[j + e]) : 0.0f;
                     a[e] = s_beta[i] * s_fk[i] * s_fk[j + e] * accA[J][rr * 2 + e] * w;
                     b[e] = s_fq[i] * s_fk[j + e] * accP[J][rr * 2 + e] * w;
-                    if (j + e < i) sL[i * LDL + j + e] = a[e];
+                    if (J == 3 && j + e < i) sD[i * LDD + ((j + e) & 15)] = a[e];
                 }
                 uint32_t hi, lo;                               // (a weight of zero where j > i)
+                if (J < 3) {
+                    split_bf16(-a[0], -a[1], hi, lo);
+                    *reinterpret_cast<uint32_t*>(sL + i * LDL + j) = hi;
+                    *reinterpret_cast<uint32_t*>(sL + CH * LDL + i * LDL + j) = lo;
+                }
                 split_bf16(b[0], b[1], hi, lo);
-                *reinterpret_cast<uint32_t*>(ph + i * CH + j) = hi;
-                *reinterpret_cast<uint32_t*>(ph + PPLANE + i * CH + j) = lo;
+                const int at = i * LDW + j;
+                *reinterpret_cast<uint32_t*>(ph + at) = hi;
+                *reinterpret_cast<uint32_t*>(ph + PPLANE + at) = lo;
             }
         }
         if (CHANNEL && lane < 28) {                            // the 8 x 8 square on the diagonal that is this warp's, a pair of rows per lane
@@ -330,313 +355,416 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(
                 a = fmaf(ki.x, x, a); a = fmaf(ki.y, y, a);
                 b = fmaf(qi.x, x, b); b = fmaf(qi.y, y, b);
             }
-            sL[i * LDL + j] = s_beta[i] * s_fk[i] * s_fk[j] * a;
+            sD[i * LDD + (j & 15)] = s_beta[i] * s_fk[i] * s_fk[j] * a;
             b *= s_fq[i] * s_fk[j];
             const bf16 hi = __float2bfloat16_rn(b);
-            ph[i * CH + j] = hi;
-            ph[PPLANE + i * CH + j] = __float2bfloat16_rn(b - __bfloat162float(hi));
+            const int at = i * LDW + j;
+            ph[at] = hi;
+            ph[PPLANE + at] = __float2bfloat16_rn(b - __bfloat162float(hi));
         }
         if (CHANNEL && tid < CH) {                             // P_ii = q_i . k_i
             const float b = s_qk[tid] * s_fq[tid] * s_fk[tid];
             const bf16 hi = __float2bfloat16_rn(b);
-            ph[tid * CH + tid] = hi;
-            ph[PPLANE + tid * CH + tid] = __float2bfloat16_rn(b - __bfloat162float(hi));
+            const int at = tid * LDW + tid;
+            ph[at] = hi;
+            ph[PPLANE + at] = __float2bfloat16_rn(b - __bfloat162float(hi));
         }
     }
     __syncthreads();
-    // ---- Q+, K exp(G_63 - G), exp(G_63)
-    {
-        for (int idx = tid; idx < CH * DQ / 2; idx += PREP_THREADS) {
-            const int i = idx / (DQ / 2), c = (idx % (DQ / 2)) * 2;
-            const float g0 = CHANNEL ? sG[i * LDG + c] : sG[i], g1 = CHANNEL ? sG[i * LDG + c + 1] : g0;
-            const float e0 = CHANNEL ? sG[(CH - 1) * LDG + c] : sG[CH - 1], e1 = CHANNEL ? sG[(CH - 1) * LDG + c + 1] : e0;
-            const float2 k2 = bf2(*reinterpret_cast<const uint32_t*>(sk + i * LDR + c)), q2 = bf2(*reinterpret_cast<const uint32_t*>(sq + i * LDR + c));
-            uint32_t hi, lo;
-            split_bf16(q2.x * s_fq[i] * ex2_approx(g0), q2.y * s_fq[i] * ex2_approx(g1), hi, lo);
-            *reinterpret_cast<uint32_t*>(out + 2 * PLANE + i * DQ + c) = hi;
-            *reinterpret_cast<uint32_t*>(out + 3 * PLANE + i * DQ + c) = lo;
-            split_bf16(k2.x * s_fk[i] * ex2_approx(e0 - g0), k2.y * s_fk[i] * ex2_approx(e1 - g1), hi, lo);
-            *reinterpret_cast<uint32_t*>(out + 4 * PLANE + i * DQ + c) = hi;
-            *reinterpret_cast<uint32_t*>(out + 5 * PLANE + i * DQ + c) = lo;
-        }
-        for (int c = tid; c < DQ; c += PREP_THREADS) fout[CH * dv + c] = ex2_approx(CHANNEL ? sG[(CH - 1) * LDG + c] : sG[CH - 1]);
-    }
-    // ---- forward substitution, a column per thread: x_i = rhs_i - sum_(j < i) L_ij x_j
-    for (int col = tid; col < DQ + dv; col += PREP_THREADS) {
-        const bool is_w = col < DQ;
-        const bf16* v = sv + (col - DQ);
-        float x[CH];
+    // ---- two warps: the inverse of each diagonal block, a column a thread (x_i = [i = j] - sum_(k < i) L_ik x_k), less its unit diagonal
+    if (warp < 2) {
+        const int b = tid >> 4, j = tid & 15;
+        float x[16];
 #pragma unroll
-        for (int i = 0; i < CH; ++i) {
-            if (is_w) x[i] = s_beta[i] * s_fk[i] * __bfloat162float(sk[i * LDR + col]) * ex2_approx(CHANNEL ? sG[i * LDG + col] : sG[i]);
-            else x[i] = s_beta[i] * __bfloat162float(v[i * (dv + 8)]);
-        }
+        for (int i = 0; i < 16; ++i) x[i] = i == j ? 1.0f : 0.0f;
 #pragma unroll
-        for (int i = 1; i < CH; ++i) {
+        for (int i = 1; i < 16; ++i) {
             float acc0 = x[i], acc1 = 0.0f;
 #pragma unroll
-            for (int j = 0; j < i; j += 4) {
-                const float4 l = *reinterpret_cast<const float4*>(sL + i * LDL + j);        // (zero from the diagonal on)
-                acc0 = fmaf(-l.x, x[j], acc0);
-                if (j + 1 < i) acc1 = fmaf(-l.y, x[j + 1], acc1);
-                if (j + 2 < i) acc0 = fmaf(-l.z, x[j + 2], acc0);
-                if (j + 3 < i) acc1 = fmaf(-l.w, x[j + 3], acc1);
+            for (int k = 0; k < i; k += 4) {
+                const float4 l = *reinterpret_cast<const float4*>(sD + (b * 16 + i) * LDD + k);       // (zero from the diagonal on)
+                acc0 = fmaf(-l.x, x[k], acc0);
+                if (k + 1 < i) acc1 = fmaf(-l.y, x[k + 1], acc1);
+                if (k + 2 < i) acc0 = fmaf(-l.z, x[k + 2], acc0);
+                if (k + 3 < i) acc1 = fmaf(-l.w, x[k + 3], acc1);
             }
             x[i] = acc0 + acc1;
         }
-        if (is_w) {
 #pragma unroll
-            for (int i = 0; i < CH; ++i) {
-                const bf16 hi = __float2bfloat16_rn(x[i]);
-                out[i * DQ + col] = hi;
-                out[PLANE + i * DQ + col] = __float2bfloat16_rn(x[i] - __bfloat162float(hi));
+        for (int i = 0; i < 16; ++i) {
+            const float v = i > j ? x[i] : 0.0f;
+            const bf16 hi = __float2bfloat16_rn(v);
+            sL[(b * 16 + i) * LDL + b * 16 + j] = hi;
+            sL[CH * LDL + (b * 16 + i) * LDL + b * 16 + j] = __float2bfloat16_rn(v - __bfloat162float(hi));
+        }
+    } else {
+        // ---- the others: Q+, K exp(G_63 - G), exp(G_63)
+        for (int idx = tid - 64; idx < CH * DQ / 8; idx += PREP_THREADS - 64) {
+            const int i = idx / (DQ / 8), c = idx % (DQ / 8) * 8;
+            const uint4 kraw = *reinterpret_cast<const uint4*>(sk + i * LDR + c), qraw = *reinterpret_cast<const uint4*>(sq + i * LDR + c);
+            const uint32_t kw[4] = {kraw.x, kraw.y, kraw.z, kraw.w}, qw[4] = {qraw.x, qraw.y, qraw.z, qraw.w};
+            uint32_t kh_[4], kl_[4], qh_[4], ql_[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float2 k2 = bf2(kw[u]), q2 = bf2(qw[u]);
+                const float2 g2 = CHANNEL ? *reinterpret_cast<const float2*>(sG + i * LDG + c + 2 * u) : make_float2(sG[i], sG[i]);
+                const float2 e2 = CHANNEL ? *reinterpret_cast<const float2*>(sG + (CH - 1) * LDG + c + 2 * u) : make_float2(sG[CH - 1], sG[CH - 1]);
+                split_bf16(k2.x * s_fk[i] * ex2_approx(e2.x - g2.x), k2.y * s_fk[i] * ex2_approx(e2.y - g2.y), kh_[u], kl_[u]);
+                split_bf16(q2.x * s_fq[i] * ex2_approx(g2.x), q2.y * s_fq[i] * ex2_approx(g2.y), qh_[u], ql_[u]);
             }
-        } else {
+            bf16* at = out + AT_K + i * LDQ + c;
+            *reinterpret_cast<uint4*>(at) = make_uint4(kh_[0], kh_[1], kh_[2], kh_[3]);
+            *reinterpret_cast<uint4*>(at + KPLANE) = make_uint4(kl_[0], kl_[1], kl_[2], kl_[3]);
+            *reinterpret_cast<uint4*>(at + 2 * KPLANE) = make_uint4(qh_[0], qh_[1], qh_[2], qh_[3]);
+            *reinterpret_cast<uint4*>(at + 3 * KPLANE) = make_uint4(ql_[0], ql_[1], ql_[2], ql_[3]);
+        }
+        for (int c = tid - 64; c < DQ; c += PREP_THREADS - 64) fout[CH * dv + c] = ex2_approx(CHANNEL ? sG[(CH - 1) * LDG + c] : sG[CH - 1]);
+    }
+    __syncthreads();
+    // ---- forward substitution by blocks of 16 tokens, transposed (the rows of a product are 16 columns of W or U0, its columns tokens):
+    //     Z_I = rhs_I - sum_(J < I) L_IJ X_J,   X_I = Z_I + (L_II^-1 - 1) Z_I.
+    // A lane holds tokens 4 q .. 4 q + 3 of a block (columns t2, t2 + 1 of both products of eight), so that sums become row operands as they lie, an
+    // operand is one 8-byte load and a result 8 or 16 bytes of a column.  (A thread a column with all its 64 numbers in registers is bound
+    // by the loads of L, the same numbers for all threads: 16,000 of the SM's cycles a chunk.)
+    const int q4 = 4 * (lane & 3), brow = 4 * (g >> 1) + (g & 1);
+    for (int tile = warp; tile < (DQ + dv) / 16; tile += PREP_THREADS / 32) {
+        const bool is_w = tile * 16 < DQ;
+        const int col = is_w ? tile * 16 + g : tile * 16 - DQ + g;
+        uint32_t xh[3][4], xl[3][4];
 #pragma unroll
-            for (int i = 0; i < CH; ++i) fout[(size_t)i * dv + col - DQ] = x[i];
+        for (int I = 0; I < 4; ++I) {
+            float z[2][4];
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int i = I * 16 + q4 + 2 * nt + (e & 1), c = col + (e >> 1) * 8;
+                    if (is_w) z[nt][e] = s_beta[i] * s_fk[i] * __bfloat162float(sk[i * LDR + c]) * ex2_approx(CHANNEL ? sG[i * LDG + c] : sG[i]);
+                    else z[nt][e] = s_beta[i] * __bfloat162float(sv[i * (dv + 8) + c]);
+                }
+#pragma unroll
+            for (int J = 0; J < 4; ++J) {
+                if (J >= I) continue;
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+                    const bf16* row = sL + (I * 16 + brow + 2 * nt) * LDL + J * 16 + q4;
+                    const uint2 bh = *reinterpret_cast<const uint2*>(row), bl = *reinterpret_cast<const uint2*>(row + CH * LDL);
+                    mma3(z[nt], xh[J], xl[J], bh.x, bh.y, bl.x, bl.y);
+                }
+            }
+            uint32_t zh[4], zl[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) split_bf16(z[u >> 1][(u & 1) * 2], z[u >> 1][(u & 1) * 2 + 1], zh[u], zl[u]);
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+                const bf16* row = sL + (I * 16 + brow + 2 * nt) * LDL + I * 16 + q4;
+                const uint2 bh = *reinterpret_cast<const uint2*>(row), bl = *reinterpret_cast<const uint2*>(row + CH * LDL);
+                mma3(z[nt], zh, zl, bh.x, bh.y, bl.x, bl.y);
+            }
+            if (is_w || I < 3)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) split_bf16(z[u >> 1][(u & 1) * 2], z[u >> 1][(u & 1) * 2 + 1], zh[u], zl[u]);
+            if (I < 3)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) { xh[I < 3 ? I : 0][u] = zh[u]; xl[I < 3 ? I : 0][u] = zl[u]; }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {                      // column col + 8 h
+                const int c = col + 8 * h, i = I * 16 + q4;
+                if (is_w) {
+                    *reinterpret_cast<uint2*>(out + c * LDW + i) = make_uint2(zh[h], zh[2 + h]);
+                    *reinterpret_cast<uint2*>(out + WPLANE + c * LDW + i) = make_uint2(zl[h], zl[2 + h]);
+                } else {
+                    *reinterpret_cast<float4*>(fout + c * CH + (i ^ TURN0(c))) = make_float4(z[0][2 * h], z[0][2 * h + 1], z[1][2 * h], z[1][2 * h + 1]);
+                }
+            }
         }
     }
 }
 
 // ---- the walk -------------------------------------------------------------------------------------------------------------------------
-#define LDQ (DQ + 8)
-#define LDS (VS + 8)
-#define LDP (CH + 8)
-#define WC (VS / 16)                  // column groups of 16
-#define WARPS (4 * WC)
-#define WALK_THREADS (32 * WARPS)
-#define MT (DQ / 16)                  // 16-row tiles of the state, tiles warp, warp + WARPS, ... belong to a warp
-#define MT_W ((MT + WARPS - 1) / WARPS)
-#define NT (VS / 8)
-#define WALK_SMEM ((6 * CH * LDQ + 2 * CH * LDP + 2 * DQ * LDS + 2 * CH * LDS) * 2)
+#define VG (VS / 16)                  // groups of 16 value channels: a pair of warps each
+#define WALK_THREADS (64 * VG)
+#define HT ((KT + 1) / 2)             // blocks of key channels a warp of a pair has
+#define STAGE_BYTES (2 * WPLANE * 2 + 2 * KPLANE * 2 + VS * CH * 4)
+#define WALK_SMEM (2 * STAGE_BYTES + VG * 2 * 16 * CH * 4)
 
-__device__ __forceinline__ void copy_plane(bf16* dst, int ld, const bf16* src, int width) {     // [64][width] into rows of ld
-    const int per = width / 8;
-    for (int idx = threadIdx.x; idx < CH * per; idx += WALK_THREADS) {
-        const int row = idx / per, c = idx - row * per;
-        cp_async16(dst + row * ld + c * 8, src + row * width + c * 8);
-    }
+__device__ __forceinline__ void bulk_in(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
-__global__ void __launch_bounds__(WALK_THREADS) walk_kernel(const bf16* __restrict__ planes, const float* __restrict__ floats, float* __restrict__ state,
-                                                            const int* __restrict__ cu_tokens, const int* __restrict__ slots, float* __restrict__ o,
-                                                            int first_req, int H, int dv) {
+// Transposed: a pair of warps has 16 value channels, a warp of it half of the key channels of their state in registers, as the sums of
+// S^T += U^T (K exp(G_63 - G)) leave them, which is how the row operand of U^T = U0^T - S^T W^T wants them; U^T goes on to the next product likewise.  Only
+// the two halves of S^T W^T meet in shared memory.  Bound by mma.sync (8 cycles of a scheduler each: 1.6 us a chunk for 64 value and 128 key channels) and the
+// operands' way from shared memory, which two chunks' worth of bulk copies fill.  64 value channels a CTA: fewer fetch W and K through L2 too often.
+__global__ void __launch_bounds__(WALK_THREADS, 1) walk_kernel(bf16* planes, float* floats, float* __restrict__ state, const int* __restrict__ cu_tokens,
+                                                               const int* __restrict__ slots, int first_req, int H, int dv, int* error_flag) {
     PDL_ENTER_WALK();
-    planes = pdl_fresh(planes); floats = pdl_fresh(floats);
-    extern __shared__ __align__(16) uint8_t smem_raw[];
-    bf16* sW = reinterpret_cast<bf16*>(smem_raw);      // [2][CH][LDQ] hi, lo
-    bf16* sQ = sW + 2 * CH * LDQ;
-    bf16* sK = sQ + 2 * CH * LDQ;
-    bf16* sP = sK + 2 * CH * LDQ;                      // [2][CH][LDP]
-    bf16* sS = sP + 2 * CH * LDP;                      // [2][DQ][LDS]
-    bf16* sU = sS + 2 * DQ * LDS;                      // [2][CH][LDS]
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    __shared__ uint64_t w_there[2], k_there[2];
     const int req = first_req + blockIdx.x, head = blockIdx.y, vs0 = blockIdx.z * VS;
     const int first = cu_tokens[req], count = cu_tokens[req + 1] - first;
     if (count <= 0) return;
     const int chunks = (count + CH - 1) / CH;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = 2 * (lane & 3);
-    const int wr = warp & 3, wc = warp >> 2;           // this warp's 16 tokens and 16 columns in the products over tokens
+    const int vg = warp >> 1, half = warp & 1;
     const size_t slot0 = (size_t)first_chunk(cu_tokens, first_req, req) * H + head;
-    float* st = state + (((size_t)slots[req] * H + head) * DQ) * dv + vs0;
-    float S[MT_W][NT][4];
-#pragma unroll
-    for (int mi = 0; mi < MT_W; ++mi) {
-        const int m0 = (warp + WARPS * mi) * 16;
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            S[mi][nt][0] = S[mi][nt][1] = S[mi][nt][2] = S[mi][nt][3] = 0.0f;
-            if (m0 < DQ) {
-                const float2 a = *reinterpret_cast<const float2*>(st + (size_t)(m0 + g) * dv + nt * 8 + t2);
-                const float2 b = *reinterpret_cast<const float2*>(st + (size_t)(m0 + g + 8) * dv + nt * 8 + t2);
-                S[mi][nt][0] = a.x; S[mi][nt][1] = a.y; S[mi][nt][2] = b.x; S[mi][nt][3] = b.y;
-            }
-        }
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; ++i) { mbar_init(&w_there[i], 1); mbar_init(&k_there[i], 1); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    auto load_w = [&](int c) {
-        if (c < chunks) {
-            const bf16* p = planes + (slot0 + (size_t)c * H) * CHUNK_BF16;
-            copy_plane(sW, LDQ, p, DQ);
-            copy_plane(sW + CH * LDQ, LDQ, p + PLANE, DQ);
-        }
-        cp_async_commit();
-    };
-    auto load_qp = [&](int c) {
-        if (c < chunks) {
-            const bf16* p = planes + (slot0 + (size_t)c * H) * CHUNK_BF16;
-            copy_plane(sQ, LDQ, p + 2 * PLANE, DQ);
-            copy_plane(sQ + CH * LDQ, LDQ, p + 3 * PLANE, DQ);
-            copy_plane(sP, LDP, p + 6 * PLANE, CH);
-            copy_plane(sP + CH * LDP, LDP, p + 6 * PLANE + PPLANE, CH);
-        }
-        cp_async_commit();
-    };
-    auto load_k = [&](int c) {
-        const bf16* p = planes + (slot0 + (size_t)c * H) * CHUNK_BF16;
-        copy_plane(sK, LDQ, p + 4 * PLANE, DQ);
-        copy_plane(sK + CH * LDQ, LDQ, p + 5 * PLANE, DQ);
-        cp_async_commit();
-    };
-    load_w(0);
-    load_qp(0);
-    const size_t o_stride = (size_t)H * dv;
-    const int a_row = wr * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, a_col = (lane >> 4) * 8;          // ldmatrix addresses: row operands ...
-    const int b_row = (lane & 7) + ((lane >> 3) & 1) * 8, b_col = (lane >> 4) * 8;                    // ... and column operands read transposed
-    const uint32_t w_addr = (uint32_t)__cvta_generic_to_shared(sW + a_row * LDQ + a_col), q_addr = (uint32_t)__cvta_generic_to_shared(sQ + a_row * LDQ + a_col);
-    const uint32_t p_addr = (uint32_t)__cvta_generic_to_shared(sP + a_row * LDP + a_col);
-    const uint32_t s_addr = (uint32_t)__cvta_generic_to_shared(sS + b_row * LDS + b_col + wc * 16), u_addr = (uint32_t)__cvta_generic_to_shared(sU + b_row * LDS + b_col);
-    const uint32_t PL_Q = CH * LDQ * 2, PL_P = CH * LDP * 2, PL_S = DQ * LDS * 2, PL_U = CH * LDS * 2;     // bytes from a hi plane to its lo plane
-    const int i0 = wr * 16 + g, i1 = i0 + 8, col = wc * 16 + t2;
-    for (int c = 0; c < chunks; ++c) {
-        const int rows = min(CH, count - c * CH);
+    __syncthreads();
+    auto load = [&](int c) {                           // (one thread) W, U0 and K of a chunk
+        if (c >= chunks) return;
+        uint8_t* stage = smem_raw + (c & 1) * STAGE_BYTES;
+        const bf16* p = planes + (slot0 + (size_t)c * H) * CHUNK_BF16(dv);
         const float* f = floats + (slot0 + (size_t)c * H) * CHUNK_F32(dv);
-        float u[2][4], last[MT_W][2];
+        mbar_expect_tx(&w_there[c & 1], 2 * WPLANE * 2 + VS * CH * 4);
+        bulk_in(stage, p, 2 * WPLANE * 2, &w_there[c & 1]);
+        bulk_in(stage + 2 * WPLANE * 2 + 2 * KPLANE * 2, f + (size_t)vs0 * CH, VS * CH * 4, &w_there[c & 1]);
+        mbar_expect_tx(&k_there[c & 1], 2 * KPLANE * 2);
+        bulk_in(stage + 2 * WPLANE * 2, p + AT_K, 2 * KPLANE * 2, &k_there[c & 1]);
+    };
+    if (threadIdx.x == 0) { load(0); load(1); }
+    // S^T: value channels g and g + 8 of the group x key channels t2, t2 + 1 of every run of eight
+    float* st = state + (((size_t)slots[req] * H + head) * DQ) * dv + vs0 + vg * 16 + g;
+    float S[HT][2][4];
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            const float2 a = *reinterpret_cast<const float2*>(f + (size_t)i0 * dv + vs0 + col + nt * 8), b = *reinterpret_cast<const float2*>(f + (size_t)i1 * dv + vs0 + col + nt * 8);
-            u[nt][0] = a.x; u[nt][1] = a.y; u[nt][2] = b.x; u[nt][3] = b.y;
-        }
+    for (int i = 0; i < HT; ++i)
 #pragma unroll
-        for (int mi = 0; mi < MT_W; ++mi) {
-            const int m0 = (warp + WARPS * mi) * 16;
-            last[mi][0] = m0 < DQ ? f[CH * dv + m0 + g] : 0.0f;
-            last[mi][1] = m0 < DQ ? f[CH * dv + m0 + g + 8] : 0.0f;
-        }
-        // the state as two bf16 operands (the products of the chunk before have read the old ones)
+        for (int n = 0; n < 2; ++n)
 #pragma unroll
-        for (int mi = 0; mi < MT_W; ++mi) {
-            const int m0 = (warp + WARPS * mi) * 16;
-            if (m0 < DQ) {
+            for (int e = 0; e < 4; ++e) {
+                const int tile = half * HT + i;
+                S[i][n][e] = tile < KT ? st[(size_t)(tile * 16 + n * 8 + t2 + (e & 1)) * dv + (e >> 1) * 8] : 0.0f;
+            }
+    const int b_row = (lane & 7) + ((lane >> 3) & 1) * 8, b_col = (lane >> 4) * 8;           // column operands that lie by their k, read transposed
+    const uint32_t w_addr = smem_u32(smem_raw) + (b_row * LDW + b_col) * 2, k_addr = smem_u32(smem_raw) + 2 * WPLANE * 2 + (b_row * LDQ + b_col) * 2;
+    float4* mine = reinterpret_cast<float4*>(smem_raw + 2 * STAGE_BYTES) + warp * (16 * CH / 4) + lane;       // [8][32 lanes]
+    const float4* other = reinterpret_cast<const float4*>(smem_raw + 2 * STAGE_BYTES) + (warp ^ 1) * (16 * CH / 4) + lane;
+    bool ok = true;
+    for (int c = 0; c < chunks; ++c) {
+        bf16* p = planes + (slot0 + (size_t)c * H) * CHUNK_BF16(dv);
+        float* f = floats + (slot0 + (size_t)c * H) * CHUNK_F32(dv);
+        const uint32_t at = (c & 1) * STAGE_BYTES, parity = (c >> 1) & 1;
+        float2 last[HT][2];
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    uint32_t hi, lo;
-                    split_bf16(S[mi][nt][0], S[mi][nt][1], hi, lo);
-                    *reinterpret_cast<uint32_t*>(sS + (m0 + g) * LDS + nt * 8 + t2) = hi;
-                    *reinterpret_cast<uint32_t*>(sS + DQ * LDS + (m0 + g) * LDS + nt * 8 + t2) = lo;
-                    split_bf16(S[mi][nt][2], S[mi][nt][3], hi, lo);
-                    *reinterpret_cast<uint32_t*>(sS + (m0 + g + 8) * LDS + nt * 8 + t2) = hi;
-                    *reinterpret_cast<uint32_t*>(sS + DQ * LDS + (m0 + g + 8) * LDS + nt * 8 + t2) = lo;
+        for (int i = 0; i < HT; ++i)
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+                last[i][n] = half * HT + i < KT ? *reinterpret_cast<const float2*>(f + CH * dv + (half * HT + i) * 16 + n * 8 + t2) : make_float2(0.0f, 0.0f);
+        ok = ok && mbar_wait(&w_there[c & 1], parity);
+        // U^T = U0^T - S^T W^T (the pair's first warp begins with U0, the second with zeros)
+        float u[8][4];
+        {
+            const float* u0 = reinterpret_cast<const float*>(smem_raw + at + 2 * WPLANE * 2 + 2 * KPLANE * 2) + (vg * 16 + g) * CH;
+#pragma unroll
+            for (int n = 0; n < 8; ++n) {
+                u[n][0] = u[n][1] = u[n][2] = u[n][3] = 0.0f;
+                if (half == 0) {
+                    const float2 a = *reinterpret_cast<const float2*>(u0 + ((n * 8 + t2) ^ TURN0(g))), b = *reinterpret_cast<const float2*>(u0 + 8 * CH + ((n * 8 + t2) ^ TURN0(g)));
+                    u[n][0] = a.x; u[n][1] = a.y; u[n][2] = b.x; u[n][3] = b.y;
                 }
             }
         }
-        cp_async_wait<1>();                            // W of this chunk (Q and P may still be on their way)
-        __syncthreads();
-        load_k(c);                                     // everyone has left the chunk before
-        // U = U0 - W S
-        {
-            Sums3 acc;
-            acc.clear();
 #pragma unroll
-            for (int kk = 0; kk < DQ / 16; ++kk) {
-                uint32_t ah[4], al[4], bh[4], bl[4];
-                ldsm_x4(w_addr + kk * 32, ah[0], ah[1], ah[2], ah[3]);
-                ldsm_x4(w_addr + PL_Q + kk * 32, al[0], al[1], al[2], al[3]);
-                ldsm_x4_trans(s_addr + kk * 16 * LDS * 2, bh[0], bh[1], bh[2], bh[3]);
-                ldsm_x4_trans(s_addr + PL_S + kk * 16 * LDS * 2, bl[0], bl[1], bl[2], bl[3]);
-                acc.add(ah, al, bh, bl);
+        for (int i = 0; i < HT; ++i) {
+            const int tile = half * HT + i;
+            if (tile >= KT) continue;
+            uint32_t sh[4], sl[4], mh[4], ml[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                split_bf16(S[i][r >> 1][(r & 1) * 2], S[i][r >> 1][(r & 1) * 2 + 1], sh[r], sl[r]);
+                mh[r] = sh[r] ^ 0x80008000u; ml[r] = sl[r] ^ 0x80008000u;          // -S
             }
+            bf16* s0 = p + AT_S + (size_t)((((vs0 >> 4) + vg) * KT + tile) * 2) * 256 + lane * 8;
+            *reinterpret_cast<uint4*>(s0) = make_uint4(sh[0], sh[1], sh[2], sh[3]);
+            *reinterpret_cast<uint4*>(s0 + 256) = make_uint4(sl[0], sl[1], sl[2], sl[3]);
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                uint32_t hi, lo;
-                split_bf16(u[nt][0] - acc.at(nt, 0), u[nt][1] - acc.at(nt, 1), hi, lo);
-                *reinterpret_cast<uint32_t*>(sU + i0 * LDS + col + nt * 8) = hi;
-                *reinterpret_cast<uint32_t*>(sU + CH * LDS + i0 * LDS + col + nt * 8) = lo;
-                split_bf16(u[nt][2] - acc.at(nt, 2), u[nt][3] - acc.at(nt, 3), hi, lo);
-                *reinterpret_cast<uint32_t*>(sU + i1 * LDS + col + nt * 8) = hi;
-                *reinterpret_cast<uint32_t*>(sU + CH * LDS + i1 * LDS + col + nt * 8) = lo;
+            for (int n = 0; n < 4; ++n) {
+                uint32_t bh[4], bl[4];
+                ldsm_x4_trans(w_addr + at + (tile * 16 * LDW + n * 16) * 2, bh[0], bh[1], bh[2], bh[3]);
+                ldsm_x4_trans(w_addr + at + WPLANE * 2 + (tile * 16 * LDW + n * 16) * 2, bl[0], bl[1], bl[2], bl[3]);
+                mma3(u[2 * n], mh, ml, bh[0], bh[1], bl[0], bl[1]);
+                mma3(u[2 * n + 1], mh, ml, bh[2], bh[3], bl[2], bl[3]);
             }
         }
-        cp_async_wait<1>();                            // Q and P (K may still be on its way)
-        __syncthreads();
-        load_w(c + 1);                                 // everyone is done with W
-        // O = Q+ S + P U
-        {
-            Sums3 acc;
-            acc.clear();
 #pragma unroll
-            for (int kk = 0; kk < DQ / 16; ++kk) {
-                uint32_t ah[4], al[4], bh[4], bl[4];
-                ldsm_x4(q_addr + kk * 32, ah[0], ah[1], ah[2], ah[3]);
-                ldsm_x4(q_addr + PL_Q + kk * 32, al[0], al[1], al[2], al[3]);
-                ldsm_x4_trans(s_addr + kk * 16 * LDS * 2, bh[0], bh[1], bh[2], bh[3]);
-                ldsm_x4_trans(s_addr + PL_S + kk * 16 * LDS * 2, bl[0], bl[1], bl[2], bl[3]);
-                acc.add(ah, al, bh, bl);
+        for (int n = 0; n < 8; ++n) mine[n * 32] = make_float4(u[n][0], u[n][1], u[n][2], u[n][3]);
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + vg) : "memory");
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            const float4 v = other[n * 32];
+            u[n][0] += v.x; u[n][1] += v.y; u[n][2] += v.z; u[n][3] += v.w;
+        }
+#pragma unroll
+        for (int i = 0; i < HT; ++i)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) { S[i][n][0] *= last[i][n].x; S[i][n][1] *= last[i][n].y; S[i][n][2] *= last[i][n].x; S[i][n][3] *= last[i][n].y; }
+        ok = ok && mbar_wait(&k_there[c & 1], parity);
+        // S^T = S^T exp(G_63) + U^T (K exp(G_63 - G))
+#pragma unroll
+        for (int kk = 0; kk < CH / 16; ++kk) {
+            uint32_t uh[4], ul[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) split_bf16(u[2 * kk + (r >> 1)][(r & 1) * 2], u[2 * kk + (r >> 1)][(r & 1) * 2 + 1], uh[r], ul[r]);
+            if ((kk >> 1) == half) {                   // in U0's place, whose copy has arrived; either warp half of it
+                bf16* u0 = reinterpret_cast<bf16*>(f) + (size_t)((((vs0 >> 4) + vg) * 4 + kk) * 2) * 256 + lane * 8;
+                *reinterpret_cast<uint4*>(u0) = make_uint4(uh[0], uh[1], uh[2], uh[3]);
+                *reinterpret_cast<uint4*>(u0 + 256) = make_uint4(ul[0], ul[1], ul[2], ul[3]);
             }
 #pragma unroll
-            for (int kk = 0; kk < CH / 16; ++kk) {
-                if (kk > wr) continue;                 // later tokens have no weight
-                uint32_t ah[4], al[4], bh[4], bl[4];
-                ldsm_x4(p_addr + kk * 32, ah[0], ah[1], ah[2], ah[3]);
-                ldsm_x4(p_addr + PL_P + kk * 32, al[0], al[1], al[2], al[3]);
-                ldsm_x4_trans(u_addr + (kk * 16 * LDS + wc * 16) * 2, bh[0], bh[1], bh[2], bh[3]);
-                ldsm_x4_trans(u_addr + PL_U + (kk * 16 * LDS + wc * 16) * 2, bl[0], bl[1], bl[2], bl[3]);
-                acc.add(ah, al, bh, bl);
-            }
-            float* dst = o + (size_t)(first + c * CH) * o_stride + (size_t)head * dv + vs0 + col;
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                if (i0 < rows) *reinterpret_cast<float2*>(dst + (size_t)i0 * o_stride + nt * 8) = make_float2(acc.at(nt, 0), acc.at(nt, 1));
-                if (i1 < rows) *reinterpret_cast<float2*>(dst + (size_t)i1 * o_stride + nt * 8) = make_float2(acc.at(nt, 2), acc.at(nt, 3));
+            for (int i = 0; i < HT; ++i) {
+                const int tile = half * HT + i;
+                if (tile >= KT) continue;
+                uint32_t bh[4], bl[4];
+                ldsm_x4_trans(k_addr + at + (kk * 16 * LDQ + tile * 16) * 2, bh[0], bh[1], bh[2], bh[3]);
+                ldsm_x4_trans(k_addr + at + KPLANE * 2 + (kk * 16 * LDQ + tile * 16) * 2, bl[0], bl[1], bl[2], bl[3]);
+                mma3(S[i][0], uh, ul, bh[0], bh[1], bl[0], bl[1]);
+                mma3(S[i][1], uh, ul, bh[2], bh[3], bl[2], bl[3]);
             }
         }
-        cp_async_wait<1>();                            // K
-        __syncthreads();
-        load_qp(c + 1);                                // everyone is done with Q and P
-        // S = exp(G_63) S + (K exp(G_63 - G))^T U
-#pragma unroll
-        for (int mi = 0; mi < MT_W; ++mi) {
-            const int m0 = (warp + WARPS * mi) * 16;
-            if (m0 < DQ) {
-                // K^T as the row operand: tokens are its columns, read transposed from the [token][channel] tile
-                const uint32_t k_addr = (uint32_t)__cvta_generic_to_shared(sK + ((lane & 7) + (lane >> 4) * 8) * LDQ + m0 + ((lane >> 3) & 1) * 8);
-                Sums3 acc[NT / 2];
-#pragma unroll
-                for (int dt = 0; dt < NT / 2; ++dt) acc[dt].clear();
-#pragma unroll
-                for (int kk = 0; kk < CH / 16; ++kk) {
-                    uint32_t ah[4], al[4];
-                    ldsm_x4_trans(k_addr + kk * 16 * LDQ * 2, ah[0], ah[1], ah[2], ah[3]);
-                    ldsm_x4_trans(k_addr + PL_Q + kk * 16 * LDQ * 2, al[0], al[1], al[2], al[3]);
-#pragma unroll
-                    for (int dt = 0; dt < NT / 2; ++dt) {
-                        uint32_t bh[4], bl[4];
-                        ldsm_x4_trans(u_addr + (kk * 16 * LDS + dt * 16) * 2, bh[0], bh[1], bh[2], bh[3]);
-                        ldsm_x4_trans(u_addr + PL_U + (kk * 16 * LDS + dt * 16) * 2, bl[0], bl[1], bl[2], bl[3]);
-                        acc[dt].add(ah, al, bh, bl);
-                    }
-                }
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) S[mi][nt][e] = fmaf(S[mi][nt][e], last[mi][e >> 1], acc[nt >> 1].at(nt & 1, e));
-            }
-        }
+        __syncthreads();                               // everyone is done with this chunk's operands (and a pair with each other's halves)
+        if (threadIdx.x == 0) load(c + 2);
     }
-    cp_async_wait<0>();
+    if (!ok && lane == 0) atomicExch(error_flag, 41);
 #pragma unroll
-    for (int mi = 0; mi < MT_W; ++mi) {
-        const int m0 = (warp + WARPS * mi) * 16;
-        if (m0 < DQ) {
+    for (int i = 0; i < HT; ++i)
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-                *reinterpret_cast<float2*>(st + (size_t)(m0 + g) * dv + nt * 8 + t2) = make_float2(S[mi][nt][0], S[mi][nt][1]);
-                *reinterpret_cast<float2*>(st + (size_t)(m0 + g + 8) * dv + nt * 8 + t2) = make_float2(S[mi][nt][2], S[mi][nt][3]);
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int tile = half * HT + i;
+                if (tile < KT) st[(size_t)(tile * 16 + n * 8 + t2 + (e & 1)) * dv + (e >> 1) * 8] = S[i][n][e];
             }
+}
+
+// ---- the outputs ----------------------------------------------------------------------------------------------------------------------
+// O^T = S0^T Q+^T + U^T P^T: a CTA per chunk, head and up to 128 value channels, a warp per 16 of them, whose operands it loads as the walk left them; Q+ and
+// P come to shared memory by bulk copies, which then holds the sums by token.  Bound by what the kernels before left (230 KB a chunk and head of 128 x 128, 150
+// of them read here).  NORM: out = O / rms(O) * weight * gate * factor (a whole head a CTA), else the sums to o.
+#define READ_THREADS 256
+#define READ_COLS 128
+#define READ_OPERANDS (2 * KPLANE * 2 + 2 * PPLANE * 2)
+#define READ_SUMS(cols) (CH * ((cols) + 4) * 4)
+
+template <bool NORM>
+__global__ void __launch_bounds__(READ_THREADS, 2) read_kernel(const bf16* __restrict__ planes, const float* __restrict__ floats, const int* __restrict__ cu_tokens,
+                                                               float* __restrict__ o, int first_req, int H, int dv, int parts, const bf16* __restrict__ gate_rows,
+                                                               int gate_stride, int gate, const float* __restrict__ norm_w, float eps, float factor,
+                                                               bf16* __restrict__ out, int out_stride, int* error_flag) {
+    PDL_ENTER();
+    planes = pdl_fresh(planes); floats = pdl_fresh(floats); gate_rows = pdl_fresh(gate_rows);
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    __shared__ uint64_t there;
+    const int req = first_req + blockIdx.z / parts, head = blockIdx.y, c0 = blockIdx.z % parts * READ_COLS, cols = min(READ_COLS, dv - c0);
+    const int tok0 = cu_tokens[req] + blockIdx.x * CH;
+    const int rows = min(CH, cu_tokens[req + 1] - tok0);
+    if (rows <= 0) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = 2 * (lane & 3);
+    const size_t slot = (size_t)(first_chunk(cu_tokens, first_req, req) + blockIdx.x) * H + head;
+    const bf16* p = planes + slot * CHUNK_BF16(dv);
+    const bf16* f = reinterpret_cast<const bf16*>(floats + slot * CHUNK_F32(dv));
+    if (threadIdx.x == 0) {
+        mbar_init(&there, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_expect_tx(&there, READ_OPERANDS);
+        bulk_in(smem_raw, p + AT_Q, READ_OPERANDS, &there);           // Q+ and, behind it, P
+    }
+    const bool some = warp * 16 < cols;                // (all lanes of a warp)
+    const int vg = (c0 >> 4) + (some ? warp : 0);
+    uint4 ah[KT], al[KT];
+#pragma unroll
+    for (int kk = 0; kk < KT; ++kk) {
+        const bf16* at = p + AT_S + (size_t)((vg * KT + kk) * 2) * 256 + lane * 8;
+        ah[kk] = *reinterpret_cast<const uint4*>(at);
+        al[kk] = *reinterpret_cast<const uint4*>(at + 256);
+    }
+    float acc[8][4];
+#pragma unroll
+    for (int n = 0; n < 8; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+    const int b_row = (lane & 7) + (lane >> 4) * 8, b_col = ((lane >> 3) & 1) * 8;             // column operands that lie by their columns
+    const uint32_t q_addr = smem_u32(smem_raw) + (b_row * LDQ + b_col) * 2, p_addr = smem_u32(smem_raw) + 2 * KPLANE * 2 + (b_row * LDW + b_col) * 2;
+    auto add = [&](const uint4& h4, const uint4& l4, uint32_t addr, int ld, int plane, int from) {
+        const uint32_t xh[4] = {h4.x, h4.y, h4.z, h4.w}, xl[4] = {l4.x, l4.y, l4.z, l4.w};
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            if (n < from) continue;
+            uint32_t bh[4], bl[4];
+            ldsm_x4(addr + n * 16 * ld * 2, bh[0], bh[1], bh[2], bh[3]);
+            ldsm_x4(addr + plane * 2 + n * 16 * ld * 2, bl[0], bl[1], bl[2], bl[3]);
+            mma3(acc[2 * n], xh, xl, bh[0], bh[1], bl[0], bl[1]);
+            mma3(acc[2 * n + 1], xh, xl, bh[2], bh[3], bl[2], bl[3]);
         }
+    };
+    __syncthreads();                                   // the barrier is set up
+    const bool ok = mbar_wait(&there, 0);
+    if (some) {
+        uint4 uh[4], ul[4];
+#pragma unroll
+        for (int kk = 0; kk < KT; ++kk) {
+            if (kk == KT / 2) {                        // (asked for where half of S's registers are free again)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const bf16* at = f + (size_t)((vg * 4 + j) * 2) * 256 + lane * 8;
+                    uh[j] = *reinterpret_cast<const uint4*>(at);
+                    ul[j] = *reinterpret_cast<const uint4*>(at + 256);
+                }
+            }
+            add(ah[kk], al[kk], q_addr + kk * 32, LDQ, KPLANE, 0);
+        }
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) add(uh[kk], ul[kk], p_addr + kk * 32, LDW, PPLANE, kk);       // (no earlier token has a weight)
+    }
+    __syncthreads();                                   // everyone has left Q+ and P
+    float* sums = reinterpret_cast<float*>(smem_raw);  // [CH][cols + 4]
+    const int ld = cols + 4;
+    if (some) {
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sums[(n * 8 + t2 + (e & 1)) * ld + warp * 16 + g + (e >> 1) * 8] = acc[n][e];
+    }
+    if (!ok && lane == 0) atomicExch(error_flag, 42);
+    __syncthreads();
+    const bool here = lane * 4 < cols;                 // four columns of a token a lane
+    for (int i = warp; i < rows; i += READ_THREADS / 32) {
+        const float4 v = here ? *reinterpret_cast<const float4*>(sums + i * ld + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!NORM) {
+            if (here) *reinterpret_cast<float4*>(o + (size_t)(tok0 + i) * H * dv + (size_t)head * dv + c0 + lane * 4) = v;
+            continue;
+        }
+        uint2 raw = make_uint2(0u, 0u);
+        if (here) raw = *reinterpret_cast<const uint2*>(gate_rows + (size_t)(tok0 + i) * gate_stride + (size_t)head * dv + lane * 4);
+        const float scale = factor / sqrtf(warp_sum((v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w)) / (float)dv + eps);
+        if (!here) continue;
+        const float4 w = *reinterpret_cast<const float4*>(norm_w + lane * 4);
+        const float2 a = bf2(raw.x), b = bf2(raw.y);
+        float4 s4 = make_float4(__fdividef(1.0f, 1.0f + __expf(-a.x)), __fdividef(1.0f, 1.0f + __expf(-a.y)), __fdividef(1.0f, 1.0f + __expf(-b.x)),
+                                __fdividef(1.0f, 1.0f + __expf(-b.y)));
+        if (gate == 1) { s4.x *= a.x; s4.y *= a.y; s4.z *= b.x; s4.w *= b.y; }
+        *reinterpret_cast<uint2*>(out + (size_t)(tok0 + i) * out_stride + (size_t)head * dv + lane * 4) =
+            make_uint2(pack_bf16(v.x * scale * w.x * s4.x, v.y * scale * w.y * s4.y), pack_bf16(v.z * scale * w.z * s4.z, v.w * scale * w.w * s4.w));
     }
 }
 
-// How many bf16 and float32 numbers a chunk and head needs between the two kernels.
-MB_API int mb_delta_chunked_scratch(int dv, int* bf16s, int* floats) { *bf16s = CHUNK_BF16; *floats = CHUNK_F32(dv); return 0; }
+// How many bf16 and float32 numbers a chunk and head needs between the kernels.
+MB_API int mb_delta_chunked_scratch(int dv, int* bf16s, int* floats) { *bf16s = CHUNK_BF16(dv); *floats = CHUNK_F32(dv); return 0; }
 
-// Requests first_req .. requests - 1.  qkv: bf16 [tokens][2 G QK_DIM + H dv] after the convolution (rows 16-byte aligned); b, a, their
-// strides, per_channel, rate_log, dt_bias, state, o as mb_delta_scan takes them; dv a multiple of V_SLICE.  planes and floats hold
-// (tokens / 64 + requests) * H pieces of mb_delta_chunked_scratch each.
+// Requests first_req .. requests - 1; which: 0 prepares, 1 walks, 2 reads (in this order).  qkv: bf16 [tokens][2 G QK_DIM + H dv] after the convolution (rows
+// 16-byte aligned); b, a, their strides, per_channel, rate_log, dt_bias and state as mb_delta_scan takes them; dv a multiple of V_SLICE.  planes and
+// floats hold (tokens / 64 + requests) * H pieces of mb_delta_chunked_scratch each.  The sums go to o as mb_delta_scan leaves them or, where out is
+// given (dv up to 128), through norm and gate to out: gate_rows, gate, norm_w, eps and factor as mb_delta_norm takes them, all three at 8-byte addresses
+// (norm_w: 16).
 MB_API int mb_delta_chunked(const void* qkv, const void* b_rows, int b_stride, const void* a_rows, int a_stride, int per_channel, const float* rate_log,
-                            const float* dt_bias, float* state, const int* cu_tokens, const int* slots, float* o, void* planes, float* floats, int first_req,
-                            int requests, int max_query_len, int H, int G, int dv, int which, cudaStream_t s) {
+                            const float* dt_bias, float* state, const int* cu_tokens, const int* slots, float* o, void* planes, float* floats,
+                            const void* gate_rows, int gate_stride, int gate, const float* norm_w, float eps, float factor, void* out, int out_stride,
+                            int* error_flag, int first_req, int requests, int max_query_len, int H, int G, int dv, int which, cudaStream_t s) {
     if (requests <= first_req || max_query_len <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G != 0 || dv <= 0 || dv % VS != 0 || first_req < 0 || ((2 * G * DQ + H * dv) % 8) != 0) return MB_ERR_BAD_SIZE;
-    if ((((uintptr_t)qkv | (uintptr_t)planes) & 15) != 0 || ((uintptr_t)floats & 7) != 0) return MB_ERR_BAD_SIZE;
+    if ((((uintptr_t)qkv | (uintptr_t)planes | (uintptr_t)floats | (uintptr_t)o) & 15) != 0) return MB_ERR_BAD_SIZE;
+    if (out != nullptr && (dv > READ_COLS || gate_rows == nullptr || norm_w == nullptr || ((gate_stride | out_stride) & 3) != 0 ||
+                           (((uintptr_t)gate_rows | (uintptr_t)out) & 7) != 0 || ((uintptr_t)norm_w & 15) != 0))
+        return MB_ERR_BAD_SIZE;
     if (which == 0) {
         const int a_vec = a_stride % 8 == 0 && (((uintptr_t)a_rows | (uintptr_t)dt_bias) & 15) == 0;      // decays per channel by 16-byte loads
         dim3 grid((max_query_len + CH - 1) / CH, H, requests - first_req);
@@ -649,7 +777,20 @@ MB_API int mb_delta_chunked(const void* qkv, const void* b_rows, int b_stride, c
         return launch_kernel(prepare_kernel<false>, grid, PREP_THREADS, PREP_SMEM(0, dv), s, 0, (const bf16*)qkv, (const bf16*)b_rows, b_stride,
                              (const bf16*)a_rows, a_stride, rate_log, dt_bias, cu_tokens, first_req, (bf16*)planes, floats, H, G, dv, a_vec);
     }
-    cudaFuncSetAttribute(walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WALK_SMEM);
-    return launch_kernel(walk_kernel, dim3(requests - first_req, H, dv / VS), WALK_THREADS, WALK_SMEM, s, 0, (const bf16*)planes, (const float*)floats,
-                         state, cu_tokens, slots, o, first_req, H, dv);
+    if (which == 1) {
+        cudaFuncSetAttribute(walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WALK_SMEM);
+        return launch_kernel(walk_kernel, dim3(requests - first_req, H, dv / VS), WALK_THREADS, WALK_SMEM, s, 0, (bf16*)planes, floats, state, cu_tokens, slots,
+                             first_req, H, dv, error_flag);
+    }
+    const int parts = (dv + READ_COLS - 1) / READ_COLS, sums = READ_SUMS(dv < READ_COLS ? dv : READ_COLS);
+    const int smem = sums > READ_OPERANDS ? sums : READ_OPERANDS;
+    const dim3 grid((max_query_len + CH - 1) / CH, H, (requests - first_req) * parts);
+    if (out != nullptr) {
+        cudaFuncSetAttribute(read_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        return launch_kernel(read_kernel<true>, grid, READ_THREADS, smem, s, 0, (const bf16*)planes, (const float*)floats, cu_tokens, o, first_req, H, dv, parts,
+                             (const bf16*)gate_rows, gate_stride, gate, norm_w, eps, factor, (bf16*)out, out_stride, error_flag);
+    }
+    cudaFuncSetAttribute(read_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return launch_kernel(read_kernel<false>, grid, READ_THREADS, smem, s, 0, (const bf16*)planes, (const float*)floats, cu_tokens, o, first_req, H, dv, parts,
+                         (const bf16*)gate_rows, gate_stride, gate, norm_w, eps, factor, (bf16*)out, out_stride, error_flag);
 }

@@ -225,7 +225,7 @@ PER_LAYOUT_SAMPLES = {
     "mb_attention_sink_fast_d160_v128_g16_vk": (["attention_sink_fast.cu"], ["HEAD_DIM=160", "V_DIM=128", "GROUP=16", "V_IN_K"]),
     "mb_attention_sigmoid_fast_d128_v128_g4": (["attention_sigmoid_fast.cu"], ["HEAD_DIM=128", "V_DIM=128", "GROUP=4"]),
     "mb_linear_attention_chunked_d128_v32": (["linear_attention_chunked.cu"], ["QK_DIM=128", "V_SLICE=32"]),
-    "mb_delta_rule_chunked_d128_v32": (["delta_rule_chunked.cu"], ["QK_DIM=128", "V_SLICE=32"]),
+    "mb_delta_rule_chunked_d128_v64": (["delta_rule_chunked.cu"], ["QK_DIM=128", "V_SLICE=64"]),
     "mb_gated_linear_chunked_d128_v128": (["gated_linear_chunked.cu"], ["QK_DIM=128", "V_SLICE=128"]),
     "mb_wkv_chunked_d64": (["gated_linear_chunked.cu"], ["QK_DIM=64", "V_SLICE=64", "TIME_MIXING"]),
     "mb_attention_sink_fast_d128_v128_g8": (["attention_sink_fast.cu"], ["HEAD_DIM=128", "V_DIM=128", "GROUP=8"]),

@@ -2481,40 +2481,63 @@ def delta_chunked_supported(dtype, d: int, dv: int) -> bool:
 
 def _delta_slice(dv: int) -> int:
     """Value channels a CTA of the walk takes (its columns of the state are independent of the others)."""
-    return 32 if dv % 32 == 0 else 16
+    return 64 if dv % 64 == 0 else 32 if dv % 32 == 0 else 16
 
 
 def _delta_chunked_job(d: int, dv: int) -> tuple:
     return (["delta_rule_chunked.cu"], [f"QK_DIM={d}", f"V_SLICE={_delta_slice(dv)}"])
 
 
+def delta_chunked_finishes(gate: torch.Tensor, norm_w: torch.Tensor, out: torch.Tensor, dv: int) -> bool:
+    """Whether the chunked form's last kernel also does norm and gate: a whole head a CTA, rows at 8-byte addresses."""
+    return dv <= 128 and (gate.stride(0) | out.stride(0)) % 4 == 0 and (gate.data_ptr() | out.data_ptr()) % 8 == 0 and norm_w.data_ptr() % 16 == 0
+
+
+def _delta_plane_numbers(d: int, dv: int) -> int:
+    """bf16 numbers a chunk and head hands over: W, K, Q and P in padded rows, the state (csrc/delta_rule_chunked.cu, CHUNK_BF16)."""
+    return 2 * d * 72 + 4 * 64 * (d + 8) + 2 * 64 * 72 + 2 * d * dv
+
+
 def delta_chunk_bytes(d: int, dv: int) -> int:
-    """Scratch memory of a chunk of 64 tokens and a head between the two kernels of the chunked form."""
-    return (6 * 64 * d + 2 * 64 * 64) * 2 + (64 * dv + d) * 4
+    """Scratch memory of a chunk of 64 tokens and a head between the kernels of the chunked form."""
+    return _delta_plane_numbers(d, dv) * 2 + (64 * dv + d) * 4
 
 
-def delta_chunked(qkv: torch.Tensor, inp: DeltaInputs, state: torch.Tensor, ctx, slots: torch.Tensor, o: torch.Tensor, H: int, G: int, d: int, dv: int,
-                  first_req: int = 0, first_token: int = 0) -> None:
+def delta_chunked(qkv: torch.Tensor, inp: DeltaInputs, state: torch.Tensor, ctx, slots: torch.Tensor, o: Optional[torch.Tensor], H: int, G: int, d: int, dv: int,
+                  first_req: int = 0, first_token: int = 0, finish=None) -> None:
     """The same recurrence as ``delta_scan``, 64 tokens at a time on the tensor cores: what does not depend on the state for all chunks and
-    heads side by side, then the chunks of a request in order (the state and every float32 factor split into two bf16 numbers where they
-    are operands)."""
-    _need_cuda(qkv, state, o, slots)
+    heads side by side, then what the chunks of a request hand on in order, then the outputs side by side (the state and every float32 factor
+    split into two bf16 numbers where they are operands).  ``finish`` (where ``delta_chunked_finishes`` says so, in place of ``o``): gate, norm
+    weight, eps, factor and output rows of ``delta_norm``."""
+    _need_cuda(qkv, state, slots)
     T = qkv.shape[0]
     assert qkv.dtype == torch.bfloat16 and qkv.shape[1] == 2 * G * d + H * dv and tuple(state.shape[1:]) == (H, d, dv)
-    assert state.dtype == o.dtype == torch.float32 and tuple(o.shape) == (T, H * dv)
+    assert state.dtype == torch.float32
+    if finish is None:
+        _need_cuda(o)
+        assert o.dtype == torch.float32 and tuple(o.shape) == (T, H * dv)
+        ending = (None, _c_int(0), _c_int(0), None, _c_float(0.0), _c_float(0.0), None, _c_int(0))
+    else:
+        gate, norm_w, eps, factor, out = finish
+        assert o is None and norm_w.dtype == torch.float32 and norm_w.numel() == dv
+        ending = (_c_void_p(inp.gate.data_ptr()), _c_int(_columns(inp.gate, T, H * dv, torch.bfloat16)), _c_int(DELTA_GATES[gate]), _ptr(norm_w), _c_float(eps),
+                  _c_float(factor), _c_void_p(out.data_ptr()), _c_int(_columns(out, T, H * dv, torch.bfloat16)))
     R, rows = ctx.num_requests - first_req, T - first_token
     chunks = rows // 64 + R                               # at most: room for a partial chunk per request
-    planes = ctx.workspace.get("delta_planes", (chunks * H, 6 * 64 * d + 2 * 64 * 64), torch.bfloat16)
+    planes = ctx.workspace.get("delta_planes", (chunks * H, _delta_plane_numbers(d, dv)), torch.bfloat16)
     floats = ctx.workspace.get("delta_floats", (chunks * H, 64 * dv + d), torch.float32)
     lib = build.load(f"mb_delta_rule_chunked_d{d}_v{_delta_slice(dv)}", *_delta_chunked_job(d, dv))
     scratch = float(rows) / 64 * H * delta_chunk_bytes(d, dv)
-    for which, what in ((0, "delta rule (chunks prepared)"), (1, "delta rule (chunks walked)")):
+    handed = float(rows) * H * dv * (2 * d / 16 + 4)            # the states and U
+    for which, what in ((0, "delta rule (chunks prepared)"), (1, "delta rule (chunks walked)"), (2, "delta rule (chunks read)")):
         if which == 0:
-            _cost(rows * qkv.shape[1] * 2 + scratch, rows * H * 64.0 * (2 * d + d + dv))
+            _cost(rows * qkv.shape[1] * 2 + scratch - rows * H * dv * d / 16, rows * H * 64.0 * (2 * d + d + dv))
+        elif which == 1:
+            _cost(rows * H * (8 * d + 4 * dv) + handed + 2.0 * R * H * d * dv * 4, rows * H * dv * 4.0 * d)
         else:
-            _cost(scratch + rows * H * dv * 4 + 2.0 * R * H * d * dv * 4, rows * H * dv * (6.0 * d + 64.0))
+            _cost(rows * H * (4 * d + 4 * 64) + handed + rows * H * dv * 4, rows * H * dv * (2.0 * d + 64.0))
         _check(lib.mb_delta_chunked(_ptr(qkv), *_delta_args(inp, T, H, d, qkv.dtype), _ptr(state), _ptr(ctx.cu_tokens), _ptr(slots), _ptr(o),
-                                    _ptr(planes), _ptr(floats), _c_int(first_req), _c_int(ctx.num_requests), _c_int(ctx.max_query_len), _c_int(H),
+                                    _ptr(planes), _ptr(floats), *ending, _ptr(_scratch_for(qkv.device).error), _c_int(first_req), _c_int(ctx.num_requests), _c_int(ctx.max_query_len), _c_int(H),
                                     _c_int(G), _c_int(dv), _c_int(which), _stream()), what)
 
 

@@ -380,7 +380,7 @@ class DeltaRule(Mixer):
 
     def workspace_per_token(self, dtype) -> int:
         """Bytes a step keeps per token beside the products' rows: the convolution's output, the heads' sums and, in chunks of 64 tokens,
-        what the two chunked kernels hand over."""
+        what the chunked kernels hand over."""
         chunked = self.heads * ops.delta_chunk_bytes(self.dim, self.vdim) // 64 if ops.delta_chunked_supported(dtype, self.dim, self.vdim) else 0
         return self.channels * element_size(dtype) + 4 * self.hv + chunked
 
@@ -422,14 +422,17 @@ class DeltaRule(Mixer):
             conv = ws.get("delta_conv", (T, self.channels), x.dtype)
             ops.delta_conv(qkv, self.conv_w, ring.state, ctx, ring.slots, conv, single, single)
             ops.stage_name = "delta rule"
-            o = ws.get("delta_o", (T, self.hv), torch.float32)
-            if (ops.use_chunked_delta_rule and ops.delta_chunked_supported(x.dtype, d, dv) and self.channels % 8 == 0
-                    and ctx.max_query_len > ops.DELTA_CHUNKED_FROM):
-                ops.delta_chunked(conv, inputs, matrices.state, ctx, matrices.slots, o, H, G, d, dv, single, single)
+            chunked = (ops.use_chunked_delta_rule and ops.delta_chunked_supported(x.dtype, d, dv) and self.channels % 8 == 0
+                       and ctx.max_query_len > ops.DELTA_CHUNKED_FROM)
+            if chunked and ops.delta_chunked_finishes(inputs.gate, self.norm_w, out, dv):
+                ops.delta_chunked(conv, inputs, matrices.state, ctx, matrices.slots, None, H, G, d, dv, single, single,
+                                  finish=(self.gate, self.norm_w, self.norm_eps, self.out_scale, out))
             else:
-                ops.delta_scan(conv, inputs, matrices.state, ctx, matrices.slots, o, H, G, d, dv, single)
-            ops.stage_name = "norm, gate"
-            ops.delta_norm(o, inputs.gate, self.gate, self.norm_w, self.norm_eps, self.out_scale, out, H, dv, single)
+                o = ws.get("delta_o", (T, self.hv), torch.float32)
+                scan = (ops.delta_chunked, single) if chunked else (ops.delta_scan,)
+                scan[0](conv, inputs, matrices.state, ctx, matrices.slots, o, H, G, d, dv, single, *scan[1:])
+                ops.stage_name = "norm, gate"
+                ops.delta_norm(o, inputs.gate, self.gate, self.norm_w, self.norm_eps, self.out_scale, out, H, dv, single)
         if joined:
             return None
         ops.stage_name = "o"
