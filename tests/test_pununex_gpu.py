@@ -214,6 +214,50 @@ def recurrence(q, k, v, beta_raw, a_raw, rate, dt_bias, state, cuts, H, G, d, dv
     return torch.cat(outs)
 
 
+@pytest.mark.parametrize("per_channel", [False, True], ids=["head", "channel"])
+@pytest.mark.parametrize("d,dv", [(128, 128), (16, 64), (80, 192), (48, 16)])
+def test_chunks_of_every_slice_and_their_norm(d, dv, per_channel):
+    """Value slices of 64, 32 and 16, an odd number of key blocks, heads wider than an output block: chunks against the recurrence token by token (both 32-bit
+    but for operands of about 16 bits, 2e-4 of the largest sum), whole and partial chunks; then norm and gate in the last kernel against the
+    separate one, which differ by the order of a sum of squares: a bf16 step (2^-8) at most."""
+    from marin_b200.engine import StepEntry
+    from marin_b200.kernels import ops
+
+    H, G, T = 4, 2, 200
+    g = torch.Generator().manual_seed(d + dv)
+    q, k = (bf(torch.randn(T, G, d, generator=g)) for _ in range(2))
+    v = bf(torch.randn(T, H, dv, generator=g))
+    beta_raw, a_raw = bf(2.0 * torch.randn(T, H, generator=g)), bf(torch.randn(T, H * d if per_channel else H, generator=g))
+    rate, dt_bias = torch.randn(H, generator=g) * 0.3, torch.randn(H * d if per_channel else H, generator=g) * 0.5 - 2.0
+    states = [0.3 * torch.randn(4, H, d, dv, generator=torch.Generator().manual_seed(1)).to(DEV) for _ in range(3)]
+    want = recurrence(q, k, v, beta_raw, a_raw, rate, dt_bias, states[0], [T], H, G, d, dv, False)
+    for cuts in ([T], [129, 64, 7]):
+        states[1].copy_(states[2])
+        got = recurrence(q, k, v, beta_raw, a_raw, rate, dt_bias, states[1], cuts, H, G, d, dv, True)
+        assert (got - want).abs().max() <= 2e-4 * want.abs().max()
+        assert (states[1] - states[0]).abs().max() <= 2e-4 * states[0].abs().max()
+    if dv > 128:
+        return
+    rt = runtime("bfloat16")
+    runner = harness([], rt)
+    runner.begin("r")
+    ctx = runner.build_context([StepEntry("r", [0] * T, [])])
+    rows = torch.cat([q.reshape(T, -1), k.reshape(T, -1), v.reshape(T, -1)], dim=1).to(DEV).contiguous()
+    inp = ops.DeltaInputs(beta_raw.to(DEV), a_raw.to(DEV), bf(torch.randn(T, H * dv, generator=g)).to(DEV), rate.to(DEV), dt_bias.to(DEV))
+    norm_w, o = torch.randn(dv, generator=g).to(DEV), torch.zeros(T, H * dv, device=DEV)
+    outs = [torch.zeros(T, H * dv + 8, device=DEV, dtype=torch.bfloat16)[:, 4:4 + H * dv] for _ in range(2)]
+    for gate in ("sigmoid", "silu"):
+        states[1].copy_(states[2])
+        ops.delta_chunked(rows, inp, states[1], ctx, ctx.state_slots, o, H, G, d, dv)
+        ops.delta_norm(o, inp.gate, gate, norm_w, 1e-5, 1.5, outs[0], H, dv)
+        states[1].copy_(states[2])
+        assert ops.delta_chunked_finishes(inp.gate, norm_w, outs[1], dv)
+        ops.delta_chunked(rows, inp, states[1], ctx, ctx.state_slots, None, H, G, d, dv, finish=(gate, norm_w, 1e-5, 1.5, outs[1]))
+        ops.check_device_errors()
+        assert ((outs[1].float() - outs[0].float()).abs() <= 2.0 ** -8 * outs[0].float().abs() + 1e-30).all()
+    runner.end("r")
+
+
 @pytest.mark.parametrize("chunked", [False, True], ids=["scan", "chunked"])
 @pytest.mark.parametrize("per_channel", [False, True], ids=["head", "channel"])
 @pytest.mark.parametrize("strength", [0.002, 0.3, 4.0, 60.0])
