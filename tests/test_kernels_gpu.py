@@ -142,6 +142,21 @@ def test_products_by_pairs_of_sms_have_the_same_bits(ops, monkeypatch, T, N, K):
     torch.testing.assert_close(results[0][1].double(), x.double() @ w.double().t(), rtol=1e-5, atol=2e-5)
 
 
+@pytest.mark.parametrize("G,T,N,K", [(4, 129, 128, 64), (5, 300, 72, 192), (2, 1031, 200, 320), (7, 2048, 130, 128)])
+def test_products_side_by_side_have_each_products_results(ops, G, T, N, K):
+    """All tiles of several products in one launch, with ragged tokens and weight rows, against float64: the float32 sums rounded to bf16 once."""
+    g = torch.Generator(device=DEV).manual_seed(G * T)
+    x = torch.randn(G, T, K, device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(G, N, K, device=DEV, generator=g) / math.sqrt(K)).to(torch.bfloat16)
+    guard = torch.full((G * T + 2, N), 7.0, device=DEV, dtype=torch.bfloat16)
+    out = guard[1:G * T + 1].view(G, T, N)
+    ops.gemm_side_by_side(x, w, out)
+    ops.check_device_errors()
+    want = x.double() @ w.double().transpose(1, 2)
+    torch.testing.assert_close(out.double(), want, rtol=2.0 ** -8, atol=1e-4)
+    assert bool((guard[0] == 7.0).all()) and bool((guard[G * T + 1] == 7.0).all())
+
+
 def test_gemm_rows_do_not_depend_on_the_batch(ops):
     """A row's result is the same alone and among 200 other rows (float32 path: bit for bit)."""
     g = torch.Generator(device=DEV).manual_seed(4)

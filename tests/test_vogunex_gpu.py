@@ -219,6 +219,57 @@ def test_single_tokens_with_every_pair_of_value_heads_in_one_block(monkeypatch):
         close(feed([part], runner, x.to(rt.dtype), [30] + [1] * (T - 30))[0], want, "bfloat16", f"from {limit} CTAs on")
 
 
+@pytest.mark.parametrize("m", [
+    _attn(32, 8, 128, 128, 0.09, size=70, pool=8, rot={"base": 10000.0, "dims": 32}, softcap=30.0),
+    _attn(16, 8, 32, 32, 0.2, size=33, pool=3, softcap=2.0),             # weights at the cap: the exponential form of tanh
+    _attn(16, 4, 16, 48, 0.25),                                          # no window, no cap
+], ids=lambda m: f"h{m['heads']}k{m['kv_heads']}d{m['dim']}")
+def test_weights_mixed_ahead_of_the_values(monkeypatch, m):
+    """The kernels that mix the heads' weights before they meet the values, against the one that mixes the heads' sums (and both against the plain form): head
+    layouts, windows shorter than, at and beside a block of keys, portions of one, two and odd tiles of 16 queries behind cached positions, and a single
+    token of another request in the same step.  Both round every weight to bf16 once, so neither may be further off than the other by more than
+    rounding goes (a quarter)."""
+    from marin_b200.engine import StepEntry
+    from marin_b200.kernels import ops
+
+    rt, hidden, T = runtime("bfloat16"), 48, 150
+    w = attention_weights(hidden, m, 31)
+    x = bf(torch.randn(T, hidden, generator=torch.Generator().manual_seed(32)))
+    want = plain.pooled_window_attention(x.double(), {k: v.double() for k, v in w.items()}, "m.mix", m, 1e-5)
+    part = build_mixer("attention", m, hidden, 1e-5, rt, w)
+    taken = []
+    inner = ops._pooled_mix
+    monkeypatch.setattr(ops, "_pooled_mix", lambda *a: (taken.append(1), inner(*a))[1])
+    for cuts in ([T], [16, 33, 1, 17, 83], [1, 64, 31, 54]):
+        off = []
+        for mixed in (True, False):
+            monkeypatch.setattr(ops, "use_pooled_mix", mixed)
+            runner = harness([part.cache_need()], rt, page=16)
+            got = feed([part], runner, x, cuts)[0]
+            close(got, want, "bfloat16", f"mixed {mixed}, cuts {cuts}")
+            off.append(float((got.double() - want).pow(2).mean()) ** 0.5)
+        assert off[0] <= 1.25 * off[1], off
+    results = []
+    for mixed in (True, False):
+        monkeypatch.setattr(ops, "use_pooled_mix", mixed)
+        runner = harness([part.cache_need()], rt, page=16)
+        for req, n in (("a", 20), ("b", 9)):
+            runner.begin(req)
+            runner.cache.reserve(req, n)
+            ctx = runner.build_context([StepEntry(req, [0] * n, [])])
+            part.forward(x[:n].to(DEV).contiguous(), ctx, runner.views.view(0, ctx), torch.zeros(n, hidden, device=DEV))
+            runner.cache.commit(req, n)
+        runner.cache.reserve("a", 21), runner.cache.reserve("b", 79)
+        ctx = runner.build_context([StepEntry("a", [0], []), StepEntry("b", [0] * 70, [])])
+        residual = torch.zeros(71, hidden, device=DEV)
+        part.forward(torch.cat([x[20:21], x[9:79]]).to(DEV).contiguous(), ctx, runner.views.view(0, ctx), residual)
+        results.append(residual.cpu())
+    for got in results:
+        close(got, torch.cat([want[20:21], want[9:79]]), "bfloat16", "a single token beside a portion")
+    assert len(taken) >= 8
+    ops.check_device_errors()
+
+
 def test_pooled_rows_live_in_the_pages_and_are_given_back_with_them():
     """Pages, their pooled rows and state slots are handed to the next request: a second request in the places of a first one
     gets what it gets alone in a fresh cache."""
