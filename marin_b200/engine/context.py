@@ -8,13 +8,20 @@ import torch
 
 
 class Workspace:
-    """Activation buffers by name, kept between steps so that a step allocates nothing once warm."""
+    """Activation buffers by name, kept between steps so that a step allocates nothing once warm.  The views handed out are kept too (a step of few
+    tokens is bound by the host, and making a view takes 2 us): at most ``VIEWS`` of them, those of a buffer only as long as it is the one in use."""
+
+    VIEWS = 512
 
     def __init__(self, device):
         self.device = device
         self._buffers: Dict[Tuple[str, torch.dtype], torch.Tensor] = {}
+        self._views: Dict[Tuple[str, Tuple[int, ...], torch.dtype], torch.Tensor] = {}
 
     def get(self, name: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
+        view = self._views.get((name, shape, dtype))
+        if view is not None:
+            return view
         count = 1
         for s in shape:
             count *= int(s)
@@ -23,7 +30,11 @@ class Workspace:
         if buf is None or buf.numel() < count:
             buf = torch.empty(max(count, 1), device=self.device, dtype=dtype)
             self._buffers[key] = buf
-        return buf[:count].view(*shape)
+            self._views = {k: v for k, v in self._views.items() if (k[0], k[2]) != key}
+        if len(self._views) >= self.VIEWS:
+            self._views = {}
+        view = self._views[(name, shape, dtype)] = buf[:count].view(*shape)
+        return view
 
 
 @dataclass

@@ -42,12 +42,14 @@ def _ptr(t: Optional[torch.Tensor]):
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+#: (a launch's tensors are on a GPU, so torch has initialised CUDA; torch.cuda.current_device asks that every time, 0.6 us)
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def _stream():
     """The current stream's handle (asked of torch on every launch: streams change under graph capture)."""
     if _raw_stream is not None:
-        return _c_void_p(_raw_stream(torch.cuda.current_device()))
+        return _c_void_p(_raw_stream(_current_device()))
     return _c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
@@ -88,7 +90,7 @@ def _cost(nbytes: float = 0, flops: float = 0.0, bytes_per_key: float = 0, flops
 
 
 def _size(t) -> int:
-    return t.numel() * t.element_size()
+    return t.nbytes
 
 
 def _check(rc: int, what: str) -> None:
@@ -106,8 +108,14 @@ def _check(rc: int, what: str) -> None:
     raise KernelError(f"{what}: CUDA error {rc} ({torch.cuda.cudart().cudaGetErrorString(rc) if hasattr(torch.cuda.cudart(), 'cudaGetErrorString') else ''})")
 
 
+_libraries: dict = {}
+
+
 def _lib(name: str):
-    return build.load(name, build.LIBRARIES[name])
+    lib = _libraries.get(name)
+    if lib is None:
+        lib = _libraries[name] = build.load(name, build.LIBRARIES[name])
+    return lib
 
 
 def embed(ids: torch.Tensor, table: torch.Tensor, out: torch.Tensor, pos_table: Optional[torch.Tensor] = None,
@@ -326,6 +334,7 @@ PERSISTENT_TILES = (128, 144, 160, 176, 192, 208, 224, 240, 256)
 STREAM_K_TILES = (128, 192, 256)
 
 
+@functools.lru_cache(maxsize=4096)
 def persistent_plan(T: int, N: int) -> int:
     """Tokens per tile for the persistent kernel: the tile width whose rounds over the SMs waste the least.
     A tile's time grows with its width plus a fixed part (ramp-up of the ring, the epilogue's tail)."""
@@ -389,22 +398,25 @@ def stream_k_plan(T: int, N: int, K: int) -> Optional[int]:
     """Tokens per tile if the product should run stream-K, else None.  The CTAs form groups, one CTA per token tile,
     and every group gets the same number of k-blocks of the weight-row tiles laid end to end: the time goes with
     row tiles / groups, without rounding up to whole rounds of tiles.  It needs at least one row tile per group."""
-    if not stream_k:
-        return None
+    return _stream_k_width(T, N, K, _KBLOCK_FIXED, _STREAM_K_FIXED, _STREAM_K_MARGIN, _STREAM_K_MAX_X_BYTES) if stream_k else None
+
+
+@functools.lru_cache(maxsize=4096)
+def _stream_k_width(T: int, N: int, K: int, kblock: int, fixed: float, margin: float, most: int) -> Optional[int]:
     best = None
     rows, nkb = -(-N // 128), -(-K // 64)
     for bn in STREAM_K_TILES:
         across = -(-T // bn)
-        if across > SM_COUNT or rows < SM_COUNT // across or (_STREAM_K_FIXED > 0 and (across < 4 or T * K * 2 > _STREAM_K_MAX_X_BYTES)):
+        if across > SM_COUNT or rows < SM_COUNT // across or (fixed > 0 and (across < 4 or T * K * 2 > most)):
             continue
-        cost = rows / (SM_COUNT // across) * nkb * (bn + _KBLOCK_FIXED) + _STREAM_K_FIXED
+        cost = rows / (SM_COUNT // across) * nkb * (bn + kblock) + fixed
         if best is None or cost <= best[0]:
             best = (cost, bn)
     if best is None:
         return None
     bn = persistent_plan(T, N)
-    whole = -(-(rows * -(-T // bn)) // SM_COUNT) * nkb * (bn + _KBLOCK_FIXED)
-    return best[1] if best[0] < _STREAM_K_MARGIN * whole else None
+    whole = -(-(rows * -(-T // bn)) // SM_COUNT) * nkb * (bn + kblock)
+    return best[1] if best[0] < margin * whole else None
 
 
 def _persistent_product(x, w, out, mode: int, T: int, N: int, K: int, s, what: str) -> None:
@@ -1935,8 +1947,8 @@ def moe_experts(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, 
     assert tuple(w_gate_up.shape) == (E, (2 if gated else 1) * ff, h) and w_gate_up.dtype == w_down.dtype == x.dtype and tuple(y.shape) == (T, h)
     assert y.dtype == torch.float32 and experts.dtype == torch.int32 and weights.dtype == torch.float32
     ends = E + identity + 1
-    ints = workspace.get("moe_ints", (ends + 3 * pairs,), torch.int32)
-    offsets, order, inv, token_sorted = ints[:ends], ints[ends:ends + pairs], ints[ends + pairs:ends + 2 * pairs], ints[ends + 2 * pairs:]
+    offsets = workspace.get("moe_offsets", (ends,), torch.int32)
+    order, inv, token_sorted = (workspace.get(name, (pairs,), torch.int32) for name in ("moe_order", "moe_inv", "moe_token_sorted"))
     if identity and weight_on_input:
         raise KernelError("experts: identity choices go with weights on the output")
     weight_sorted = workspace.get("moe_weight_sorted", (pairs,), torch.float32)
