@@ -1182,14 +1182,10 @@ static int persistent_dispatch(const void* x, const void* w, void* out, int mode
 #define PAIR_CASE(BN, STAGES) \
     case -BN: return launch_persistent<BN, STAGES, false, true>(mw, mx, out, mode, T, N, K, ctas, error_flag, norm, scale, sk, s, glu, heads, rope)
     switch (bn) {
-        PAIR_CASE(128, 8);
-        PAIR_CASE(144, 8);
+        PAIR_CASE(128, 8);                               // (an MMA over two SMs takes tokens in steps of 32)
         PAIR_CASE(160, 7);
-        PAIR_CASE(176, 7);
         PAIR_CASE(192, 7);
-        PAIR_CASE(208, 7);
         PAIR_CASE(224, 6);
-        PAIR_CASE(240, 6);
         PAIR_CASE(256, 6);
         case 128: return launch_persistent<128, 6, false>(mw, mx, out, mode, T, N, K, ctas, error_flag, norm, scale, sk, s, glu, heads, rope);
         case 144: return launch_persistent<144, 6, false>(mw, mx, out, mode, T, N, K, ctas, error_flag, norm, scale, sk, s, glu, heads, rope);
@@ -1217,7 +1213,7 @@ static int sm_count_of_current_device() {
     return known[device];
 }
 
-// The persistent kernel: bn tokens per tile (a multiple of 16 from 128 to 256; negative: -bn, by CTAs in pairs), `ctas` CTAs (one per SM).
+// The persistent kernel: bn tokens per tile (a multiple of 16 from 128 to 256; negative: -bn, a multiple of 32, by CTAs in pairs), `ctas` CTAs (one per SM).
 MB_API int mb_gemm_tc_persistent(const void* x, const void* w, void* out, int mode, int T, int N, int K, int bn, int ctas,
                                  int* error_flag, cudaStream_t s) {
     return persistent_dispatch(x, w, out, mode, T, N, K, bn, ctas, error_flag, TcNormOut{}, TcRowScale{}, TcStreamK{}, s);

@@ -351,13 +351,19 @@ PAIRS_FROM = 1 << 34
 
 
 def paired_plan(T: int, N: int, K: int) -> int:
-    """``persistent_plan``'s width, negative where CTAs work in pairs on 256 weight rows of it: from ``PAIRS_FROM`` multiply-adds on, wherever that
-    takes no more rounds (each pair is two SMs; an odd last row tile leaves one idle)."""
-    bn = persistent_plan(T, N)
-    if not pair_tiles or T * N * K < PAIRS_FROM:
-        return bn
-    rows, across = -(-N // 128), -(-T // bn)
-    return -bn if -(-(-(-rows // 2) * across) // (SM_COUNT // 2)) <= -(-(rows * across) // SM_COUNT) else bn
+    """``persistent_plan``'s width, or a negative one: CTAs then work in pairs on 256 weight rows of it.  From ``PAIRS_FROM`` multiply-adds on, at widths
+    in steps of 32, wherever ``persistent_plan``'s measure, less 7 %, comes out no larger than the single tiles' (each pair is two SMs, and an odd last row
+    tile leaves one of them idle).  7 %: pairs of 256 against single tiles of 240 took 227 us for 231 (1,184 tokens, 24,576 rows of 4,096) and 61.0 for 63.7
+    (2,048, 6,144 of 2,560), where the measure has 6 % more for them; at equal widths they save 2 to 4 %."""
+    return _paired_width(T, N) if pair_tiles and T * N * K >= PAIRS_FROM else persistent_plan(T, N)
+
+
+@functools.lru_cache(maxsize=4096)
+def _paired_width(T: int, N: int) -> int:
+    cost, single = _tile_by_tile(T, N)
+    rows = -(-N // 256)
+    paired, bn = min((-(-(rows * -(-T // bn)) // (SM_COUNT // 2)) * (bn + 24), bn) for bn in PERSISTENT_TILES if bn % 32 == 0)
+    return -bn if 0.93 * paired <= cost else single
 
 
 def _tile_by_tile(T: int, N: int):

@@ -9,7 +9,8 @@ from marin_b200.kernels import ops
 def test_stream_k_is_planned_only_where_the_kernel_takes_it(T, N, K):
     bn = ops.stream_k_plan(T, N, K)
     assert ops.persistent_plan(T, N) in ops.PERSISTENT_TILES
-    assert abs(ops.paired_plan(T, N, K)) == ops.persistent_plan(T, N)
+    paired = ops.paired_plan(T, N, K)
+    assert paired == ops.persistent_plan(T, N) or (-paired in ops.PERSISTENT_TILES and paired % 32 == 0)
     if bn is None:
         return
     assert bn in ops.STREAM_K_TILES
