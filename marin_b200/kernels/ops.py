@@ -2010,10 +2010,13 @@ def _experts_tc(x, xs, w_gate_up, w_down, offsets, act, inv, weights, y, weight_
     mode = 0 if capped else _GLU_MODES["silu"] if gated else 4
     first = workspace.get("moe_gate_up", (pairs, 2 * ff), x.dtype) if capped else act
     N = w_gate_up.shape[1]
+    # by pairs of SMs from PAIRS_FROM multiply-adds on (2,048 tokens, 8 experts of 2,560 x 3,648, two chosen, a shared one of 2,432: 292 us alone, 269 in pairs)
+    tile1, tile2 = (-tile if pair_tiles and tile == 256 and parts == 1 and h * (pairs * n + n2 * n_shared) >= PAIRS_FROM else tile
+                    for n, n_shared in ((N, first2.shape[0] if n2 else 0), (ff, ff2)))
     _cost(touched * N * h * size + pairs * (h + ff) * size + (_size(first2) + _size(x) + _size(act2) if n2 else 0),
           2.0 * pairs * N * h + (2.0 * T * first2.numel() if n2 else 0.0))
     _check(lib.mb_moe_grouped_tc(_ptr(xs), _ptr(w_gate_up), _ptr(offsets), _c_int(E), _c_int(pairs), _c_int(N), _c_int(h), _ptr(first), _ptr(x if n2 else None),
-                                 _ptr(first2), _c_int(n2), _c_int(first2.shape[0] if n2 else 0), _c_int(h), _ptr(act2), _c_int(mode), _c_int(tile),
+                                 _ptr(first2), _c_int(n2), _c_int(first2.shape[0] if n2 else 0), _c_int(h), _ptr(act2), _c_int(mode), _c_int(tile1),
                                  _c_int(1), _c_int(SM_COUNT), _ptr(s.error), _stream()),
            "experts, gate|up (grouped, tcgen05)" if gated else "experts, up, relu squared (grouped, tcgen05)")
     if capped:
@@ -2022,7 +2025,7 @@ def _experts_tc(x, xs, w_gate_up, w_down, offsets, act, inv, weights, y, weight_
     _cost(touched * ff * h * size + pairs * ff * size + _size(rows) + (_size(down2) + _size(act2) + _size(rows2) if n2 else 0),
           2.0 * pairs * ff * h + (2.0 * T * down2.numel() if n2 else 0.0))
     _check(lib.mb_moe_grouped_tc(_ptr(act), _ptr(w_down), _ptr(offsets), _c_int(E), _c_int(pairs), _c_int(h), _c_int(ff), _ptr(rows), _ptr(act2), _ptr(down2),
-                                 _c_int(n2), _c_int(h if n2 else 0), _c_int(ff2), _ptr(rows2), _c_int(1), _c_int(tile), _c_int(parts), _c_int(SM_COUNT),
+                                 _c_int(n2), _c_int(h if n2 else 0), _c_int(ff2), _ptr(rows2), _c_int(1), _c_int(tile2), _c_int(parts), _c_int(SM_COUNT),
                                  _ptr(s.error), _stream()), "experts, down (grouped, tcgen05)")
     _cost(_size(rows) + 2 * _size(y) + (_size(rows2) if n2 else 0))
     _check(_lib("mb_moe").mb_moe_combine(_ptr(rows), _ptr(inv), _ptr(None if weight_on_input else weights), _ptr(y), _c_int(T), _c_int(h), _c_int(top), *same,

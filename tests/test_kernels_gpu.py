@@ -935,6 +935,30 @@ def test_grouped_expert_products_on_tcgen05_match_the_plain_twin(ops, request, a
     assert float(off.max()) <= 0.05 * float((want - y0).abs().max())
 
 
+@pytest.mark.parametrize("counts,h,ff,shared_ff", [((300, 0, 257, 256, 40), 192, 320, 128), ((540, 3), 128, 128, 64), ((1, 700, 33), 320, 448, 0)])
+def test_grouped_products_by_pairs_of_sms_have_the_same_bits(ops, monkeypatch, counts, h, ff, shared_ff):
+    """Odd tiles of 128 weight rows (the next expert's rows lie behind them), shares that fill no tile and several, the shared expert: K in the same order."""
+    from marin_b200.engine.context import Workspace
+
+    E, T = len(counts), sum(counts)
+    g = torch.Generator(device=DEV).manual_seed(T + h)
+    experts = torch.tensor([e for e, n in enumerate(counts) for _ in range(n)], dtype=torch.int32, device=DEV)[torch.randperm(T, generator=g, device=DEV)].view(T, 1).contiguous()
+    weights = torch.rand(T, 1, generator=g, device=DEV)
+    rnd = lambda *shape: (torch.randn(*shape, generator=g, device=DEV) * shape[-1] ** -0.5).to(torch.bfloat16)
+    x, w1, w2 = rnd(T, h), rnd(E, 2 * ff, h), rnd(E, h, ff)
+    shared = (rnd(2 * shared_ff, h), rnd(h, shared_ff)) if shared_ff else None
+    assert ops._expert_tile(T, E) == 256
+    monkeypatch.setattr(ops, "PAIRS_FROM", 0)
+    results = []
+    for pairs in (True, False):
+        monkeypatch.setattr(ops, "pair_tiles", pairs)
+        y = torch.zeros(T, h, device=DEV)
+        ops.moe_experts(x, w1, w2, experts, weights, y, False, Workspace(DEV), True, "swiglu", None, 0, shared)
+        ops.check_device_errors()
+        results.append(y)
+    assert torch.equal(*results) and float(results[0].abs().max()) > 0
+
+
 @pytest.mark.parametrize("T,h,E", [(1183, 96, 3), (1184, 96, 8), (1187, 2560, 9), (2049, 52, 20), (5, 2560, 64), (3, 132, 7), (301, 96, 8), (603, 132, 5)])
 def test_router_straight_from_memory_has_the_staged_kernels_bits(ops, T, h, E):
     """Eight, four, two tokens a block (from 1,184, 592, 296 on) and one, and the kernel that stages the row (taken for rows that are not at 8-byte addresses)."""
