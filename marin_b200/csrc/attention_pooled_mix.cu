@@ -95,16 +95,22 @@ __device__ __forceinline__ int pools_seen(int p, int window, int pool) { return 
 // The tiles of 16 queries of request r start at this tile of the step's portions (room is left for a partial tile per request).
 __device__ __forceinline__ int first_tile(const int* cu_tokens, int first_req, int r) { return (cu_tokens[r] - cu_tokens[first_req]) / NQ + (r - first_req); }
 
-// Blocks of a tile whose queries are at positions q_first .. q_last: pooled ones first, then positions from the block of the first one seen.
+// Blocks of a tile whose queries are at positions q_first .. q_last: pooled ones first, then positions from the block of the first one seen.  Of a
+// block only the rows from `begin` to `end` are read, what lies beside them counts as zero: a page that the window has passed may belong to another
+// request, and a number there that is not finite would reach the sums through a weight of zero.
 struct Blocks {
-    int pooled, first, count, nb_most;
-    __device__ Blocks(int q_first, int q_last, int window, int pool, int size) {
+    int pooled, first, count, nb_most, seen, q_last;
+    __device__ Blocks(int q_first, int q_last_, int window, int pool, int size) {
+        q_last = q_last_;
         nb_most = pools_seen(q_last, window, pool);
         pooled = (nb_most + size - 1) / size;
-        first = first_seen(q_first, window) / size;
+        seen = first_seen(q_first, window);
+        first = seen / size;
         count = pooled + q_last / size - first + 1;
     }
     __device__ bool is_pooled(int b) const { return b < pooled; }
+    __device__ int begin(int b) const { return b < pooled ? 0 : seen; }
+    __device__ int end(int b) const { return b < pooled ? nb_most - 1 : q_last; }
     __device__ int key0(int b, int size) const { return b < pooled ? b * size : (first + b - pooled) * size; }
 };
 
@@ -145,11 +151,11 @@ __global__ void __launch_bounds__(256, 2) stats_kernel(
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     auto fetch = [&](int b) {
         const bool pooled = blocks.is_pooled(b);
-        const int key0 = blocks.key0(b, SN), last = pooled ? blocks.nb_most - 1 : pos0 + here - 1;
+        const int key0 = blocks.key0(b, SN);
         const bf16* src = pooled ? k_pool : k_cache;
         bf16* dst = sK + (b & 1) * SN * LDK;
         const int row = tid >> 2, key = key0 + row;            // four threads a row
-        if (key <= last) {
+        if (key >= blocks.begin(b) && key <= blocks.end(b)) {
             const bf16* from = src + row_at(table, key, pooled, kh, page_shift, pool, pool_rows) * D;
 #pragma unroll
             for (int c = tid & 3; c < D / 8; c += 4) cp_async16(dst + row * LDK + c * 8, from + c * 8);
@@ -283,13 +289,13 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
     bf16* myK = sK + kv * NK * LDK;
     auto fetch = [&](int b) {                                  // this warp's part of its kv head's keys: 16 bytes a lane
         const bool pooled = blocks.is_pooled(b);
-        const int key0 = blocks.key0(b, NK), last = pooled ? blocks.nb_most - 1 : pos0 + here - 1;
+        const int key0 = blocks.key0(b, NK), begin = blocks.begin(b), end = blocks.end(b);
         const bf16* src = pooled ? k_pool : k_cache;
         constexpr int PER = D / 8;
 #pragma unroll 4
         for (int idx = warp % WK * 32 + lane; idx < NK * PER; idx += 32 * WK) {
             const int row = idx / PER, c = idx % PER, key = key0 + row;
-            if (key <= last) cp_async16(myK + row * LDK + c * 8, src + row_at(table, key, pooled, kv, page_shift, pool, pool_rows) * D + c * 8);
+            if (key >= begin && key <= end) cp_async16(myK + row * LDK + c * 8, src + row_at(table, key, pooled, kv, page_shift, pool, pool_rows) * D + c * 8);
             else *reinterpret_cast<uint4*>(myK + row * LDK + c * 8) = make_uint4(0, 0, 0, 0);
         }
         cp_async_commit();
@@ -459,12 +465,12 @@ __global__ void __launch_bounds__(VALUE_THREADS) value_kernel(
                 }
             }
             const bool pooled = all.is_pooled(b);
-            const int key0 = all.key0(b, NK), last = pooled ? all.nb_most - 1 : pos0 + here - 1;
+            const int key0 = all.key0(b, NK), begin = all.begin(b), end = all.end(b);
             const bf16* from = pooled ? v_pool : v_cache;
             constexpr int PER = DV / 8;
             for (int idx = tid; idx < NK * PER; idx += VALUE_THREADS) {
                 const int row = idx / PER, c = idx % PER, key = key0 + row;
-                if (key <= last) cp_async16(sV + row * LDV + c * 8, from + row_at(table, key, pooled, kh, page_shift, pool, pool_rows) * DV + c * 8);
+                if (key >= begin && key <= end) cp_async16(sV + row * LDV + c * 8, from + row_at(table, key, pooled, kh, page_shift, pool, pool_rows) * DV + c * 8);
                 else *reinterpret_cast<uint4*>(sV + row * LDV + c * 8) = make_uint4(0, 0, 0, 0);
             }
         }

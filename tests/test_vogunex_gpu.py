@@ -270,6 +270,32 @@ def test_weights_mixed_ahead_of_the_values(monkeypatch, m):
     ops.check_device_errors()
 
 
+def test_rows_that_the_window_has_passed_are_another_requests():
+    """A window without pooled blocks, portions behind it long enough for the kernels that mix the weights ahead of the values: the pages ahead of the
+    window are given back, and their places in the block table read as page 0, here another request's, whose numbers are large, infinite or not
+    numbers: every bit is what it is with zeros there.  Window and cuts leave up to 28 rows of the first block ahead of the first position seen."""
+    from marin_b200.kernels import ops
+
+    m = _attn(16, 4, 32, 32, 0.2, size=10, softcap=2.0)
+    rt, hidden, cuts = runtime("bfloat16"), 48, [100, 400, 325, 17]
+    part = build_mixer("attention", m, hidden, 1e-5, rt, attention_weights(hidden, m, 33))
+    x = bf(torch.randn(sum(cuts), hidden, generator=torch.Generator().manual_seed(34)))
+    results = []
+    for other in (0.0, math.nan, math.inf, 3e38):
+        runner = harness([part.cache_need()], rt, page=8, pages=160)
+        runner.begin("other")
+        runner.cache.reserve("other", 8)
+        assert list(runner.cache.block_table("other", 0)) == [0]
+        group = runner.cache.groups[0]
+        group.k[:, 0], group.v[:, 0] = other, other
+        results.append(feed([part], runner, x, cuts)[0])
+        runner.end("other")
+    assert bool(torch.isfinite(results[0]).all())
+    for got in results[1:]:
+        assert torch.equal(got, results[0])
+    ops.check_device_errors()
+
+
 def test_pooled_rows_live_in_the_pages_and_are_given_back_with_them():
     """Pages, their pooled rows and state slots are handed to the next request: a second request in the places of a first one
     gets what it gets alone in a fresh cache."""
