@@ -1913,15 +1913,23 @@ def _expert_tile(pairs: int, E: int) -> int:
     return 32 if average <= 20 else 64 if average <= 44 else 128 if average <= 100 else 256
 
 
-def _down_parts(touched: int, shared_rows: int, average: float, tile: int, h: int, ff: int, shared_ff: int) -> int:
+#: the further parts' results take no more memory than this (working memory that steps of any size are planned with)
+EXPERTS_PARTS_BYTES = 32 << 20
+
+
+def _down_parts(touched: int, pairs: int, shared_rows: int, tile: int, h: int, ff: int, shared_ff: int) -> int:
     """Parts of K the experts' last products are cut into: with few rows there are few tiles (8 experts of width 2,560: 160 for 148 SMs, two rounds), and the parts
-    make the rounds finer.  A part keeps at least eight k-blocks; beyond a hundred rows an expert the tensor pipe, not the rounds, sets the time."""
-    if average > 100:
+    make the rounds finer.  In bytes that the device moves meanwhile: a round of tiles is an SM's 128 weight rows of K each; a further part is one more
+    float32 row a pair (and shared row) written and read.  A part keeps at least eight k-blocks; beyond a hundred rows an expert the tensor pipe, not the
+    rounds, sets the time."""
+    if pairs > 100 * touched:
         return 1
     tiles = -(-h // 128) * (touched + -(-shared_rows // tile))
     kbs = [k // 64 for k in (ff, shared_ff) if k]
-    fits = [p for p in (1, 2, 3, 4) if all(-(-n // p) >= 8 and (p - 1) * -(-n // p) < n for n in kbs)] or [1]
-    return min(fits, key=lambda p: (-(-tiles * p // SM_COUNT) / p + 0.02 * p, p))
+    further = (pairs + shared_rows) * h * 4
+    fits = [p for p in (1, 2, 3, 4) if all(-(-n // p) >= 8 and (p - 1) * -(-n // p) < n for n in kbs) and (p - 1) * further <= EXPERTS_PARTS_BYTES] or [1]
+    round_bytes = SM_COUNT * 128 * max(ff, shared_ff) * 2
+    return min(fits, key=lambda p: (-(-tiles * p // SM_COUNT) / p * round_bytes + (p - 1) * 2 * further, p))
 
 
 def moe_joins_shared(x: torch.Tensor, h: int, ff: int, shared_ff: int, E: int, top: int, interleaved: bool, activation: str) -> bool:
@@ -2003,7 +2011,7 @@ def _experts_tc(x, xs, w_gate_up, w_down, offsets, act, inv, weights, y, weight_
         first2, down2 = shared
         ff2 = down2.shape[1]
     n2 = T if shared is not None else 0
-    parts = _down_parts(touched, T if n2 else 0, pairs / E, tile, h, ff, ff2)
+    parts = _down_parts(touched, pairs, n2, tile, h, ff, ff2)
     if n2:
         act2, rows2 = workspace.get("moe_shared_act", (T, ff2), x.dtype), workspace.get("moe_shared_rows", (parts, T, h), torch.float32)
     capped = activation == "glu_capped"

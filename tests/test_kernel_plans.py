@@ -33,3 +33,20 @@ def test_few_token_plan_keeps_every_slice_in_use(T, N, K):
     nkb = -(-K // 64)
     per = -(-nkb // splits)
     assert (splits - 1) * per < nkb                            # no slice without k-blocks
+
+
+@pytest.mark.parametrize("E", [1, 8, 16, 32, 60, 128, 384, 512])
+@pytest.mark.parametrize("h,ff,shared_ff", [(2560, 3648, 2432), (4096, 2048, 0), (2048, 768, 768), (256, 512, 1024)])
+def test_parts_of_the_experts_last_products_cost_less_than_the_round_they_save(E, h, ff, shared_ff):
+    """Whatever the experts' number and shares: no part is empty or short, what further parts write and read again is less than a round of weight tiles, and it
+    fits the memory set aside for it."""
+    for rows in (1, 2, 5, 12, 20, 33, 60, 96, 99, 150):                       # an expert's average share
+        pairs = rows * E
+        for shared_rows in ((0, pairs // 2 + 1) if shared_ff else (0,)):
+            tile = ops._expert_tile(pairs, E)
+            parts = ops._down_parts(min(pairs, E), pairs, shared_rows, tile, h, ff, shared_ff if shared_rows else 0)
+            further = (parts - 1) * (pairs + shared_rows) * h * 4
+            assert 2 * further <= ops.SM_COUNT * 128 * max(ff, shared_ff) * 2 and further <= ops.EXPERTS_PARTS_BYTES
+            for k in (ff, shared_ff if shared_rows else 0):
+                n = k // 64
+                assert k == 0 or parts == 1 or (-(-n // parts) >= 8 and (parts - 1) * -(-n // parts) < n)
