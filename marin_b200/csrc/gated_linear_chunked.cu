@@ -261,8 +261,9 @@ __global__ void __launch_bounds__(256) carry_kernel(float* floats, float* __rest
     const int chunks = (count + CH - 1) / CH, n = at / dv;
     const size_t step = (size_t)H * CHUNK_F32(dv);
     float* base = floats + ((size_t)first_chunk(cu_tokens, first_req, req) * H + head) * CHUNK_F32(dv);
-    float4* kept = reinterpret_cast<float4*>(state + (size_t)slots[req] * state_stride + (size_t)head * DQ * dv + at);
-    float4 s = *kept;
+    float* kept = state + (size_t)slots[req] * state_stride + (size_t)head * DQ * dv + at;
+    const bool whole = (((uintptr_t)kept) & 15) == 0;          // (a slot's row may be of any length: time mixing over an odd hidden size)
+    float4 s = whole ? *reinterpret_cast<const float4*>(kept) : make_float4(kept[0], kept[1], kept[2], kept[3]);
     float4 add[CARRY_AHEAD];
     float decay[CARRY_AHEAD];
     for (int c0 = 0; c0 < chunks; c0 += CARRY_AHEAD) {
@@ -281,7 +282,8 @@ __global__ void __launch_bounds__(256) carry_kernel(float* floats, float* __rest
                 s.x = fmaf(s.x, e, add[u].x); s.y = fmaf(s.y, e, add[u].y); s.z = fmaf(s.z, e, add[u].z); s.w = fmaf(s.w, e, add[u].w);
             }
     }
-    *kept = s;
+    if (whole) *reinterpret_cast<float4*>(kept) = s;
+    else { kept[0] = s.x; kept[1] = s.y; kept[2] = s.z; kept[3] = s.w; }
 }
 
 // ---- the outputs -------------------------------------------------------------------------------------------------------------------
@@ -631,7 +633,7 @@ MB_API int mb_gla_chunked(int which, const void* q, const void* k, const void* v
 #else
 // Time mixing over requests first_req .. requests - 1; which: 0 adds, 1 carries, 2 reads (in this order).  r, k, v, gate_rows, out bf16 [tokens][H * QK_DIM]; the
 // decays' numbers either as float32 rows wraw likewise, or (wraw null) as l W_2^T of l bf16 [tokens][rank] and w2 bf16 [H * QK_DIM][rank], rank a multiple of 16
-// up to 128; w0, u and norm_w float32 [H * QK_DIM]; all 16-byte aligned.  A slot's row of `state_stride` floats (a multiple of 4) has the heads'
+// up to 128; w0, u and norm_w float32 [H * QK_DIM]; all 16-byte aligned.  A slot's row of `state_stride` floats has the heads'
 // matrices at `state` and the last row of h ([tokens][width]) at `last`.  floats holds (tokens / 64 + requests) * H pieces of mb_gla_chunked_scratch.
 MB_API int mb_wkv_chunked(int which, const void* r, const void* k, const void* v, const float* wraw, const void* l, const void* w2, int rank, const float* w0,
                           const float* u, float* state,
@@ -639,10 +641,10 @@ MB_API int mb_wkv_chunked(int which, const void* r, const void* k, const void* v
                           const void* gate_rows, const float* norm_w, float eps, void* out, int first_req, int requests, int max_query_len, int H, cudaStream_t s) {
     static_assert(VS == DQ, "time mixing: values as wide as keys, a whole head a CTA");
     if (requests <= first_req || max_query_len <= 0) return 0;
-    if (H <= 0 || first_req < 0 || width <= 0 || state_stride % 4 != 0) return MB_ERR_BAD_SIZE;
+    if (H <= 0 || first_req < 0 || width <= 0) return MB_ERR_BAD_SIZE;
     if (wraw != nullptr) rank = 0;
     else if (l == nullptr || w2 == nullptr || rank <= 0 || rank % 16 != 0 || rank > 128) return MB_ERR_BAD_SIZE;
-    if ((((uintptr_t)r | (uintptr_t)k | (uintptr_t)v | (uintptr_t)wraw | (uintptr_t)l | (uintptr_t)w2 | (uintptr_t)w0 | (uintptr_t)u | (uintptr_t)floats | (uintptr_t)state | (uintptr_t)gate_rows |
+    if ((((uintptr_t)r | (uintptr_t)k | (uintptr_t)v | (uintptr_t)wraw | (uintptr_t)l | (uintptr_t)w2 | (uintptr_t)w0 | (uintptr_t)u | (uintptr_t)floats | (uintptr_t)gate_rows |
           (uintptr_t)norm_w | (uintptr_t)out) & 15) != 0)
         return MB_ERR_BAD_SIZE;
     const int count = requests - first_req, stride = H * DQ;

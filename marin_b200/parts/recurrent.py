@@ -174,7 +174,7 @@ class WKV(Mixer):
         ops.tanh_cap(low, 1.0)
         out = ws.get("wkv_out", (T, n), x.dtype)
         # prompt portions 64 tokens at a time on the tensor cores; single tokens (and sizes those kernels are not made for, and the 32-bit path) token by token
-        chunked = ops.wkv_goes_chunked(ctx, x.dtype, self.dim, state, rkvg[0], rkvg[1], rkvg[2], rkvg[3], low)
+        chunked = ops.wkv_goes_chunked(ctx, x.dtype, self.dim, *rkvg, low)
         inside = chunked and self.low_dim <= 128                # the chunked kernels apply the decays' second matrix themselves
         walked = ctx.num_decode if chunked else None            # the requests that are walked: all, or those with a single token
         wraw = None

@@ -228,25 +228,88 @@ def test_wkv_alone(dtype, heads, dim, rank):
         close(feed(mixer, harness(mixer, rt), x, cuts), want, dtype, f"cuts {cuts[:4]}")
 
 
-@pytest.mark.parametrize("heads, dim", [(2, 64), (1, 128), (2, 32), (3, 16)])
-def test_wkv_long_portions_in_blocks_side_by_side(heads, dim):
-    """Portions long enough to be cut into blocks that are walked side by side (bfloat16), cut at and around block edges,
-    with single tokens and short portions (one walk) in between: all of them carry the same state and the same last row."""
-    from marin_b200.kernels import ops
+def wkv_mixer(heads, dim, rank, hidden, seed, rt):
     from marin_b200.parts import lookup
 
-    dtype = "bfloat16"
-    rt = runtime(dtype)
+    mixer = lookup("mixer", "wkv")(hidden=hidden, heads=heads, dim=dim, decay_rank=rank, name="m", norm_eps=1e-5)
+    w = mixer_weights(mixer, "bfloat16", seed)
+    w["m.w0"] = (torch.rand(heads * dim, generator=torch.Generator().manual_seed(seed + 1)) * 5.0 - 4.5).to(torch.bfloat16)
+    return mixer, w
+
+
+@pytest.mark.parametrize("chunked", [True, False], ids=["chunks", "walk"])
+@pytest.mark.parametrize("heads, dim", [(2, 64), (1, 128), (2, 32), (3, 16), (2, 48)])
+def test_wkv_long_portions(monkeypatch, heads, dim, chunked):
+    """Long portions in chunks of 64 tokens and token by token (bfloat16), cut at and around chunk edges, with single tokens and short portions (the walk)
+    in between: all of them carry the same state and the same last row."""
+    from marin_b200.kernels import ops
+
+    rt = runtime("bfloat16")
     hidden, T = 40, 700
-    mixer = lookup("mixer", "wkv")(hidden=hidden, heads=heads, dim=dim, decay_rank=8, name="m", norm_eps=1e-5)
-    w = mixer_weights(mixer, dtype, 12)
-    w["m.w0"] = (torch.rand(heads * dim, generator=torch.Generator().manual_seed(13)) * 5.0 - 4.5).to(torch.bfloat16)
+    mixer, w = wkv_mixer(heads, dim, 8, hidden, 12, rt)
     mixer.load(dict(w), rt)
     x = torch.randn(T, hidden, generator=torch.Generator().manual_seed(14)).to(rt.dtype)
     want = plain.wkv(x.double(), {k: v.double() for k, v in w.items()}, "m", heads, dim, 1e-5)
-    assert ops.WKV_BLOCKS_FROM <= 256 and ops.WKV_BLOCK_TOKENS == 128
-    for cuts in ([700], [256, 444], [257, 1, 1, 441], [300, 100, 300], [383, 317]):
-        close(feed(mixer, harness(mixer, rt, ctx_len=1024), x, cuts), want, dtype, f"cuts {cuts}")
+    monkeypatch.setattr(ops, "use_chunked_wkv", chunked)
+    taken, inner = [], ops.wkv_chunked
+    monkeypatch.setattr(ops, "wkv_chunked", lambda *a: (taken.append(1), inner(*a))[1])
+    for cuts in ([700], [256, 444], [257, 1, 1, 441], [300, 100, 300], [383, 317], [17, 64, 16, 603]):
+        close(feed(mixer, harness(mixer, rt, ctx_len=1024), x, cuts), want, "bfloat16", f"cuts {cuts}")
+    assert len(taken) == (13 if chunked else 0)
+
+
+@pytest.mark.parametrize("heads, dim, rank, hidden, spread", [
+    (2, 64, 8, 40, 1.0),
+    (1, 128, 144, 40, 1.0),                  # the decays' second matrix by itself: too many numbers between the two
+    (3, 16, 16, 42, 1.0), (1, 80, 24, 43, 1.0),      # slots' rows at odd addresses
+    (2, 32, 32, 40, 5.0), (1, 64, 8, 40, 5.0),       # decays from nearly one to nothing, token by token in every channel
+])
+def test_wkv_chunks_beside_single_tokens(monkeypatch, heads, dim, rank, hidden, spread):
+    """Two portions and a single token of a third request in one step, portions at the edges of chunks, against the plain implementation; then the states and last
+    rows against the walk's.  States: products of pairs of bf16 numbers, about 2^-17 a factor, and sums of a chunk's logarithms, some hundreds where most decays
+    are ordinary (half a last place of 512 is 3e-5 in log2): 2e-4 of the largest number holds both, as it does for the delta rule's chunks.  The last row is copied."""
+    from marin_b200.engine import StepEntry
+    from marin_b200.kernels import ops
+
+    rt = runtime("bfloat16")
+    mixer, w = wkv_mixer(heads, dim, rank, hidden, 15, rt)
+    w["m.w2"] = w["m.w2"] * spread
+    mixer.load(dict(w), rt)
+    steps = [[("a", 63), ("b", 65), ("c", 30)], [("c", 1), ("a", 64), ("b", 129)], [("b", 1), ("c", 1), ("a", 130)], [("a", 1), ("b", 17), ("c", 200)]]
+    total = {r: sum(n for step in steps for q, n in step if q == r) for r in "abc"}
+    x = {r: torch.randn(total[r], hidden, generator=torch.Generator().manual_seed(ord(r))).to(rt.dtype) for r in "abc"}
+    want = {r: plain.wkv(x[r].double(), {k: v.double() for k, v in w.items()}, "m", heads, dim, 1e-5) for r in "abc"}
+    taken, inner = [], ops.wkv_chunked
+    monkeypatch.setattr(ops, "wkv_chunked", lambda *a: (taken.append(a[-1] is None), inner(*a))[1])
+    kept = []
+    for chunked in (True, False):
+        monkeypatch.setattr(ops, "use_chunked_wkv", chunked)
+        runner = harness(mixer, rt, pages=200, ctx_len=1024)
+        at, got, states = dict.fromkeys("abc", 0), {r: [] for r in "abc"}, []
+        for r in "abc":
+            runner.begin(r)
+        for step in steps:
+            for r, n in step:
+                runner.cache.reserve(r, at[r] + n)
+            ctx = runner.build_context([StepEntry(r, [0] * n, []) for r, n in step])
+            view = runner.views.view(0, ctx)
+            rows = torch.cat([x[r][at[r]:at[r] + n] for r, n in step]).to(DEV)
+            residual = torch.zeros(rows.shape[0], hidden, device=DEV)
+            mixer.forward(rows, ctx, view, residual)
+            for (r, n), out, span in zip(step, residual.cpu().split([n for _, n in step]), ctx.spans):
+                got[r].append(out)
+                at[r] += n
+                runner.cache.commit(r, at[r])
+                states.append(view.state[span.slot].clone())
+        for r in "abc":
+            close(torch.cat(got[r]), want[r], "bfloat16", f"request {r}, chunked {chunked}")
+        kept.append(states)
+        ops.check_device_errors()
+    assert taken == [rank <= 128] * 4
+    m = heads * dim * dim
+    for a, b in zip(*kept):
+        assert torch.equal(a[m:], b[m:])
+        assert float((a[:m] - b[:m]).abs().max()) <= 2e-4 * float(b[:m].abs().max())
 
 
 def attention_mixer(hidden, H, K, d, dv, rows, farthest, coef=0.3, every=5, scale=0.25):
