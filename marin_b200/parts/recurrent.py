@@ -176,22 +176,24 @@ class WKV(Mixer):
         # prompt portions 64 tokens at a time on the tensor cores; single tokens (and sizes those kernels are not made for, and the 32-bit path) token by token
         chunked = ops.wkv_goes_chunked(ctx, x.dtype, self.dim, *rkvg, low)
         inside = chunked and self.low_dim <= 128                # the chunked kernels apply the decays' second matrix themselves
-        walked = ctx.num_decode if chunked else None            # the requests that are walked: all, or those with a single token
+        walked = ctx.num_decode if chunked else T               # the step's first so many tokens are walked: all, or the single ones
+        rows = walked if inside else T                          # ... and so many decays are asked for
         wraw = None
-        if not inside or walked:
-            wraw = ws.get("wkv_wraw", (T, n), torch.float32)
-            ops.gemm(low, self.w_2, wraw)
+        if rows > 0:
+            wraw = ws.get("wkv_wraw", (rows, n), torch.float32)
+            ops.gemm(low[:rows], self.w_2, wraw)
         if chunked:
             ops.stage_name = "recurrence, norm, gate"
             ops.wkv_chunked(rkvg[0], rkvg[1], rkvg[2], rkvg[3], low, self.w_2, self.w0, self.u, self.norm_w, self.norm_eps, state, carry, x, ctx, cache.slots,
                             out, self.heads, self.dim, None if inside else wraw)
-        if walked != 0:
+        if walked > 0:
             ops.stage_name = "recurrence"
-            o = ws.get("wkv_o", (T, n), torch.float32)
-            ops.wkv_scan(rkvg[0], rkvg[1], rkvg[2], wraw, self.w0, self.u, state, carry, x, ctx, cache.slots, o, self.heads, self.dim, walked)
+            o = ws.get("wkv_o", (walked, n), torch.float32)
+            r, k, v, g = (t[:walked] for t in rkvg)
+            ops.wkv_scan(r, k, v, wraw[:walked], self.w0, self.u, state, carry, x[:walked], ctx, cache.slots, o, self.heads, self.dim,
+                         walked if chunked else None)
             ops.stage_name = "norm, gate"
-            rows = T if walked is None else walked
-            ops.head_norm_gate(o[:rows], self.norm_w, rkvg[3][:rows], self.norm_eps, out[:rows], self.heads, self.dim)
+            ops.head_norm_gate(o, self.norm_w, g, self.norm_eps, out[:walked], self.heads, self.dim)
         ops.stage_name = "o"
         ops.gemm(out, self.w_o, residual, accumulate=True)
         return None

@@ -281,6 +281,8 @@ def test_wkv_chunks_beside_single_tokens(monkeypatch, heads, dim, rank, hidden, 
     want = {r: plain.wkv(x[r].double(), {k: v.double() for k, v in w.items()}, "m", heads, dim, 1e-5) for r in "abc"}
     taken, inner = [], ops.wkv_chunked
     monkeypatch.setattr(ops, "wkv_chunked", lambda *a: (taken.append(a[-1] is None), inner(*a))[1])
+    decays, product = [], ops.gemm                             # tokens whose decays' numbers are asked for by themselves
+    monkeypatch.setattr(ops, "gemm", lambda x, w, *a, **k: (decays.append(x.shape[0]) if w is mixer.w_2 else None, product(x, w, *a, **k))[1])
     kept = []
     for chunked in (True, False):
         monkeypatch.setattr(ops, "use_chunked_wkv", chunked)
@@ -306,6 +308,8 @@ def test_wkv_chunks_beside_single_tokens(monkeypatch, heads, dim, rank, hidden, 
         kept.append(states)
         ops.check_device_errors()
     assert taken == [rank <= 128] * 4
+    everything = [sum(n for _, n in step) for step in steps]
+    assert decays == ([1, 2, 1] if rank <= 128 else everything) + everything       # (the single tokens' where the chunks make their own)
     m = heads * dim * dim
     for a, b in zip(*kept):
         assert torch.equal(a[m:], b[m:])
