@@ -730,7 +730,9 @@ __global__ void __launch_bounds__(READ_THREADS, 2) read_kernel(const bf16* __res
     for (int i = warp; i < rows; i += READ_THREADS / 32) {
         const float4 v = here ? *reinterpret_cast<const float4*>(sums + i * ld + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
         if (!NORM) {
-            if (here) *reinterpret_cast<float4*>(o + (size_t)(tok0 + i) * H * dv + (size_t)head * dv + c0 + lane * 4) = v;
+            float* to = o + (size_t)(tok0 + i) * H * dv + (size_t)head * dv + c0 + lane * 4;
+            if (here && (((uintptr_t)to) & 15) == 0) *reinterpret_cast<float4*>(to) = v;
+            else if (here) { to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w; }
             continue;
         }
         uint2 raw = make_uint2(0u, 0u);
@@ -761,7 +763,7 @@ MB_API int mb_delta_chunked(const void* qkv, const void* b_rows, int b_stride, c
                             int* error_flag, int first_req, int requests, int max_query_len, int H, int G, int dv, int which, cudaStream_t s) {
     if (requests <= first_req || max_query_len <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G != 0 || dv <= 0 || dv % VS != 0 || first_req < 0 || ((2 * G * DQ + H * dv) % 8) != 0) return MB_ERR_BAD_SIZE;
-    if ((((uintptr_t)qkv | (uintptr_t)planes | (uintptr_t)floats | (uintptr_t)o) & 15) != 0) return MB_ERR_BAD_SIZE;
+    if ((((uintptr_t)qkv | (uintptr_t)planes | (uintptr_t)floats) & 15) != 0) return MB_ERR_BAD_SIZE;
     if (out != nullptr && (dv > READ_COLS || gate_rows == nullptr || norm_w == nullptr || ((gate_stride | out_stride) & 3) != 0 ||
                            (((uintptr_t)gate_rows | (uintptr_t)out) & 7) != 0 || ((uintptr_t)norm_w & 15) != 0))
         return MB_ERR_BAD_SIZE;

@@ -225,7 +225,10 @@ MB_API int mb_moe_route(const void* h_rows, int dtype, const float* router, cons
     if (dtype == MB_BF16 && h % 4 == 0 && (((uintptr_t)h_rows) & 7) == 0 && (((uintptr_t)router) & 15) == 0) {
         // as many tokens a block as still give every SM a block or two (148 SMs), if their rows fit
         const size_t per = (size_t)(2 * E + groups) * sizeof(float);
-#define MR_CASE(PER, FROM)                                                                                                                                        if (tokens >= FROM && (PER == 1 || PER * (per + (size_t)h * 2) + 16 <= 48 * 1024))                                                                                return launch_kernel(moe_route_rows_kernel<PER>, (tokens + PER - 1) / PER, MR_THREADS, PER * per + (PER > 1 ? (size_t)PER * h * 2 + 16 : 0), s, 0,                                 (const bf16*)h_rows, router, router_bias, expert_out, weight_out, tokens, h, E, top, score_mode, renorm, correction, groups, keep, factor);
+#define MR_CASE(PER, FROM)                                                                                                                       \
+        if (tokens >= FROM && (PER == 1 || PER * (per + (size_t)h * 2) + 16 <= 48 * 1024))                                                       \
+            return launch_kernel(moe_route_rows_kernel<PER>, (tokens + PER - 1) / PER, MR_THREADS, PER * per + (PER > 1 ? (size_t)PER * h * 2 + 16 : 0), s, 0, \
+                                 (const bf16*)h_rows, router, router_bias, expert_out, weight_out, tokens, h, E, top, score_mode, renorm, correction, groups, keep, factor);
         MR_CASE(8, 8 * 148) MR_CASE(4, 4 * 148) MR_CASE(2, 2 * 148) MR_CASE(1, 1)
 #undef MR_CASE
     }
@@ -586,7 +589,7 @@ __global__ void __launch_bounds__(128) moe_grouped_kernel(const bf16* __restrict
 // y[t][c] += sum over the token's choices, in choice order, of rows[inv[t top + choice]][c] (times the choice's weight, if given);
 // a choice numbered E or above is the identity: its row is h_rows[t] times identity_weight.  more (null: none): rows [tokens][h] added last.
 // rows and more may come in `parts` parts, rows_part and more_part numbers apart: a row is their sum, in order.
-// Bound by the bytes: four columns a thread by 16-byte accesses (h a multiple of 4).
+// Bound by the bytes: four columns a thread by 16-byte accesses (h a multiple of 4; y may lie at any float's address).
 __global__ void moe_combine_kernel(const float* __restrict__ rows, const int* __restrict__ inv, const float* __restrict__ weight_of,
                                    float* __restrict__ y, int h, int top, const int* __restrict__ expert_of, const bf16* __restrict__ h_rows,
                                    const float* __restrict__ identity_weight, int E, const float* __restrict__ more, int parts,
@@ -595,8 +598,10 @@ __global__ void moe_combine_kernel(const float* __restrict__ rows, const int* __
     rows = pdl_fresh(rows); inv = pdl_fresh(inv); y = pdl_fresh(y); weight_of = pdl_fresh(weight_of);
     expert_of = pdl_fresh(expert_of); h_rows = pdl_fresh(h_rows); identity_weight = pdl_fresh(identity_weight); more = pdl_fresh(more);
     const int t = blockIdx.x;
+    const bool whole = (((uintptr_t)y) & 15) == 0;
     for (int c = 4 * (blockIdx.y * blockDim.x + threadIdx.x); c < h; c += 4 * gridDim.y * blockDim.x) {
-        float4 a = *reinterpret_cast<const float4*>(y + (size_t)t * h + c);
+        float* at = y + (size_t)t * h + c;
+        float4 a = whole ? *reinterpret_cast<const float4*>(at) : make_float4(at[0], at[1], at[2], at[3]);
         for (int k = 0; k < top; ++k) {
             if (h_rows != nullptr && expert_of[t * top + k] >= E) {
                 const float w = identity_weight[t * top + k];
@@ -622,7 +627,8 @@ __global__ void moe_combine_kernel(const float* __restrict__ rows, const int* __
             }
             a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
         }
-        *reinterpret_cast<float4*>(y + (size_t)t * h + c) = a;
+        if (whole) *reinterpret_cast<float4*>(at) = a;
+        else { at[0] = a.x; at[1] = a.y; at[2] = a.z; at[3] = a.w; }
     }
 }
 
@@ -688,7 +694,7 @@ MB_API int mb_moe_grouped_down(const void* act, const void* w_down, const int* o
 MB_API int mb_moe_combine(const float* rows, const int* inv, const float* weight_of, float* y, int tokens, int h, int top, const int* expert_of,
                           const void* h_rows, const float* identity_weight, int E, const float* more, int parts, cudaStream_t s) {
     if (tokens <= 0) return 0;
-    if (parts < 1 || h % 4 != 0 || (((uintptr_t)rows | (uintptr_t)y | (uintptr_t)more) & 15) != 0) return MB_ERR_BAD_SIZE;
+    if (parts < 1 || h % 4 != 0 || (((uintptr_t)rows | (uintptr_t)more) & 15) != 0) return MB_ERR_BAD_SIZE;
     return launch_kernel(moe_combine_kernel, dim3(tokens, tokens >= 512 ? 1 : (h / 4 + 127) / 128), tokens >= 512 ? 256 : 128, 0, s, 0, rows, inv, weight_of, y, h, top,
                          expert_of, (const bf16*)h_rows, identity_weight, E, more, parts, (long long)tokens * top * h, (long long)tokens * h);
 }

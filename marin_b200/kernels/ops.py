@@ -2482,7 +2482,8 @@ DELTA_CHUNKED_FROM = 8
 
 
 def delta_chunked_supported(dtype, d: int, dv: int) -> bool:
-    return dtype == torch.bfloat16 and d % 16 == 0 and 16 <= d <= 128 and dv % 16 == 0
+    prepared = 8 * 64 * (d + 8) + 2 * 64 * 72 * 2 + 4 * 16 * 20 * 4 + 4 * 64 * 4 + 2 * 64 * (dv + 8) + 16       # csrc/delta_rule_chunked.cu, PREP_SMEM
+    return dtype == torch.bfloat16 and d % 16 == 0 and 16 <= d <= 128 and dv % 16 == 0 and prepared <= 227 * 1024
 
 
 def _delta_slice(dv: int) -> int:

@@ -972,3 +972,22 @@ def test_router_straight_from_memory_has_the_staged_kernels_bits(ops, T, h, E):
     ops.moe_route(x, router, *out[0], "softmax", True, None, corr)
     ops.moe_route(odd, router, *out[1], "softmax", True, None, corr)
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("T,identity", [(5, 0), (600, 2)])
+def test_expert_results_are_added_to_rows_at_any_address(ops, T, identity):
+    """Rows that are not at 16-byte addresses get what aligned ones get, bit for bit."""
+    from marin_b200.engine.context import Workspace
+
+    E, h, ff = 4, 128, 64
+    g = torch.Generator(device=DEV).manual_seed(T)
+    rnd = lambda *shape: (torch.randn(*shape, generator=g, device=DEV) * shape[-1] ** -0.5).to(torch.bfloat16)
+    x, w1, w2 = rnd(T, h), rnd(E, 2 * ff, h), rnd(E, h, ff)
+    experts = torch.randint(0, E + identity, (T, 2), generator=g, device=DEV, dtype=torch.int32)
+    weights, y0 = torch.rand(T, 2, generator=g, device=DEV), torch.randn(T, h, generator=g, device=DEV)
+    want, odd = y0.clone(), torch.zeros(T * h + 1, device=DEV)[1:].view(T, h)
+    odd.copy_(y0)
+    for y in (want, odd):
+        ops.moe_experts(x, w1, w2, experts, weights, y, False, Workspace(DEV), True, "swiglu", None, identity)
+    ops.check_device_errors()
+    assert torch.equal(odd, want) and not torch.equal(want, y0)

@@ -246,9 +246,13 @@ def test_chunks_of_every_slice_and_their_norm(d, dv, per_channel):
     inp = ops.DeltaInputs(beta_raw.to(DEV), a_raw.to(DEV), bf(torch.randn(T, H * dv, generator=g)).to(DEV), rate.to(DEV), dt_bias.to(DEV))
     norm_w, o = torch.randn(dv, generator=g).to(DEV), torch.zeros(T, H * dv, device=DEV)
     outs = [torch.zeros(T, H * dv + 8, device=DEV, dtype=torch.bfloat16)[:, 4:4 + H * dv] for _ in range(2)]
+    odd = torch.zeros(T * H * dv + 1, device=DEV)[1:].view(T, H * dv)          # (sums may go to any float's address)
     for gate in ("sigmoid", "silu"):
         states[1].copy_(states[2])
+        ops.delta_chunked(rows, inp, states[1], ctx, ctx.state_slots, odd, H, G, d, dv)
+        states[1].copy_(states[2])
         ops.delta_chunked(rows, inp, states[1], ctx, ctx.state_slots, o, H, G, d, dv)
+        assert torch.equal(odd, o)
         ops.delta_norm(o, inp.gate, gate, norm_w, 1e-5, 1.5, outs[0], H, dv)
         states[1].copy_(states[2])
         assert ops.delta_chunked_finishes(inp.gate, norm_w, outs[1], dv)
