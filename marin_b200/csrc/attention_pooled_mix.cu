@@ -7,15 +7,18 @@
 // times the products with V, and a float32 [tokens][H][KV_HEADS][V_DIM] that a second kernel reads.)  Mixing needs the weights already
 // divided by their sums, so three kernels:
 //   stats_kernel  (a CTA per kv head and 128 rows = queries x its heads): the logarithm of every row's sum of weights;
-//   mix_kernel    (a CTA per 16 queries, two heads a warp, 32 keys at a time): the weights of all heads, mixed, to scratch memory as bf16;
+//   mix_kernel    (a CTA per 16 queries, two heads a warp, 32 keys at a time): the weights of all heads, mixed, to scratch memory in 16 bits;
 //   value_kernel  (a CTA per 32 queries and kv head, a warp per head and 16 queries): mixed weights x values.
 // Exactness: the weights p are float32 and enter the mixing product as pairs of bf16 numbers (p = hi + lo), as does talk; the three larger of the four
-// products are taken, so about 16 bits of each enter, and the mixed weights are rounded to bf16 once, where the other kernel rounds every head's.
-// Scratch: [tile][block][H][16][32] bf16, a tile of 16 queries of one request, its blocks of 32 pooled rows, then of 32 positions.
+// products are taken, so about 16 bits of each enter.  The mixed weights, bounded numbers, wait as halves under one power of two for all of them (11 bits) and
+// meet the values as two bf16 numbers that hold the 11 bits exactly: they add next to nothing to the error that rounding the results
+// makes, where weights rounded to bf16 (every head's, in the other kernel) made it 1.17 times as large.
+// Scratch: [tile][block][H][16][32] halves, a tile of 16 queries of one request, its blocks of 32 pooled rows, then of 32 positions.
 // Measured on B200, 2,048 tokens, 32 heads of 128 over 8, window 1,024, pools of 64: the other kernel and its mixing 1,189 us;
-// these 95 + 216 + 100 us.  mix_kernel is bound by the instructions that make a weight (about fourteen a score, with the cap) and its two mixing products.
+// these 95 + 216 + 141 us (the values 100 with weights rounded to bf16, one product a block instead of two).  mix_kernel is bound by the instructions that make a weight (about fourteen a score, with the cap) and its two mixing products.
 #define MB_LIB "attention_pooled_mix"
 #define MB_LIB_ID 25
+#include <cuda_fp16.h>
 #include "common.cuh"
 #include "launch.cuh"
 #include "mma_helpers.cuh"
@@ -264,10 +267,25 @@ __device__ __forceinline__ void split_bf16(float x, float y, uint32_t& hi, uint3
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = pack_bf16(x - back.x, y - back.y);
 }
+__device__ __forceinline__ uint32_t pack_half(float lo, float hi) {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// A mixed weight is at most NH times the largest |talk| (every weight is at most 1); this power of two brings it below 2^15, so that its 11 bits as a
+// half are there down to 2^-29 of the bound (a bf16 has 8).  Found by every warp from all of talk: the largest of numbers does not depend on their order.
+__device__ __forceinline__ int mixed_shift(const float* __restrict__ talk, int lane) {
+    float top = 0.0f;
+    for (int i = lane; i < NH * NH; i += 32) top = fmaxf(top, fabsf(talk[i]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    return min(100, max(-100, 14 - ilogbf(fmaxf(top, 1e-30f) * NH)));
+}
+__device__ __forceinline__ float two_to(int n) { return __int_as_float((127 + n) << 23); }
 
 __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
     const bf16* __restrict__ q, const bf16* __restrict__ k_cache, const bf16* __restrict__ k_pool, const float* __restrict__ lse,
-    const float* __restrict__ talk, bf16* __restrict__ mixed, const int* __restrict__ block_table, int max_pages, const int* __restrict__ cu_tokens,
+    const float* __restrict__ talk, __half* __restrict__ mixed, const int* __restrict__ block_table, int max_pages, const int* __restrict__ cu_tokens,
     const int* __restrict__ seq_lens, int first_req, int page_shift, float scale, float cap, int window, int pool, int pool_rows, int most_blocks) {
     PDL_ENTER();
     q = pdl_fresh(q); k_cache = pdl_fresh(k_cache); k_pool = pdl_fresh(k_pool); lse = pdl_fresh(lse);
@@ -283,7 +301,7 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
     const int here = min(NQ, n - qt * NQ), pos0 = seq_lens[r] - n + qt * NQ;
     const int* table = block_table + (size_t)r * max_pages;
     const Blocks blocks(pos0, pos0 + here - 1, window, pool, NK);
-    bf16* dst = mixed + (size_t)(first_tile(cu_tokens, first_req, r) + qt) * most_blocks * (NH * NQ * NK);
+    __half* dst = mixed + (size_t)(first_tile(cu_tokens, first_req, r) + qt) * most_blocks * (NH * NQ * NK);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t2 = 2 * (lane & 3);
     const int kv = warp / WK;
     bf16* myK = sK + kv * NK * LDK;
@@ -331,6 +349,7 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
         for (int kk = 0; kk < D / 16; ++kk) q_fragment(qa[h][kk], r0, r1, kk * 16 + t2);
     }
     const Cap c(scale, cap);
+    const float up = two_to(mixed_shift(talk, lane));
     const uint32_t k_addr = (uint32_t)__cvta_generic_to_shared(myK + ((lane & 7) + (lane >> 4) * 8) * LDK + ((lane >> 3) & 1) * 8);
     // a pair's row read as a B operand: eight keys of one query, 8 weights a matrix, up to 32 weights at a time
     const uint32_t p_addr = (uint32_t)__cvta_generic_to_shared(sPh + (lane & 7) * P_PITCH + (lane >> 3) * 16);
@@ -402,8 +421,8 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
                 mma_bf16_16816(acc, ah, pl[2 * ks], pl[2 * ks + 1]);
             }
             uint8_t* w = sW + (mt * 16 + g8) * W_HEAD + query * W_PITCH + (k8 + t2) * 2;
-            *reinterpret_cast<uint32_t*>(w) = pack_bf16(acc[0], acc[1]);
-            *reinterpret_cast<uint32_t*>(w + 8 * W_HEAD) = pack_bf16(acc[2], acc[3]);
+            *reinterpret_cast<uint32_t*>(w) = pack_half(acc[0] * up, acc[1] * up);
+            *reinterpret_cast<uint32_t*>(w + 8 * W_HEAD) = pack_half(acc[2] * up, acc[3] * up);
         }
         cp_async_wait<0>();
         __syncthreads();                                       // the mixed rows and the next block's keys are there; the pairs' rows may be written again
@@ -419,14 +438,15 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
 // Bound by what a CTA fetches through L2: two neighbouring tiles share every block of values (their ranges of blocks differ by one at most at either end).
 #define V_STAGES 4
 #define VT 2                          // tiles of 16 queries a CTA
+static_assert(VT == 2, "a tile's blocks are one of two");
 #define A_PITCH (NK + 8)              // elements of a row of mixed weights in shared memory
 #define A_TILE (G * NQ * A_PITCH)
 #define V_STAGE_BYTES (VT * A_TILE * 2 + NK * LDV * 2)
 #define VALUE_SMEM (V_STAGES * V_STAGE_BYTES)
 #define VALUE_THREADS (32 * G * VT)
 
-__global__ void __launch_bounds__(VALUE_THREADS) value_kernel(
-    const bf16* __restrict__ mixed, const bf16* __restrict__ v_cache, const bf16* __restrict__ v_pool, bf16* __restrict__ out,
+__global__ void __launch_bounds__(VALUE_THREADS, 2) value_kernel(
+    const __half* __restrict__ mixed, const float* __restrict__ talk, const bf16* __restrict__ v_cache, const bf16* __restrict__ v_pool, bf16* __restrict__ out,
     const int* __restrict__ block_table, int max_pages, const int* __restrict__ cu_tokens, const int* __restrict__ seq_lens, int first_req, int page_shift,
     int window, int pool, int pool_rows, int most_blocks) {
     PDL_ENTER();
@@ -442,18 +462,18 @@ __global__ void __launch_bounds__(VALUE_THREADS) value_kernel(
     // block b of the CTA as a tile's own block (negative: the tile has no such block)
     auto block_of = [&](int b, int tile) {
         if (tile * NQ >= here) return -1;
-        const Blocks& o = own[tile];
-        if (all.is_pooled(b)) return b < o.pooled ? b : -1;
-        const int at = all.first + b - all.pooled - o.first;
-        return at >= 0 && at < o.count - o.pooled ? o.pooled + at : -1;
+        const int o_pooled = tile == 0 ? own[0].pooled : own[1].pooled, o_first = tile == 0 ? own[0].first : own[1].first;
+        if (all.is_pooled(b)) return b < o_pooled ? b : -1;
+        const int at = all.first + b - all.pooled - o_first, o_count = tile == 0 ? own[0].count : own[1].count;
+        return at >= 0 && at < o_count - o_pooled ? o_pooled + at : -1;
     };
-    const bf16* src = mixed + (size_t)(first_tile(cu_tokens, first_req, r) + qt) * most_blocks * (NH * NQ * NK) + (size_t)kh * G * NQ * NK;
+    const __half* src = mixed + (size_t)(first_tile(cu_tokens, first_req, r) + qt) * most_blocks * (NH * NQ * NK) + (size_t)kh * G * NQ * NK;
     const size_t per_tile = (size_t)most_blocks * (NH * NQ * NK);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tile = warp / G;
     auto fetch = [&](int b) {
         if (b < all.count) {
-            bf16* sA = reinterpret_cast<bf16*>(smem_raw + (b % V_STAGES) * V_STAGE_BYTES);
-            bf16* sV = sA + VT * A_TILE;
+            __half* sA = reinterpret_cast<__half*>(smem_raw + (b % V_STAGES) * V_STAGE_BYTES);
+            bf16* sV = reinterpret_cast<bf16*>(sA + VT * A_TILE);
             constexpr int PER_TILE = G * NQ * (NK / 8);
 #pragma unroll
             for (int t = 0; t < VT; ++t) {
@@ -478,6 +498,7 @@ __global__ void __launch_bounds__(VALUE_THREADS) value_kernel(
     };
 #pragma unroll
     for (int b = 0; b < V_STAGES - 1; ++b) fetch(b);
+    const float down = two_to(-mixed_shift(talk, lane));
     float o[DV / 8][4];
 #pragma unroll
     for (int i = 0; i < DV / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
@@ -486,19 +507,26 @@ __global__ void __launch_bounds__(VALUE_THREADS) value_kernel(
         __syncthreads();                                       // block b is there, and everyone is done with the stage that is filled next
         fetch(b + V_STAGES - 1);
         if (block_of(b, tile) < 0) continue;
-        const bf16* sA = reinterpret_cast<const bf16*>(smem_raw + (b % V_STAGES) * V_STAGE_BYTES);
+        const __half* sA = reinterpret_cast<const __half*>(smem_raw + (b % V_STAGES) * V_STAGE_BYTES);
         const uint32_t a_addr = (uint32_t)__cvta_generic_to_shared(sA + (warp * NQ + (lane & 7) + ((lane >> 3) & 1) * 8) * A_PITCH + (lane >> 4) * 8);
         const uint32_t v_addr = (uint32_t)__cvta_generic_to_shared(sA + VT * A_TILE + ((lane & 7) + ((lane >> 3) & 1) * 8) * LDV + (lane >> 4) * 8);
 #pragma unroll
         for (int ks = 0; ks < NK / 16; ++ks) {
-            uint32_t a[4];
+            uint32_t a[4], hi[4], lo[4];
             ldsm_x4(a_addr + ks * 32, a[0], a[1], a[2], a[3]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {                      // 11 bits as two bf16 numbers, exactly
+                const float2 w = __half22float2(*reinterpret_cast<const __half2*>(&a[i]));
+                split_bf16(w.x * down, w.y * down, hi[i], lo[i]);
+            }
 #pragma unroll
             for (int dt = 0; dt < DV / 8; dt += 2) {
                 uint32_t b0, b1, b2, b3;
                 ldsm_x4_trans(v_addr + (uint32_t)(ks * 16 * LDV * 2 + dt * 16), b0, b1, b2, b3);
-                mma_bf16_16816(o[dt], a, b0, b1);
-                mma_bf16_16816(o[dt + 1], a, b2, b3);
+                mma_bf16_16816(o[dt], hi, b0, b1);
+                mma_bf16_16816(o[dt + 1], hi, b2, b3);
+                mma_bf16_16816(o[dt], lo, b0, b1);
+                mma_bf16_16816(o[dt + 1], lo, b2, b3);
             }
         }
     }
@@ -520,7 +548,7 @@ static int page_shift_of(int page_size) {
 }
 
 // Requests first_req .. first_req + count - 1 of the step; which: 0 the rows' sums (lse float32 [tokens][H]), 1 the mixed weights, 2 the results (in this
-// order).  mixed: bf16, (tokens / 16 + count) tiles of most_blocks blocks of H * 512; most_blocks: at least the blocks of 32 any tile of the step has.
+// order).  mixed: halves, (tokens / 16 + count) tiles of most_blocks blocks of H * 512; most_blocks: at least the blocks of 32 any tile of the step has.
 // q, caches, out and mixed 16-byte aligned.
 MB_API int mb_attn_pooled_mix(int which, const void* q, const void* k_cache, const void* v_cache, const void* k_pool, const void* v_pool, float* lse,
                               const float* talk, void* mixed, void* out, const int* block_table, int max_pages, const int* cu_tokens, const int* seq_lens,
@@ -540,9 +568,9 @@ MB_API int mb_attn_pooled_mix(int which, const void* q, const void* k_cache, con
     if (which == 1) {
         cudaFuncSetAttribute(mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MIX_SMEM);
         return launch_kernel(mix_kernel, dim3(tiles_of, 1, count), MIX_THREADS, MIX_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache, (const bf16*)k_pool, (const float*)lse, talk,
-                             (bf16*)mixed, block_table, max_pages, cu_tokens, seq_lens, first_req, shift, scale, cap, window, pool, pool_rows, most_blocks);
+                             (__half*)mixed, block_table, max_pages, cu_tokens, seq_lens, first_req, shift, scale, cap, window, pool, pool_rows, most_blocks);
     }
     cudaFuncSetAttribute(value_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VALUE_SMEM);
-    return launch_kernel(value_kernel, dim3((tiles_of + VT - 1) / VT, KH, count), VALUE_THREADS, VALUE_SMEM, s, 0, (const bf16*)mixed, (const bf16*)v_cache, (const bf16*)v_pool, (bf16*)out, block_table,
+    return launch_kernel(value_kernel, dim3((tiles_of + VT - 1) / VT, KH, count), VALUE_THREADS, VALUE_SMEM, s, 0, (const __half*)mixed, talk, (const bf16*)v_cache, (const bf16*)v_pool, (bf16*)out, block_table,
                          max_pages, cu_tokens, seq_lens, first_req, shift, window, pool, pool_rows, most_blocks);
 }

@@ -2138,7 +2138,7 @@ def _pooled_mix(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table, H: i
     nd, T, ws = ctx.num_decode, q.shape[0], ctx.workspace
     count = ctx.num_requests - nd
     lse = ws.get("pooled_lse", (T, H), torch.float32)
-    mixed = ws.get("pooled_mixed", (((T - nd) // 16 + count) * blocks * H * 512,), q.dtype)
+    mixed = ws.get("pooled_mixed", (((T - nd) // 16 + count) * blocks * H * 512,), torch.float16)
     lib = build.load(_pooled_mix_name(d, dv, H, K), *_pooled_mix_job(d, dv, H, K))
     args = (_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(k_pool), _ptr(v_pool), _ptr(lse), _ptr(talk), _ptr(mixed), _ptr(out), _ptr(block_table),
             _c_int(block_table.shape[1]), _ptr(ctx.cu_tokens), _ptr(ctx.seq_lens), _c_int(nd), _c_int(count), _c_int(ctx.max_query_len),

@@ -270,6 +270,44 @@ def test_weights_mixed_ahead_of_the_values(monkeypatch, m):
     ops.check_device_errors()
 
 
+@pytest.mark.parametrize("gain", [1.0, 2.0 ** -12, 300.0])
+def test_mixed_weights_are_held_to_more_bits_than_the_results(gain):
+    """The attention's rows against float64 from the same queries, keys, values and pooled rows: they are off by the rounding of the result to bf16 (relative
+    2^-9 at most a number) and by little else.  A mixed weight of 11 bits adds at most an eighth of that, in squares 1/64; the pairs of bf16 numbers that weights and
+    matrix are mixed as, the cap and the exponentials less than 1e-4: 1.15 in all leaves room.  (Weights of 8 bits made it 1.17.)"""
+    from marin_b200.engine import StepEntry
+    from marin_b200.kernels import ops
+
+    H, K, d, window, pool, page = 32, 8, 128, 70, 8, 16
+    m = _attn(H, K, d, d, 0.09, size=window, pool=pool, rot={"base": 10000.0, "dims": 32}, softcap=30.0)
+    rt, hidden, T = runtime("bfloat16"), 48, 400
+    w = attention_weights(hidden, m, 35)
+    w["m.mix.talk"] = bf(gain * w["m.mix.talk"].float())
+    part = build_mixer("attention", m, hidden, 1e-5, rt, w)
+    runner = harness([part.cache_need()], rt, page=page)
+    runner.begin("r")
+    runner.cache.reserve("r", T)
+    ctx = runner.build_context([StepEntry("r", [0] * T, [])])
+    view = runner.views.view(0, ctx)
+    part.forward(bf(torch.randn(T, hidden, generator=torch.Generator().manual_seed(36))).to(DEV), ctx, view, torch.zeros(T, hidden, device=DEV))
+    ops.check_device_errors()
+    q = ctx.workspace.get("q", (T, H * d), torch.bfloat16).view(T, K, H // K, d).double()
+    got = ctx.workspace.get("attn_out", (T, H * d), torch.bfloat16).view(T, H, d).double()
+    table, at = torch.tensor(runner.cache.block_table("r", 0), device=DEV), torch.arange(T, device=DEV)
+    ends = torch.arange(T // pool, device=DEV) * pool + pool - 1
+    rows = lambda one, pooled: torch.cat([one[table[at // page], :, at % page], pooled[table[ends // page], :, ends % page // pool]]).double()
+    keys, values = rows(view.k, view.k_pool), rows(view.v, view.v_pool)
+    far = at[:, None] - at[None, :]
+    seen = torch.cat([(far >= 0) & (far < window), ends[None, :] <= at[:, None] - window], dim=1)
+    s = torch.einsum("nkgd,mkd->kgnm", q, keys).reshape(H, T, -1) * 0.09
+    p = (30.0 * torch.tanh(s / 30.0)).masked_fill(~seen, -math.inf).softmax(dim=-1)
+    p = torch.einsum("hg,gnm->hnm", part.talk_w.double(), p).view(K, H // K, T, -1)
+    want = torch.einsum("kgnm,mkd->nkgd", p, values).reshape(T, H, d)
+    rms = lambda x: float(x.pow(2).mean().sqrt())
+    assert rms(got - want) <= 1.15 * rms(want.to(torch.bfloat16).double() - want)
+    runner.end("r")
+
+
 def test_rows_that_the_window_has_passed_are_another_requests():
     """A window without pooled blocks, portions behind it long enough for the kernels that mix the weights ahead of the values: the pages ahead of the
     window are given back, and their places in the block table read as page 0, here another request's, whose numbers are large, infinite or not
