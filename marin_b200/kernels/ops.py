@@ -2486,13 +2486,22 @@ def delta_chunked_supported(dtype, d: int, dv: int) -> bool:
     return dtype == torch.bfloat16 and d % 16 == 0 and 16 <= d <= 128 and dv % 16 == 0 and prepared <= 227 * 1024
 
 
-def _delta_slice(dv: int) -> int:
-    """Value channels a CTA of the walk takes (its columns of the state are independent of the others)."""
-    return 64 if dv % 64 == 0 else 32 if dv % 32 == 0 else 16
+#: up to this many CTAs of 64 value channels (half of the SMs, so that twice as many still are one round) the walk takes 32 a CTA: a chunk then has half the products
+#: and, with SMs idle, nothing costs more.  A whole mixer over one prompt of 2,048 tokens, 20 heads of 128 x 128, a decay per head: 64 channels 408 us, 32 367; 16
+#: heads 291 and 251, two prompts 265 and 240; beyond, three prompts and 20 heads (120 CTAs) 304 and 308, four and 16 (128) 215 and 219
+DELTA_NARROW_UP_TO = 74
 
 
-def _delta_chunked_job(d: int, dv: int) -> tuple:
-    return (["delta_rule_chunked.cu"], [f"QK_DIM={d}", f"V_SLICE={_delta_slice(dv)}"])
+def _delta_slice(dv: int, walks: int = 1 << 30) -> int:
+    """Value channels a CTA of the walk takes (its columns of the state are independent of the others) with so many requests and heads to walk."""
+    if dv % 64 == 0:
+        return 32 if walks * (dv // 64) <= DELTA_NARROW_UP_TO else 64
+    return 32 if dv % 32 == 0 else 16
+
+
+def _delta_chunked_lib(d: int, slice: int):
+    """Name and job of the chunked kernels with this many value channels a CTA of the walk."""
+    return f"mb_delta_rule_chunked_d{d}_v{slice}", (["delta_rule_chunked.cu"], [f"QK_DIM={d}", f"V_SLICE={slice}"])
 
 
 def delta_chunked_finishes(gate: torch.Tensor, norm_w: torch.Tensor, out: torch.Tensor, dv: int) -> bool:
@@ -2533,7 +2542,8 @@ def delta_chunked(qkv: torch.Tensor, inp: DeltaInputs, state: torch.Tensor, ctx,
     chunks = rows // 64 + R                               # at most: room for a partial chunk per request
     planes = ctx.workspace.get("delta_planes", (chunks * H, _delta_plane_numbers(d, dv)), torch.bfloat16)
     floats = ctx.workspace.get("delta_floats", (chunks * H, 64 * dv + d), torch.float32)
-    lib = build.load(f"mb_delta_rule_chunked_d{d}_v{_delta_slice(dv)}", *_delta_chunked_job(d, dv))
+    name, job = _delta_chunked_lib(d, _delta_slice(dv, R * H))
+    lib = build.load(name, *job)
     scratch = float(rows) / 64 * H * delta_chunk_bytes(d, dv)
     handed = float(rows) * H * dv * (2 * d / 16 + 4)            # the states and U
     for which, what in ((0, "delta rule (chunks prepared)"), (1, "delta rule (chunks walked)"), (2, "delta rule (chunks read)")):
@@ -2553,7 +2563,7 @@ def delta_rule_jobs(dtype, d: int, dv: int) -> dict:
     chunked tensor-core kernels for prompt portions."""
     jobs = library_jobs("mb_delta_rule")
     if use_chunked_delta_rule and delta_chunked_supported(dtype, d, dv):
-        jobs[f"mb_delta_rule_chunked_d{d}_v{_delta_slice(dv)}"] = _delta_chunked_job(d, dv)
+        jobs.update(_delta_chunked_lib(d, slice) for slice in {_delta_slice(dv), _delta_slice(dv, 1)})
     return jobs
 
 

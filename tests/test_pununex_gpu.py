@@ -262,6 +262,26 @@ def test_chunks_of_every_slice_and_their_norm(d, dv, per_channel):
     runner.end("r")
 
 
+@pytest.mark.parametrize("d,dv", [(128, 128), (48, 64)])
+def test_walks_of_32_and_64_value_channels_have_the_same_bits(monkeypatch, d, dv):
+    """A state's columns are independent and 16 of them are worked out alike in both: the same outputs and states, whole and partial chunks."""
+    from marin_b200.kernels import ops
+
+    H, G, T = 6, 2, 300
+    g = torch.Generator().manual_seed(d)
+    q, k = (bf(torch.randn(T, G, d, generator=g)) for _ in range(2))
+    v, beta_raw, a_raw = bf(torch.randn(T, H, dv, generator=g)), bf(2.0 * torch.randn(T, H, generator=g)), bf(torch.randn(T, H * d, generator=g))
+    rate, dt_bias = torch.randn(H, generator=g) * 0.3, torch.randn(H * d, generator=g) * 0.5 - 2.0
+    start = 0.3 * torch.randn(4, H, d, dv, generator=g)
+    results = []
+    for most, width in ((0, 64), (1 << 20, 32)):
+        monkeypatch.setattr(ops, "DELTA_NARROW_UP_TO", most)
+        assert ops._delta_slice(dv, H) == width
+        state = start.to(DEV)
+        results.append((recurrence(q, k, v, beta_raw, a_raw, rate, dt_bias, state, [129, 171], H, G, d, dv, True), state))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
 @pytest.mark.parametrize("chunked", [False, True], ids=["scan", "chunked"])
 @pytest.mark.parametrize("per_channel", [False, True], ids=["head", "channel"])
 @pytest.mark.parametrize("strength", [0.002, 0.3, 4.0, 60.0])
