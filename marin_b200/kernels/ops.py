@@ -766,7 +766,8 @@ def _attention_cost(q, rows: int, H: int, K: int, d: int, which: str) -> None:
 
 #: 32-bit prompt portions go to the tile kernel (False: the plain kernel takes every row)
 use_attention_tiles = True
-#: ... when the step's longest portion has at least this many tokens (a tile's 32 rows are then at least a quarter full for two heads a kv head)
+#: ... when the step's longest portion has at least this many tokens (a tile's 32 rows are then at least a quarter full for two heads a kv head; a layer of 16 heads
+#: over 8, four tokens behind 60, 500 and 4,000 cached ones: 178, 252 and 892 us, by the plain kernel 175, 290 and 1,825)
 ATTENTION_TILES_FROM = 4
 
 
@@ -1154,7 +1155,8 @@ def linear_attention_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, 
 
 #: bf16 prompt portions of time mixing go 64 tokens at a time through the tensor-core kernels (False: the walk token by token)
 use_chunked_wkv = True
-#: ... when the step's longest portion has more tokens than this (a walk takes about 1.3 us a token, the three kernels some 20 us however few there are)
+#: ... when the step's longest portion has more tokens than this (a walk takes about 1.3 us a token, the three kernels some 20 us however few there are; a whole mixer
+#: of 40 heads of 64 over 17, 32 and 64 tokens: 157, 146 and 146 us, by the walk 168, 155 and 156)
 WKV_CHUNKED_FROM = 16
 
 
@@ -1866,26 +1868,25 @@ def moe_jobs(dtype, h: int, ff: int) -> dict:
     return library_jobs("mb_moe", "mb_moe_tc") if dtype == torch.bfloat16 and fast_experts_supported(h, ff) else library_jobs("mb_moe")
 
 
-#: from this many (token, choice) pairs on, the experts' products go to the persistent tcgen05 kernel; below, to the grouped mma.sync kernel,
-#: whose smaller tiles put more CTAs on the few experts that are read
-EXPERTS_TC_FROM = 1
-
-
 #: the capped form runs behind the plain product, whose rows are bf16: only with many pairs an expert (the mma.sync kernel applies it to its float32 sums)
 EXPERTS_CAPPED_TC_FROM = 96
 
 
 def _experts_on_tcgen05(E: int, pairs: int, interleaved: bool, activation: str) -> bool:
-    """Whether the grouped tcgen05 products take these experts (up to 512; a gated form that its epilogue applies needs gate and up rows in alternating
-    blocks)."""
+    """Whether the grouped tcgen05 products take these experts, from one token on (a whole call, 8 experts of 2,560 x 3,648, two chosen, a shared one of 2,432: 1, 4,
+    8, 16 tokens 88, 94, 104, 117 us, by mma.sync 141, 112, 140, 143; 64 of 1,024, four chosen: 76, 122, 145, 174 and 110, 125, 167, 219; 128 of 2,048 x 768,
+    eight chosen, one token: 120 and 117).  The mma.sync kernel keeps more than 512 experts, a gated form whose gate and up rows do not alternate, and the
+    capped form with few pairs an expert or in a step that is being captured, where its float32 sums are what earlier captured steps had."""
     if activation == "glu_capped" and (pairs < EXPERTS_CAPPED_TC_FROM * E or torch.cuda.is_current_stream_capturing()):
         return False
-    return use_tensor_cores and E <= 512 and pairs >= EXPERTS_TC_FROM and (interleaved or activation != "swiglu")
+    return use_tensor_cores and E <= 512 and (interleaved or activation != "swiglu")
 
 
 def _expert_tile(pairs: int, E: int) -> int:
     """The widest tile of rows, from the experts' average share: one tile holds an ordinary expert's rows while the rows are few (its weights are then
-    read once, and a small tile leaves room for a deep ring); equal tiles of at most 256 beyond."""
+    read once, and a small tile leaves room for a deep ring); equal tiles of at most 256 beyond.  A whole call, 8 experts of 2,560 x 3,648, two chosen, a shared one
+    of 2,432, by tiles of 32, 64, 128 and 256: shares of 12 rows 118, 122, 123, 128 us; 20 125, 123, 127, 133; 25 140, 126, 129, 134; 44 199, 136, 131, 143;
+    64 236, 175, 129, 140; 100 335, 233, 155, 148."""
     average = pairs / E
     return 32 if average <= 20 else 64 if average <= 44 else 128 if average <= 100 else 256
 

@@ -155,6 +155,13 @@ def test_products_side_by_side_have_each_products_results(ops, G, T, N, K):
     ops.check_device_errors()
     want = x.double() @ w.double().transpose(1, 2)
     torch.testing.assert_close(out.double(), want, rtol=2.0 ** -8, atol=1e-4)
+    ops.use_side_by_side = False                                # one after the other: sums in another kernel's order, a bf16 step at most where they round apart
+    try:
+        single = torch.empty_like(out)
+        ops.gemm_side_by_side(x, w, single)
+    finally:
+        ops.use_side_by_side = True
+    torch.testing.assert_close(out.float(), single.float(), rtol=2.0 ** -7, atol=1e-4)
     assert bool((guard[0] == 7.0).all()) and bool((guard[G * T + 1] == 7.0).all())
 
 
@@ -573,6 +580,40 @@ def test_qkv_product_finishes_its_heads(ops, T, H, K, hidden, norm, rope, write)
     torch.testing.assert_close(caches[1].float(), caches[3].float(), **tol)
     if write:
         assert float(caches[0].float().abs().sum()) > 0 and float(caches[1].float().abs().sum()) > 0
+
+
+@pytest.mark.parametrize("H,K,T,width", [(5, 1, 1500, 256), (5, 3, 1000, 160), (1, 1, 3300, 224), (7, 1, 1100, 128)])
+def test_heads_finished_by_pairs_of_sms_have_the_same_bits(ops, monkeypatch, H, K, T, width):
+    """An odd number of heads leaves the last pair's second SM without one (its 128 weight rows lie past the last): queries, keys and values bit for bit, and
+    what lies around them untouched."""
+    from marin_b200.engine.context import Workspace
+
+    d, page, hidden = 128, 16, 320
+    g = torch.Generator(device=DEV).manual_seed(T)
+    n = (H + 2 * K) * d
+    x = torch.randn(T, hidden, device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(n, hidden, device=DEV, generator=g) / math.sqrt(hidden)).to(torch.bfloat16)
+    qw, kw = (1 + 0.1 * torch.randn(d, device=DEV, generator=g) for _ in range(2))
+    positions = torch.randint(0, 4000, (T,), device=DEV, generator=g, dtype=torch.int32)
+    inv_freq = torch.pow(torch.tensor(1e6), -(torch.arange(d // 2, dtype=torch.float32) * 2.0 / d)).to(DEV)
+    pages = T // page + 3
+    slots = torch.randperm(pages * page, device=DEV, generator=g)[:T].to(torch.int32)
+    monkeypatch.setattr(ops, "PAIRS_FROM", 0)
+    monkeypatch.setattr(ops, "_paired_width", lambda T, N: -width)
+    monkeypatch.setattr(ops, "persistent_plan", lambda T, N: width)
+    results = []
+    for pairs in (True, False):
+        monkeypatch.setattr(ops, "pair_tiles", pairs)
+        assert ops.paired_plan(T, n, hidden) == (-width if pairs else width)
+        step = SimpleNamespace(extras={}, workspace=Workspace(DEV))
+        q = torch.full((T + 2, H * d), 7.0, device=DEV, dtype=torch.bfloat16)
+        caches = [torch.full((pages, K, page, d), 7.0, device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+        assert ops.gemm_qkv_heads(x, w, q[1:T + 1], qw, kw, 1e-6, positions, inv_freq, d, False, slots, *caches, H, K, d, True, step)
+        ops.check_device_errors()
+        results.append([q, *caches])
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    assert bool((results[0][0][[0, T + 1]] == 7.0).all()) and int((results[0][0] != 7.0).sum()) > T * H * d * 0.9
 
 
 def test_qkv_product_declines_what_it_cannot_finish(ops):
