@@ -2052,8 +2052,9 @@ def attention_pooled(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table,
     rows = -(-page_size // pool) if pool else 0
     if talk is not None and ctx.num_requests > ctx.num_decode:
         blocks = _pooled_mix_blocks(ctx, window, pool)
-        if (use_pooled_mix and pooled_mix_supported(q.dtype, H, K, d, dv) and page_size & (page_size - 1) == 0 and blocks * 32 <= 2 * K * dv
-                and ctx.max_query_len >= POOLED_MIX_FROM and scale > 0 and all(t is None or t.data_ptr() % 16 == 0 for t in (q, k_cache, v_cache, k_pool, v_pool, out))):
+        if (use_pooled_mix and pooled_mix_supported(q.dtype, H, K, d, dv) and page_size & (page_size - 1) == 0 and scale > 0
+                and _pooled_mix_pays(T - ctx.num_decode, ctx.num_requests - ctx.num_decode, ctx.max_query_len, blocks, K, dv)
+                and all(t is None or t.data_ptr() % 16 == 0 for t in (q, k_cache, v_cache, k_pool, v_pool, out))):
             _pooled_mix(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table, H, K, d, dv, scale, softcap or 0.0, window, pool, rows, talk, blocks)
             if ctx.num_decode == 0:
                 return
@@ -2093,8 +2094,25 @@ def attention_pooled(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table,
 #: prompt portions with mixed head weights go to the kernels that mix the weights ahead of the values (False: every head's sums over every kv head's values,
 #: mixed afterwards)
 use_pooled_mix = True
-#: ... when the step's longest portion fills at least one tile of queries
-POOLED_MIX_FROM = 16
+#: ... where that costs less, in us on B200 with 32 heads of 128 over 8: this way a block of 32 keys of the longest tile (a tile of 16 queries walks its keys in one
+#: CTA), the other way a token (its sums written and mixed) and a token's block.  Whole mixers, this way and the other: one portion behind 2,000 positions, window
+#: 1,024, pools of 64, 256, 384, 512 and 2,048 tokens 386, 403, 429 and 640 against 300, 406, 539 and 1,723; window 512 247, 258, 277 and 439 against 223, 289,
+#: 383 and 1,175; nothing before them, one portion of 192, 320 and 512 tokens 124, 163 and 240 against 128, 172 and 275, four of 80 115 against 153
+POOLED_MIX_COSTS = (9.0, 0.17, 0.022)
+
+
+def _pooled_mix_tiles(tokens: int, portions: int) -> int:
+    """Tiles of 16 queries that ``tokens`` of so many portions have room for (a partial one each)."""
+    return tokens // 16 + portions
+
+
+def _pooled_mix_pays(tokens: int, portions: int, longest: int, blocks: int, K: int, dv: int) -> bool:
+    """Whether portions of so many tokens (in all) go to the kernels that mix the weights first: a portion that fills a tile, enough tokens for their ``blocks`` (with
+    2, 10, 19 and 35 of them from 84, 231, 291 and 335 tokens on), and mixed weights (H x 16 x 32 numbers of 16 bits a tile and block) that take no more
+    memory than the heads' sums would (H x K x dv of 32 bits a token), which is what a step's working memory is planned with.  By that a window of
+    1,024 passes with 8 kv heads of 128, one of 2,048 or none over more than 2,000 positions does not."""
+    block, token, both = POOLED_MIX_COSTS
+    return longest >= 16 and block * blocks <= tokens * (token + both * blocks) and _pooled_mix_tiles(tokens, portions) * blocks * 256 <= tokens * K * dv
 
 
 def pooled_mix_supported(dtype, H: int, K: int, d: int, dv: int) -> bool:
@@ -2139,7 +2157,8 @@ def _pooled_mix(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table, H: i
     nd, T, ws = ctx.num_decode, q.shape[0], ctx.workspace
     count = ctx.num_requests - nd
     lse = ws.get("pooled_lse", (T, H), torch.float32)
-    mixed = ws.get("pooled_mixed", (((T - nd) // 16 + count) * blocks * H * 512,), torch.float16)
+    # (in the place of the heads' sums of another step: 16-bit numbers of which there are never more bytes, _pooled_mix_pays)
+    mixed = ws.get("pooled_parts", (_pooled_mix_tiles(T - nd, count) * blocks * H * 256,), torch.float32)
     lib = build.load(_pooled_mix_name(d, dv, H, K), *_pooled_mix_job(d, dv, H, K))
     args = (_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(k_pool), _ptr(v_pool), _ptr(lse), _ptr(talk), _ptr(mixed), _ptr(out), _ptr(block_table),
             _c_int(block_table.shape[1]), _ptr(ctx.cu_tokens), _ptr(ctx.seq_lens), _c_int(nd), _c_int(count), _c_int(ctx.max_query_len),

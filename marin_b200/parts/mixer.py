@@ -809,8 +809,8 @@ class PooledAttention(Mixer):
 
     def workspace_per_token(self, dtype) -> int:
         """Bytes a step keeps per token beside the products' rows: with mixed weights, every head's float32 sum over every kv
-        head's values."""
-        return 4 * self.heads * self.kv_heads * self.v_head_dim if self.talk else 0
+        head's values (or, in their place and never more, the mixed weights) and the logarithm of its weights' sum."""
+        return 4 * self.heads * (self.kv_heads * self.v_head_dim + 1) if self.talk else 0
 
     def kernel_jobs(self, dtype) -> Dict[str, tuple]:
         return ops.pooled_attention_jobs(dtype, self.heads, self.kv_heads, self.head_dim, self.v_head_dim)

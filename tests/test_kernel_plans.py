@@ -50,3 +50,22 @@ def test_parts_of_the_experts_last_products_cost_less_than_the_round_they_save(E
             for k in (ff, shared_ff if shared_rows else 0):
                 n = k // 64
                 assert k == 0 or parts == 1 or (-(-n // parts) >= 8 and (parts - 1) * -(-n // parts) < n)
+
+
+@pytest.mark.parametrize("H,K,dv", [(32, 8, 128), (16, 8, 32), (16, 4, 48)])
+def test_mixed_weights_never_take_more_memory_than_the_heads_sums(H, K, dv):
+    """Where a step's portions go to the kernels that mix the weights first, those fit what the heads' sums of as many tokens would take (the working memory's
+    plan); few tokens for the keys they meet, and none that fills a tile of 16 queries, never go there."""
+    for tokens in (16, 84, 200, 400, 512, 2048, 8192):
+        for portions in (1, 2, 4, 19, 60):
+            for blocks in (1, 6, 18, 35, 64, 200):
+                longest = -(-tokens // portions)
+                if not ops._pooled_mix_pays(tokens, portions, longest, blocks, K, dv):
+                    continue
+                assert longest >= 16
+                tiles = sum(-(-n // 16) for n in [tokens // portions] * (portions - 1) + [tokens - tokens // portions * (portions - 1)])
+                assert tiles <= ops._pooled_mix_tiles(tokens, portions)
+                assert ops._pooled_mix_tiles(tokens, portions) * blocks * H * 16 * 32 * 2 <= tokens * H * K * dv * 4
+    assert ops._pooled_mix_pays(2048, 1, 2048, 35, 8, 128) and not ops._pooled_mix_pays(2048, 1, 2048, 64, 8, 128)
+    for blocks, few, many in ((2, 80, 90), (10, 224, 240), (35, 320, 352)):
+        assert not ops._pooled_mix_pays(few, 1, few, blocks, 8, 128) and ops._pooled_mix_pays(many, 1, many, blocks, 8, 128)

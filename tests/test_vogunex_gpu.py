@@ -239,6 +239,7 @@ def test_weights_mixed_ahead_of_the_values(monkeypatch, m):
     part = build_mixer("attention", m, hidden, 1e-5, rt, w)
     taken = []
     inner = ops._pooled_mix
+    monkeypatch.setattr(ops, "POOLED_MIX_COSTS", (0.0, 0.0, 0.0))
     monkeypatch.setattr(ops, "_pooled_mix", lambda *a: (taken.append(1), inner(*a))[1])
     for cuts in ([T], [16, 33, 1, 17, 83], [1, 64, 31, 54]):
         off = []
@@ -306,6 +307,32 @@ def test_mixed_weights_are_held_to_more_bits_than_the_results(gain):
     rms = lambda x: float(x.pow(2).mean().sqrt())
     assert rms(got - want) <= 1.15 * rms(want.to(torch.bfloat16).double() - want)
     runner.end("r")
+
+
+def test_both_ways_over_portions_share_their_memory(monkeypatch):
+    """What a step's portions keep, mixed ahead of the values or afterwards, one portion or many short ones, stays within what is planned per token."""
+    from marin_b200.engine import StepEntry
+    from marin_b200.kernels import ops
+
+    m = _attn(32, 8, 128, 128, 0.09, size=700, pool=8, softcap=30.0)
+    rt, hidden, T = runtime("bfloat16"), 48, 960
+    part = build_mixer("attention", m, hidden, 1e-5, rt, attention_weights(hidden, m, 37))
+    runner = harness([part.cache_need()], rt, page=16, pages=160)
+    x, taken, inner = bf(torch.randn(T, hidden, generator=torch.Generator().manual_seed(38))).to(DEV), [], ops._pooled_mix
+    monkeypatch.setattr(ops, "_pooled_mix", lambda *a: (taken.append(1), inner(*a))[1])
+    for lens, ahead, ways in (([T], True, 1), ([T], False, 1), ([900, 20, 20, 20], True, 2)):
+        monkeypatch.setattr(ops, "use_pooled_mix", ahead)
+        for i, n in enumerate(lens):
+            runner.begin(i)
+            runner.cache.reserve(i, n)
+        ctx = runner.build_context([StepEntry(i, [0] * n, []) for i, n in enumerate(lens)])
+        part.forward(x, ctx, runner.views.view(0, ctx), torch.zeros(T, hidden, device=DEV))
+        for i in range(len(lens)):
+            runner.end(i)
+        assert len(taken) == ways
+        held = sum(buf.nbytes for (name, _), buf in ctx.workspace._buffers.items() if name.startswith("pooled"))
+        assert held <= part.workspace_per_token(torch.bfloat16) * T
+    ops.check_device_errors()
 
 
 def test_rows_that_the_window_has_passed_are_another_requests():
