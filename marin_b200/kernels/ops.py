@@ -1873,9 +1873,9 @@ EXPERTS_CAPPED_TC_FROM = 96
 
 
 def _experts_on_tcgen05(E: int, pairs: int, interleaved: bool, activation: str) -> bool:
-    """Whether the grouped tcgen05 products take these experts, from one token on (a whole call, 8 experts of 2,560 x 3,648, two chosen, a shared one of 2,432: 1, 4,
-    8, 16 tokens 88, 94, 104, 117 us, by mma.sync 141, 112, 140, 143; 64 of 1,024, four chosen: 76, 122, 145, 174 and 110, 125, 167, 219; 128 of 2,048 x 768,
-    eight chosen, one token: 120 and 117).  The mma.sync kernel keeps more than 512 experts, a gated form whose gate and up rows do not alternate, and the
+    """Whether the grouped tcgen05 products take these experts, from one token on (a whole call replayed from a graph, 8 experts of 2,560 x 3,648, two
+    chosen, a shared one of 2,432: 1, 4, 8, 16 tokens 66, 93, 106, 114 us, by mma.sync 98, 119, 138, 140; 64 of 1,024, four chosen, 1, 4, 8: 94, 122, 140 and 107,
+    126, 164; 128 of 2,048 x 768, eight chosen, one token: 131 and 133).  The mma.sync kernel keeps more than 512 experts, a gated form whose gate and up rows do not alternate, and the
     capped form with few pairs an expert or in a step that is being captured, where its float32 sums are what earlier captured steps had."""
     if activation == "glu_capped" and (pairs < EXPERTS_CAPPED_TC_FROM * E or torch.cuda.is_current_stream_capturing()):
         return False
