@@ -1,7 +1,7 @@
 // Matrix product on the CUDA cores: out[t, n] = sum_k x[t, k] * w[n, k], float32 accumulate.  Every output is one fixed chain (or,
 // for few weight rows, a fixed number of chains added in order) of fused multiply-adds over increasing k that depends on N and K
-// alone, so a row's result does not depend on how many other rows the batch holds.  This is the whole 32-bit path's matrix product (no
-// tensor cores, no reduced-precision mode) and the plain twin the tensor-core kernel is tested against.  The reference's
+// alone, so a row's result does not depend on how many other rows the batch holds.  This is the 32-bit path's product where rows of K
+// numbers are not whole 16-byte units (gemm_f32.cu has the others) and the plain twin the tensor-core kernels are tested against.  The reference's
 // counterpart is its warp-per-row kernel (crates/cuda/src/kernels.cu:73-116).
 //
 // Bound by the multiply-adds (128 a clock and SM: 72 TFLOP/s at 1.9 GHz) and by shared memory: a 16-byte load of a warp takes four of its

@@ -149,6 +149,7 @@ def load(name: str, sources: Sequence[str], defines: Sequence[str] = ()) -> ctyp
 LIBRARIES: Dict[str, List[str]] = {
     "mb_elementwise": ["elementwise.cu"],
     "mb_gemm_simple": ["gemm_simple.cu"],
+    "mb_gemm_f32": ["gemm_f32.cu"],
     "mb_attention_simple": ["attention_simple.cu"],
     "mb_sampling": ["sampling.cu"],
     "mb_gemm_tc": ["gemm_tc.cu"],
@@ -256,6 +257,8 @@ def build_for(model, dtype, verbose: bool = True) -> List[str]:
 
     jobs = {"mb_elementwise": (LIBRARIES["mb_elementwise"], []), "mb_sampling": (LIBRARIES["mb_sampling"], []),
             "mb_gemm_simple": (LIBRARIES["mb_gemm_simple"], [])}
+    if dtype == torch.float32:
+        jobs["mb_gemm_f32"] = (LIBRARIES["mb_gemm_f32"], [])
     if dtype == torch.bfloat16:
         jobs["mb_gemm_tc"] = (LIBRARIES["mb_gemm_tc"], [])
     if hasattr(model, "kernel_jobs"):

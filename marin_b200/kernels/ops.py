@@ -438,6 +438,34 @@ def _persistent_product(x, w, out, mode: int, T: int, N: int, K: int, s, what: s
                                      _c_int(paired_plan(T, N, K)), _c_int(SM_COUNT), _ptr(s.error), _stream()), what)
 
 
+@functools.lru_cache(maxsize=4096)
+def f32_plan(T: int, N: int, K: int):
+    """Tokens a tile and CTAs a tile of the 32-bit product on the tensor cores (neither changes a bit of the result): the least rounds of CTAs over the SMs times
+    a CTA's clocks.  Measured on B200: a stage of 64 k 1,750 + 10 a token (3,200 at 128), up to 32 tokens 2,750, or 4,500 with two CTAs an SM; 4,000 to begin
+    and end; where a cluster adds its sums 3,000 and a clock for every 16 bytes of them that a CTA reads.  Clusters of eight find room for 112 CTAs at once, of
+    four for 132 (1,024 rows of 2,048 and 64 tokens: 16 clusters of eight 23.6 us, 8 of them 13.5)."""
+    groups = 8 if N <= F32_FEW_ROWS else 4
+    chunks = -(-K // 64)
+    per = -(-chunks // groups)
+    rows = -(-N // 128)
+    best = None
+    for width in (16, 32) if T <= 32 else (32, 48, 64, 80, 96, 112, 128):
+        for splits in (1, groups // 2, groups):
+            few = width <= 32
+            ctas = rows * -(-T // width) * splits
+            at_once = {8: 112, 4: 132}.get(splits, SM_COUNT)
+            stage = (2750 if ctas <= at_once else 4500) if few else 1750 + 10 * width + (170 if width > 112 else 0)
+            adding = 3000 + width * 128 * 4 * groups // splits // 16 if splits > 1 else 0
+            cost = -(-ctas // (at_once * (2 if few else 1))) * (min(chunks, per * groups // splits) * stage + 4000 + adding)
+            if best is None or cost < best[0]:
+                best = (cost, width, splits)
+    return best[1:]
+
+
+#: up to so many weight rows the 32-bit product cuts K into eight chains, beyond into four (gemm_f32.cu: GF_FEW_ROWS)
+F32_FEW_ROWS = 3072
+
+
 class NormOut:
     """An RMS norm that may ride on a ``+=`` product: ``rows`` (activation dtype ``[T, N]``) is where the normed
     rows are wanted, ``weight`` float32 ``[N]``."""
@@ -471,7 +499,8 @@ COUPLED_NORM_MAX_TOKENS = 16
 def gemm(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, then_norm: Optional[NormOut] = None,
          activation: Optional[str] = None):
     """``out[t, n] (+)= sum_k x[t, k] * w[n, k]``.  bfloat16 inputs run on the tensor cores (tcgen05, float32
-    accumulate); float32 inputs run on the CUDA cores in true float32.  ``activation`` "relu2": ``out = max(x w^T, 0)^2`` in
+    accumulate); float32 inputs too, every number as three bfloat16 ones, with the error of float32 sums (rows that are not whole 16-byte
+    units: on the CUDA cores).  ``activation`` "relu2": ``out = max(x w^T, 0)^2`` in
     the activation dtype, applied to the float32 sums in the tensor-core product's epilogue (as a kernel of its own behind
     the plain product).
 
@@ -536,6 +565,15 @@ def gemm(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, then_n
             _ptr(s.error), _stream()), "gemm (tensor cores, coupled with a norm)")
         return carried
     assert scaled is None, "rows with a pending norm reach only the tensor-core product"
+    if (use_tensor_cores and x.dtype == w.dtype == out.dtype == torch.float32 and K % 4 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
+        width, splits = f32_plan(T, N, K)
+        _check(_lib("mb_gemm_f32").mb_gemm_f32(_ptr(x), _ptr(w), _ptr(out), _c_int(T), _c_int(N), _c_int(K), _c_int(int(accumulate)), _c_int(width),
+                                               _c_int(splits), _ptr(_scratch_for(x.device).error), _stream()), "gemm (float32, tensor cores)")
+        if activation is not None:
+            if activation != "relu2" or accumulate:
+                raise KernelError(f"gemm: activation {activation!r} goes with a plain output")
+            relu2(out)
+        return None
     _check(_lib("mb_gemm_simple").mb_gemm_simple(_ptr(x), _code(x), _ptr(w), _code(w), _ptr(out), _code(out), _c_int(T),
                                                 _c_int(N), _c_int(K), _c_int(int(accumulate)), _stream()), "gemm")
     if activation is not None:

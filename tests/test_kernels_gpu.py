@@ -936,6 +936,69 @@ def test_float32_product_at_tile_edges(ops, T, N, K):
     assert torch.equal(added, out + out)
 
 
+@pytest.mark.parametrize("T,N,K", [(1, 1, 4), (16, 127, 60), (17, 129, 64), (33, 3072, 68), (113, 3073, 132), (129, 300, 260), (40, 640, 2052), (200, 128, 576)])
+def test_float32_product_on_tensor_cores(ops, monkeypatch, T, N, K):
+    """Every width and share of a tile gives the same bits, and they lie no further from 64 bits than a chain of multiply-adds does.  Bound: an accumulator drops
+    what lies below its last bit (2^-23 of it) at each of a stage's four large additions and at twenty of numbers 2^-8 as large; then the
+    stages' and the groups' additions round, at most K / 64 + 8 times 2^-24; what no product is made of is below 2^-25."""
+    g = torch.Generator().manual_seed(T + N + K)
+    x, w = torch.randn(T, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    want, scale = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    first = None
+    groups = 8 if N <= ops.F32_FEW_ROWS else 4
+    for width, splits in [(width, splits) for width in (16, 32, 48, 112, 128) for splits in (1, groups // 2, groups)]:
+        monkeypatch.setattr(ops, "f32_plan", lambda *a: (width, splits))
+        out = torch.full((T, N), math.nan, device=DEV)
+        ops.gemm(x, w, out)
+        first = out if first is None else first
+        assert torch.equal(out, first), (width, splits)
+        added = out.clone()
+        ops.gemm(x, w, added, accumulate=True)
+        assert torch.equal(added, out + out), (width, splits)
+    monkeypatch.undo()
+    assert float(((first - want).abs() / scale).max()) <= (5 + (K / 64 + 8) / 2) * 2.0 ** -23
+    chain = torch.empty_like(first)
+    monkeypatch.setattr(ops, "use_tensor_cores", False)
+    ops.gemm(x, w, chain)
+    if T * N > 1000:
+        assert float((first - want).norm()) <= 1.05 * float((chain - want).norm())
+    ops.check_device_errors()
+
+
+def test_float32_product_of_numbers_that_do_not_split(ops, monkeypatch):
+    """Infinities, not-a-numbers, numbers above bf16's range and numbers too small for three parts: the plain chain's result for their rows (or one as near to 64
+    bits), and the other rows' bits as if they were not there."""
+    g = torch.Generator().manual_seed(3)
+    T, N, K = 70, 200, 192
+    x, w = torch.randn(T, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    clean = torch.empty(T, N, device=DEV)
+    ops.gemm(x, w, clean)
+    rows = [3, 4, 5, 6, 8, 31]
+    x[3, 5], x[4, 7], x[6, 1] = math.inf, math.nan, 3.4e38
+    x[5] *= 1e-38
+    x[8] = 1e-41
+    x[31, 60] = 1e-39
+    w[9, 3], w[10] = -math.inf, w[10] * 1e-36
+    x[7] = 0.0
+    want, scale = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    chain = torch.empty_like(clean)
+    monkeypatch.setattr(ops, "use_tensor_cores", False)
+    ops.gemm(x, w, chain)
+    monkeypatch.undo()
+    for plan in [(16, 1), (32, 8), (64, 1), (128, 4), (128, 8)]:
+        monkeypatch.setattr(ops, "f32_plan", lambda *a: plan)
+        out = torch.full((T, N), 7.0, device=DEV)
+        ops.gemm(x, w, out)
+        finite = torch.isfinite(chain)
+        assert torch.equal(torch.isnan(out), torch.isnan(chain)) and torch.equal(torch.isposinf(out), torch.isposinf(chain)) and torch.equal(torch.isneginf(out), torch.isneginf(chain))
+        assert bool(((out - want).abs()[finite] <= (2.0 ** -16 * scale + 2.0 ** -149 * K)[finite]).all())      # (a chain of 192 roundings, and of the smallest numbers)
+        assert bool((out[7][finite[7]] == 0.0).all())
+        whole = [t for t in range(T) if t not in rows + [7]]
+        assert torch.equal(out[whole][:, 128:], clean[whole][:, 128:])                  # (a tile of 128 weight rows goes together)
+        first = out if plan == (16, 1) else first
+        assert torch.equal(torch.nan_to_num(out, 5.0), torch.nan_to_num(first, 5.0))
+
+
 @pytest.mark.parametrize("activation,form", [("swiglu", None), ("relu2", None), ("glu_capped", (2.0, 1.5, 1.0))])
 @pytest.mark.parametrize("counts,h,ff,shared_ff", [((1,), 64, 64, 0), ((0, 16, 17, 0, 33, 1), 128, 192, 64), ((300, 0, 257, 256, 40), 192, 320, 128),
                                                    ((64, 65, 31, 60), 320, 64, 192), ((2,) * 100, 64, 128, 0), ((540, 3), 128, 128, 64)])
