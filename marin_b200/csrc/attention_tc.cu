@@ -167,12 +167,13 @@ __device__ __forceinline__ void mbar_arrive_one(uint64_t* bar) {
 }
 
 // The MMA with its A operand in tensor memory (row m in lane m, two bf16 per 32-bit column) and B in shared memory.
-__device__ __forceinline__ void umma_bf16_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_bf16_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t elected) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected)
         : "memory");
 }
 
@@ -303,6 +304,7 @@ __global__ void __launch_bounds__(256, 2) attn_prefill_tc_kernel(
         return j < kept ? j : kb_first + j - kept;
     };
 
+    const int role = warp_same(warp);
     if (warp == 5 || (warp == 6 && !TA_V_IN_K)) {
         // ---- the loader warps: warp 5 asks for Q once and then for every block of K, warp 6 for every block of V, each
         // as soon as the block's buffer is free.  Lanes 0..3 each ask for one box of a block, so that one instruction
@@ -365,83 +367,60 @@ __global__ void __launch_bounds__(256, 2) attn_prefill_tc_kernel(
                 ok = __all_sync(0xffffffffu, ok);
             }
         }
-    } else if (warp == 4) {
-        // ---- the issuer of S: one lane issues S(i) = Q K(i)^T as soon as the block's keys have landed and P V of block
-        // i - 2 is done (S(i) goes where P(i - 2) lies).  Issuing an MMA costs the thread over a hundred cycles, and a
-        // block has twelve: one thread for all of them set the kernel's pace (1,600 of a block's 1,620 cycles busy), so
-        // S and P V have an issuer each. ----
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TA_BN >> 3) << 17) | ((uint32_t)(TA_BM >> 4) << 24);
-            const uint32_t sq = smem_u32(sQ);
-            uint64_t qdesc[D / 16], kdesc[2][D / 16];
+    } else if (role == 4) {
+        // ---- the issuer of S: one warp issues S(i) = Q K(i)^T as soon as the block's keys have landed and P V of block
+        // i - 2 is done (S(i) goes where P(i - 2) lies).  S and P V have an issuer each: neither's MMAs wait
+        // behind the other's barriers. ----
+        constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TA_BN >> 3) << 17) | ((uint32_t)(TA_BM >> 4) << 24);
+        const uint32_t elected = elect_one(), tmem_s = warp_same(tmem_base);
+        const int blocks = warp_same(nblk);
+        bool ok = __all_sync(0xffffffffu, wait_or_abort(q_full, 0, abort, error_flag, 21));
+        const long long start = TA_T();
+        long long m_idle = 0;
+        for (int i = 0; ok && i < blocks; ++i) {
+            const long long m_t0 = TA_T();
+            ok = __all_sync(0xffffffffu, wait_or_abort(&k_full[i & 1], (i >> 1) & 1, abort, error_flag, 29));
+            if (ok && i >= 2) ok = __all_sync(0xffffffffu, wait_or_abort(&v_free[i & 1], ((i - 2) >> 1) & 1, abort, error_flag, 29));
+            m_idle += TA_T() - m_t0;
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t qdesc = umma_desc(smem_u32(sQ)), kdesc = umma_desc(smem_u32(sKV + (size_t)(i & 1) * TA_BUF_BYTES));
 #pragma unroll
-            for (int kk = 0; kk < D / 16; ++kk) {
-                qdesc[kk] = umma_desc(sq + (kk / 4) * (TA_BM * 128)) + 2 * (kk % 4);
-#pragma unroll
-                for (int b = 0; b < 2; ++b)
-                    kdesc[b][kk] = umma_desc(smem_u32(sKV + (size_t)b * TA_BUF_BYTES) + (kk / 4) * (TA_BN * 128)) + 2 * (kk % 4);
-            }
-            bool ok = wait_or_abort(q_full, 0, abort, error_flag, 21);
-            const long long start = TA_T();
-            long long m_idle = 0;
-            for (int i = 0; ok && i < nblk; ++i) {
-                const long long m_t0 = TA_T();
-                ok = wait_or_abort(&k_full[i & 1], (i >> 1) & 1, abort, error_flag, 29);
-                if (ok && i >= 2) ok = wait_or_abort(&v_free[i & 1], ((i - 2) >> 1) & 1, abort, error_flag, 29);
-                m_idle += TA_T() - m_t0;
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (i & 1) {
-#pragma unroll
-                    for (int kk = 0; kk < D / 16; ++kk) umma_bf16(tmem_base + (uint32_t)TA_BN, qdesc[kk], kdesc[1][kk], idesc_s, kk > 0 ? 1u : 0u);
-                } else {
-#pragma unroll
-                    for (int kk = 0; kk < D / 16; ++kk) umma_bf16(tmem_base, qdesc[kk], kdesc[0][kk], idesc_s, kk > 0 ? 1u : 0u);
-                }
-                umma_commit(&s_done[i & 1]);
-            }
-            TA_OUT(3, m_idle); TA_OUT(4, TA_T() - start); TA_OUT(5, (long long)nblk);
+            for (int kk = 0; kk < D / 16; ++kk)
+                umma_bf16(tmem_s + (uint32_t)((i & 1) * TA_BN), qdesc + (uint32_t)((kk / 4) * (TA_BM * 128 >> 4) + 2 * (kk % 4)),
+                          kdesc + (uint32_t)((kk / 4) * (TA_BN * 128 >> 4) + 2 * (kk % 4)), idesc_s, kk > 0 ? 1u : 0u, elected);
+            umma_commit(&s_done[i & 1], elected);
         }
+        if (lane == 0) { TA_OUT(3, m_idle); TA_OUT(4, TA_T() - start); TA_OUT(5, (long long)nblk); }
     } else if (warp == 6) {
         // (rows that are keys and values both: nothing to ask for)
-    } else if (warp == 7) {
+    } else if (role == 7) {
         // ---- the issuer of P V: O += P(i) V(i) once the rows have put P(i) into tensor memory and the values have landed
         // (any rescaling of O by the rows happened before they arrived) ----
-        if (lane == 0) {
-            constexpr uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(DV >> 3) << 17) | ((uint32_t)(TA_BM >> 4) << 24);
-            uint64_t vdesc[2][TA_BN / 16];
+        constexpr uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(DV >> 3) << 17) | ((uint32_t)(TA_BM >> 4) << 24);
+        const uint32_t elected = elect_one(), tmem_pv = warp_same(tmem_base);
+        const int blocks = warp_same(nblk);
+        bool ok = true;
+        const long long start = TA_T();
+        long long m_idle = 0;
+        for (int i = 0; ok && i < blocks; ++i) {
+            const int buf = i & 1;
+            const long long m_t0 = TA_T();
+            ok = __all_sync(0xffffffffu, wait_or_abort(&p_ready[buf], (i >> 1) & 1, abort, error_flag, 29));
+            // (rows that are keys and values both landed before S was issued: the wait returns at once)
+            if (ok) ok = __all_sync(0xffffffffu, wait_or_abort(TA_V_IN_K ? &k_full[buf] : &v_full[buf], (i >> 1) & 1, abort, error_flag, 29));
+            m_idle += TA_T() - m_t0;
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // P is the A operand straight from tensor memory: row = lane, two bf16 per 32-bit column
+            const uint32_t tp = tmem_pv + (uint32_t)(buf * TA_BN);
+            const uint64_t vdesc = umma_desc_mn(smem_u32(sKV + (size_t)buf * TA_BUF_BYTES) + TA_V_OFF, TA_BN * 128);
 #pragma unroll
             for (int kk = 0; kk < TA_BN / 16; ++kk)
-#pragma unroll
-                for (int b = 0; b < 2; ++b)
-                    vdesc[b][kk] = umma_desc_mn(smem_u32(sKV + (size_t)b * TA_BUF_BYTES) + TA_V_OFF + kk * 2048, TA_BN * 128);
-            bool ok = true;
-            const long long start = TA_T();
-            long long m_idle = 0;
-            for (int i = 0; ok && i < nblk; ++i) {
-                const int buf = i & 1;
-                const long long m_t0 = TA_T();
-                ok = wait_or_abort(&p_ready[buf], (i >> 1) & 1, abort, error_flag, 29);
-                // (rows that are keys and values both landed before S was issued: the wait returns at once)
-                if (ok) ok = wait_or_abort(TA_V_IN_K ? &k_full[buf] : &v_full[buf], (i >> 1) & 1, abort, error_flag, 29);
-                m_idle += TA_T() - m_t0;
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                // P is the A operand straight from tensor memory: row = lane, two bf16 per 32-bit column
-                const uint32_t tp = tmem_base + (uint32_t)(buf * TA_BN);
-                if (buf) {
-#pragma unroll
-                    for (int kk = 0; kk < TA_BN / 16; ++kk)
-                        umma_bf16_tmem_a(tmem_base + TA_O_COL, tp + (uint32_t)(kk * 8), vdesc[1][kk], idesc_pv, (i > 0 || kk > 0) ? 1u : 0u);
-                } else {
-#pragma unroll
-                    for (int kk = 0; kk < TA_BN / 16; ++kk)
-                        umma_bf16_tmem_a(tmem_base + TA_O_COL, tp + (uint32_t)(kk * 8), vdesc[0][kk], idesc_pv, (i > 0 || kk > 0) ? 1u : 0u);
-                }
-                umma_commit(&v_free[buf]);
-            }
-            TA_OUT(6, m_idle); TA_OUT(7, TA_T() - start);
+                umma_bf16_tmem_a(tmem_pv + TA_O_COL, tp + (uint32_t)(kk * 8), vdesc + (uint32_t)(kk * (2048 >> 4)), idesc_pv, (i > 0 || kk > 0) ? 1u : 0u, elected);
+            umma_commit(&v_free[buf], elected);
         }
+        if (lane == 0) { TA_OUT(6, m_idle); TA_OUT(7, TA_T() - start); }
     } else {
         // ---- the rows: thread t owns query row t ----
         const int row_t = TA_PAIR ? threadIdx.x & (TA_TOK - 1) : threadIdx.x;

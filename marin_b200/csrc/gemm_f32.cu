@@ -93,23 +93,6 @@ template <int PLANE> __device__ __forceinline__ void gf_put(uint32_t at, const f
     gf_st(at + 2 * PLANE, l0, l1);
 }
 
-// One MMA by the elected lane of a whole warp.  The choice of the lane is a predicate of the instruction and no branch, so that descriptors and addresses stay in
-// uniform registers: 24 of them behind a branch took their warp 2,550 cycles whatever their width, so 1,140 (width 64) to 1,360 (112), what they run for.
-__device__ __forceinline__ void gf_umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t elected) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected)
-        : "memory");
-}
-__device__ __forceinline__ uint32_t gf_elect() {
-    uint32_t e;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
-    return e;
-}
-
 __device__ __noinline__ float gf_chain(const float* x, const float* w, int K) {
     float sum = 0.0f;
     for (int k = 0; k < K; ++k) sum = fmaf(x[k], w[k], sum);
@@ -260,7 +243,7 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
             load(i, more);
         }
     };
-    const uint32_t elected = gf_elect();
+    const uint32_t elected = elect_one();
     auto issue = [&](int c) {                                     // a whole warp: a stage's MMAs
         const int st = c % STAGES;
         if (ok && !mbar_wait(&full[st], (c / STAGES) & 1)) { atomicExch(error_flag, 32); ok = false; }
@@ -272,18 +255,18 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
         // the smallest products first: each addition drops what lies below the accumulator's last bit
 #pragma unroll
         for (int kk = 0; kk < GF_BK / 16; ++kk) {
-            gf_umma(d, da + 2 * AP + 2 * kk, db + 2 * kk, idesc, kk > 0 ? 1u : 0u, elected);
-            gf_umma(d, da + 2 * kk, db + 2 * BP + 2 * kk, idesc, 1u, elected);
-            gf_umma(d, da + AP + 2 * kk, db + BP + 2 * kk, idesc, 1u, elected);
+            umma_bf16(d, da + 2 * AP + 2 * kk, db + 2 * kk, idesc, kk > 0 ? 1u : 0u, elected);
+            umma_bf16(d, da + 2 * kk, db + 2 * BP + 2 * kk, idesc, 1u, elected);
+            umma_bf16(d, da + AP + 2 * kk, db + BP + 2 * kk, idesc, 1u, elected);
         }
 #pragma unroll
         for (int kk = 0; kk < GF_BK / 16; ++kk) {
-            gf_umma(d, da + AP + 2 * kk, db + 2 * kk, idesc, 1u, elected);
-            gf_umma(d, da + 2 * kk, db + BP + 2 * kk, idesc, 1u, elected);
+            umma_bf16(d, da + AP + 2 * kk, db + 2 * kk, idesc, 1u, elected);
+            umma_bf16(d, da + 2 * kk, db + BP + 2 * kk, idesc, 1u, elected);
         }
 #pragma unroll
-        for (int kk = 0; kk < GF_BK / 16; ++kk) gf_umma(d, da + 2 * kk, db + 2 * kk, idesc, 1u, elected);
-        if (elected) umma_commit(&done[st]);
+        for (int kk = 0; kk < GF_BK / 16; ++kk) umma_bf16(d, da + 2 * kk, db + 2 * kk, idesc, 1u, elected);
+        umma_commit(&done[st], elected);
         __syncwarp();
     };
     const int role = __shfl_sync(0xffffffffu, warp, 0);           // (known to be the same in a whole warp)

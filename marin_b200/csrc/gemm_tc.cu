@@ -4,8 +4,8 @@
 // (BN = 16..256 tokens per CTA), so that a decode step with a handful of tokens still fills the 128-row
 // datapath and streams every weight exactly once.  Both operands are K-major in global memory (w is
 // [N, K], x is [T, K]) and are brought into shared memory by TMA (cp.async.bulk.tensor, 128-byte swizzle,
-// no multicast) through a ring of STAGES buffers guarded by mbarriers; one thread issues the MMAs (two, into two
-// accumulators that the epilogue adds, with up to 64 tokens), whose float32 accumulator lives in tensor memory; four
+// no multicast) through a ring of STAGES buffers guarded by mbarriers; one warp issues the MMAs, whose float32 accumulator
+// lives in tensor memory; four
 // warps read it back with tcgen05.ld and write out[t, n] (32 consecutive n per warp and token: coalesced).
 //
 // Split-K: with few tokens and few weight rows there are fewer tiles than SMs, so blockIdx.z cuts K into
@@ -235,22 +235,15 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
     const int kb_begin = blockIdx.z * kb_per_split;
     const int kb_end = min(total_kb, kb_begin + kb_per_split);
     const int nkb = kb_end - kb_begin;
-    // Starting an MMA costs the issuing thread on the order of a hundred cycles, whatever its size, and with few tokens
-    // that, not the data, sets the pace once the weights have landed: up to 64 tokens two threads issue, even k-blocks
-    // into one accumulator and odd ones into a second, and the epilogue adds the two.
-    constexpr bool DUAL = BN <= 64;
-    // With two issuers the ring must have an even number of stages: a stage then belongs to one issuer for good.  With
-    // an odd number the issuers take turns on a stage, and an issuer's first wait on it can be for the barrier's
-    // second phase: a parity wait cannot tell "the second phase is over" from "the first has not ended yet", so the
-    // issuer that is ahead would run MMAs on a stage that is still being filled and give it back once too often
-    // (seen with five stages at 32 tokens: a launch failure once in a few hundred steps).
-    static_assert(!DUAL || STAGES % 2 == 0, "two MMA issuers need an even number of stages");
-    constexpr int NSC = DUAL ? 32 : 64;                               // threads that work out the per-token factors
-    constexpr uint32_t TMEM_COLS = (DUAL ? 2 * BN : BN) < 32 ? 32 : (DUAL ? 2 * BN : BN);
+    // (One warp issues the MMAs.  While each cost its thread a hundred cycles, two with an accumulator each were faster up to 64 tokens; now the second is
+    // only one more that has to come to its end: a decode step of one sequence, 8 layers of the 0.6B layout, 311 us with two and 284 with one; of eight
+    // sequences, 4 layers of the 4B layout, 426 and 427.)
+    constexpr int NSC = 64;                                           // threads that work out the per-token factors
+    constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        mbar_init(accum, DUAL ? 2 : 1);
+        mbar_init(accum, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -265,6 +258,7 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
 
     MB_TRACE_MARK();
     pdl_launch_dependents();
+    const int role = warp_same(warp);
     if (warp == 0 && lane == 0) {
         // ---- producer: TMA loads into the ring.  The weights are written by no kernel, so the first tiles of w
         // are asked for before the wait on the kernels ahead in the stream; x is read only after it. ----
@@ -286,27 +280,26 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
             tma_load_2d(a, &map_w, k, n0, &full[s]);
             tma_load_2d(a + L::A_BYTES, &map_x, k, t0, &full[s]);
         }
-    } else if ((warp == 1 || (DUAL && warp == 3)) && lane == 0) {
-        // ---- MMA issuers: thread `which` takes the k-blocks i = which, which + step, ... into accumulator `which` ----
+    } else if (role == 1) {
+        // ---- the MMAs ----
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
-        const int which = warp == 1 ? 0 : 1, step = DUAL ? 2 : 1;
-        const uint32_t tmem_d = tmem_base + (uint32_t)(which * BN);
+        const uint32_t tmem_d = warp_same(tmem_base), elected = elect_one();
         bool ok = true;
-        for (int i = which; i < nkb && ok; i += step) {
+        for (int i = 0; i < nkb && ok; ++i) {
             const int s = i % STAGES;
             const uint32_t phase = (i / STAGES) & 1;
-            if (!mbar_wait(&full[s], phase)) { atomicExch(error_flag, 2); ok = false; break; }
+            if (!mbar_wait_warp(&full[s], phase)) { atomicExch(error_flag, 2); ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t a = smem_u32(smem + s * L::STAGE_BYTES);
             const uint64_t adesc = umma_desc(a), bdesc = umma_desc(a + L::A_BYTES);
 #pragma unroll
             for (int kk = 0; kk < TC_BK / 16; ++kk)
-                umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (i > which || kk > 0) ? 1u : 0u);
-            if (i + STAGES < nkb) umma_commit(&empty[s]);             // only a stage that is filled again needs to be given back
+                umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (i > 0 || kk > 0) ? 1u : 0u, elected);
+            if (i + STAGES < nkb) umma_commit(&empty[s], elected);    // only a stage that is filled again needs to be given back
         }
-        umma_commit(accum);
-    } else if ((DUAL ? warp == 2 : warp >= 2) && scale.sumsq != nullptr) {
-        // ---- the per-token factors of the norm ahead of this product: warp 2 (and 3, with one issuer) adds the slots, in slot order ----
+        umma_commit(accum, elected);
+    } else if (warp >= 2 && scale.sumsq != nullptr) {
+        // ---- the per-token factors of the norm ahead of this product: warps 2 and 3 add the slots, in slot order ----
         pdl_wait();
         // warps 2 and 3: `tpt` threads per token (a power of two, at most 32), each adds its share of the slots in
         // slot order, up to 24 loads in flight at a time; then the shares are added in a fixed tree
@@ -359,12 +352,6 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
             float v[16];
             if (have) {
                 tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-                if (DUAL && nkb >= 2) {                               // the odd k-blocks' accumulator
-                    float v2[16];
-                    tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(BN + c0), v2);
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] += v2[j];
-                }
             }
             else {
 #pragma unroll
@@ -537,12 +524,6 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
         float v[16];
         if (have) {
             tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-            if (DUAL && nkb >= 2) {                                   // the odd k-blocks' accumulator
-                float v2[16];
-                tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(BN + c0), v2);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] += v2[j];
-            }
         }
         else {
 #pragma unroll
@@ -732,6 +713,7 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
     const uint32_t tmem_base = *tmem_slot;
     PDL_ENTER_EARLY();
 
+    const int role = warp_same(warp);
     if (warp == 0 && lane == 0) {
         int it = 0;                                                   // k-blocks issued so far, over all tiles
         bool ok = true;
@@ -761,7 +743,8 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
             }
         }
         PROBE_OUT(0, p_wait); PROBE_OUT(1, p_issue);
-    } else if (warp == 1 && lane == 0 && rank == 0) {
+    } else if (role == 1 && rank == 0) {
+        const uint32_t elected = elect_one(), tmem_mma = warp_same(tmem_base);
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(CTAS * TC_BM >> 4) << 24);
         int it = 0, local = 0;
         bool ok = true;
@@ -772,29 +755,29 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
             const int buf = local & 1;
             const uint32_t acc_phase = (local >> 1) & 1;
             const long long mt0 = PROBE_T();
-            if (!mbar_wait(&acc_empty[buf], acc_phase ^ 1)) { atomicExch(error_flag, 12); ok = false; break; }
+            if (!mbar_wait_warp(&acc_empty[buf], acc_phase ^ 1)) { atomicExch(error_flag, 12); ok = false; break; }
             PROBE_ADD(m_acc, mt0);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BN);
+            const uint32_t tmem_d = tmem_mma + (uint32_t)(buf * BN);
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
                 const int s = it % STAGES;
                 const uint32_t phase = (it / STAGES) & 1;
                 const long long mt1 = PROBE_T();
-                if (!mbar_wait(&full[s], phase)) { atomicExch(error_flag, 13); ok = false; break; }
+                if (!mbar_wait_warp(&full[s], phase)) { atomicExch(error_flag, 13); ok = false; break; }
                 PROBE_ADD(m_full, mt1);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t a = smem_u32(smem + s * L::STAGE_BYTES);
                 const uint64_t adesc = umma_desc(a), bdesc = umma_desc(a + L::A_BYTES);
 #pragma unroll
                 for (int kk = 0; kk < TC_BK / 16; ++kk) {
-                    if (PAIR) umma_bf16_pair(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
-                    else umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
+                    if (PAIR) umma_bf16_pair(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u, elected);
+                    else umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u, elected);
                 }
-                if (PAIR) umma_commit_pair(&empty[s]);
-                else umma_commit(&empty[s]);
+                if (PAIR) umma_commit_pair(&empty[s], elected);
+                else umma_commit(&empty[s], elected);
             }
-            if (PAIR) umma_commit_pair(&acc_full[buf]);
-            else umma_commit(&acc_full[buf]);
+            if (PAIR) umma_commit_pair(&acc_full[buf], elected);
+            else umma_commit(&acc_full[buf], elected);
         }
         PROBE_ADD(m_all, mt_start);
         PROBE_OUT(2, m_full); PROBE_OUT(3, m_acc); PROBE_OUT(4, m_all);

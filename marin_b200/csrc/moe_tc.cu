@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(320) moe_grouped_tc_kernel(const __grid_consta
     auto begin_of = [&](int nkb) { return part * ((nkb + parts - 1) / parts); };
     auto end_of = [&](int nkb) { return min(nkb, (part + 1) * ((nkb + parts - 1) / parts)); };
 
+    const int role = warp_same(warp);
     if (warp == 0 && lane == 0) {
         int it = 0;                                                   // k-blocks issued so far, over all tiles
         bool ok = true;
@@ -152,33 +153,35 @@ __global__ void __launch_bounds__(320) moe_grouped_tc_kernel(const __grid_consta
                 }
             }
         }
-    } else if (warp == 1 && lane == 0 && rank == 0) {
+    } else if (role == 1 && rank == 0) {
+        const uint32_t elected = elect_one(), tmem_mma = warp_same(tmem_base);
         int it = 0, local = 0;
         bool ok = true;
-        for (; ok && walk.next(row0, rows_end, width, n0, part); ++local) {
+        for (; ok && warp_same((int)walk.next(row0, rows_end, width, n0, part)); ++local) {
             const int buf = local & 1;
-            const int nkb = (walk.g == 0 ? sh.K : ex.K) / TC_BK;
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(width >> 3) << 17) | ((uint32_t)(CTAS * TC_BM >> 4) << 24);
-            if (!mbar_wait(&acc_empty[buf], ((local >> 1) & 1) ^ 1)) { atomicExch(error_flag, 22); ok = false; break; }
+            part = warp_same(part);
+            const int nkb = warp_same(walk.g == 0 ? sh.K : ex.K) / TC_BK;
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(warp_same(width) >> 3) << 17) | ((uint32_t)(CTAS * TC_BM >> 4) << 24);
+            if (!mbar_wait_warp(&acc_empty[buf], ((local >> 1) & 1) ^ 1)) { atomicExch(error_flag, 22); ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BNM);
+            const uint32_t tmem_d = tmem_mma + (uint32_t)(buf * BNM);
             const int kb0 = begin_of(nkb), kb1 = end_of(nkb);
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
                 const int s = it % STAGES;
-                if (!mbar_wait(&full[s], (it / STAGES) & 1)) { atomicExch(error_flag, 23); ok = false; break; }
+                if (!mbar_wait_warp(&full[s], (it / STAGES) & 1)) { atomicExch(error_flag, 23); ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t a = smem_u32(smem + s * R::STAGE);
                 const uint64_t adesc = umma_desc(a), bdesc = umma_desc(a + R::A_BYTES);
 #pragma unroll
                 for (int kk = 0; kk < TC_BK / 16; ++kk) {
-                    if (PAIR) umma_bf16_pair(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
-                    else umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
+                    if (PAIR) umma_bf16_pair(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u, elected);
+                    else umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u, elected);
                 }
-                if (PAIR) umma_commit_pair(&empty[s]);
-                else umma_commit(&empty[s]);
+                if (PAIR) umma_commit_pair(&empty[s], elected);
+                else umma_commit(&empty[s], elected);
             }
-            if (PAIR) umma_commit_pair(&acc_full[buf]);
-            else umma_commit(&acc_full[buf]);
+            if (PAIR) umma_commit_pair(&acc_full[buf], elected);
+            else umma_commit(&acc_full[buf], elected);
         }
     } else if (warp >= 2) {
         const int quarter = warp & 3;                                 // the 32 TMEM lanes this warp may read
