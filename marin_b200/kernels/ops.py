@@ -314,20 +314,41 @@ def check_device_errors(device=None) -> None:
             s.check()
 
 
+@functools.lru_cache(maxsize=4096)
 def gemm_plan(T: int, N: int, K: int):
     """Tokens per CTA and the number of K slices (1, 2, 4 or 8: the CTAs of one cluster) for the tensor-core
-    kernel.  K is cut when there are fewer tiles than SMs, as far as every slice keeps at least 4 k-blocks."""
+    kernel.  K is cut when there are fewer tiles than SMs, as far as every slice keeps at least 4 k-blocks: up to 128 tokens into as many as
+    there is room for, beyond by ``_cluster_microseconds``."""
     bn = 16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 else 128
     tiles = -(-N // 128) * -(-T // bn)
     nkb = -(-K // 64)
-    splits = 1
-    if tiles < SM_COUNT:
-        for cand in (8, 4, 2):
-            per = -(-nkb // cand)
-            if tiles * cand <= 2 * SM_COUNT + 32 and per >= 4 and (cand - 1) * per < nkb:
-                splits = cand
-                break
-    return bn, splits
+    if tiles >= SM_COUNT:
+        return bn, 1
+    fits = [s for s in (8, 4, 2) if tiles * s <= 2 * SM_COUNT + 32 and -(-nkb // s) >= 4 and (s - 1) * -(-nkb // s) < nkb]
+    if T > 128:
+        return bn, min(fits + [1], key=lambda s: _cluster_microseconds(tiles, nkb, s))
+    return bn, fits[0] if fits else 1
+
+
+def _cluster_microseconds(tiles: int, nkb: int, splits: int) -> float:
+    """What a product of tiles of 128 x 128 takes with K in so many slices (B200, 136 to 640 tokens): 0.4 us a k-block with a CTA an SM, 0.5 with two, and
+    more than 148 CTAs in clusters of eight do not all find room (2,560 rows of 2,048, 256 tokens: 12.5 us in four slices, 18.8 in eight)."""
+    ctas, per = tiles * splits, -(-nkb // splits)
+    if ctas <= SM_COUNT:
+        return 7.0 + 0.4 * per
+    return (8.3 + 0.5 * per * -(-ctas // (2 * SM_COUNT))) * (1.6 if splits == 8 else 1.0)
+
+
+@functools.lru_cache(maxsize=4096)
+def half_round(T: int, N: int, K: int) -> bool:
+    """Whether a product with fewer tiles than SMs goes to the persistent kernel all the same: one round of whole tiles there is 4.9 us and 0.236 a k-block,
+    without the slices' sums (B200: 6,144 rows of 1,024, 256 tokens 9.0 us for 12.2 in two slices; of 4,096 20.4 for 22.1; but 4,096 rows of 4,096 20.4
+    for 16.6 in four)."""
+    if T <= 128 or N <= 0:
+        return False
+    bn, splits = gemm_plan(T, N, K)
+    nkb = -(-K // 64)
+    return 4.9 + 0.236 * nkb <= _cluster_microseconds(-(-N // 128) * -(-T // bn), nkb, splits)
 
 
 PERSISTENT_TILES = (128, 144, 160, 176, 192, 208, 224, 240, 256)
@@ -343,34 +364,32 @@ def persistent_plan(T: int, N: int) -> int:
 
 #: two SMs on one tile of 256 weight rows in the persistent kernel
 pair_tiles = True
-#: from this many multiply-adds on: what pairs save is a share of the time (a third less operand traffic, so less power and a higher clock), what they cost
-#: is about 2 us a launch (clusters to place, two SMs' ends to wait for).  Measured on B200 back to back, one and two SMs a tile of the same width: 2,048 tokens,
-#: 24,576 rows of 4,096 362 and 349 us; 6,144 of 2,560 63.7 and 62.0; 2,560 of 4,096 (2.1e10) 54.0 and 53.1; 2,560 of 2,560 (1.2e10) 35.8 and
-#: 35.3, but 2,560 of 1,024 16.7 and 17.5; 10,240 of 256 25.0 and 28.8; 1,900 tokens, 5,120 rows of 128 12.1 and 14.5.
-PAIRS_FROM = 1 << 34
+#: from this many multiply-adds on (pairs take clusters to place and two SMs' ends to wait for; measured on B200, 36 to 2e11 multiply-adds: see ``_paired_width``)
+PAIRS_FROM = 1 << 33
 
 
 def paired_plan(T: int, N: int, K: int) -> int:
     """``persistent_plan``'s width, or a negative one: CTAs then work in pairs on 256 weight rows of it.  From ``PAIRS_FROM`` multiply-adds on, at widths
-    in steps of 32, wherever ``persistent_plan``'s measure, less 7 %, comes out no larger than the single tiles' (each pair is two SMs, and an odd last row
-    tile leaves one of them idle).  7 %: pairs of 256 against single tiles of 240 took 227 us for 231 (1,184 tokens, 24,576 rows of 4,096) and 61.0 for 63.7
-    (2,048, 6,144 of 2,560), where the measure has 6 % more for them; at equal widths they save 2 to 4 %."""
+    in steps of 32, wherever the pairs' rounds come out cheaper."""
     return _paired_width(T, N) if pair_tiles and T * N * K >= PAIRS_FROM else persistent_plan(T, N)
 
 
 @functools.lru_cache(maxsize=4096)
 def _paired_width(T: int, N: int) -> int:
+    """Rounds of pairs over the SMs times width + 112, 0.7 of that and 30 more, against rounds of single tiles times width + 96.  Fitted to 85 shapes of 300 to 2,048
+    tokens on B200: the choice costs 1.5 % on average over the best width of each (2,048 tokens, 4,096 rows of 4,096: 57 us by pairs of 256, 60 by single tiles of
+    240; 19,456 of 2,560: 148 and 171; 1,184 tokens, 6,144 of 2,560: 34 by pairs of 224, 33 by single tiles of 208)."""
     cost, single = _tile_by_tile(T, N)
     rows = -(-N // 256)
-    paired, bn = min((-(-(rows * -(-T // bn)) // (SM_COUNT // 2)) * (bn + 24), bn) for bn in PERSISTENT_TILES if bn % 32 == 0)
-    return -bn if 0.93 * paired <= cost else single
+    paired, bn = min((-(-(rows * -(-T // bn)) // (SM_COUNT // 2)) * (bn + 112), bn) for bn in PERSISTENT_TILES if bn % 32 == 0)
+    return -bn if 0.7 * paired + 30 <= cost else single
 
 
 def _tile_by_tile(T: int, N: int):
     best = None
     for bn in PERSISTENT_TILES:
         tiles = -(-N // 128) * -(-T // bn)
-        cost = -(-tiles // SM_COUNT) * (bn + 24)
+        cost = -(-tiles // SM_COUNT) * (bn + 96)
         if best is None or cost < best[0]:
             best = (cost, bn)
     return best
@@ -378,26 +397,22 @@ def _tile_by_tile(T: int, N: int):
 
 def many_tokens(T: int, N: int, with_heads: bool = False) -> bool:
     """Whether a product of T tokens and N weight rows goes to the persistent kernel (else: one CTA per tile, K cut
-    over the CTAs of a cluster where tiles are few).  It needs a round of tiles to be worth it: with fewer tiles than SMs
-    the clusters' many CTAs ask for more at once (measured at Qwen3-4B sizes: the down product at 512 tokens 43 us
-    against 52, at 768 tokens 45 against 53; o at 768 tokens 23 against 26).  The q|k|v product that finishes its heads
-    stays persistent from half a round on: beyond 128 tokens only that kernel can finish them (17.6 us at 256 tokens
-    against 18.2 plus the q/k kernel)."""
+    over the CTAs of a cluster where tiles are few, unless ``half_round`` finds one round of whole tiles shorter).  The q|k|v product that finishes its heads
+    stays persistent from a third of a round on: beyond 128 tokens only that kernel can finish them, which saves the q/k kernel."""
     tiles = -(-N // 128) * -(-T // 128)
-    return T > 128 and tiles >= (SM_COUNT // 2 if with_heads else SM_COUNT)
+    return T > 128 and tiles >= (SM_COUNT // 3 if with_heads else SM_COUNT)
 
 
 #: the persistent kernel deals k-blocks instead of tiles over the SMs where whole tiles would leave SMs idle
 stream_k = True
 
 
-#: Stream-K against tile by tile, fitted to timings on B200 (2,048 and 1,024 tokens, layer sizes of 4B to 14B models):
-#: a k-block of a 128 x bn tile costs about bn + 138 (the weight tile is fetched whatever the width), and stream-K
-#: pays a fixed part worth 7,700 such units (about 8 us: every CTA parks a partial tile at the start and the last
-#: epilogue, which nothing overlaps, is longer).  Measured times came out up to 0.1 above the predicted ratio, hence
-#: the margin.  Groups walk different k at the same time, so x has to stay in L2 (at 71 MB stream-K lost 6 % where
-#: the fit promised 9 %; at 57 and 67 MB and 20 row tiles it gained 22 and 17 %), and with fewer than four token tiles the fit did not hold (0.98 and 1.07 for 0.75 and 0.91).
-_KBLOCK_FIXED, _STREAM_K_FIXED, _STREAM_K_MARGIN, _STREAM_K_MAX_X_BYTES = 138, 7700, 0.87, 64 << 20
+#: Stream-K against whole tiles, fitted to timings on B200 (300 to 2,048 tokens, layer sizes of 0.6B to 8B models): a k-block of a 128 x bn tile costs
+#: about bn + 64, which stream-K's CTAs do at 0.87 of it (no empty last round); pairs at 0.73, and a round of tiles 1,600 (pairs 2,400) more, a launch of pairs
+#: 4,200.  Stream-K pays 9,000 (every CTA parks a partial tile at the start and the last epilogue, which nothing overlaps, is longer): 2,048 tokens by 2,560 rows
+#: of 9,728 89 us for 92 by pairs, of 4,096 41 for 40.  Groups walk different k at the same time, so x has to stay in L2; with fewer than four token tiles
+#: the fit does not hold, nor from two rounds on (2,048 by 7,680 of 2,560 79 us, 70 by pairs), where little is left of an empty last one.
+_KBLOCK_FIXED, _STREAM_K_FIXED, _STREAM_K_MARGIN, _STREAM_K_MAX_X_BYTES = 64, 9000, 0.98, 64 << 20
 
 
 def stream_k_plan(T: int, N: int, K: int) -> Optional[int]:
@@ -413,15 +428,18 @@ def _stream_k_width(T: int, N: int, K: int, kblock: int, fixed: float, margin: f
     rows, nkb = -(-N // 128), -(-K // 64)
     for bn in STREAM_K_TILES:
         across = -(-T // bn)
-        if across > SM_COUNT or rows < SM_COUNT // across or (fixed > 0 and (across < 4 or T * K * 2 > most)):
+        if across > SM_COUNT or rows < SM_COUNT // across or (fixed > 0 and (across < 4 or rows >= 2 * (SM_COUNT // across) or T * K * 2 > most)):
             continue
-        cost = rows / (SM_COUNT // across) * nkb * (bn + kblock) + fixed
+        cost = 0.87 * rows / (SM_COUNT // across) * nkb * (bn + kblock) + fixed
         if best is None or cost <= best[0]:
             best = (cost, bn)
     if best is None:
         return None
-    bn = persistent_plan(T, N)
-    whole = -(-(rows * -(-T // bn)) // SM_COUNT) * nkb * (bn + kblock)
+    bn = paired_plan(T, N, K)
+    if bn > 0:
+        whole = -(-(rows * -(-T // bn)) // SM_COUNT) * (nkb * (bn + kblock) + 1600)
+    else:
+        whole = 0.73 * -(-(-(-rows // 2) * -(-T // -bn)) // (SM_COUNT // 2)) * (nkb * (kblock - bn) + 2400) + 4200
     return best[1] if best[0] < margin * whole else None
 
 
@@ -523,7 +541,7 @@ def gemm(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, then_n
             if activation != "relu2" or accumulate or out.dtype != torch.bfloat16 or then_norm is not None:
                 raise KernelError(f"gemm: activation {activation!r} goes with a plain bfloat16 output")
             mode = 4
-        if many_tokens(T, N):
+        if many_tokens(T, N) or half_round(T, N, K):
             s = _scratch_for(x.device)
             lib = _lib("mb_gemm_tc")
             carried = None
@@ -923,7 +941,7 @@ def gemm_glu_rows(x: torch.Tensor, w: torch.Tensor, rows: Optional[torch.Tensor]
     _cost(_size(w) + _size(x) + T * (I + P) * 2, 2.0 * T * N * K)
     parked = flags = None
     ctas, floats, what = 0, 0, "gemm+glu (tensor cores"
-    if many_tokens(T, N):
+    if T > 128:                                                     # (gated rows: K is not cut, and whole tiles are the persistent kernel's)
         ctas, bn = SM_COUNT, stream_k_plan(T, N, K)
         what += ", persistent"
         if bn is not None:
@@ -965,7 +983,7 @@ def gemm_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, out: torch.Tensor,
     s = _scratch_for(x.device)
     mode = _GLU_MODES[activation]
     _cost(_size(w_interleaved) + _size(x) + _size(out), 2.0 * T * N * K)
-    if many_tokens(T, N):
+    if T > 128:                                                     # (as in gemm_glu_rows)
         if scaled is not None:
             _check(_lib("mb_gemm_tc").mb_gemm_tc_persistent_coupled(
                 _ptr(x), _ptr(w_interleaved), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K), _c_int(persistent_plan(T, N)),
@@ -1920,13 +1938,16 @@ def _experts_on_tcgen05(E: int, pairs: int, interleaved: bool, activation: str) 
     return use_tensor_cores and E <= 512 and (interleaved or activation != "swiglu")
 
 
-def _expert_tile(pairs: int, E: int) -> int:
-    """The widest tile of rows, from the experts' average share: one tile holds an ordinary expert's rows while the rows are few (its weights are then
-    read once, and a small tile leaves room for a deep ring); equal tiles of at most 256 beyond.  A whole call, 8 experts of 2,560 x 3,648, two chosen, a shared one
-    of 2,432, by tiles of 32, 64, 128 and 256: shares of 12 rows 118, 122, 123, 128 us; 20 125, 123, 127, 133; 25 140, 126, 129, 134; 44 199, 136, 131, 143;
-    64 236, 175, 129, 140; 100 335, 233, 155, 148."""
+def _expert_tile(pairs: int, E: int, shared_rows: int = 0) -> int:
+    """The widest tile of rows, from the experts' average share and a shared expert's rows: one tile holds an ordinary expert's rows while the rows are few (its
+    weights are then read once, and a small tile leaves room for a deep ring); equal tiles of at most 256 beyond.  A whole call by tiles of 32, 64, 128 and 256: 8
+    experts of 2,560 x 3,648, two chosen, a shared one of 2,432: shares of 12 rows 111, 115, 116, 124 us; 20 122, 120, 120, 128; 25 136, 124, 122, 130; 44 199,
+    134, 125, 139; 64 232, 168, 124, 137; 100 335, 238, 154, 146.  16 experts of 2,048 x 1,280, one chosen, a shared one of 1,024: 4 77, 79, 79, 84; 5 81, 78, 79,
+    84; 8 84, 80, 82, 86; 11 87, 86, 82, 89; 44 178, 122, 101, 106; 62 207, 154, 116, 111."""
     average = pairs / E
-    return 32 if average <= 20 else 64 if average <= 44 else 128 if average <= 100 else 256
+    if average <= 20 and shared_rows <= 128:
+        return 32 if shared_rows <= 64 else 64
+    return 128 if average <= (50 if shared_rows > 512 else 80) else 256
 
 
 #: the further parts' results take no more memory than this (working memory that steps of any size are planned with)
@@ -2020,7 +2041,7 @@ def _experts_tc(x, xs, w_gate_up, w_down, offsets, act, inv, weights, y, weight_
     E, h, ff = w_down.shape
     pairs, size, touched = xs.shape[0], x.element_size(), min(xs.shape[0], w_down.shape[0])
     gated = activation != "relu2"
-    lib, s, tile = _lib("mb_moe_tc"), _scratch_for(x.device), _expert_tile(pairs, E)
+    lib, s, tile = _lib("mb_moe_tc"), _scratch_for(x.device), _expert_tile(pairs, E, T if shared is not None else 0)
     first2 = down2 = act2 = rows2 = None
     ff2 = 0
     if shared is not None:

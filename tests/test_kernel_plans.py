@@ -35,6 +35,20 @@ def test_few_token_plan_keeps_every_slice_in_use(T, N, K):
     assert (splits - 1) * per < nkb                            # no slice without k-blocks
 
 
+@pytest.mark.parametrize("T", [129, 136, 200, 384, 700, 1184, 2048])
+@pytest.mark.parametrize("N,K", [(1, 8), (128, 64), (1024, 3072), (2560, 9728), (3232, 2560), (4096, 1024), (6144, 4096), (19456, 2560)])
+def test_plans_beyond_128_tokens_are_launches_the_kernels_take(T, N, K):
+    """Slices of K that all have work, whole tiles instead only where there are fewer of them than SMs or many tokens say so anyway."""
+    bn, splits = ops.gemm_plan(T, N, K)
+    nkb = -(-K // 64)
+    assert bn == 128 and splits in (1, 2, 4, 8) and (splits - 1) * -(-nkb // splits) < nkb
+    tiles = -(-N // 128) * -(-T // 128)
+    assert splits == 1 or (tiles < ops.SM_COUNT and -(-nkb // splits) >= 4)
+    if tiles < ops.SM_COUNT and ops.half_round(T, N, K):
+        assert 4.9 + 0.236 * nkb <= ops._cluster_microseconds(tiles, nkb, splits)
+    assert not ops.half_round(128, N, K) and not ops.many_tokens(128, N, True)
+
+
 @pytest.mark.parametrize("E", [1, 8, 16, 32, 60, 128, 384, 512])
 @pytest.mark.parametrize("h,ff,shared_ff", [(2560, 3648, 2432), (4096, 2048, 0), (2048, 768, 768), (256, 512, 1024)])
 def test_parts_of_the_experts_last_products_cost_less_than_the_round_they_save(E, h, ff, shared_ff):

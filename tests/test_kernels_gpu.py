@@ -936,6 +936,27 @@ def test_float32_product_at_tile_edges(ops, T, N, K):
     assert torch.equal(added, out + out)
 
 
+@pytest.mark.parametrize("T,N,K", [(129, 96, 64), (200, 4096, 256), (257, 672, 1032), (384, 3232, 72), (130, 160, 4160)])
+def test_products_of_less_than_a_round_of_tiles(ops, T, N, K):
+    """Beyond 128 tokens, whole tiles or slices of K, whichever is planned, and a gated product, against float64: float32 sums (K roundings of 2^-24) rounded to bf16 once."""
+    g = torch.Generator(device=DEV).manual_seed(T + N)
+    x = torch.randn(T, K, device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(N, K, device=DEV, generator=g) / math.sqrt(K)).to(torch.bfloat16)
+    want = x.double() @ w.double().t()
+    out, added = torch.zeros(T, N, device=DEV, dtype=torch.bfloat16), torch.ones(T, N, device=DEV)
+    ops.gemm(x, w, out)
+    ops.gemm(x, w, added, accumulate=True)
+    scale = x.double().abs() @ w.double().abs().t()
+    assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -24 * K * scale + 1e-30).all())
+    assert bool(((added.double() - 1.0 - want).abs() <= 2.0 ** -24 * (K * scale + 4.0)).all())
+    rows = w.view(N // 32, 2, 16, K)
+    gate, up = x.double() @ rows[:, 0].reshape(-1, K).double().t(), x.double() @ rows[:, 1].reshape(-1, K).double().t()
+    act = torch.empty(T, N // 2, device=DEV, dtype=torch.bfloat16)
+    ops.gemm_swiglu(x, w, act)
+    torch.testing.assert_close(act.double(), torch.nn.functional.silu(gate) * up, rtol=1.6e-2, atol=1e-3)
+    ops.check_device_errors()
+
+
 @pytest.mark.parametrize("T,N,K", [(1, 1, 4), (16, 127, 60), (17, 129, 64), (33, 3072, 68), (113, 3073, 132), (129, 300, 260), (40, 640, 2052), (200, 128, 576)])
 def test_float32_product_on_tensor_cores(ops, monkeypatch, T, N, K):
     """Every width and share of a tile gives the same bits, and they lie no further from 64 bits than a chain of multiply-adds does.  Bound: an accumulator drops
