@@ -318,6 +318,73 @@ __global__ void __launch_bounds__(256) qk_norm_rope_write_fast_kernel(
     }
 }
 
+// The same for float32 heads of 32 M elements (M even) with the rotation over the whole head (half-split pairs): a warp a head, lane l holds elements l + 32 m, so that
+// an element's rotation partner (m +- M / 2) lies in the same lane.  The same arithmetic in the same order as the general kernel: the same bits.
+// Bound by latency: a warp asks for all of its heads before it works on the first, 8 warps a token (few tokens: a CTA has fewer heads).  Measured on
+// B200, 333 tokens of 32 heads of 128: 6.8 us (the general kernel, a head after another in four warps, 30).
+#define QKR_HEADS 4
+template <int M>
+__global__ void __launch_bounds__(256) qk_norm_rope_write_rows_kernel(
+    const float* __restrict__ qkv, int row_stride, float* __restrict__ q_out, const float* __restrict__ q_w, const float* __restrict__ k_w, float eps,
+    const int* __restrict__ positions, const float* __restrict__ inv_freq, const int* __restrict__ slot_mapping, float* __restrict__ k_cache,
+    float* __restrict__ v_cache, int H, int K, int page_size, int heads_total, int heads_per_warp) {
+    PDL_ENTER();
+    qkv = pdl_fresh(qkv);
+    constexpr int d = 32 * M, half = d / 2;
+    __shared__ float cs_tab[half], sn_tab[half];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x;
+    const int first = (blockIdx.y * 8 + warp) * heads_per_warp, last = min(heads_total, first + heads_per_warp);
+    float v[QKR_HEADS][M];
+#pragma unroll
+    for (int h = 0; h < QKR_HEADS; ++h)
+#pragma unroll
+        for (int m = 0; m < M; ++m) v[h][m] = first + h < last ? qkv[(size_t)t * row_stride + (size_t)(first + h) * d + lane + 32 * m] : 0.0f;
+    const int slot = heads_total > H ? slot_mapping[t] : -1;
+    if (inv_freq != nullptr) {
+        const float pos = (float)positions[t];
+        for (int i = threadIdx.x; i < half; i += 256) {
+            float sn, cs;
+            sincosf(pos * inv_freq[i], &sn, &cs);
+            cs_tab[i] = cs;
+            sn_tab[i] = sn;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < QKR_HEADS; ++h) {
+        const int head = first + h;
+        if (head >= last) break;
+        const bool is_q = head < H, is_k = !is_q && head < H + K;
+        const float* w = is_q ? q_w : (is_k ? k_w : nullptr);
+        if (w != nullptr) {
+            float ss = 0.0f;
+#pragma unroll
+            for (int m = 0; m < M; ++m) ss += v[h][m] * v[h][m];
+            const float scale = 1.0f / sqrtf(warp_sum(ss) / (float)d + eps);
+#pragma unroll
+            for (int m = 0; m < M; ++m) v[h][m] = v[h][m] * scale * w[lane + 32 * m];
+        }
+        if ((is_q || is_k) && inv_freq != nullptr) {
+#pragma unroll
+            for (int m = 0; m < M / 2; ++m) {
+                const float cs = cs_tab[lane + 32 * m], sn = sn_tab[lane + 32 * m], a = v[h][m], b = v[h][m + M / 2];
+                v[h][m] = a * cs - b * sn;
+                v[h][m + M / 2] = b * cs + a * sn;
+            }
+        }
+        float* dst = nullptr;
+        if (is_q) {
+            dst = q_out + ((size_t)t * H + head) * d;
+        } else if (slot >= 0) {
+            const int kh = is_k ? head - H : head - H - K;
+            dst = (is_k ? k_cache : v_cache) + (((size_t)(slot / page_size) * K + kh) * page_size + (size_t)(slot % page_size)) * d;
+        }
+        if (dst == nullptr) continue;
+#pragma unroll
+        for (int m = 0; m < M; ++m) dst[lane + 32 * m] = v[h][m];
+    }
+}
+
 MB_API int mb_qk_norm_rope_write(const void* qkv, int dtype, void* q_out, const float* q_w, const float* k_w, float eps,
                                  const int* positions, const float* inv_freq, int rotary_dim, int interleaved,
                                  const int* slot_mapping, void* k_cache, void* v_cache, int tokens, int H, int K, int d,
@@ -337,6 +404,14 @@ MB_API int mb_qk_norm_rope_write(const void* qkv, int dtype, void* q_out, const 
                                  eps, positions, inv_freq, slot_mapping, (bf16*)k_cache, (bf16*)v_cache, H, K, page_size, heads_total);
         return launch_kernel(qk_norm_rope_write_fast_kernel<32>, tokens, 256, 0, s, 0, (const bf16*)qkv, row_stride, (bf16*)q_out, q_w, k_w,
                              eps, positions, inv_freq, slot_mapping, (bf16*)k_cache, (bf16*)v_cache, H, K, page_size, heads_total);
+    }
+    if (dtype == MB_F32 && (d == 64 || d == 128 || d == 256) && !interleaved && (inv_freq == nullptr || rotary_dim == d)) {
+        // (from 256 tokens on there are CTAs enough: eight warps share a token's angles and take up to four heads each)
+        const int per = tokens >= 256 ? min(QKR_HEADS, (heads_total + 7) / 8) : 1;
+        const dim3 grid(tokens, (heads_total + 8 * per - 1) / (8 * per));
+        const auto kernel = d == 64 ? qk_norm_rope_write_rows_kernel<2> : d == 128 ? qk_norm_rope_write_rows_kernel<4> : qk_norm_rope_write_rows_kernel<8>;
+        return launch_kernel(kernel, grid, 256, 0, s, 0, (const float*)qkv, row_stride, (float*)q_out, q_w, k_w, eps, positions, inv_freq, slot_mapping,
+                             (float*)k_cache, (float*)v_cache, H, K, page_size, heads_total, per);
     }
     const int warps = 4;
     // few tokens: a warp per head, the heads spread over CTAs; many tokens: one CTA per token walks all heads and

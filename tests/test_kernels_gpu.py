@@ -957,6 +957,35 @@ def test_products_of_less_than_a_round_of_tiles(ops, T, N, K):
     ops.check_device_errors()
 
 
+@pytest.mark.parametrize("H,K,d", [(16, 8, 128), (3, 1, 64), (33, 2, 256)])
+def test_float32_heads_do_not_depend_on_how_many_share_a_block(ops, H, K, d):
+    """From 256 tokens on a warp takes several heads: the bits of one token alone, and the plain formula's numbers (a sum of d squares and two products: 2^-24 d)."""
+    import kernel_refs
+
+    g = torch.Generator(device=DEV).manual_seed(d)
+    T, page = 257, 16
+    x = torch.randn(T, (H + 2 * K) * d, device=DEV, generator=g)
+    qw, kw = (1 + 0.1 * torch.randn(d, device=DEV, generator=g) for _ in range(2))
+    positions = torch.randint(0, 4000, (T,), device=DEV, generator=g, dtype=torch.int32)
+    inv_freq = torch.pow(torch.tensor(1e6), -(torch.arange(d // 2, dtype=torch.float32) * 2.0 / d)).to(DEV)
+    slots = torch.randperm(T + 40, device=DEV, generator=g)[:T].to(torch.int32)
+    slots[7] = -1
+
+    def run(t0, t1, fn):
+        caches = [torch.zeros((T + 40) // page + 1, K, page, d, device=DEV) for _ in range(2)]
+        q = torch.empty(t1 - t0, H * d, device=DEV)
+        fn(x[t0:t1].contiguous(), q, qw, kw, 1e-6, positions[t0:t1].contiguous(), inv_freq, d, False, slots[t0:t1].contiguous(), *caches, H, K, d)
+        return q, *caches
+
+    whole, plain = run(0, T, ops.qk_norm_rope_write), run(0, T, kernel_refs.qk_norm_rope_write)
+    for got, want in zip(whole, plain):
+        torch.testing.assert_close(got, want, rtol=1e-4, atol=2e-4)
+    parts = [run(0, 1, ops.qk_norm_rope_write), run(1, T, ops.qk_norm_rope_write)]
+    assert torch.equal(torch.cat([p[0] for p in parts]), whole[0])
+    for n in (1, 2):
+        assert torch.equal(parts[0][n] + parts[1][n], whole[n])
+
+
 @pytest.mark.parametrize("T,N,K", [(1, 1, 4), (16, 127, 60), (17, 129, 64), (33, 3072, 68), (113, 3073, 132), (129, 300, 260), (40, 640, 2052), (200, 128, 576)])
 def test_float32_product_on_tensor_cores(ops, monkeypatch, T, N, K):
     """Every width and share of a tile gives the same bits, and they lie no further from 64 bits than a chain of multiply-adds does.  Bound: an accumulator drops
