@@ -90,21 +90,23 @@ __global__ void __launch_bounds__(AS_THREADS) attention_simple_kernel(
 // sum as its warps' butterflies, values added key by key, chunks from position 0 on; a chunk behind a row's position changes nothing),
 // so a token's result is the same bits whichever kernel it went through and however the prompt was cut.
 // Bound by shared memory and the multiply-adds: a 16-byte load takes four cycles of a warp whatever it reads, so scores are made 4 rows x 4 keys a thread
-// and values added 4 rows x 8 columns (1.5 to 2 cycles of loads for one of multiply-adds).  The keys' and values' half chunks arrive by cp.async one
-// ahead of the arithmetic.  Measured on B200 (333 tokens, 16 heads of 128 over 8 kv heads): attention_simple_kernel 605 us, this
-// one 88 us; with 2 x 4 and 2 x 8 a thread, or a lane a row with its query in registers and every key read by the whole warp, 115 us.
-#define AT_ROWS 32
-#define AT_THREADS 128
-#define AT_WARPS (AT_THREADS / 32)
+// and values added 4 rows x 8 columns (half a cycle of loads for one of multiply-adds).  The keys' and values' half chunks arrive by cp.async one
+// ahead of the arithmetic.  A few hundred tokens are few blocks, and the block with the last queries walks all keys while the first ones are long done: such a
+// step goes by 16 rows and 64 threads a block, twice as many blocks of half the length.  Measured on B200 (333 tokens, 16 heads of 128 over 8 kv heads):
+// attention_simple_kernel 605 us; by 32 rows, a half's rows looked up behind a division each (2,300 clocks a half) and the softmax row by row
+// (6,000 a chunk) 88 us; rows looked up side by side 72; the softmax's rows interleaved and 16 rows a block 57 (400 tokens, 32 heads over 8, 32 rows
+// a block: 109 and 91).  With 4 x 2 and 4 x 4 a thread and twice the threads 65.
 #define AT_CHUNK AS_THREADS
 #define AT_HALF 64
 #define AT_LD 132                     // floats a row of 128 takes in shared memory
-#define AT_SMEM ((2 * AT_ROWS * AT_LD + 2 * AT_HALF * AT_LD + AT_ROWS) * 4)
+#define AT_SMEM(rows) ((2 * (rows) * AT_LD + 2 * AT_HALF * AT_LD + (rows)) * 4)
 
-__global__ void __launch_bounds__(AT_THREADS, 2) attention_tile_kernel(
+template <int AT_ROWS>
+__global__ void __launch_bounds__(4 * AT_ROWS, 2) attention_tile_kernel(
     const float* __restrict__ q, const float* __restrict__ k_cache, const float* __restrict__ v_cache, float* __restrict__ out,
     const int* __restrict__ block_table, int max_pages, const int* __restrict__ cu_tokens, const int* __restrict__ seq_lens,
-    int first_req, int H, int K, int d, int page_size, float scale) {
+    int first_req, int H, int K, int d, int page_size, int page_shift, float scale) {
+    constexpr int AT_WARPS = AT_ROWS / 8, OWN = AT_ROWS / AT_WARPS;
     PDL_ENTER();
     q = pdl_fresh(q); k_cache = pdl_fresh(k_cache); v_cache = pdl_fresh(v_cache);
     extern __shared__ __align__(16) float at_smem[];
@@ -127,12 +129,15 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tile_kernel(
         const float* src = (stage & 2) ? v_cache : k_cache;
         float* dst = sKV + (stage & 1) * AT_HALF * AT_LD;
         const int key0 = (stage >> 2) * AT_CHUNK + (stage & 1) * AT_HALF;
-        for (int row = warp; row < AT_HALF; row += AT_WARPS) {               // a warp a row
-            const int key = key0 + row;
-            float* to = dst + row * AT_LD + 4 * lane;
-            if (lane >= d4) continue;
-            if (key <= last) cp_async16(to, src + (((size_t)table[key / page_size] * K + kh) * page_size + (size_t)(key % page_size)) * d + 4 * lane);
-            else *reinterpret_cast<float4*>(to) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        // a warp a row; where its rows lie is looked up by as many lanes side by side (pages of a power of two: page_shift, else -1; a key behind the last one
+        // repeats it: nobody adds what comes of it)
+        constexpr int MINE = AT_HALF / AT_WARPS;
+        const int key = min(key0 + warp + AT_WARPS * (lane % MINE), last), page = page_shift >= 0 ? key >> page_shift : key / page_size;
+        const long long at = (((long long)table[page] * K + kh) * page_size + (key - page * page_size)) * d;
+#pragma unroll
+        for (int i = 0; i < MINE; ++i) {
+            const long long from = __shfl_sync(0xffffffffu, at, i);
+            if (lane < d4) cp_async16(dst + (warp + AT_WARPS * i) * AT_LD + 4 * lane, src + from + 4 * lane);
         }
         cp_async_commit();
     };
@@ -144,9 +149,9 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tile_kernel(
         if (row < rows) v = *reinterpret_cast<const float4*>(q + ((size_t)(tok0 + q0 + row / G) * H + kh * G + row % G) * d + 4 * lane);
         *reinterpret_cast<float4*>(sQ + row * AT_LD + 4 * lane) = v;
     }
-    // scores: rows ty + 8 i x keys tx + 16 j; values: rows 4 ty + i x columns 4 tx.. and 64 + 4 tx..; softmax: rows 8 warp ..
+    // scores: rows ty + AT_ROWS / 4 i x keys tx + 16 j; values: rows 4 ty + i x columns 4 tx.. and 64 + 4 tx..; softmax: rows 8 warp .., the warp's of the values
     const int tx = tid & 15, ty = tid >> 4;
-    constexpr int OWN = AT_ROWS / AT_WARPS;
+    constexpr int RT = AT_ROWS / 4;
     float m[OWN], l[OWN], acc[4][8];
     int row_pos[4];                                        // (of rows that are not there: nobody reads their results)
 #pragma unroll
@@ -169,22 +174,45 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tile_kernel(
             for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
-#pragma unroll 2
-            for (int c = 0; c < d4; ++c) {
-                float4 a[4];
+            // (the next four columns on their way while these are multiplied)
+            float4 a[2][4], k[2][4];
+            auto take = [&](int c, int to) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(sQ + (ty + 8 * i) * AT_LD + 4 * c);
+                for (int i = 0; i < 4; ++i) a[to][i] = *reinterpret_cast<const float4*>(sQ + (ty + RT * i) * AT_LD + 4 * c);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float4 k = *reinterpret_cast<const float4*>(kv + (tx + 16 * j) * AT_LD + 4 * c);
+                for (int j = 0; j < 4; ++j) k[to][j] = *reinterpret_cast<const float4*>(kv + (tx + 16 * j) * AT_LD + 4 * c);
+            };
+            auto add = [&](int of) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        s[i][j] = fmaf(a[i].w, k.w, fmaf(a[i].z, k.z, fmaf(a[i].y, k.y, fmaf(a[i].x, k.x, s[i][j]))));
-                }
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) s[i][j] = fmaf(a[of][i].x, k[of][j].x, s[i][j]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) s[i][j] = fmaf(a[of][i].y, k[of][j].y, s[i][j]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) s[i][j] = fmaf(a[of][i].z, k[of][j].z, s[i][j]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) s[i][j] = fmaf(a[of][i].w, k[of][j].w, s[i][j]);
+            };
+            take(0, 0);
+            int c = 0;
+#pragma unroll 1
+            for (; c + 2 <= d4; c += 2) {
+                take(c + 1, 1);
+                add(0);
+                take(c + 2 < d4 ? c + 2 : c, 0);
+                add(1);
             }
+            if (c < d4) add(0);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int row = ty + 8 * i, pos = pos0 + row / G;
+                const int row = ty + RT * i, pos = pos0 + row / G;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const int key = off + tx + 16 * j;
@@ -194,64 +222,113 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tile_kernel(
             if (!(stage & 1)) continue;
             __syncthreads();                               // the chunk's scores are all there
 #pragma unroll
-            for (int i = 0; i < OWN; ++i) {
-                const int row = OWN * warp + i, pos = pos0 + row / G;
-                if (row >= rows) continue;
-                float* p = sP + row * AT_LD + lane;        // a lane a key
-                const float s0 = p[0], s1 = p[32], s2 = p[64], s3 = p[96];
-                const float m_new = fmaxf(m[i], warp_max(fmaxf(fmaxf(s0, s1), fmaxf(s2, s3))));
-                const float corr = expf(m[i] - m_new);
-                const int key = base + lane;
-                const float p0 = key <= pos ? expf(s0 - m_new) : 0.0f, p1 = key + 32 <= pos ? expf(s1 - m_new) : 0.0f;
-                const float p2 = key + 64 <= pos ? expf(s2 - m_new) : 0.0f, p3 = key + 96 <= pos ? expf(s3 - m_new) : 0.0f;
-                p[0] = p0; p[32] = p1; p[64] = p2; p[96] = p3;
-                const float sum = (warp_sum(p0) + warp_sum(p2)) + (warp_sum(p1) + warp_sum(p3));      // block_sum's order
-                l[i] = fmaf(l[i], corr, sum);
-                m[i] = m_new;
-                if (lane == 0) sCorr[row] = corr;
+            for (int half = 0; half < OWN; half += 4) {    // four rows side by side, a lane a key
+                const int row0 = OWN * warp + half;
+                float* p = sP + row0 * AT_LD + lane;
+                float w[4][4], corr[4], top[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) w[i][e] = p[i * AT_LD + 32 * e];
+                    top[i] = fmaxf(fmaxf(w[i][0], w[i][1]), fmaxf(w[i][2], w[i][3]));
+                }
+                {
+                    // four rows' maxima at once: half of the lanes go on with half of the rows
+                    const bool up = (lane & 16) != 0, on = (lane & 8) != 0;
+                    const float u0 = fmaxf(up ? top[2] : top[0], __shfl_xor_sync(0xffffffffu, up ? top[0] : top[2], 16));
+                    const float u1 = fmaxf(up ? top[3] : top[1], __shfl_xor_sync(0xffffffffu, up ? top[1] : top[3], 16));
+                    float u = fmaxf(on ? u1 : u0, __shfl_xor_sync(0xffffffffu, on ? u0 : u1, 8));
+                    u = fmaxf(u, __shfl_xor_sync(0xffffffffu, u, 4));
+                    u = fmaxf(u, __shfl_xor_sync(0xffffffffu, u, 2));
+                    u = fmaxf(u, __shfl_xor_sync(0xffffffffu, u, 1));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) top[i] = __shfl_sync(0xffffffffu, u, 8 * i);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float m_new = fmaxf(m[half + i], top[i]);
+                    const int pos = pos0 + (row0 + i) / G;
+                    corr[i] = expf(m[half + i] - m_new);
+                    m[half + i] = m_new;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        w[i][e] = base + lane + 32 * e <= pos ? expf(w[i][e] - m_new) : 0.0f;
+                        p[i * AT_LD + 32 * e] = w[i][e];
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    // the four warps' butterflies of block_sum at once (half of the lanes go on with half of them), then their sums in its order
+                    const bool up = (lane & 16) != 0, on = (lane & 8) != 0;
+                    const float u0 = (up ? w[i][2] : w[i][0]) + __shfl_xor_sync(0xffffffffu, up ? w[i][0] : w[i][2], 16);
+                    const float u1 = (up ? w[i][3] : w[i][1]) + __shfl_xor_sync(0xffffffffu, up ? w[i][1] : w[i][3], 16);
+                    float sum = (on ? u1 : u0) + __shfl_xor_sync(0xffffffffu, on ? u0 : u1, 8);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 16);              // 0 and 2; 1 and 3
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+                    l[half + i] = fmaf(l[half + i], corr[i], sum);
+                    if (lane == 0) sCorr[row0 + i] = corr[i];
+                }
             }
-            continue;                                      // (the barrier at the top of the next stage publishes the weights)
-        }
-        if (!(stage & 1)) {
+            __syncwarp();
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float corr = 4 * ty + i < rows ? sCorr[4 * ty + i] : 1.0f;
+                const float corr = sCorr[4 * ty + i];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) acc[i][j] *= corr;
             }
+            continue;                                      // (the barrier at the top of the next stage publishes the weights)
         }
         const float* p = sP + 4 * ty * AT_LD + off;
         const int first = base + off;
         // four keys at a time; `all`: every row of the tile sees them
-        auto add = [&](int j, bool all) {
+        auto add = [&](int j, bool all, const float4* v) {
             float w[4][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(w[i]) = *reinterpret_cast<const float4*>(p + i * AT_LD + j);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const float* row = kv + (j + e) * AT_LD + 4 * tx;
-                const float4 lo = *reinterpret_cast<const float4*>(row), hi = *reinterpret_cast<const float4*>(row + 64);
-                const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+                const float x[8] = {v[2 * e].x, v[2 * e].y, v[2 * e].z, v[2 * e].w, v[2 * e + 1].x, v[2 * e + 1].y, v[2 * e + 1].z, v[2 * e + 1].w};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     if (!all && first + j + e > row_pos[i]) continue;
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) acc[i][c] = fmaf(w[i][e], v[c], acc[i][c]);
+                    for (int c = 0; c < 8; ++c) acc[i][c] = fmaf(w[i][e], x[c], acc[i][c]);
                 }
+            }
+        };
+        auto take = [&](int j, float4* v) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float* row = kv + (j + e) * AT_LD + 4 * tx;
+                v[2 * e] = *reinterpret_cast<const float4*>(row);
+                v[2 * e + 1] = *reinterpret_cast<const float4*>(row + 64);
             }
         };
         const int whole = min(AT_HALF, max(0, pos0 - first + 1)) & ~3, most = min(AT_HALF, last - first + 1);
         int j = 0;
+        float4 v0[8], v1[8];                               // (the next four keys' values on their way while these are added)
+        take(0, v0);
 #pragma unroll 1
-        for (; j < whole; j += 4) add(j, true);
+        for (; j + 8 <= whole; j += 8) {
+            take(j + 4, v1);
+            add(j, true, v0);
+            take(min(j + 8, AT_HALF - 4), v0);
+            add(j + 4, true, v1);
+        }
 #pragma unroll 1
-        for (; j < most; j += 4) add(j, false);
+        for (; j < most; j += 4) {
+            add(j, j < whole, v0);
+            take(min(j + 4, AT_HALF - 4), v0);
+        }
     }
-    __syncthreads();                                       // (sCorr takes the sums now)
+    __syncwarp();                                          // (sCorr takes the sums now)
 #pragma unroll
     for (int i = 0; i < OWN; ++i)
         if (lane == 0) sCorr[OWN * warp + i] = l[i];
-    __syncthreads();
+    __syncwarp();
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int row = 4 * ty + i;
@@ -272,13 +349,23 @@ MB_API int mb_attention_tile(const void* q, const void* k_cache, const void* v_c
                              const int* cu_tokens, const int* seq_lens, int first_req, int count, int max_query_len, int H, int K, int d,
                              int page_size, float scale, cudaStream_t s) {
     if (count <= 0 || max_query_len <= 0) return 0;
-    if (d <= 0 || d > 128 || d % 4 != 0 || K <= 0 || H % K != 0 || H / K > AT_ROWS || page_size <= 0) return MB_ERR_BAD_SIZE;
-    const int per_tile = AT_ROWS / (H / K);
+    if (d <= 0 || d > 128 || d % 4 != 0 || K <= 0 || H % K != 0 || H / K > 32 || page_size <= 0) return MB_ERR_BAD_SIZE;
     if ((((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) & 15) != 0) return MB_ERR_BAD_SIZE;
-    cudaFuncSetAttribute(attention_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM);
-    dim3 grid((max_query_len + per_tile - 1) / per_tile, K, count);
-    return launch_kernel(attention_tile_kernel, grid, AT_THREADS, AT_SMEM, s, 0, (const float*)q, (const float*)k_cache, (const float*)v_cache,
-                         (float*)out, block_table, max_pages, cu_tokens, seq_lens, first_req, H, K, d, page_size, scale);
+    int page_shift = -1, sms = 0, device = 0;
+    for (int i = 0; i < 31; ++i)
+        if ((1 << i) == page_size) page_shift = i;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    // 32 rows a block where that makes two blocks an SM (what a block fetches is then shared by twice the rows); a row's bits do not depend on it
+    const int G = H / K, tiles = (max_query_len + 32 / G - 1) / (32 / G);
+    const bool wide = G > 16 || (long long)tiles * K * count >= 2 * sms;
+    const int per_tile = (wide ? 32 : 16) / G;
+    const dim3 grid((max_query_len + per_tile - 1) / per_tile, K, count);
+    const auto kernel = wide ? attention_tile_kernel<32> : attention_tile_kernel<16>;
+    const int rows = wide ? 32 : 16;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM(rows));
+    return launch_kernel(kernel, grid, 4 * rows, AT_SMEM(rows), s, 0, (const float*)q, (const float*)k_cache, (const float*)v_cache, (float*)out, block_table,
+                         max_pages, cu_tokens, seq_lens, first_req, H, K, d, page_size, page_shift, scale);
 }
 
 MB_API int mb_attention_simple(const void* q, const void* k_cache, const void* v_cache, void* out, int dtype,
