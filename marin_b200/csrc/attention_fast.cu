@@ -528,7 +528,7 @@ __global__ void __launch_bounds__(128, PF_MIN_CTAS) attn_prefill_kernel(
     bf16* sQ = reinterpret_cast<bf16*>(pf_smem);
     bf16* sKV = sQ + PF_BM * PF_LD;                  // [2 buffers][K then V][64][PF_LD]
     const int H = K * GROUP;
-    const int r = first_req + blockIdx.z, h = blockIdx.y, qt = gridDim.x - 1 - blockIdx.x;   // long tiles first
+    const int r = first_req + blockIdx.y, h = blockIdx.x, qt = gridDim.z - 1 - blockIdx.z;   // all heads' long tiles first
     const int tok0 = cu_tokens[r], n = cu_tokens[r + 1] - tok0;
     if (qt * PF_BM >= n) return;
     const int len = seq_lens[r], pos0 = len - n;
@@ -805,7 +805,7 @@ MB_API int mb_attn_prefill(const void* q, const void* k_cache, const void* v_cac
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    dim3 grid((max_query_len + PF_BM - 1) / PF_BM, K * GROUP, requests);
+    dim3 grid(K * GROUP, requests, (max_query_len + PF_BM - 1) / PF_BM);
     return launch_kernel(attn_prefill_kernel, grid, 128, PF_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache,
                          (bf16*)out, block_table, max_pages, cu_tokens, seq_lens, first_req, K, page_shift, scale, window);
 }

@@ -9,10 +9,10 @@
 // positions; the scores use the keys of g's kv head, the weights (one running softmax per row) multiply the values of
 // `VALUE_HEADS` kv heads at a time: with mixing (`all_heads`) every query head needs its weighted sum over every kv head's
 // values, A[g][c] (float32 [tokens][H][K][V_DIM]), which a second kernel mixes, out_h = sum_g talk[h][g] A[g][kv(h)]; a CTA
-// then takes the kv heads c0 .. c0 + VALUE_HEADS - 1 (blockIdx.y counts (g, c0 / VALUE_HEADS)) and repeats the scores for
+// then takes the kv heads c0 .. c0 + VALUE_HEADS - 1 (blockIdx.x counts (g, c0 / VALUE_HEADS)) and repeats the scores for
 // each such slice.  Without mixing a CTA sums the values of g's own kv head and writes bf16 [tokens][H][V_DIM].
 // Single tokens (`single`: every request of the step brings one token): the tile's rows are the GROUP query heads of one kv
-// head instead of 64 queries of one head (blockIdx.y counts (kv head, slice)), so the heads that share keys share their loads.
+// head instead of 64 queries of one head (blockIdx.x counts (kv head, slice)), so the heads that share keys share their loads.
 // `single` = 2 (mixing, at most four slices): a CTA takes a kv head's query heads with *all* slices, warp w working out the
 // sums of slice w over the one copy of the keys (the scores are cheap enough to repeat per warp); the value buffer then holds
 // every kv head's block.
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(128) attn_pooled_prefill_kernel(
     // (single: `h` is the first query head of the kv head, and row i of the tile is head h + i at the one position)
     const bool by_warp = single == 2;                        // every slice in this CTA, a warp each
     const int per_y = by_warp ? 1 : slices;
-    const int r = first_req + blockIdx.z, h = single ? (blockIdx.y / per_y) * GROUP : blockIdx.y / per_y, qt = gridDim.x - 1 - blockIdx.x;
+    const int r = first_req + blockIdx.y, h = single ? (blockIdx.x / per_y) * GROUP : blockIdx.x / per_y, qt = gridDim.z - 1 - blockIdx.z;   // all heads' long tiles first
     const int tok0 = cu_tokens[r], n = cu_tokens[r + 1] - tok0;
     if (qt * BM >= n) return;
     const int len = seq_lens[r], pos0 = len - n;
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(128) attn_pooled_prefill_kernel(
     const int kh = h / GROUP;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // c0, nvh: the kv heads whose values this warp sums; load_c0, load_n: those the CTA's value buffer holds
-    const int c0 = by_warp ? min(warp, slices - 1) * VH : all_heads ? (blockIdx.y % slices) * VH : kh;
+    const int c0 = by_warp ? min(warp, slices - 1) * VH : all_heads ? (blockIdx.x % slices) * VH : kh;
     const int nvh = all_heads ? min(VH, K - c0) : 1;
     const int load_c0 = by_warp ? 0 : c0, load_n = by_warp ? K : nvh;
     const int* table = block_table + (size_t)r * max_pages;
@@ -360,7 +360,7 @@ MB_API int mb_attn_pooled_prefill(const void* q, const void* k_cache, const void
         if (wide <= 200 * 1024) { single = 2; smem = wide > smem ? wide : smem; }
     }
     cudaFuncSetAttribute(attn_pooled_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    dim3 grid((max_query_len + BM - 1) / BM, single == 2 ? K : (single ? K : K * GROUP) * slices, count);
+    dim3 grid(single == 2 ? K : (single ? K : K * GROUP) * slices, count, (max_query_len + BM - 1) / BM);
     return launch_kernel(attn_pooled_prefill_kernel, grid, 128, smem, s, 0, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache,
                          (const bf16*)k_pool, (const bf16*)v_pool, parts, (bf16*)out, block_table, max_pages, cu_tokens, seq_lens, first_req, K,
                          shift, scale, cap, window, pool, pool_rows, all_heads, single);

@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(AS_THREADS) attention_simple_kernel(
 // step goes by 16 rows and 64 threads a block, twice as many blocks of half the length.  Measured on B200 (333 tokens, 16 heads of 128 over 8 kv heads):
 // attention_simple_kernel 605 us; by 32 rows, a half's rows looked up behind a division each (2,300 clocks a half) and the softmax row by row
 // (6,000 a chunk) 88 us; rows looked up side by side 72; the softmax's rows interleaved and 16 rows a block 57 (400 tokens, 32 heads over 8, 32 rows
-// a block: 109 and 91).  With 4 x 2 and 4 x 4 a thread and twice the threads 65.
+// a block: 109 and 91); all heads' last tiles first 45.  With 4 x 2 and 4 x 4 a thread and twice the threads 65.
 #define AT_CHUNK AS_THREADS
 #define AT_HALF 64
 #define AT_LD 132                     // floats a row of 128 takes in shared memory
@@ -115,9 +115,9 @@ __global__ void __launch_bounds__(4 * AT_ROWS, 2) attention_tile_kernel(
     float* sKV = sP + AT_ROWS * AT_LD;                     // two half chunks of keys or values in turn
     float* sCorr = sKV + 2 * AT_HALF * AT_LD;              // [rows]
     const int G = H / K, per_tile = AT_ROWS / G;
-    const int r = first_req + blockIdx.z, kh = blockIdx.y;
+    const int r = first_req + blockIdx.y, kh = blockIdx.x % K;
     const int tok0 = cu_tokens[r], n = cu_tokens[r + 1] - tok0;
-    const int q0 = (gridDim.x - 1 - blockIdx.x) * per_tile;                   // (the longest walks first)
+    const int q0 = (gridDim.x - 1 - blockIdx.x) / K * per_tile;               // (the longest walks first, of all heads)
     if (q0 >= n) return;
     const int queries = min(per_tile, n - q0), rows = queries * G;
     const int pos0 = seq_lens[r] - n + q0, last = pos0 + queries - 1;         // positions of the tile's first and last query
@@ -360,7 +360,7 @@ MB_API int mb_attention_tile(const void* q, const void* k_cache, const void* v_c
     const int G = H / K, tiles = (max_query_len + 32 / G - 1) / (32 / G);
     const bool wide = G > 16 || (long long)tiles * K * count >= 2 * sms;
     const int per_tile = (wide ? 32 : 16) / G;
-    const dim3 grid((max_query_len + per_tile - 1) / per_tile, K, count);
+    const dim3 grid((max_query_len + per_tile - 1) / per_tile * K, count);
     const auto kernel = wide ? attention_tile_kernel<32> : attention_tile_kernel<16>;
     const int rows = wide ? 32 : 16;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM(rows));

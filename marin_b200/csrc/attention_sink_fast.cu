@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(128, 2) attn_sink_prefill_kernel(
     bf16* sV = sK + BN * LDK;
 #endif
     const int H = K * GROUP;
-    const int r = first_req + blockIdx.z, h = blockIdx.y, qt = gridDim.x - 1 - blockIdx.x;   // long tiles first
+    const int r = first_req + blockIdx.y, h = blockIdx.x, qt = gridDim.z - 1 - blockIdx.z;   // all heads' long tiles first
     const int tok0 = cu_tokens[r], count = cu_tokens[r + 1] - tok0;
     if (qt * BM >= count) return;
     const int len = seq_lens[r], pos0 = len - count;
@@ -646,7 +646,7 @@ MB_API int mb_attn_sink_prefill(const void* q, const void* k_cache, const void* 
     const int shift = page_shift_of(page_size);
     if (shift < 0 || window < 0 || chunk < 0 || keep < 0 || (wide_out == nullptr && (out_stride < K * GROUP * DV || out_stride % 2 != 0))) return MB_ERR_BAD_SIZE;
     cudaFuncSetAttribute(attn_sink_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM);
-    dim3 grid((max_query_len + BM - 1) / BM, K * GROUP, count);
+    dim3 grid(K * GROUP, count, (max_query_len + BM - 1) / BM);
     return launch_kernel(attn_sink_prefill_kernel, grid, 128, PF_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache,
                          (bf16*)out, block_table, max_pages, cu_tokens, seq_lens, first_req, K, shift, scale, window, chunk, sink, sink_logit,
                          (const bf16*)gate, gate_stride, keep, softcap, out_scale, out_stride, wide_out);

@@ -89,14 +89,6 @@ __device__ __forceinline__ float ta_exp2(float x) {
     return y;
 }
 
-// MN-major B operand (V: rows are keys, 64 head columns contiguous per 128-byte swizzled row): 8-key groups 1024 bytes
-// apart (stride offset), 64-column halves `half_bytes` apart (leading offset).
-__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t smem_addr, uint32_t half_bytes) {
-    const uint32_t lo = ((smem_addr & 0x3FFFFu) >> 4) | ((half_bytes >> 4) << 16);
-    const uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);
-    return ((uint64_t)hi << 32) | lo;
-}
-
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
     uint32_t r[32];
     asm volatile(
@@ -207,13 +199,13 @@ __device__ __forceinline__ void tmem_st32_bits(uint32_t taddr, const uint32_t* v
 }
 
 #ifdef TA_PROBE
-// Where the roles wait (a build for measuring only, -DTA_PROBE): per CTA (x + gridDim.x * y of request 0), clock ticks
+// Where the roles wait (a build for measuring only, -DTA_PROBE): per CTA (x + gridDim.x * z of request 0), clock ticks
 // of [0] row 0 waiting for S, [1] row 0 waiting for O before a rescale, [2] row 0's loop in all, [3] the MMA thread
 // finding nothing to issue, [4] the MMA thread's loop in all, [5] the key blocks.
 __device__ long long ta_probe[4096 * 8];
 MB_API int mb_attn_prefill_tc_probe_read(long long* host) { return (int)cudaMemcpyFromSymbol(host, ta_probe, sizeof(ta_probe)); }
 #define TA_T() clock64()
-#define TA_OUT(slot, v) do { const int cta_ = blockIdx.x + gridDim.x * blockIdx.y; if (blockIdx.z == 0 && cta_ < 4096) ta_probe[cta_ * 8 + (slot)] = (v); } while (0)
+#define TA_OUT(slot, v) do { const int cta_ = blockIdx.x + gridDim.x * blockIdx.z; if (blockIdx.y == 0 && cta_ < 4096) ta_probe[cta_ * 8 + (slot)] = (v); } while (0)
 #else
 #define TA_T() 0LL
 #define TA_OUT(slot, v) do { (void)(v); } while (0)
@@ -257,7 +249,9 @@ __global__ void __launch_bounds__(256, 2) attn_prefill_tc_kernel(
     volatile int* abort = (volatile int*)(tmem_slot + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     PDL_ENTER_EARLY();
-    const int r = first_req + blockIdx.z, h = blockIdx.y * (TA_PAIR + 1), qt = gridDim.x - 1 - blockIdx.x;   // long tiles first
+    // all heads' long tiles first (head by head the last heads' long tiles began when the first heads' short ones were done: 2,048 tokens of 32 heads 64 us,
+    // so 49)
+    const int r = first_req + blockIdx.y, h = blockIdx.x * (TA_PAIR + 1), qt = gridDim.z - 1 - blockIdx.z;
     const int tok0 = cu_tokens[r], n = cu_tokens[r + 1] - tok0;
     if (qt * TA_TOK >= n) return;                           // nothing to do here (before any tensor memory is taken)
     if ((smem_u32(smem) & 1023u) != 0) { if (threadIdx.x == 0) atomicExch(error_flag, 20); return; }
@@ -297,7 +291,7 @@ __global__ void __launch_bounds__(256, 2) attn_prefill_tc_kernel(
     // The online softmax does not care about the order of the key blocks.  Every CTA starts at another block, so that
     // the many CTAs that read the same keys and values (the query tiles of a request, the heads of a group) do not
     // all ask the L2 for the same lines at the same moment.
-    const int rot = (int)(((unsigned)(h * gridDim.x + qt) * 37u) % (unsigned)nblk);
+    const int rot = (int)(((unsigned)(h * gridDim.z + qt) * 37u) % (unsigned)nblk);
     auto block_of = [&](int i) {
         int j = i + rot;
         j = j >= nblk ? j - nblk : j;
@@ -682,7 +676,7 @@ MB_API int mb_attn_prefill_tc(const void* q, const void* k_cache, const void* v_
     if (rc) return rc;
     rc = TA_V_IN_K ? map_2d(&mv, k_cache, cache_rows, D, box_rows) : map_2d(&mv, v_cache, cache_rows, DV, box_rows);
     if (rc) return rc;
-    dim3 grid((max_query_len + TA_TOK - 1) / TA_TOK, K * GROUP / (TA_PAIR + 1), requests);
+    dim3 grid(K * GROUP / (TA_PAIR + 1), requests, (max_query_len + TA_TOK - 1) / TA_TOK);
     return launch_kernel(softcap > 0.0f ? attn_prefill_tc_kernel<true> : attn_prefill_tc_kernel<false>, grid, 256, TA_SMEM, s, 0, mq, mk, mv, (bf16*)out,
                          block_table, max_pages, cu_tokens, seq_lens, first_req, K, page_shift, scale, window, error_flag, box_rows, chunk, sink, sink_logit,
                          (const bf16*)gate, gate_stride, keep, softcap, out_scale, out_stride, lam, eps);

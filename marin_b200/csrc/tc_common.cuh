@@ -49,6 +49,14 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
     return ((uint64_t)hi << 32) | lo;
 }
 
+// MN-major B operand (V: rows are keys, 64 head columns contiguous per 128-byte swizzled row): 8-key groups 1024 bytes
+// apart (stride offset), 64-column halves `half_bytes` apart (leading offset).
+__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t smem_addr, uint32_t half_bytes) {
+    const uint32_t lo = ((smem_addr & 0x3FFFFu) >> 4) | ((half_bytes >> 4) << 16);
+    const uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);
+    return ((uint64_t)hi << 32) | lo;
+}
+
 // MMAs are issued by a whole warp, for which one elected lane acts: the choice of the lane is a predicate of the instruction and no branch, and what decides
 // about loops and branches around it is the same in all lanes for all the compiler knows (warp_same, mbar_wait_warp).  Descriptors and addresses then stay in
 // uniform registers, where the instruction wants them.  Behind a branch of one lane every MMA carried them over first: about 106 cycles each whatever
