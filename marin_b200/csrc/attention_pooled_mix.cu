@@ -7,19 +7,20 @@
 // times the products with V, and a float32 [tokens][H][KV_HEADS][V_DIM] that a second kernel reads.)  Mixing needs the weights already
 // divided by their sums, so three kernels:
 //   stats_kernel  (a CTA per kv head and 128 rows = queries x its heads): the logarithm of every row's sum of weights;
-//   mix_kernel    (a CTA per 16 queries, two heads a warp, 32 keys at a time): the weights of all heads, mixed, to scratch memory in 16 bits;
-//   value_kernel  (a CTA per 32 queries and kv head, a warp per head and 16 queries): mixed weights x values.
+//   mix_kernel    (equal runs of the tiles' blocks a CTA, two heads a warp, 16 queries x 16 keys a step): the weights of all heads, mixed, to scratch memory in 16 bits;
+//   value_kernel  (a CTA per 128 rows of a kv head, tcgen05): mixed weights x values.
 // Exactness: the weights p are float32 and enter the mixing product as pairs of bf16 numbers (p = hi + lo), as does talk; the three larger of the four
 // products are taken, so about 16 bits of each enter.  The mixed weights, bounded numbers, wait as halves under one power of two for all of them (11 bits) and
 // meet the values as two bf16 numbers that hold the 11 bits exactly: they add next to nothing to the error that rounding the results
 // makes, where weights rounded to bf16 (every head's, in the other kernel) made it 1.17 times as large.
-// Scratch: [tile][block][H][16][32] halves, a tile of 16 queries of one request, its blocks of 32 pooled rows, then of 32 positions.
+// Scratch: [tile][block][kv head][query][8 keys][its head][key] halves, a tile of 16 queries of one request, its blocks of 32 pooled rows, then of 32 positions.
 // Measured on B200, 2,048 tokens, 32 heads of 128 over 8, window 1,024, pools of 64: the other kernel and its mixing 1,189 us;
-// these 95 + 216 + 141 us (the values 100 with weights rounded to bf16, one product a block instead of two).  mix_kernel is bound by the instructions that make a weight (about fourteen a score, with the cap) and its two mixing products.
+// these 79 + 166 + 72 us (95 + 216 + 141 with a CTA a tile in the mixing, three barriers a block and the values on mma.sync).  mix_kernel is bound by issue: about a
+// thousand instructions a warp and block (cap, exponential, two parts, their stores) behind which its products of 3,600 clocks a block hide.
 #define MB_LIB "attention_pooled_mix"
 #define MB_LIB_ID 25
 #include <cuda_fp16.h>
-#include "common.cuh"
+#include "tc_common.cuh"
 #include "launch.cuh"
 #include "mma_helpers.cuh"
 
@@ -47,7 +48,6 @@ static_assert(GROUP * KV_HEADS == 16 || GROUP * KV_HEADS == 32, "16 or 32 query 
 #define NQ 16                         // queries a tile
 #define NK 32                         // keys a block
 #define LDK (D + 8)                   // padded rows in shared memory (elements): ldmatrix without bank conflicts
-#define LDV (DV + 8)
 #define LOG2E 1.4426950408889634f
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256, 2) stats_kernel(
     q = pdl_fresh(q); k_cache = pdl_fresh(k_cache); k_pool = pdl_fresh(k_pool);
     extern __shared__ __align__(16) uint8_t smem_raw[];
     bf16* sK = reinterpret_cast<bf16*>(smem_raw);
-    const int r = first_req + blockIdx.z, kh = blockIdx.y, qt = gridDim.x - 1 - blockIdx.x;
+    const int r = first_req + blockIdx.y, kh = blockIdx.x, qt = gridDim.z - 1 - blockIdx.z;          // all heads' long tiles first
     const int tok0 = cu_tokens[r], n = cu_tokens[r + 1] - tok0;
     if (qt * SQ >= n) return;
     const int here = min(SQ, n - qt * SQ), pos0 = seq_lens[r] - n + qt * SQ;
@@ -252,14 +252,17 @@ __global__ void __launch_bounds__(256, 2) stats_kernel(
 #define WK (G / HW)                   // warps a kv head
 #define MIX_WARPS (KH * WK)
 #define MIX_THREADS (32 * MIX_WARPS)
+#define HK 16                         // keys a step: half a block
 #define P_PITCH (2 * NH + 16)         // bytes of a pair's row of H weights
-#define P_QUERY (NK * P_PITCH + 16)   // bytes between queries (ldmatrix over a query's keys and the stores over queries both spread over the banks)
-#define P_BYTES (NQ * P_QUERY)
-#define W_PITCH (2 * NK + 16)         // bytes of a mixed row (one head and query)
-#define W_HEAD (NQ * W_PITCH + 16)
+#define P_BYTES (NQ * HK * P_PITCH + NQ / 4 * 16)
 #define TALK_FRAGS ((NH / 16) * (NH / 16))
-#define MIX_SMEM (KH * NK * LDK * 2 + 2 * P_BYTES + NH * W_HEAD + 2 * TALK_FRAGS * 512)
-static_assert(MIX_SMEM <= 227 * 1024, "the mixing kernel's tiles do not fit shared memory");
+#define MIX_SMEM (2 * KH * HK * LDK * 2 + 4 * P_BYTES + 2 * TALK_FRAGS * 4 * 512)
+static_assert(MIX_SMEM <= 220 * 1024, "the mixing kernel's tiles do not fit shared memory");
+// Where a query's row of pairs begins: a group of four queries 16 bytes further on, and a query's heads two by two turned by query % 4 within 16 bytes, so that the
+// 32 rows a warp writes a word of lie in 32 banks (rows of whole 16 bytes alone: four of them a bank).  talk's columns are turned alike.
+struct MixWhole { static constexpr bool value = false; };
+struct MixMasked { static constexpr bool value = true; };
+__device__ __forceinline__ int p_row(int query) { return query * HK * P_PITCH + (query >> 2) * 16; }
 
 __device__ __forceinline__ void split_bf16(float x, float y, uint32_t& hi, uint32_t& lo) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
@@ -283,262 +286,428 @@ __device__ __forceinline__ int mixed_shift(const float* __restrict__ talk, int l
 }
 __device__ __forceinline__ float two_to(int n) { return __int_as_float((127 + n) << 23); }
 
+// The blocks of a step's tiles end to end, dealt out in equal runs over the CTAs: a tile ahead of a whole window has few blocks, and one CTA a tile left
+// SMs idle for a third of the time.
 __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
     const bf16* __restrict__ q, const bf16* __restrict__ k_cache, const bf16* __restrict__ k_pool, const float* __restrict__ lse,
     const float* __restrict__ talk, __half* __restrict__ mixed, const int* __restrict__ block_table, int max_pages, const int* __restrict__ cu_tokens,
-    const int* __restrict__ seq_lens, int first_req, int page_shift, float scale, float cap, int window, int pool, int pool_rows, int most_blocks) {
+    const int* __restrict__ seq_lens, int first_req, int reqs, int page_shift, float scale, float cap, int window, int pool, int pool_rows, int most_blocks) {
     PDL_ENTER();
     q = pdl_fresh(q); k_cache = pdl_fresh(k_cache); k_pool = pdl_fresh(k_pool); lse = pdl_fresh(lse);
     extern __shared__ __align__(16) uint8_t smem_raw[];
-    bf16* sK = reinterpret_cast<bf16*>(smem_raw);              // [KH][NK][LDK]: a kv head's block is fetched and read by its own warps
-    uint8_t* sPh = smem_raw + KH * NK * LDK * 2;               // [NQ][NK] rows of H weights: the larger part ...
-    uint8_t* sPl = sPh + P_BYTES;                              // ... and what it leaves
-    uint8_t* sW = sPl + P_BYTES;                               // [H][NQ] rows of NK mixed weights
-    uint4* sT = reinterpret_cast<uint4*>(sW + NH * W_HEAD);    // talk as A operands: [2 parts][H / 16][H / 16][lane]
-    const int r = first_req + blockIdx.z, qt = gridDim.x - 1 - blockIdx.x;
-    const int tok0 = cu_tokens[r], n = cu_tokens[r + 1] - tok0;
-    if (qt * NQ >= n) return;
-    const int here = min(NQ, n - qt * NQ), pos0 = seq_lens[r] - n + qt * NQ;
-    const int* table = block_table + (size_t)r * max_pages;
-    const Blocks blocks(pos0, pos0 + here - 1, window, pool, NK);
-    __half* dst = mixed + (size_t)(first_tile(cu_tokens, first_req, r) + qt) * most_blocks * (NH * NQ * NK);
+    __shared__ int s_before[MIX_THREADS], s_warp[MIX_WARPS];
+    bf16* sK = reinterpret_cast<bf16*>(smem_raw);              // two of [KH][HK][LDK]: a kv head's keys are fetched and read by its own warps
+    uint8_t* sP = smem_raw + 2 * KH * HK * LDK * 2;            // two of [2][NQ][HK] rows of H weights: the larger part and what it leaves
+    uint4* sT = reinterpret_cast<uint4*>(sP + 4 * P_BYTES);    // talk as A operands: [turned by][2 parts][H / 16][H / 16][lane]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t2 = 2 * (lane & 3);
-    const int kv = warp / WK;
-    bf16* myK = sK + kv * NK * LDK;
-    auto fetch = [&](int b) {                                  // this warp's part of its kv head's keys: 16 bytes a lane
-        const bool pooled = blocks.is_pooled(b);
-        const int key0 = blocks.key0(b, NK), begin = blocks.begin(b), end = blocks.end(b);
-        const bf16* src = pooled ? k_pool : k_cache;
-        constexpr int PER = D / 8;
-#pragma unroll 4
-        for (int idx = warp % WK * 32 + lane; idx < NK * PER; idx += 32 * WK) {
-            const int row = idx / PER, c = idx % PER, key = key0 + row;
-            if (key >= begin && key <= end) cp_async16(myK + row * LDK + c * 8, src + row_at(table, key, pooled, kv, page_shift, pool, pool_rows) * D + c * 8);
-            else *reinterpret_cast<uint4*>(myK + row * LDK + c * 8) = make_uint4(0, 0, 0, 0);
+    const int last_req = first_req + reqs - 1, tiles_all = first_tile(cu_tokens, first_req, last_req + 1);
+    // the tile of this number: its request, and how many of it there are before (-1: none has this number)
+    auto request_of = [&](int tile) {
+        int lo = first_req, hi = last_req;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (first_tile(cu_tokens, first_req, mid) <= tile) lo = mid;
+            else hi = mid - 1;
         }
-        cp_async_commit();
+        return lo;
     };
-    fetch(0);
-    for (int idx = tid; idx < TALK_FRAGS * 32; idx += MIX_THREADS) {
-        const int frag = idx / 32, l = idx % 32, row = frag / (NH / 16) * 16 + (l >> 2), col = frag % (NH / 16) * 16 + 2 * (l & 3);
+    auto blocks_of = [&](int tile) {
+        if (tile >= tiles_all) return 0;
+        const int r = request_of(tile), q0 = (tile - first_tile(cu_tokens, first_req, r)) * NQ, n = cu_tokens[r + 1] - cu_tokens[r];
+        if (q0 >= n) return 0;
+        const int pos0 = seq_lens[r] - n + q0;
+        return Blocks(pos0, pos0 + min(NQ, n - q0) - 1, window, pool, NK).count;
+    };
+    const int per = (tiles_all + MIX_THREADS - 1) / MIX_THREADS;
+    int units;                                                 // blocks of all tiles
+    {
+        int mine = 0;
+        for (int i = 0; i < per; ++i) mine += blocks_of(tid * per + i);
+        int sum = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+        }
+        if (lane == 31) s_warp[warp] = sum;
+        __syncthreads();
+        int before = 0;
+        units = 0;
+        for (int w = 0; w < MIX_WARPS; ++w) {
+            if (w < warp) before += s_warp[w];
+            units += s_warp[w];
+        }
+        s_before[tid] = before + sum - mine;
+    }
+    int unit = (int)((long long)units * blockIdx.x / gridDim.x);
+    const int unit_end = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
+    if (unit >= unit_end) return;
+    constexpr int MT = NH / 16;                                // 16 mixed heads at a time: a warp keeps to one of the MT
+    const int mt = warp % MT, turned = (warp / MT) & 3;        // and to queries that are turned alike
+    for (int idx = tid; idx < 4 * TALK_FRAGS * 32; idx += MIX_THREADS) {
+        const int turn = idx / (TALK_FRAGS * 32), frag = idx / 32 % TALK_FRAGS, l = idx % 32, row = frag / MT * 16 + (l >> 2);
+        const int col = frag % MT * 16 + 2 * ((l - turn) & 3);
         uint4 hi, lo;
         split_bf16(talk[row * NH + col], talk[row * NH + col + 1], hi.x, lo.x);
         split_bf16(talk[(row + 8) * NH + col], talk[(row + 8) * NH + col + 1], hi.y, lo.y);
         split_bf16(talk[row * NH + col + 8], talk[row * NH + col + 9], hi.z, lo.z);
         split_bf16(talk[(row + 8) * NH + col + 8], talk[(row + 8) * NH + col + 9], hi.w, lo.w);
-        sT[idx] = hi;
-        sT[TALK_FRAGS * 32 + idx] = lo;
+        sT[(turn * 2) * TALK_FRAGS * 32 + frag * 32 + l] = hi;
+        sT[(turn * 2 + 1) * TALK_FRAGS * 32 + frag * 32 + l] = lo;
     }
-    // the queries of this warp's heads stay in registers; a thread's rows are queries g8 and g8 + 8
-    uint32_t qa[HW][D / 16][4];
-    float base[HW][2];
-    int qp[2], lo[2], nb[2];
-#pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-        qp[rr] = g8 + 8 * rr < here ? pos0 + g8 + 8 * rr : -1;          // (a query that is not there sees nothing)
-        lo[rr] = first_seen(qp[rr], window);
-        nb[rr] = qp[rr] >= 0 ? pools_seen(qp[rr], window, pool) : 0;
-    }
-#pragma unroll
-    for (int h = 0; h < HW; ++h) {
-        const size_t a0 = (size_t)(tok0 + qt * NQ + g8) * NH + warp * HW + h, a1 = a0 + (size_t)8 * NH;
-        const bf16 *r0 = qp[0] >= 0 ? q + a0 * D : nullptr, *r1 = qp[1] >= 0 ? q + a1 * D : nullptr;
-        base[h][0] = qp[0] >= 0 ? lse[a0] : 0.0f;
-        base[h][1] = qp[1] >= 0 ? lse[a1] : 0.0f;
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) q_fragment(qa[h][kk], r0, r1, kk * 16 + t2);
-    }
-    const Cap c(scale, cap);
     const float up = two_to(mixed_shift(talk, lane));
+    const Cap c(scale, cap);
+    const int kv = warp / WK;
+    bf16* myK = sK + kv * HK * LDK;
     const uint32_t k_addr = (uint32_t)__cvta_generic_to_shared(myK + ((lane & 7) + (lane >> 4) * 8) * LDK + ((lane >> 3) & 1) * 8);
     // a pair's row read as a B operand: eight keys of one query, 8 weights a matrix, up to 32 weights at a time
-    const uint32_t p_addr = (uint32_t)__cvta_generic_to_shared(sPh + (lane & 7) * P_PITCH + (lane >> 3) * 16);
-    constexpr int MT = NH / 16;                                // 16 mixed heads at a time: a warp keeps to one of the MT, whose operands it loads once a block
-    const int mt = warp % MT;
-    cp_async_wait<0>();
-    __syncthreads();                                           // the first block's keys and talk are there
-    for (int b = 0; b < blocks.count; ++b) {
-        const bool pooled = blocks.is_pooled(b);
-        const int key0 = blocks.key0(b, NK);
-        float s[HW][NK / 8][4];
-#pragma unroll
-        for (int h = 0; h < HW; ++h)
-#pragma unroll
-            for (int j = 0; j < NK / 8; ++j) s[h][j][0] = s[h][j][1] = s[h][j][2] = s[h][j][3] = 0.0f;
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
-#pragma unroll
-            for (int j = 0; j < NK / 8; j += 2) {
-                uint32_t b0, b1, b2, b3;
-                ldsm_x4(k_addr + (uint32_t)(j * 8 * LDK * 2 + kk * 32), b0, b1, b2, b3);
-#pragma unroll
-                for (int h = 0; h < HW; ++h) {
-                    mma_bf16_16816(s[h][j], qa[h][kk], b0, b1);
-                    mma_bf16_16816(s[h][j + 1], qa[h][kk], b2, b3);
-                }
-            }
-        c.apply<HW * NK / 8>(&s[0][0]);
-        const bool inside = pooled ? key0 + NK <= nb[0] && qp[1] >= 0 : key0 + NK - 1 <= qp[0] && key0 >= lo[1] && qp[1] >= 0;
-        // the weights, in two parts, to the pairs' rows
-#pragma unroll
-        for (int j = 0; j < NK / 8; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int rr = e >> 1, in = j * 8 + t2 + (e & 1), kj = key0 + in;
-                float w0 = ex2_approx(fmaf(s[0][j][e], c.sl2, -base[0][rr])), w1 = ex2_approx(fmaf(s[1][j][e], c.sl2, -base[1][rr]));
-                if (!inside && !(pooled ? kj < nb[rr] : (kj <= qp[rr] && kj >= lo[rr]))) w0 = w1 = 0.0f;
-                uint32_t hi, low;
-                split_bf16(w0, w1, hi, low);
-                const int at = (g8 + 8 * rr) * P_QUERY + in * P_PITCH + warp * HW * 2;
-                *reinterpret_cast<uint32_t*>(sPh + at) = hi;
-                *reinterpret_cast<uint32_t*>(sPl + at) = low;
-            }
-        __syncthreads();                                       // every head's weights of the block are there; its keys and the last mixed rows are done with
-        if (b + 1 < blocks.count) fetch(b + 1);
-        // talk x weights: eight pairs (one query, eight keys) at a time
-        uint4 th[MT], tl[MT];
-#pragma unroll
-        for (int ks = 0; ks < MT; ++ks) { th[ks] = sT[(mt * MT + ks) * 32 + lane]; tl[ks] = sT[(TALK_FRAGS + mt * MT + ks) * 32 + lane]; }
-#pragma unroll 4
-        for (int job = warp / MT; job < NQ * (NK / 8); job += MIX_WARPS / MT) {
-            const int query = job / (NK / 8), k8 = job % (NK / 8) * 8;
-            uint32_t ph[4], pl[4];
-            const uint32_t row = p_addr + (uint32_t)(query * P_QUERY + k8 * P_PITCH);
-            if (NH == 32) {
-                ldsm_x4(row, ph[0], ph[1], ph[2], ph[3]);
-                ldsm_x4(row + P_BYTES, pl[0], pl[1], pl[2], pl[3]);
-            } else {
-                // (16 heads: two matrices; the upper lanes' addresses are not used)
-                asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(ph[0]), "=r"(ph[1]) : "r"(row));
-                asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(pl[0]), "=r"(pl[1]) : "r"(row + P_BYTES));
-            }
-            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-            for (int ks = 0; ks < MT; ++ks) {
-                const uint32_t ah[4] = {th[ks].x, th[ks].y, th[ks].z, th[ks].w}, al[4] = {tl[ks].x, tl[ks].y, tl[ks].z, tl[ks].w};
-                mma_bf16_16816(acc, ah, ph[2 * ks], ph[2 * ks + 1]);
-                mma_bf16_16816(acc, al, ph[2 * ks], ph[2 * ks + 1]);
-                mma_bf16_16816(acc, ah, pl[2 * ks], pl[2 * ks + 1]);
-            }
-            uint8_t* w = sW + (mt * 16 + g8) * W_HEAD + query * W_PITCH + (k8 + t2) * 2;
-            *reinterpret_cast<uint32_t*>(w) = pack_half(acc[0] * up, acc[1] * up);
-            *reinterpret_cast<uint32_t*>(w + 8 * W_HEAD) = pack_half(acc[2] * up, acc[3] * up);
+    const uint32_t p_addr = (uint32_t)__cvta_generic_to_shared(sP + (lane & 7) * P_PITCH + (lane >> 3) * 16);
+    const int p_at = p_row(g8) + t2 * P_PITCH + ((warp * HW / 2) & ~3) * 4 + ((warp * HW / 2 + g8) & 3) * 4;   // where this warp's pair of heads lies in query g8's rows
+    __syncthreads();                                           // s_before and talk are there
+    int tile;                                                  // the tile this CTA begins in
+    {
+        int lo = 0, hi = MIX_THREADS - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (s_before[mid] <= unit) lo = mid;
+            else hi = mid - 1;
         }
-        cp_async_wait<0>();
-        __syncthreads();                                       // the mixed rows and the next block's keys are there; the pairs' rows may be written again
-        for (int idx = tid; idx < NH * NQ * (NK / 8); idx += MIX_THREADS) {
-            const int row = idx / (NK / 8), c8 = idx % (NK / 8);
-            *reinterpret_cast<uint4*>(dst + (size_t)b * (NH * NQ * NK) + row * NK + c8 * 8) =
-                *reinterpret_cast<const uint4*>(sW + (row / NQ) * W_HEAD + (row % NQ) * W_PITCH + c8 * 16);
+        tile = lo * per;
+        int before = s_before[lo];
+        for (int n; before + (n = blocks_of(tile)) <= unit; ++tile) before += n;
+        unit -= before;                                        // (from here on: the first block of the tile; unit_end counts down with it)
+        lo = before;
+        hi = unit_end - before;
+        for (int left = hi; left > 0; ++tile, unit = 0) {
+            const int count = blocks_of(tile);
+            if (count == 0) continue;
+            const int b_end = min(count, left);
+            left -= count;
+            const int r = request_of(tile), qt = tile - first_tile(cu_tokens, first_req, r), tok0 = cu_tokens[r], n = cu_tokens[r + 1] - tok0;
+            const int here = min(NQ, n - qt * NQ), pos0 = seq_lens[r] - n + qt * NQ;
+            const int* table = block_table + (size_t)r * max_pages;
+            const Blocks blocks(pos0, pos0 + here - 1, window, pool, NK);
+            __half* dst = mixed + (size_t)tile * most_blocks * (NH * NQ * NK);
+            const int steps = 2 * (b_end - unit), b0 = unit;
+            auto fetch = [&](int step) {                       // this warp's part of its kv head's keys: 16 bytes a lane
+                if (step < steps) {
+                    const int b = b0 + (step >> 1);
+                    const bool pooled = blocks.is_pooled(b);
+                    const int key0 = blocks.key0(b, NK) + (step & 1) * HK, begin = blocks.begin(b), end = blocks.end(b);
+                    const bf16* src = pooled ? k_pool : k_cache;
+                    bf16* to = myK + (step & 1) * KH * HK * LDK;
+                    constexpr int PER = D / 8;
+                    if (!pooled && page_shift >= 4 && key0 >= begin && key0 + HK - 1 <= end) {          // rows of one page, one behind the other
+                        const bf16* from = src + row_at(table, key0, false, kv, page_shift, pool, pool_rows) * D;
+#pragma unroll
+                        for (int i = 0; i < HK * PER; i += 32 * WK) {
+                            const int idx = i + warp % WK * 32 + lane;
+                            if (HK * PER % (32 * WK) == 0 || idx < HK * PER) cp_async16(to + idx / PER * LDK + idx % PER * 8, from + idx * 8);
+                        }
+                    } else {
+#pragma unroll 1
+                        for (int idx = warp % WK * 32 + lane; idx < HK * PER; idx += 32 * WK) {
+                            const int row = idx / PER, c8 = idx % PER, key = key0 + row;
+                            if (key >= begin && key <= end) cp_async16(to + row * LDK + c8 * 8, src + row_at(table, key, pooled, kv, page_shift, pool, pool_rows) * D + c8 * 8);
+                            else *reinterpret_cast<uint4*>(to + row * LDK + c8 * 8) = make_uint4(0, 0, 0, 0);
+                        }
+                    }
+                }
+                cp_async_commit();
+            };
+            fetch(0);
+            fetch(1);
+            // the queries of this warp's heads stay in registers; a thread's rows are queries g8 and g8 + 8
+            uint32_t qa[HW][D / 16][4];
+            float base[HW][2];
+            int qp[2], seen[2], nb[2];
+#pragma unroll
+            for (int rr = 0; rr < 2; ++rr) {
+                qp[rr] = g8 + 8 * rr < here ? pos0 + g8 + 8 * rr : -1;          // (a query that is not there sees nothing)
+                seen[rr] = first_seen(qp[rr], window);
+                nb[rr] = qp[rr] >= 0 ? pools_seen(qp[rr], window, pool) : 0;
+            }
+#pragma unroll
+            for (int h = 0; h < HW; ++h) {
+                const size_t a0 = (size_t)(tok0 + qt * NQ + g8) * NH + warp * HW + h, a1 = a0 + (size_t)8 * NH;
+                const bf16 *r0 = qp[0] >= 0 ? q + a0 * D : nullptr, *r1 = qp[1] >= 0 ? q + a1 * D : nullptr;
+                base[h][0] = qp[0] >= 0 ? lse[a0] : 0.0f;
+                base[h][1] = qp[1] >= 0 ? lse[a1] : 0.0f;
+#pragma unroll
+                for (int kk = 0; kk < D / 16; ++kk) q_fragment(qa[h][kk], r0, r1, kk * 16 + t2);
+            }
+            float s[HW][HK / 8][4];
+            auto scores = [&](int step) {
+                const uint32_t at = k_addr + (uint32_t)((step & 1) * KH * HK * LDK * 2);
+#pragma unroll
+                for (int h = 0; h < HW; ++h)
+#pragma unroll
+                    for (int j = 0; j < HK / 8; ++j) s[h][j][0] = s[h][j][1] = s[h][j][2] = s[h][j][3] = 0.0f;
+#pragma unroll
+                for (int kk = 0; kk < D / 16; ++kk) {
+                    uint32_t b0, b1, b2, b3;
+                    ldsm_x4(at + (uint32_t)(kk * 32), b0, b1, b2, b3);
+#pragma unroll
+                    for (int h = 0; h < HW; ++h) {
+                        mma_bf16_16816(s[h][0], qa[h][kk], b0, b1);
+                        mma_bf16_16816(s[h][1], qa[h][kk], b2, b3);
+                    }
+                }
+            };
+            auto put = [&](uint8_t* to, int key0, bool pooled, auto masked) {     // in two parts, to the pairs' rows
+#pragma unroll
+                for (int j = 0; j < HK / 8; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int rr = e >> 1, in = j * 8 + t2 + (e & 1), kj = key0 + in;
+                        float w0 = ex2_approx(fmaf(s[0][j][e], c.sl2, -base[0][rr])), w1 = ex2_approx(fmaf(s[1][j][e], c.sl2, -base[1][rr]));
+                        if (decltype(masked)::value && !(pooled ? kj < nb[rr] : (kj <= qp[rr] && kj >= seen[rr]))) w0 = w1 = 0.0f;
+                        uint32_t hi, low;
+                        split_bf16(w0, w1, hi, low);
+                        const int at = (8 * rr * HK + j * 8 + (e & 1)) * P_PITCH + 2 * rr * 16;
+                        *reinterpret_cast<uint32_t*>(to + at) = hi;
+                        *reinterpret_cast<uint32_t*>(to + P_BYTES + at) = low;
+                    }
+            };
+            auto weights = [&](int step) {
+                const int b = b0 + (step >> 1);
+                const bool pooled = blocks.is_pooled(b);
+                const int key0 = blocks.key0(b, NK) + (step & 1) * HK;
+                c.apply<HW * HK / 8>(&s[0][0]);
+                const bool inside = pooled ? key0 + HK <= nb[0] && qp[1] >= 0 : key0 + HK - 1 <= qp[0] && key0 >= seen[1] && qp[1] >= 0;
+                uint8_t* to = sP + (step & 1) * 2 * P_BYTES + p_at;
+                if (__all_sync(0xffffffffu, inside)) put(to, key0, pooled, MixWhole());
+                else put(to, key0, pooled, MixMasked());
+            };
+            // talk x weights: eight pairs (one query, eight keys) at a time, straight to memory: [kv head][query][8 keys][its head][key]
+            auto mix = [&](int step) {
+                const uint4* t = sT + turned * 2 * TALK_FRAGS * 32 + mt * MT * 32 + lane;
+                uint4 th[MT], tl[MT];
+#pragma unroll
+                for (int ks = 0; ks < MT; ++ks) { th[ks] = t[ks * 32]; tl[ks] = t[(TALK_FRAGS + ks) * 32]; }
+                __half* to = dst + (size_t)(b0 + (step >> 1)) * (NH * NQ * NK) + (mt * 16 + g8) / G * (NQ * NK * G) + ((step & 1) * (HK / 8) * G + g8 % G) * 8 + t2;
+                constexpr int GROUPS = MIX_WARPS / MT;         // (eight or more: a warp's queries are turned alike)
+                static_assert(GROUPS % 4 == 0, "queries that are turned alike");
+#pragma unroll
+                for (int query = warp / MT; query < NQ; query += GROUPS)
+#pragma unroll
+                    for (int k8 = 0; k8 < HK / 8; ++k8) {
+                        uint32_t ph[4], pl[4];
+                        const uint32_t row = p_addr + (uint32_t)((step & 1) * 2 * P_BYTES + p_row(query) + k8 * 8 * P_PITCH);
+                        if (NH == 32) {
+                            ldsm_x4(row, ph[0], ph[1], ph[2], ph[3]);
+                            ldsm_x4(row + P_BYTES, pl[0], pl[1], pl[2], pl[3]);
+                        } else {
+                            // (16 heads: two matrices; the upper lanes' addresses are not used)
+                            asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(ph[0]), "=r"(ph[1]) : "r"(row));
+                            asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(pl[0]), "=r"(pl[1]) : "r"(row + P_BYTES));
+                        }
+                        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                        for (int ks = 0; ks < MT; ++ks) {
+                            const uint32_t ah[4] = {th[ks].x, th[ks].y, th[ks].z, th[ks].w}, al[4] = {tl[ks].x, tl[ks].y, tl[ks].z, tl[ks].w};
+                            mma_bf16_16816(acc, ah, ph[2 * ks], ph[2 * ks + 1]);
+                            mma_bf16_16816(acc, al, ph[2 * ks], ph[2 * ks + 1]);
+                            mma_bf16_16816(acc, ah, pl[2 * ks], pl[2 * ks + 1]);
+                        }
+                        __half* w = to + (query * (NK / 8) + k8) * G * 8;
+                        *reinterpret_cast<uint32_t*>(w) = pack_half(acc[0] * up, acc[1] * up);
+                        *reinterpret_cast<uint32_t*>(w + 8 / G * (NQ * NK * G)) = pack_half(acc[2] * up, acc[3] * up);
+                    }
+            };
+            cp_async_wait<1>();
+            __syncthreads();                                   // the first step's keys are there (and nobody mixes the tile before any more)
+            scores(0);
+            weights(0);
+            cp_async_wait<0>();
+            __syncthreads();
+            // one barrier a step: behind it lie the step's weights and the next step's keys; the products of both and the next step's weights run side by side
+            for (int step = 0; step < steps; ++step) {
+                fetch(step + 2);
+                if (step + 1 < steps) scores(step + 1);
+                mix(step);
+                if (step + 1 < steps) weights(step + 1);
+                cp_async_wait<0>();
+                __syncthreads();
+            }
         }
     }
 }
 
 // ---- mixed weights x values -----------------------------------------------------------------------------------------------------------------
-// Bound by what a CTA fetches through L2: two neighbouring tiles share every block of values (their ranges of blocks differ by one at most at either end).
+// On tcgen05: 128 rows (neighbouring tiles' queries x the heads of a kv head) x 32 keys a block, the weights' 11 bits as two bf16 numbers side by side in a row
+// of 128 bytes (32 keys' larger parts, then what they leave), the values as the other operand for both.  Eight warps bring the weights (four blocks
+// ahead, in registers) and the values (two ahead, by cp.async), one issues the MMAs.  Bound by the bytes of the mixed weights, most of which come back from HBM.
 #define V_STAGES 4
-#define VT 2                          // tiles of 16 queries a CTA
-static_assert(VT == 2, "a tile's blocks are one of two");
-#define A_PITCH (NK + 8)              // elements of a row of mixed weights in shared memory
-#define A_TILE (G * NQ * A_PITCH)
-#define V_STAGE_BYTES (VT * A_TILE * 2 + NK * LDV * 2)
-#define VALUE_SMEM (V_STAGES * V_STAGE_BYTES)
-#define VALUE_THREADS (32 * G * VT)
+#define VT (8 / G)                    // tiles of 16 queries a CTA: 128 rows
+#define V_AHEAD 4                     // blocks of mixed weights on their way in registers
+#define V_PAGE_BLOCKS 48              // blocks whose rows' pages are kept in shared memory (of those behind them they are looked up in the walk)
+#define V_HALVES ((DV + 63) / 64)
+#define V_A_BYTES (128 * 128)
+#define V_B_HALF (NK * 128)           // 64 columns of 32 keys
+#define V_STAGE_BYTES (V_A_BYTES + V_HALVES * V_B_HALF)
+#define VALUE_SMEM (V_STAGES * V_STAGE_BYTES + 1024)
+#define VALUE_WORKERS 256
+#define V_CHUNKS (VT * G * NQ * (NK / 8) / VALUE_WORKERS)      // 16-byte pieces of a block's mixed weights a thread
+static_assert(VT * G * NQ == 128 && V_CHUNKS == 2, "128 rows, two pieces a thread");
+#define V_COLS (DV <= 32 ? 32 : DV <= 64 ? 64 : 128)
 
-__global__ void __launch_bounds__(VALUE_THREADS, 2) value_kernel(
+__global__ void __launch_bounds__(VALUE_WORKERS + 32, 2) value_kernel(
     const __half* __restrict__ mixed, const float* __restrict__ talk, const bf16* __restrict__ v_cache, const bf16* __restrict__ v_pool, bf16* __restrict__ out,
     const int* __restrict__ block_table, int max_pages, const int* __restrict__ cu_tokens, const int* __restrict__ seq_lens, int first_req, int page_shift,
-    int window, int pool, int pool_rows, int most_blocks) {
+    int window, int pool, int pool_rows, int most_blocks, int* __restrict__ error_flag) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t full[V_STAGES], done[V_STAGES];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_page[V_PAGE_BLOCKS * NK];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     PDL_ENTER();
     mixed = pdl_fresh(mixed); v_cache = pdl_fresh(v_cache); v_pool = pdl_fresh(v_pool);
-    extern __shared__ __align__(16) uint8_t smem_raw[];
-    const int r = first_req + blockIdx.z, kh = blockIdx.y, qt = (gridDim.x - 1 - blockIdx.x) * VT;
+    const int r = first_req + blockIdx.y, kh = blockIdx.x, qt = (gridDim.z - 1 - blockIdx.z) * VT;
     const int tok0 = cu_tokens[r], n = cu_tokens[r + 1] - tok0;
     if (qt * NQ >= n) return;
+    if (tid == 0) {
+        for (int i = 0; i < V_STAGES; ++i) { mbar_init(&full[i], VALUE_WORKERS / 32); mbar_init(&done[i], 1); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) tmem_alloc<false>(&tmem_slot, V_COLS);
     const int here = min(VT * NQ, n - qt * NQ), pos0 = seq_lens[r] - n + qt * NQ;
     const int* table = block_table + (size_t)r * max_pages;
     const Blocks all(pos0, pos0 + here - 1, window, pool, NK);
-    const Blocks own[VT] = {Blocks(pos0, pos0 + min(here, NQ) - 1, window, pool, NK), Blocks(pos0 + min(here - 1, NQ), pos0 + here - 1, window, pool, NK)};
-    // block b of the CTA as a tile's own block (negative: the tile has no such block)
-    auto block_of = [&](int b, int tile) {
-        if (tile * NQ >= here) return -1;
-        const int o_pooled = tile == 0 ? own[0].pooled : own[1].pooled, o_first = tile == 0 ? own[0].first : own[1].first;
-        if (all.is_pooled(b)) return b < o_pooled ? b : -1;
-        const int at = all.first + b - all.pooled - o_first, o_count = tile == 0 ? own[0].count : own[1].count;
-        return at >= 0 && at < o_count - o_pooled ? o_pooled + at : -1;
-    };
-    const __half* src = mixed + (size_t)(first_tile(cu_tokens, first_req, r) + qt) * most_blocks * (NH * NQ * NK) + (size_t)kh * G * NQ * NK;
-    const size_t per_tile = (size_t)most_blocks * (NH * NQ * NK);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tile = warp / G;
-    auto fetch = [&](int b) {
-        if (b < all.count) {
-            __half* sA = reinterpret_cast<__half*>(smem_raw + (b % V_STAGES) * V_STAGE_BYTES);
-            bf16* sV = reinterpret_cast<bf16*>(sA + VT * A_TILE);
-            constexpr int PER_TILE = G * NQ * (NK / 8);
+    // the pages of the blocks' rows, looked up ahead of all else: a look-up in the walk waits behind the weights that are on their way (500 to 1,500 clocks a block)
+    for (int i = tid; i < min(all.count, V_PAGE_BLOCKS) * NK; i += VALUE_WORKERS + 32) {
+        const int b = i / NK, key = all.key0(b, NK) + i % NK;
+        s_page[i] = key >= all.begin(b) && key <= all.end(b) ? table[(all.is_pooled(b) ? key * pool + pool - 1 : key) >> page_shift] : 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    bool ok = true;
+    if (warp_same(warp) == VALUE_WORKERS / 32) {
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(DV >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint32_t elected = elect_one(), d = warp_same(tmem);
+        const int blocks = warp_same(all.count);
+        for (int b = 0; b < blocks; ++b) {
+            const int st = b % V_STAGES;
+            if (ok && !mbar_wait_warp(&full[st], (b / V_STAGES) & 1)) { atomicExch(error_flag, 41); ok = false; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a = smem_u32(smem) + st * V_STAGE_BYTES;
+            const uint64_t da = umma_desc(a), db = umma_desc_mn(a + V_A_BYTES, V_B_HALF);
 #pragma unroll
-            for (int t = 0; t < VT; ++t) {
-                const int mine = block_of(b, t);
-                if (mine < 0) continue;
-                for (int idx = tid; idx < PER_TILE; idx += VALUE_THREADS) {
-                    const int row = idx / (NK / 8), c8 = idx % (NK / 8) * 8;
-                    cp_async16(sA + t * A_TILE + row * A_PITCH + c8, src + t * per_tile + (size_t)mine * (NH * NQ * NK) + row * NK + c8);
+            for (int part = 0; part < 2; ++part)
+#pragma unroll
+                for (int kk = 0; kk < NK / 16; ++kk)
+                    umma_bf16(d, da + (uint32_t)(4 * part + 2 * kk), db + (uint32_t)(kk * (2048 >> 4)), idesc, (b > 0 || part > 0 || kk > 0) ? 1u : 0u, elected);
+            umma_commit(&done[st], elected);
+        }
+    } else {
+        // this thread's pieces of a block: (tile, 16 bytes of it); row = query of the CTA * G + head
+        const __half* from[V_CHUNKS];
+        uint32_t at[V_CHUNKS];
+        int o_pooled[V_CHUNKS], shift_by[V_CHUNKS], last[V_CHUNKS];      // a tile's own blocks: its pooled ones, how far its positions' lie from the CTA's, its last
+#pragma unroll
+        for (int i = 0; i < V_CHUNKS; ++i) {
+            const int piece = tid + VALUE_WORKERS * i, tile = piece / (G * NQ * (NK / 8)), idx = piece % (G * NQ * (NK / 8));
+            const int head = idx % G, query = idx / G / (NK / 8), k8 = idx / G % (NK / 8), row = (tile * NQ + query) * G + head;
+            from[i] = mixed + ((size_t)(first_tile(cu_tokens, first_req, r) + qt + tile) * most_blocks) * (NH * NQ * NK) + kh * (G * NQ * NK) + idx * 8;
+            at[i] = (uint32_t)(row * 128 + ((k8 ^ (row & 7)) << 4));
+            const int first = min(tile * NQ, here - 1), count = min(NQ, here - tile * NQ);
+            const Blocks own(pos0 + first, pos0 + first + max(count, 1) - 1, window, pool, NK);
+            o_pooled[i] = count > 0 ? own.pooled : 0;
+            shift_by[i] = all.first - all.pooled - own.first + own.pooled;
+            last[i] = count > 0 ? own.count : 0;
+        }
+        uint4 raw[V_AHEAD][V_CHUNKS];
+        auto load = [&](int b, uint4* to) {
+#pragma unroll
+            for (int i = 0; i < V_CHUNKS; ++i) {
+                const int mine = all.is_pooled(b) ? b : b + shift_by[i];
+                const bool there = b < all.count && (all.is_pooled(b) ? b < o_pooled[i] : mine >= o_pooled[i] && mine < last[i]);
+                to[i] = there ? *reinterpret_cast<const uint4*>(from[i] + (size_t)mine * (NH * NQ * NK)) : make_uint4(0, 0, 0, 0);
+            }
+        };
+        constexpr int PER = DV / 8, PASSES = (NK * PER + VALUE_WORKERS - 1) / VALUE_WORKERS;
+        auto values = [&](int b) {
+            if (b < all.count) {
+                uint8_t* to = smem + (b % V_STAGES) * V_STAGE_BYTES + V_A_BYTES;
+                const bool pooled = all.is_pooled(b);
+                const int key0 = all.key0(b, NK), begin = all.begin(b), end = all.end(b), mask = (1 << page_shift) - 1;
+                const bf16* src = pooled ? v_pool : v_cache;
+#pragma unroll
+                for (int i = 0; i < PASSES; ++i) {
+                    const int idx = tid + VALUE_WORKERS * i, row = idx / PER, c = idx % PER, key = key0 + row;
+                    if (NK * PER % VALUE_WORKERS != 0 && idx >= NK * PER) break;
+                    uint8_t* dst = to + c / 8 * V_B_HALF + row * 128 + (((c ^ row) & 7) << 4);
+                    const bool there = key >= begin && key <= end;
+                    const int p = pooled ? key * pool + pool - 1 : key;
+                    const int page = b < V_PAGE_BLOCKS ? s_page[b * NK + row] : there ? table[p >> page_shift] : 0;
+                    const size_t head_page = (size_t)page * KH + kh;
+                    const size_t at_row = pooled ? head_page * (size_t)pool_rows + (size_t)((p & mask) / pool) : (head_page << page_shift) + (size_t)(p & mask);
+                    if (there) cp_async16(dst, src + at_row * DV + c * 8);
+                    else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
                 }
             }
-            const bool pooled = all.is_pooled(b);
-            const int key0 = all.key0(b, NK), begin = all.begin(b), end = all.end(b);
-            const bf16* from = pooled ? v_pool : v_cache;
-            constexpr int PER = DV / 8;
-            for (int idx = tid; idx < NK * PER; idx += VALUE_THREADS) {
-                const int row = idx / PER, c = idx % PER, key = key0 + row;
-                if (key >= begin && key <= end) cp_async16(sV + row * LDV + c * 8, from + row_at(table, key, pooled, kh, page_shift, pool, pool_rows) * DV + c * 8);
-                else *reinterpret_cast<uint4*>(sV + row * LDV + c * 8) = make_uint4(0, 0, 0, 0);
+            cp_async_commit();
+        };
+        const float down = two_to(-mixed_shift(talk, lane));
+#pragma unroll
+        for (int i = 0; i < V_AHEAD; ++i) load(i, raw[i]);
+        values(0);
+        values(1);
+        for (int b0 = 0; b0 < all.count; b0 += V_AHEAD) {
+#pragma unroll
+            for (int u = 0; u < V_AHEAD; ++u) {
+                const int b = b0 + u, st = b % V_STAGES;
+                if (b >= all.count) break;
+                // (the stage of block b - 2 is the one that block b + 2's values go to; block b's was free before)
+                if (b >= 2 && ok && !mbar_wait(&done[(b - 2) % V_STAGES], ((b - 2) / V_STAGES) & 1)) { atomicExch(error_flag, 42); ok = false; }
+                values(b + 2);
+                uint8_t* to = smem + st * V_STAGE_BYTES;
+#pragma unroll
+                for (int i = 0; i < V_CHUNKS; ++i) {
+                    const uint32_t w[4] = {raw[u][i].x, raw[u][i].y, raw[u][i].z, raw[u][i].w};
+                    uint32_t hi[4], lo[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {              // 11 bits as two bf16 numbers, exactly
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+                        split_bf16(f.x * down, f.y * down, hi[e], lo[e]);
+                    }
+                    *reinterpret_cast<uint4*>(to + at[i]) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                    *reinterpret_cast<uint4*>(to + (at[i] ^ 64)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                }
+                load(b + V_AHEAD, raw[u]);
+                cp_async_wait<2>();
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[st])) : "memory");
             }
         }
-        cp_async_commit();
-    };
+        cp_async_wait<0>();
+        const int end = all.count - 1;
+        if (ok && !mbar_wait(&done[end % V_STAGES], (end / V_STAGES) & 1)) { atomicExch(error_flag, 43); ok = false; }
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // two warps share 32 rows: each takes every other 16 columns
+        const int row = (warp & 3) * 32 + lane, query = row / G;
+        bf16* to = out + ((size_t)(tok0 + qt * NQ + query) * NH + kh * G + row % G) * DV;
 #pragma unroll
-    for (int b = 0; b < V_STAGES - 1; ++b) fetch(b);
-    const float down = two_to(-mixed_shift(talk, lane));
-    float o[DV / 8][4];
+        for (int c = 0; c < DV; c += 16) {
+            if (((c >> 4) & 1) != (warp >> 2)) continue;
+            float v[16];
+            tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c, v);
+            if (query >= here) continue;
+            uint32_t p[8];
 #pragma unroll
-    for (int i = 0; i < DV / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
-    for (int b = 0; b < all.count; ++b) {
-        cp_async_wait<V_STAGES - 2>();
-        __syncthreads();                                       // block b is there, and everyone is done with the stage that is filled next
-        fetch(b + V_STAGES - 1);
-        if (block_of(b, tile) < 0) continue;
-        const __half* sA = reinterpret_cast<const __half*>(smem_raw + (b % V_STAGES) * V_STAGE_BYTES);
-        const uint32_t a_addr = (uint32_t)__cvta_generic_to_shared(sA + (warp * NQ + (lane & 7) + ((lane >> 3) & 1) * 8) * A_PITCH + (lane >> 4) * 8);
-        const uint32_t v_addr = (uint32_t)__cvta_generic_to_shared(sA + VT * A_TILE + ((lane & 7) + ((lane >> 3) & 1) * 8) * LDV + (lane >> 4) * 8);
-#pragma unroll
-        for (int ks = 0; ks < NK / 16; ++ks) {
-            uint32_t a[4], hi[4], lo[4];
-            ldsm_x4(a_addr + ks * 32, a[0], a[1], a[2], a[3]);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {                      // 11 bits as two bf16 numbers, exactly
-                const float2 w = __half22float2(*reinterpret_cast<const __half2*>(&a[i]));
-                split_bf16(w.x * down, w.y * down, hi[i], lo[i]);
-            }
-#pragma unroll
-            for (int dt = 0; dt < DV / 8; dt += 2) {
-                uint32_t b0, b1, b2, b3;
-                ldsm_x4_trans(v_addr + (uint32_t)(ks * 16 * LDV * 2 + dt * 16), b0, b1, b2, b3);
-                mma_bf16_16816(o[dt], hi, b0, b1);
-                mma_bf16_16816(o[dt + 1], hi, b2, b3);
-                mma_bf16_16816(o[dt], lo, b0, b1);
-                mma_bf16_16816(o[dt + 1], lo, b2, b3);
-            }
+            for (int e = 0; e < 8; ++e) p[e] = pack_bf16(v[2 * e], v[2 * e + 1]);
+            *reinterpret_cast<uint4*>(to + c) = make_uint4(p[0], p[1], p[2], p[3]);
+            *reinterpret_cast<uint4*>(to + c + 8) = make_uint4(p[4], p[5], p[6], p[7]);
         }
     }
-    cp_async_wait<0>();
-#pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-        const int row = tile * NQ + (lane >> 2) + 8 * rr;
-        if (row >= here) continue;
-        bf16* to = out + ((size_t)(tok0 + qt * NQ + row) * NH + kh * G + warp % G) * DV + 2 * (lane & 3);
-#pragma unroll
-        for (int i = 0; i < DV / 8; ++i) *reinterpret_cast<uint32_t*>(to + i * 8) = pack_bf16(o[i][2 * rr], o[i][2 * rr + 1]);
-    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) tmem_free<false>(tmem, V_COLS);
 }
 
 static int page_shift_of(int page_size) {
@@ -553,7 +722,7 @@ static int page_shift_of(int page_size) {
 MB_API int mb_attn_pooled_mix(int which, const void* q, const void* k_cache, const void* v_cache, const void* k_pool, const void* v_pool, float* lse,
                               const float* talk, void* mixed, void* out, const int* block_table, int max_pages, const int* cu_tokens, const int* seq_lens,
                               int first_req, int count, int max_query_len, int page_size, float scale, float cap, int window, int pool, int pool_rows,
-                              int most_blocks, cudaStream_t s) {
+                              int most_blocks, int* error_flag, cudaStream_t s) {
     if (count <= 0 || max_query_len <= 0) return 0;
     const int shift = page_shift_of(page_size);
     if (shift < 0 || window < 0 || pool < 0 || (pool > 0 && (k_pool == nullptr || v_pool == nullptr)) || most_blocks <= 0) return MB_ERR_BAD_SIZE;
@@ -561,16 +730,19 @@ MB_API int mb_attn_pooled_mix(int which, const void* q, const void* k_cache, con
     if ((((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)mixed | (uintptr_t)out) & 15) != 0) return MB_ERR_BAD_SIZE;
     if (which == 0) {
         cudaFuncSetAttribute(stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STATS_SMEM);
-        return launch_kernel(stats_kernel, dim3((max_query_len + SQ - 1) / SQ, KH, count), 256, STATS_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache,
+        return launch_kernel(stats_kernel, dim3(KH, count, (max_query_len + SQ - 1) / SQ), 256, STATS_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache,
                              (const bf16*)k_pool, lse, block_table, max_pages, cu_tokens, seq_lens, first_req, shift, scale, cap, window, pool, pool_rows);
     }
     const int tiles_of = (max_query_len + NQ - 1) / NQ;
     if (which == 1) {
         cudaFuncSetAttribute(mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MIX_SMEM);
-        return launch_kernel(mix_kernel, dim3(tiles_of, 1, count), MIX_THREADS, MIX_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache, (const bf16*)k_pool, (const float*)lse, talk,
-                             (__half*)mixed, block_table, max_pages, cu_tokens, seq_lens, first_req, shift, scale, cap, window, pool, pool_rows, most_blocks);
+        int device = 0, sms = 0;
+        cudaGetDevice(&device);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        return launch_kernel(mix_kernel, dim3(sms > 0 ? sms : 1), MIX_THREADS, MIX_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache, (const bf16*)k_pool, (const float*)lse, talk,
+                             (__half*)mixed, block_table, max_pages, cu_tokens, seq_lens, first_req, count, shift, scale, cap, window, pool, pool_rows, most_blocks);
     }
     cudaFuncSetAttribute(value_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VALUE_SMEM);
-    return launch_kernel(value_kernel, dim3((tiles_of + VT - 1) / VT, KH, count), VALUE_THREADS, VALUE_SMEM, s, 0, (const __half*)mixed, talk, (const bf16*)v_cache, (const bf16*)v_pool, (bf16*)out, block_table,
-                         max_pages, cu_tokens, seq_lens, first_req, shift, window, pool, pool_rows, most_blocks);
+    return launch_kernel(value_kernel, dim3(KH, count, (tiles_of + VT - 1) / VT), VALUE_WORKERS + 32, VALUE_SMEM, s, 0, (const __half*)mixed, talk, (const bf16*)v_cache, (const bf16*)v_pool, (bf16*)out, block_table,
+                         max_pages, cu_tokens, seq_lens, first_req, shift, window, pool, pool_rows, most_blocks, error_flag);
 }

@@ -2112,7 +2112,8 @@ def attention_pooled(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table,
     if talk is not None and ctx.num_requests > ctx.num_decode:
         blocks = _pooled_mix_blocks(ctx, window, pool)
         if (use_pooled_mix and pooled_mix_supported(q.dtype, H, K, d, dv) and page_size & (page_size - 1) == 0 and scale > 0
-                and _pooled_mix_pays(T - ctx.num_decode, ctx.num_requests - ctx.num_decode, ctx.max_query_len, blocks, K, dv)
+                and _pooled_mix_pays(T - ctx.num_decode, ctx.num_requests - ctx.num_decode, ctx.max_query_len, blocks, K, dv,
+                                     _pooled_mix_walk(T - ctx.num_decode, ctx.num_requests - ctx.num_decode, blocks))
                 and all(t is None or t.data_ptr() % 16 == 0 for t in (q, k_cache, v_cache, k_pool, v_pool, out))):
             _pooled_mix(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table, H, K, d, dv, scale, softcap or 0.0, window, pool, rows, talk, blocks)
             if ctx.num_decode == 0:
@@ -2153,10 +2154,10 @@ def attention_pooled(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table,
 #: prompt portions with mixed head weights go to the kernels that mix the weights ahead of the values (False: every head's sums over every kv head's values,
 #: mixed afterwards)
 use_pooled_mix = True
-#: ... where that costs less, in us on B200 with 32 heads of 128 over 8: this way a block of 32 keys of the longest tile (a tile of 16 queries walks its keys in one
-#: CTA), the other way a token (its sums written and mixed) and a token's block.  Whole mixers, this way and the other: one portion behind 2,000 positions, window
-#: 1,024, pools of 64, 256, 384, 512 and 2,048 tokens 386, 403, 429 and 640 against 300, 406, 539 and 1,723; window 512 247, 258, 277 and 439 against 223, 289,
-#: 383 and 1,175; nothing before them, one portion of 192, 320 and 512 tokens 124, 163 and 240 against 128, 172 and 275, four of 80 115 against 153
+#: ... where that costs less, in us on B200 with 32 heads of 128 over 8: this way a block of 32 keys that a CTA walks, the other way a token (its sums written and
+#: mixed) and a token's block.  Whole mixers, this way and the other: one portion behind 2,000 positions, window 1,024, pools of 64, 128, 256, 512 and 2,048 tokens
+#: 144, 171, 219 and 517 against 160, 276, 493 and 1,652; window 512 109, 132, 171 and 370 against 119, 198, 333 and 1,102; nothing before them, one portion of 128,
+#: 160, 192, 320 and 512 tokens 92, 94, 94, 99 and 131 against 84, 92, 98, 138 and 211, four of 100 96 against 144
 POOLED_MIX_COSTS = (9.0, 0.17, 0.022)
 
 
@@ -2165,13 +2166,18 @@ def _pooled_mix_tiles(tokens: int, portions: int) -> int:
     return tokens // 16 + portions
 
 
-def _pooled_mix_pays(tokens: int, portions: int, longest: int, blocks: int, K: int, dv: int) -> bool:
-    """Whether portions of so many tokens (in all) go to the kernels that mix the weights first: a portion that fills a tile, enough tokens for their ``blocks`` (with
-    2, 10, 19 and 35 of them from 84, 231, 291 and 335 tokens on), and mixed weights (H x 16 x 32 numbers of 16 bits a tile and block) that take no more
+def _pooled_mix_walk(tokens: int, portions: int, blocks: int) -> float:
+    """Blocks a CTA of the mixing kernel walks: an equal share of all tiles' (a few for its start and for a tile's)."""
+    return 4.0 + _pooled_mix_tiles(tokens, portions) * blocks / SM_COUNT
+
+
+def _pooled_mix_pays(tokens: int, portions: int, longest: int, blocks: int, K: int, dv: int, walk: Optional[float] = None) -> bool:
+    """Whether portions of so many tokens (in all) go to the kernels that mix the weights first: a portion that fills a tile, enough tokens for the blocks a CTA
+    walks (``walk``; all ``blocks`` of a tile where it is not given: with 2, 10, 19 and 35 of them from 84, 231, 291 and 335 tokens on), and mixed weights (H x 16 x 32 numbers of 16 bits a tile and block) that take no more
     memory than the heads' sums would (H x K x dv of 32 bits a token), which is what a step's working memory is planned with.  By that a window of
     1,024 passes with 8 kv heads of 128, one of 2,048 or none over more than 2,000 positions does not."""
     block, token, both = POOLED_MIX_COSTS
-    return longest >= 16 and block * blocks <= tokens * (token + both * blocks) and _pooled_mix_tiles(tokens, portions) * blocks * 256 <= tokens * K * dv
+    return longest >= 16 and block * (blocks if walk is None else walk) <= tokens * (token + both * blocks) and _pooled_mix_tiles(tokens, portions) * blocks * 256 <= tokens * K * dv
 
 
 def pooled_mix_supported(dtype, H: int, K: int, d: int, dv: int) -> bool:
@@ -2180,8 +2186,8 @@ def pooled_mix_supported(dtype, H: int, K: int, d: int, dv: int) -> bool:
 
 
 def _pooled_mix_smem(H: int, K: int, d: int) -> int:
-    """Bytes of shared memory the mixing kernel needs (its keys, the weights of 512 pairs in two parts, the mixed rows, the mixing matrix)."""
-    return K * 32 * (d + 8) * 2 + 2 * 16 * (32 * (2 * H + 16) + 16) + H * (16 * 80 + 16) + 2 * (H // 16) ** 2 * 512
+    """Bytes of shared memory the mixing kernel needs (two steps' keys, the weights of their 256 pairs each in two parts, the mixing matrix turned in four ways)."""
+    return 2 * K * 16 * (d + 8) * 2 + 4 * (16 * 16 * (2 * H + 16) + 64) + 8 * (H // 16) ** 2 * 512
 
 
 def _pooled_mix_blocks(ctx, window: int, pool: int) -> int:
@@ -2221,7 +2227,8 @@ def _pooled_mix(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table, H: i
     lib = build.load(_pooled_mix_name(d, dv, H, K), *_pooled_mix_job(d, dv, H, K))
     args = (_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(k_pool), _ptr(v_pool), _ptr(lse), _ptr(talk), _ptr(mixed), _ptr(out), _ptr(block_table),
             _c_int(block_table.shape[1]), _ptr(ctx.cu_tokens), _ptr(ctx.seq_lens), _c_int(nd), _c_int(count), _c_int(ctx.max_query_len),
-            _c_int(k_cache.shape[2]), _c_float(scale), _c_float(softcap), _c_int(window), _c_int(pool), _c_int(rows), _c_int(blocks), _stream())
+            _c_int(k_cache.shape[2]), _c_float(scale), _c_float(softcap), _c_int(window), _c_int(pool), _c_int(rows), _c_int(blocks),
+            _ptr(_scratch_for(q.device).error), _stream())
     size = q.element_size()
     # what the algorithm needs is shared out: the queries and keys with the sums, the mixing of a pair's weights, the values and results with the last
     for which, what, nbytes, per_key, per_pair in (
