@@ -435,10 +435,11 @@ __global__ void __launch_bounds__(RUNS <= 2 ? 1024 : 256) qkv_finish_vec_kernel(
 // cosines then sines).  With a convolution the thread's weights and last TAPS - 1 inputs stay in registers, so that every row is read once a run.
 // TAPS 0: no convolution.
 #define FR_THREADS 128
-#define FR_RUN 8
+#define FR_RUN(taps) ((taps) > 0 ? 8 : 2)    // rows a thread has in flight (without a convolution nothing is shared along a run: two, and twice the
+                                             // threads an SM: 2,048 tokens of 48 heads of 128 22 us where eight took 35)
 
 template <int TAPS>
-__global__ void __launch_bounds__(FR_THREADS, 3) qkv_finish_runs_kernel(
+__global__ void __launch_bounds__(FR_THREADS, TAPS > 0 ? 3 : 6) qkv_finish_runs_kernel(
     const bf16* __restrict__ row, int row_stride, bf16* __restrict__ q_out, const float* __restrict__ q_b, const float* __restrict__ k_b,
     const float* __restrict__ v_b, int norm, const float* __restrict__ q_w, const float* __restrict__ k_w, float eps, const int* __restrict__ positions,
     const float* __restrict__ rope, int rot_dim, const int* __restrict__ slot_mapping, bf16* __restrict__ k_cache, bf16* __restrict__ v_cache, int H, int K,
@@ -470,16 +471,16 @@ __global__ void __launch_bounds__(FR_THREADS, 3) qkv_finish_runs_kernel(
     if (TAPS > 0 && active)
 #pragma unroll
         for (int j = 0; j < TAPS; ++j) load8(cv.w + (size_t)j * cv.channels + c, wt[j]);
-    uint4 raw[FR_RUN];                                         // every row of the run in flight at once
+    uint4 raw[FR_RUN(TAPS)];                                   // every row of the run in flight at once
 #pragma unroll
-    for (int u = 0; u < FR_RUN; ++u) {
+    for (int u = 0; u < FR_RUN(TAPS); ++u) {
         raw[u] = make_uint4(0, 0, 0, 0);
         if (active && t0 + u < t1) raw[u] = *reinterpret_cast<const uint4*>(row + (size_t)(t0 + u) * row_stride + c);
     }
     int first = 0, end = 0;
     float* kept = nullptr;
 #pragma unroll
-    for (int u = 0; u < FR_RUN; ++u) {
+    for (int u = 0; u < FR_RUN(TAPS); ++u) {
         const int t = t0 + u;
         if (t >= t1) break;                                    // (the same for the whole block)
         float x[8];
@@ -599,7 +600,7 @@ MB_API int mb_qkv_finish(const void* row, int row_stride, int dtype, void* q_out
         aligned16(q_b) && aligned16(k_b) && aligned16(v_b) && aligned16(q_w) && aligned16(k_w) && aligned16(k_cache) && aligned16(v_cache) && aligned16(conv_w) &&
         aligned16(ring) && aligned16(rope)) {
         const int cols = H * d + (write_kv ? K * d + K / maps * dv : 0);
-        const int run = tokens >= 256 ? FR_RUN : tokens >= 64 ? 2 : 1;
+        const int run = tokens >= 256 ? FR_RUN(conv_w == nullptr ? 0 : taps) : tokens >= 64 ? 2 : 1;
         dim3 grid((tokens + run - 1) / run, (cols / 8 + FR_THREADS - 1) / FR_THREADS);
 #define FR_CASE(TAPS)                                                                                                                                \
     if ((conv_w == nullptr ? 0 : taps) == TAPS)                                                                                                      \

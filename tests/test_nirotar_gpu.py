@@ -622,3 +622,50 @@ def test_the_command_line_takes_a_nirotar_folder(tmp_path):
     for stage in ("embedding", "q|k|v|g", "q|dkv", "heads", "q into the latent", "attention", "v from the latent", "router",
                   "experts", "head", "sampling"):
         assert stage in e.stdout, stage
+
+
+@pytest.mark.parametrize("H,dn,dr,r,rot,interleaved", [(32, 64, 32, 128, 32, True), (3, 8, 16, 8, 16, False), (5, 16, 24, 224, 16, False), (1, 0, 8, 64, 0, True), (40, 8, 64, 96, 40, True)])
+@pytest.mark.parametrize("own_rows", [False, True])
+def test_latent_heads_by_runs_of_eight_numbers(H, dn, dr, r, rot, interleaved, own_rows):
+    """bf16 rows that go by 16-byte pieces against the float32 kernel over the same numbers, rounded once (2^-8) after sums of r squares (2^-24 r); nothing beside
+    the rows is written."""
+    from marin_b200.kernels import ops
+
+    g = torch.Generator(device=DEV).manual_seed(H + r)
+    T, D, page = 37, r + dr, 16
+    rows = torch.randn(T, H * (dn + dr) + (0 if own_rows else D), device=DEV, generator=g).to(torch.bfloat16)
+    kv = torch.randn(T, D + 8, device=DEV, generator=g).to(torch.bfloat16)[:, :D] if own_rows else None
+    cw = 1 + 0.1 * torch.randn(r, device=DEV, generator=g)
+    positions = torch.randint(0, 3000, (T,), device=DEV, generator=g, dtype=torch.int32)
+    inv_freq = torch.pow(torch.tensor(1e4), -(torch.arange(max(1, rot // 2), dtype=torch.float32) * 2.0 / max(1, rot))).to(DEV) if rot else None
+    slots = torch.randperm(T + 11, device=DEV, generator=g)[:T].to(torch.int32)
+    slots[5] = -1
+
+    def run(dtype, write):
+        q = torch.full((T, H * D), 3.0, device=DEV, dtype=dtype)
+        cache = torch.full(((T + 11) // page + 1, 1, page, D), 3.0, device=DEV, dtype=dtype)
+        ops.latent_finish(rows.to(dtype), q, cw, 1e-6, positions, inv_freq, rot, interleaved, slots if write else None, cache if write else None, H, dn, dr, r, write,
+                          None if kv is None else kv if dtype == torch.bfloat16 else kv.float())
+        return q.float(), cache.float()
+
+    for write in (True, False):
+        for got, want in zip(run(torch.bfloat16, write), run(torch.float32, write)):
+            torch.testing.assert_close(got, want, rtol=2.0 ** -8, atol=1e-5)
+
+
+@pytest.mark.parametrize("T,H,N,K,o_head", [(16, 2, 128, 64, 136), (65, 3, 64, 128, 64), (200, 1, 129, 72, 132), (100, 2, 8, 8, 8), (64, 1, 72, 200, 73)])
+def test_products_per_head_at_tile_edges(T, H, N, K, o_head):
+    """Whole and ragged tiles of tokens, columns and k, results in 16-byte pieces and not, against float64 (float32 sums of K products, rounded once)."""
+    from marin_b200.kernels import ops
+
+    g = torch.Generator(device=DEV).manual_seed(T + N)
+    x = torch.randn(T, H * (K + 8), device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(H, N, K, device=DEV, generator=g) * K ** -0.5).to(torch.bfloat16)
+    out = torch.full((T, H * o_head + (H * o_head) % 2), 7.0, device=DEV, dtype=torch.bfloat16)
+    ops.heads_product(x, K + 8, K, w, out, o_head)
+    for a in range(H):
+        xa = x[:, a * (K + 8):a * (K + 8) + K].double()
+        want, scale = xa @ w[a].double().t(), xa.abs() @ w[a].double().abs().t()
+        got = out[:, a * o_head:a * o_head + N].double()
+        assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -23 * K * scale).all())
+        assert bool((out[:, a * o_head + N:(a + 1) * o_head] == 7.0).all())
