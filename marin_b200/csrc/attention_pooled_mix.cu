@@ -15,7 +15,7 @@
 // makes, where weights rounded to bf16 (every head's, in the other kernel) made it 1.17 times as large.
 // Scratch: [tile][block][kv head][query][8 keys][its head][key] halves, a tile of 16 queries of one request, its blocks of 32 pooled rows, then of 32 positions.
 // Measured on B200, 2,048 tokens, 32 heads of 128 over 8, window 1,024, pools of 64: the other kernel and its mixing 1,189 us;
-// these 79 + 166 + 72 us (95 + 216 + 141 with a CTA a tile in the mixing, three barriers a block and the values on mma.sync).  mix_kernel is bound by issue: about a
+// these 79 + 166 + 63 us (95 + 216 + 141 with a CTA a tile in the mixing, three barriers a block and the values on mma.sync).  mix_kernel is bound by issue: about a
 // thousand instructions a warp and block (cap, exponential, two parts, their stores) behind which its products of 3,600 clocks a block hide.
 #define MB_LIB "attention_pooled_mix"
 #define MB_LIB_ID 25
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(MIX_THREADS, 1) mix_kernel(
 #define V_STAGES 4
 #define VT (8 / G)                    // tiles of 16 queries a CTA: 128 rows
 #define V_AHEAD 4                     // blocks of mixed weights on their way in registers
-#define V_PAGE_BLOCKS 48              // blocks whose rows' pages are kept in shared memory (of those behind them they are looked up in the walk)
+#define V_ROW_BLOCKS 48               // blocks whose rows' places are kept in shared memory (of those behind them they are looked up in the walk)
 #define V_HALVES ((DV + 63) / 64)
 #define V_A_BYTES (128 * 128)
 #define V_B_HALF (NK * 128)           // 64 columns of 32 keys
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(VALUE_WORKERS + 32, 2) value_kernel(
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t full[V_STAGES], done[V_STAGES];
     __shared__ uint32_t tmem_slot;
-    __shared__ int s_page[V_PAGE_BLOCKS * NK];
+    __shared__ unsigned s_row[V_ROW_BLOCKS * NK];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     PDL_ENTER();
@@ -575,11 +575,12 @@ __global__ void __launch_bounds__(VALUE_WORKERS + 32, 2) value_kernel(
     const int here = min(VT * NQ, n - qt * NQ), pos0 = seq_lens[r] - n + qt * NQ;
     const int* table = block_table + (size_t)r * max_pages;
     const Blocks all(pos0, pos0 + here - 1, window, pool, NK);
-    // the pages of the blocks' rows, looked up ahead of all else: a look-up in the walk waits behind the weights that are on their way (500 to 1,500 clocks a block)
-    for (int i = tid; i < min(all.count, V_PAGE_BLOCKS) * NK; i += VALUE_WORKERS + 32) {
-        const int b = i / NK, key = all.key0(b, NK) + i % NK;
-        s_page[i] = key >= all.begin(b) && key <= all.end(b) ? table[(all.is_pooled(b) ? key * pool + pool - 1 : key) >> page_shift] : 0;
-    }
+    // where the blocks' rows lie (~0: not there), looked up ahead of all else: in the walk it would be a third of its instructions
+    auto row_of = [&](int b, int n) {
+        const int key = all.key0(b, NK) + n;
+        return key >= all.begin(b) && key <= all.end(b) ? (unsigned)row_at(table, key, all.is_pooled(b), kh, page_shift, pool, pool_rows) : ~0u;
+    };
+    for (int i = tid; i < min(all.count, V_ROW_BLOCKS) * NK; i += VALUE_WORKERS + 32) s_row[i] = row_of(i / NK, i % NK);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -625,33 +626,31 @@ __global__ void __launch_bounds__(VALUE_WORKERS + 32, 2) value_kernel(
             for (int i = 0; i < V_CHUNKS; ++i) {
                 const int mine = all.is_pooled(b) ? b : b + shift_by[i];
                 const bool there = b < all.count && (all.is_pooled(b) ? b < o_pooled[i] : mine >= o_pooled[i] && mine < last[i]);
-                to[i] = there ? *reinterpret_cast<const uint4*>(from[i] + (size_t)mine * (NH * NQ * NK)) : make_uint4(0, 0, 0, 0);
+                to[i] = there ? *reinterpret_cast<const uint4*>(from[i] + (size_t)(unsigned)(mine * (NH * NQ * NK))) : make_uint4(0, 0, 0, 0);
             }
         };
         constexpr int PER = DV / 8, PASSES = (NK * PER + VALUE_WORKERS - 1) / VALUE_WORKERS;
+        uint32_t v_at[PASSES];
+#pragma unroll
+        for (int i = 0; i < PASSES; ++i) {
+            const int idx = tid + VALUE_WORKERS * i, row = idx / PER, c = idx % PER;
+            v_at[i] = V_A_BYTES + c / 8 * V_B_HALF + row * 128 + (((c ^ row) & 7) << 4);
+        }
         auto values = [&](int b) {
             if (b < all.count) {
-                uint8_t* to = smem + (b % V_STAGES) * V_STAGE_BYTES + V_A_BYTES;
-                const bool pooled = all.is_pooled(b);
-                const int key0 = all.key0(b, NK), begin = all.begin(b), end = all.end(b), mask = (1 << page_shift) - 1;
-                const bf16* src = pooled ? v_pool : v_cache;
+                const uint32_t to = smem_u32(smem) + (b % V_STAGES) * V_STAGE_BYTES;
+                const bf16* src = all.is_pooled(b) ? v_pool : v_cache;
 #pragma unroll
                 for (int i = 0; i < PASSES; ++i) {
-                    const int idx = tid + VALUE_WORKERS * i, row = idx / PER, c = idx % PER, key = key0 + row;
-                    if (NK * PER % VALUE_WORKERS != 0 && idx >= NK * PER) break;
-                    uint8_t* dst = to + c / 8 * V_B_HALF + row * 128 + (((c ^ row) & 7) << 4);
-                    const bool there = key >= begin && key <= end;
-                    const int p = pooled ? key * pool + pool - 1 : key;
-                    const int page = b < V_PAGE_BLOCKS ? s_page[b * NK + row] : there ? table[p >> page_shift] : 0;
-                    const size_t head_page = (size_t)page * KH + kh;
-                    const size_t at_row = pooled ? head_page * (size_t)pool_rows + (size_t)((p & mask) / pool) : (head_page << page_shift) + (size_t)(p & mask);
-                    if (there) cp_async16(dst, src + at_row * DV + c * 8);
-                    else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+                    const int row = (tid + VALUE_WORKERS * i) / PER;
+                    if (NK * PER % VALUE_WORKERS != 0 && row >= NK) break;
+                    const unsigned at_row = b < V_ROW_BLOCKS ? s_row[b * NK + row] : row_of(b, row);
+                    if (at_row != ~0u) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + v_at[i]), "l"(src + (size_t)at_row * DV + (tid + VALUE_WORKERS * i) % PER * 8) : "memory");
+                    else asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(to + v_at[i]), "r"(0) : "memory");
                 }
             }
             cp_async_commit();
         };
-        const float down = two_to(-mixed_shift(talk, lane));
 #pragma unroll
         for (int i = 0; i < V_AHEAD; ++i) load(i, raw[i]);
         values(0);
@@ -670,9 +669,9 @@ __global__ void __launch_bounds__(VALUE_WORKERS + 32, 2) value_kernel(
                     const uint32_t w[4] = {raw[u][i].x, raw[u][i].y, raw[u][i].z, raw[u][i].w};
                     uint32_t hi[4], lo[4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {              // 11 bits as two bf16 numbers, exactly
+                    for (int e = 0; e < 4; ++e) {              // 11 bits as two bf16 numbers, exactly (the power of two comes off the sums)
                         const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
-                        split_bf16(f.x * down, f.y * down, hi[e], lo[e]);
+                        split_bf16(f.x, f.y, hi[e], lo[e]);
                     }
                     *reinterpret_cast<uint4*>(to + at[i]) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
                     *reinterpret_cast<uint4*>(to + (at[i] ^ 64)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
@@ -691,6 +690,7 @@ __global__ void __launch_bounds__(VALUE_WORKERS + 32, 2) value_kernel(
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // two warps share 32 rows: each takes every other 16 columns
         const int row = (warp & 3) * 32 + lane, query = row / G;
+        const float down = two_to(-mixed_shift(talk, lane));
         bf16* to = out + ((size_t)(tok0 + qt * NQ + query) * NH + kh * G + row % G) * DV;
 #pragma unroll
         for (int c = 0; c < DV; c += 16) {
@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(VALUE_WORKERS + 32, 2) value_kernel(
             if (query >= here) continue;
             uint32_t p[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) p[e] = pack_bf16(v[2 * e], v[2 * e + 1]);
+            for (int e = 0; e < 8; ++e) p[e] = pack_bf16(v[2 * e] * down, v[2 * e + 1] * down);
             *reinterpret_cast<uint4*>(to + c) = make_uint4(p[0], p[1], p[2], p[3]);
             *reinterpret_cast<uint4*>(to + c + 8) = make_uint4(p[4], p[5], p[6], p[7]);
         }
