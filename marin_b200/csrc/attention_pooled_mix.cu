@@ -6,7 +6,7 @@
 // head multiplies its own kv head's values once.  (attention_pooled_fast.cu sums every head over every kv head's values and mixes the sums: KV_HEADS
 // times the products with V, and a float32 [tokens][H][KV_HEADS][V_DIM] that a second kernel reads.)  Mixing needs the weights already
 // divided by their sums, so three kernels:
-//   stats_kernel  (a CTA per kv head and 128 rows = queries x its heads): the logarithm of every row's sum of weights;
+//   stats_kernel  (a CTA per kv head and 128 rows = queries x its heads, tcgen05): the logarithm of every row's sum of weights;
 //   mix_kernel    (equal runs of the tiles' blocks a CTA, two heads a warp, 16 queries x 16 keys a step): the weights of all heads, mixed, to scratch memory in 16 bits;
 //   value_kernel  (a CTA per 128 rows of a kv head, tcgen05): mixed weights x values.
 // Exactness: the weights p are float32 and enter the mixing product as pairs of bf16 numbers (p = hi + lo), as does talk; the three larger of the four
@@ -15,7 +15,7 @@
 // makes, where weights rounded to bf16 (every head's, in the other kernel) made it 1.17 times as large.
 // Scratch: [tile][block][kv head][query][8 keys][its head][key] halves, a tile of 16 queries of one request, its blocks of 32 pooled rows, then of 32 positions.
 // Measured on B200, 2,048 tokens, 32 heads of 128 over 8, window 1,024, pools of 64: the other kernel and its mixing 1,189 us;
-// these 79 + 166 + 63 us (95 + 216 + 141 with a CTA a tile in the mixing, three barriers a block and the values on mma.sync).  mix_kernel is bound by issue: about a
+// these 55 + 166 + 63 us (95 + 216 + 141 with a CTA a tile in the mixing, three barriers a block and the sums and values on mma.sync).  mix_kernel is bound by issue: about a
 // thousand instructions a warp and block (cap, exponential, two parts, their stores) behind which its products of 3,600 clocks a block hide.
 #define MB_LIB "attention_pooled_mix"
 #define MB_LIB_ID 25
@@ -133,117 +133,162 @@ __device__ __forceinline__ void q_fragment(uint32_t* a, const bf16* lo, const bf
 }
 
 // ---- the logarithm (base 2) of every row's sum of weights ---------------------------------------------------------------------------------
-#define SQ (128 / G)                  // queries a CTA: 128 rows with the kv head's query heads
+// On tcgen05: 128 rows (queries x the heads of a kv head) x 64 keys a block into one of four buffers of tensor memory; a thread has a row, two warps of 32
+// rows take the blocks in turn and add their sums at the end.  Four warps bring the keys, one issues the MMAs.  Bound by the rows' instructions (62% of the issue slots,
+// tensor cores 13%); on mma.sync, where a warp also loaded fragments and shared its rows' maxima, 79 us, now 55 (2,048 tokens, 32 heads of 128, window 1,024).
+#define SQ (128 / G)                  // queries a CTA
 #define SN 64                         // keys a block
-#define STATS_SMEM (2 * SN * LDK * 2)
+#define S_STAGES 4                    // blocks of keys, and buffers of scores
+#define S_HALVES ((D + 63) / 64)
+#define S_Q_HALF (128 * 128)
+#define S_K_HALF (SN * 128)
+#define S_K_BYTES (S_HALVES * S_K_HALF)
+#define STATS_SMEM (S_HALVES * S_Q_HALF + S_STAGES * S_K_BYTES + 1024)
+#define S_ROW_WARPS 8
+#define S_LOAD_WARPS 4
+#define STATS_THREADS (32 * (S_ROW_WARPS + S_LOAD_WARPS + 1))
+#define S_ROW_BLOCKS 24               // blocks whose rows' places are kept in shared memory
 
-__global__ void __launch_bounds__(256, 2) stats_kernel(
+__global__ void __launch_bounds__(STATS_THREADS, 2) stats_kernel(
     const bf16* __restrict__ q, const bf16* __restrict__ k_cache, const bf16* __restrict__ k_pool, float* __restrict__ lse,
     const int* __restrict__ block_table, int max_pages, const int* __restrict__ cu_tokens, const int* __restrict__ seq_lens, int first_req,
-    int page_shift, float scale, float cap, int window, int pool, int pool_rows) {
+    int page_shift, float scale, float cap, int window, int pool, int pool_rows, int* __restrict__ error_flag) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t k_full[S_STAGES], s_done[S_STAGES], s_free[S_STAGES];
+    __shared__ uint32_t tmem_slot;
+    __shared__ unsigned s_row[S_ROW_BLOCKS * SN];
+    __shared__ float2 s_other[128];
+    uint8_t* sQ = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* sK = sQ + S_HALVES * S_Q_HALF;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     PDL_ENTER_EARLY();
     q = pdl_fresh(q); k_cache = pdl_fresh(k_cache); k_pool = pdl_fresh(k_pool);
-    extern __shared__ __align__(16) uint8_t smem_raw[];
-    bf16* sK = reinterpret_cast<bf16*>(smem_raw);
     const int r = first_req + blockIdx.y, kh = blockIdx.x, qt = gridDim.z - 1 - blockIdx.z;          // all heads' long tiles first
     const int tok0 = cu_tokens[r], n = cu_tokens[r + 1] - tok0;
     if (qt * SQ >= n) return;
+    if (tid == 0) {
+        for (int i = 0; i < S_STAGES; ++i) { mbar_init(&k_full[i], S_LOAD_WARPS); mbar_init(&s_done[i], 1); mbar_init(&s_free[i], 4); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) tmem_alloc<false>(&tmem_slot, S_STAGES * SN);
     const int here = min(SQ, n - qt * SQ), pos0 = seq_lens[r] - n + qt * SQ;
     const int* table = block_table + (size_t)r * max_pages;
     const Blocks blocks(pos0, pos0 + here - 1, window, pool, SN);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    auto fetch = [&](int b) {
-        const bool pooled = blocks.is_pooled(b);
-        const int key0 = blocks.key0(b, SN);
-        const bf16* src = pooled ? k_pool : k_cache;
-        bf16* dst = sK + (b & 1) * SN * LDK;
-        const int row = tid >> 2, key = key0 + row;            // four threads a row
-        if (key >= blocks.begin(b) && key <= blocks.end(b)) {
-            const bf16* from = src + row_at(table, key, pooled, kh, page_shift, pool, pool_rows) * D;
-#pragma unroll
-            for (int c = tid & 3; c < D / 8; c += 4) cp_async16(dst + row * LDK + c * 8, from + c * 8);
-        } else {
-#pragma unroll
-            for (int c = tid & 3; c < D / 8; c += 4) *reinterpret_cast<uint4*>(dst + row * LDK + c * 8) = make_uint4(0, 0, 0, 0);
-        }
-        cp_async_commit();
+    for (int idx = tid; idx < 128 * (D / 8); idx += STATS_THREADS) {
+        const int row = idx / (D / 8), c = idx % (D / 8), ql = row / G;
+        uint8_t* dst = sQ + c / 8 * S_Q_HALF + row * 128 + (((c ^ row) & 7) << 4);
+        if (ql < here) cp_async16(dst, q + ((size_t)(tok0 + qt * SQ + ql) * NH + kh * G + row % G) * D + c * 8);
+        else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+    }
+    cp_async_commit();
+    auto row_of = [&](int b, int i) {
+        const int key = blocks.key0(b, SN) + i;
+        return key >= blocks.begin(b) && key <= blocks.end(b) ? (unsigned)row_at(table, key, blocks.is_pooled(b), kh, page_shift, pool, pool_rows) : ~0u;
     };
-    fetch(0);
-    // this thread's rows: warp * 16 + lane / 4 and 8 on; row = query * G + head of the group
-    uint32_t qa[D / 16][4];
-    int qp[2], lo[2], nb[2], at[2];
-    {
-        const bf16* rows[2];
+    for (int i = tid; i < min(blocks.count, S_ROW_BLOCKS) * SN; i += STATS_THREADS) s_row[i] = row_of(i / SN, i % SN);
+    cp_async_wait<0>();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    const int role = warp_same(warp), count = warp_same(blocks.count);
+    bool ok = true;
+    float m_run = -INFINITY, l_run = 0.0f;
+    if (role == S_ROW_WARPS + S_LOAD_WARPS) {
+        // ---- the MMAs: S(b) = Q K(b)^T once the keys have landed and the rows have read what lay in its buffer ----
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(SN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint32_t elected = elect_one(), d = warp_same(tmem);
+        for (int b = 0; b < count; ++b) {
+            const int st = b % S_STAGES;
+            if (ok && !mbar_wait_warp(&k_full[st], (b / S_STAGES) & 1)) { atomicExch(error_flag, 44); ok = false; }
+            if (ok && b >= S_STAGES && !mbar_wait_warp(&s_free[st], (b / S_STAGES - 1) & 1)) { atomicExch(error_flag, 45); ok = false; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t da = umma_desc(smem_u32(sQ)), db = umma_desc(smem_u32(sK) + st * S_K_BYTES);
 #pragma unroll
-        for (int rr = 0; rr < 2; ++rr) {
-            const int row = warp * 16 + (lane >> 2) + 8 * rr, ql = row / G;
-            const bool there = ql < here;
-            at[rr] = there ? (tok0 + qt * SQ + ql) * NH + kh * G + row % G : -1;
-            rows[rr] = there ? q + (size_t)at[rr] * D : nullptr;
-            qp[rr] = pos0 + ql;
-            lo[rr] = first_seen(qp[rr], window);
-            nb[rr] = pools_seen(qp[rr], window, pool);
+            for (int kk = 0; kk < D / 16; ++kk)
+                umma_bf16(d + (uint32_t)(st * SN), da + (uint32_t)(kk / 4 * (S_Q_HALF >> 4) + 2 * (kk % 4)), db + (uint32_t)(kk / 4 * (S_K_HALF >> 4) + 2 * (kk % 4)), idesc,
+                          kk > 0 ? 1u : 0u, elected);
+            umma_commit(&s_done[st], elected);
         }
+    } else if (role >= S_ROW_WARPS) {
+        // ---- the keys: a block's loads two blocks ahead of its arrival ----
+        const int t = tid - 32 * S_ROW_WARPS;
+        constexpr int PER = D / 8, THREADS = 32 * S_LOAD_WARPS;
+        for (int b = 0; b < count + 2; ++b) {
+            if (b < count) {
+                const int st = b % S_STAGES;
+                if (b >= S_STAGES && ok && !mbar_wait(&s_done[st], (b / S_STAGES - 1) & 1)) { atomicExch(error_flag, 46); ok = false; }
+                uint8_t* to = sK + st * S_K_BYTES;
+                const bf16* src = blocks.is_pooled(b) ? k_pool : k_cache;
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) q_fragment(qa[kk], rows[0], rows[1], kk * 16 + 2 * (lane & 3));
-    }
-    const Cap c(scale, cap);
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.0f, 0.0f};
-    for (int b = 0; b < blocks.count; ++b) {
-        const bool pooled = blocks.is_pooled(b);
-        const int key0 = blocks.key0(b, SN);
-        cp_async_wait<0>();
-        __syncthreads();                                       // this block is there, and everyone is done with the other buffer
-        if (b + 1 < blocks.count) fetch(b + 1);
-        float s[SN / 8][4];
-#pragma unroll
-        for (int j = 0; j < SN / 8; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.0f;
-        const uint32_t k_addr = (uint32_t)__cvta_generic_to_shared(sK + (b & 1) * SN * LDK + ((lane & 7) + (lane >> 4) * 8) * LDK + ((lane >> 3) & 1) * 8);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
-#pragma unroll
-            for (int j = 0; j < SN / 8; j += 2) {
-                uint32_t b0, b1, b2, b3;
-                ldsm_x4(k_addr + (uint32_t)(j * 8 * LDK * 2 + kk * 32), b0, b1, b2, b3);
-                mma_bf16_16816(s[j], qa[kk], b0, b1);
-                mma_bf16_16816(s[j + 1], qa[kk], b2, b3);
-            }
-        c.apply<SN / 8>(s);
-        float mx[2] = {-INFINITY, -INFINITY};
-        const bool inside = pooled ? key0 + SN <= nb[0] : key0 + SN - 1 <= qp[0] && key0 >= lo[1];      // (rows that are not there: positions beyond)
-        if (!inside) {
-#pragma unroll
-            for (int j = 0; j < SN / 8; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int rr = e >> 1, kj = key0 + j * 8 + 2 * (lane & 3) + (e & 1);
-                    if (!(pooled ? kj < nb[rr] : (kj <= qp[rr] && kj >= lo[rr]))) s[j][e] = -INFINITY;
+                for (int i = 0; i < SN * PER; i += THREADS) {
+                    const int idx = i + t, row = idx / PER, c = idx % PER;
+                    const unsigned at = b < S_ROW_BLOCKS ? s_row[b * SN + row] : row_of(b, row);
+                    uint8_t* dst = to + c / 8 * S_K_HALF + row * 128 + (((c ^ row) & 7) << 4);
+                    if (at != ~0u) cp_async16(dst, src + (size_t)at * D + c * 8);
+                    else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
                 }
-        }
-#pragma unroll
-        for (int j = 0; j < SN / 8; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                mx[e >> 1] = fmaxf(mx[e >> 1], s[j][e]);
             }
-#pragma unroll
-        for (int rr = 0; rr < 2; ++rr) {
-            mx[rr] = fmaxf(mx[rr], __shfl_xor_sync(0xffffffffu, mx[rr], 1));
-            mx[rr] = fmaxf(mx[rr], __shfl_xor_sync(0xffffffffu, mx[rr], 2));
-            const float m_new = fmaxf(m_run[rr], mx[rr] * c.sl2), base = m_new == -INFINITY ? 0.0f : m_new;
-            float sum = 0.0f;
-#pragma unroll
-            for (int j = 0; j < SN / 8; ++j) sum += ex2_approx(fmaf(s[j][2 * rr], c.sl2, -base)) + ex2_approx(fmaf(s[j][2 * rr + 1], c.sl2, -base));
-            l_run[rr] = l_run[rr] * ex2_approx(m_run[rr] - base) + sum;
-            m_run[rr] = m_new;
+            cp_async_commit();
+            if (b < 2) continue;
+            cp_async_wait<2>();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&k_full[(b - 2) % S_STAGES])) : "memory");
         }
-    }
+    } else {
+        // ---- the rows ----
+        const int row = (warp & 3) * 32 + lane, qp = row / G < here ? pos0 + row / G : -1;       // (a query that is not there sees nothing)
+        const int lo = first_seen(qp, window), nb = qp >= 0 ? pools_seen(qp, window, pool) : 0;
+        const Cap c(scale, cap);
+        for (int b = warp >> 2; b < count; b += 2) {
+            const int st = b % S_STAGES;
+            if (ok && !mbar_wait(&s_done[st], (b / S_STAGES) & 1)) { atomicExch(error_flag, 47); ok = false; }
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const bool pooled = blocks.is_pooled(b);
+            const int key0 = blocks.key0(b, SN);
+            const bool inside = __all_sync(0xffffffffu, pooled ? key0 + SN <= nb : key0 + SN - 1 <= qp && key0 >= lo);
 #pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-        float l = l_run[rr];
-        l += __shfl_xor_sync(0xffffffffu, l, 1);
-        l += __shfl_xor_sync(0xffffffffu, l, 2);
-        if ((lane & 3) == 0 && at[rr] >= 0) lse[at[rr]] = m_run[rr] + log2f(l);
+            for (int half = 0; half < SN; half += 32) {
+                float s[32];
+                tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(st * SN + half), s);
+                tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(st * SN + half + 16), s + 16);
+                if (half + 32 == SN) {                         // the buffer may be written again
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&s_free[st])) : "memory");
+                }
+                c.apply<8>(reinterpret_cast<float(*)[4]>(s));
+                if (!inside) {
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) {
+                        const int kj = key0 + half + e;
+                        if (!(pooled ? kj < nb : (kj <= qp && kj >= lo))) s[e] = -INFINITY;
+                    }
+                }
+                float top[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+                for (int e = 4; e < 32; ++e) top[e & 3] = fmaxf(top[e & 3], s[e]);
+                const float m_new = fmaxf(m_run, fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * c.sl2), base = m_new == -INFINITY ? 0.0f : m_new;
+                float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                for (int e = 0; e < 32; ++e) sum[e & 3] += ex2_approx(fmaf(s[e], c.sl2, -base));
+                l_run = fmaf(l_run, ex2_approx(m_run - base), (sum[0] + sum[1]) + (sum[2] + sum[3]));
+                m_run = m_new;
+            }
+        }
+        if (warp >= 4) s_other[row] = make_float2(m_run, l_run);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) tmem_free<false>(tmem, S_STAGES * SN);
+    if (warp < 4) {
+        const int row = tid, ql = row / G;
+        const float2 o = s_other[row];
+        const float m = fmaxf(m_run, o.x), base = m == -INFINITY ? 0.0f : m;
+        if (ql < here) lse[(size_t)(tok0 + qt * SQ + ql) * NH + kh * G + row % G] = m + log2f(fmaf(l_run, ex2_approx(m_run - base), o.y * ex2_approx(o.x - base)));
     }
 }
 
@@ -730,8 +775,8 @@ MB_API int mb_attn_pooled_mix(int which, const void* q, const void* k_cache, con
     if ((((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)mixed | (uintptr_t)out) & 15) != 0) return MB_ERR_BAD_SIZE;
     if (which == 0) {
         cudaFuncSetAttribute(stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STATS_SMEM);
-        return launch_kernel(stats_kernel, dim3(KH, count, (max_query_len + SQ - 1) / SQ), 256, STATS_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache,
-                             (const bf16*)k_pool, lse, block_table, max_pages, cu_tokens, seq_lens, first_req, shift, scale, cap, window, pool, pool_rows);
+        return launch_kernel(stats_kernel, dim3(KH, count, (max_query_len + SQ - 1) / SQ), STATS_THREADS, STATS_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache,
+                             (const bf16*)k_pool, lse, block_table, max_pages, cu_tokens, seq_lens, first_req, shift, scale, cap, window, pool, pool_rows, error_flag);
     }
     const int tiles_of = (max_query_len + NQ - 1) / NQ;
     if (which == 1) {

@@ -271,6 +271,35 @@ def test_weights_mixed_ahead_of_the_values(monkeypatch, m):
     ops.check_device_errors()
 
 
+@pytest.mark.parametrize("m", [_attn(32, 16, 48, 112, 0.15, size=1400, pool=2, softcap=5.0), _attn(32, 8, 128, 128, 0.09, size=1400, pool=2, softcap=30.0)],
+                         ids=["h32k16d48v112", "h32k8d128v128"])
+def test_mixed_weights_behind_the_blocks_that_are_looked_up_ahead(monkeypatch, m):
+    """Three requests of uneven length in one step, the first with more blocks of keys and values than the kernels keep the rows' places of (24 of 64 keys, 48 of
+    32), head sizes that are no multiple of 64, two and four query heads a kv head, the same tokens in each, so each is held to the plain form's first rows."""
+    from marin_b200.engine import StepEntry
+    from marin_b200.kernels import ops
+
+    rt, hidden, T, page = runtime("bfloat16"), 48, 1750, 16
+    w = attention_weights(hidden, m, 41)
+    x = bf(torch.randn(T, hidden, generator=torch.Generator().manual_seed(42)))
+    want = plain.pooled_window_attention(x.double(), {k: v.double() for k, v in w.items()}, "m.mix", m, 1e-5)
+    part = build_mixer("attention", m, hidden, 1e-5, rt, w)
+    taken = []
+    inner = ops._pooled_mix
+    monkeypatch.setattr(ops, "POOLED_MIX_COSTS", (0.0, 0.0, 0.0))
+    monkeypatch.setattr(ops, "_pooled_mix", lambda *a: (taken.append(1), inner(*a))[1])
+    runner, lengths = harness([part.cache_need()], rt, page=page, pages=160), {"a": T, "b": 41, "c": 193}
+    for req, n in lengths.items():
+        runner.begin(req)
+        runner.cache.reserve(req, n)
+    ctx = runner.build_context([StepEntry(req, [0] * n, []) for req, n in lengths.items()])
+    residual = torch.zeros(sum(lengths.values()), hidden, device=DEV)
+    part.forward(torch.cat([x[:n] for n in lengths.values()]).to(DEV).contiguous(), ctx, runner.views.view(0, ctx), residual)
+    close(residual.cpu(), torch.cat([want[:n] for n in lengths.values()]), "bfloat16", "uneven requests")
+    assert taken
+    ops.check_device_errors()
+
+
 @pytest.mark.parametrize("gain", [1.0, 2.0 ** -12, 300.0])
 def test_mixed_weights_are_held_to_more_bits_than_the_results(gain):
     """The attention's rows against float64 from the same queries, keys, values and pooled rows: they are off by the rounding of the result to bf16 (relative
