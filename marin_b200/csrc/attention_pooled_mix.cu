@@ -1,5 +1,5 @@
 // bf16 attention over a window and pooled blocks with mixed head weights (attention_pooled.cu) over prompt portions, on the tensor cores
-// (mma.sync), compiled for one head layout: -DHEAD_DIM, -DV_DIM (multiples of 16 up to 128), -DGROUP (2 or 4 query heads a kv head), -DKV_HEADS
+// (tcgen05; the mixing mma.sync), compiled for one head layout: -DHEAD_DIM, -DV_DIM (multiples of 16 up to 128), -DGROUP (2 or 4 query heads a kv head), -DKV_HEADS
 // (with GROUP * KV_HEADS 16 or 32).
 //
 // out_h = sum_j (sum_g talk[h, g] p_g[j]) v_kv(h)[j]: the heads' weights of a (query, key) pair are mixed before they meet the values, so every
