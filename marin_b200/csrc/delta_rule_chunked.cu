@@ -18,7 +18,7 @@
 // the substitution adds up and the state are float32; where a float32 number has to be an operand of a product it is split into two bf16
 // numbers (value = hi + lo) and the three larger products are taken, so that about 16 bits of it enter (of a block's inverse only what lies
 // below its unit diagonal).
-// Measured on B200, two prompts of 712 and 1,188 tokens, 20 heads of 128 x 128, a decay per channel: prepare 101 us (141 with a column of the substitution a
+// Measured on B200, two prompts of 712 and 1,188 tokens, 20 heads of 128 x 128, a decay per channel: prepare 91 us (141 with a column of the substitution a
 // thread), walk 65 (124 with the outputs made in it, 32 value channels a CTA and operands from shared memory on both sides), read 39 (with the norm, 12 us as a
 // kernel of its own).
 #define MB_LIB "delta_rule_chunked"
@@ -205,18 +205,27 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(
         float run = 0.0f;
         for (int i = 0; i < CH; ++i) { run += sG[i]; sG[i] = run; }
     }
-    for (int row = warp; row < CH; row += PREP_THREADS / 32) {
+    {                                                          // eight rows a warp side by side, four lanes a row
+        const int row = warp * 8 + g;
         float qq = 0.0f, kk = 0.0f, qk = 0.0f;
-        for (int c = lane; c < DQ; c += 32) {
-            const float x = __bfloat162float(sq[row * LDR + c]), y = __bfloat162float(sk[row * LDR + c]);
-            qq = fmaf(x, x, qq);
-            kk = fmaf(y, y, kk);
-            qk = fmaf(x, y, qk);
+        for (int c = lane & 3; c < DQ / 8; c += 4) {
+            const uint4 q8 = *reinterpret_cast<const uint4*>(sq + row * LDR + c * 8), k8 = *reinterpret_cast<const uint4*>(sk + row * LDR + c * 8);
+            const uint32_t qw[4] = {q8.x, q8.y, q8.z, q8.w}, kw[4] = {k8.x, k8.y, k8.z, k8.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float2 x = bf2(qw[u]), y = bf2(kw[u]);
+                qq = fmaf(x.x, x.x, qq); qq = fmaf(x.y, x.y, qq);
+                kk = fmaf(y.x, y.x, kk); kk = fmaf(y.y, y.y, kk);
+                qk = fmaf(x.x, y.x, qk); qk = fmaf(x.y, y.y, qk);
+            }
         }
-        qq = warp_sum(qq);
-        kk = warp_sum(kk);
-        qk = warp_sum(qk);
-        if (lane == 0) {
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            qq += __shfl_xor_sync(0xffffffffu, qq, o);
+            kk += __shfl_xor_sync(0xffffffffu, kk, o);
+            qk += __shfl_xor_sync(0xffffffffu, qk, o);
+        }
+        if ((lane & 3) == 0) {
             s_fq[row] = 1.0f / (sqrtf((float)DQ) * sqrtf(qq + UNIT_EPS));
             s_fk[row] = 1.0f / sqrtf(kk + UNIT_EPS);
             s_qk[row] = qk;
@@ -231,21 +240,28 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(
         *reinterpret_cast<uint4*>(ph + PPLANE + at) = make_uint4(0, 0, 0, 0);
     }
     __syncthreads();
-    // ---- A and P: two warps make the rows 16 I .. 16 I + 15, each eight columns of every block of sixteen
+    // ---- A and P: two warps make the rows 16 I .. 16 I + 15, with one decay per head each eight columns of every block of sixteen.  With one per channel each
+    // half of the channels (so that no row's exponentials and splits are made twice), and they exchange the halves of the sums: with the
+    // rows' lengths found four lanes a row, 102 -> 91 us for 620 chunks and heads (the rows of the last block had 2.6 times the first one's work).
     {
         const int I = warp >> 1, half = warp & 1;
         const int i0 = I * 16 + g, i1 = i0 + 8;
+        constexpr int NH = CHANNEL ? 2 : 1;                    // runs of eight columns
         float accA[4][4], accP[4][4];                          // [block of columns]; the fourth: this block's own
+        float farA[3][4], farP[3][4];                          // the run of eight columns that the other warp will finish
 #pragma unroll
         for (int J = 0; J < 4; ++J)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) { accA[J][e] = 0.0f; accP[J][e] = 0.0f; }
+            for (int e = 0; e < 4; ++e) {
+                accA[J][e] = 0.0f; accP[J][e] = 0.0f;
+                if (J < 3) { farA[J < 3 ? J : 0][e] = 0.0f; farP[J < 3 ? J : 0][e] = 0.0f; }
+            }
         // a reference for the rows of this block against earlier ones: the sum at the last row before it; for its rows 8 .. 15 against
         // its rows 0 .. 7 (worked out by the first of the two warps): the sum at its row 7
         const float* ref = sG + (I > 0 ? I * 16 - 1 : 0) * LDG;
         const float* mid = sG + (I * 16 + 7) * LDG;
 #pragma unroll 1
-        for (int kk = 0; kk < DQ / 16; ++kk) {
+        for (int kk = CHANNEL ? half * ((KT + 1) / 2) : 0; kk < (CHANNEL && half == 0 ? (KT + 1) / 2 : KT); ++kk) {
             uint32_t rk[4], rq[4];                             // raw bf16 pairs: rows i0, i1 at channels c, c + 8
             const int c = kk * 16 + t2;
 #pragma unroll
@@ -280,17 +296,20 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(
 #pragma unroll
                     for (int J = 0; J < 3; ++J) {
                         if (J >= I) continue;
-                        const int j = J * 16 + half * 8 + g;
-                        const float2 ga = *reinterpret_cast<const float2*>(sG + j * LDG + c), gb = *reinterpret_cast<const float2*>(sG + j * LDG + c + 8);
-                        const float2 x = bf2(*reinterpret_cast<const uint32_t*>(sk + j * LDR + c)), y = bf2(*reinterpret_cast<const uint32_t*>(sk + j * LDR + c + 8));
-                        uint32_t bh0, bl0, bh1, bl1;
-                        split_bf16(x.x * ex2_approx(r[0] - ga.x), x.y * ex2_approx(r[1] - ga.y), bh0, bl0);
-                        split_bf16(y.x * ex2_approx(r[2] - gb.x), y.y * ex2_approx(r[3] - gb.y), bh1, bl1);
-                        mma3(accA[J], kh_, kl_, bh0, bh1, bl0, bl1);
-                        mma3(accP[J], qh_, ql_, bh0, bh1, bl0, bl1);
+#pragma unroll
+                        for (int far = 0; far < NH; ++far) {
+                            const int j = J * 16 + (half ^ far) * 8 + g;
+                            const float2 ga = *reinterpret_cast<const float2*>(sG + j * LDG + c), gb = *reinterpret_cast<const float2*>(sG + j * LDG + c + 8);
+                            const float2 x = bf2(*reinterpret_cast<const uint32_t*>(sk + j * LDR + c)), y = bf2(*reinterpret_cast<const uint32_t*>(sk + j * LDR + c + 8));
+                            uint32_t bh0, bl0, bh1, bl1;
+                            split_bf16(x.x * ex2_approx(r[0] - ga.x), x.y * ex2_approx(r[1] - ga.y), bh0, bl0);
+                            split_bf16(y.x * ex2_approx(r[2] - gb.x), y.y * ex2_approx(r[3] - gb.y), bh1, bl1);
+                            mma3(far ? farA[J] : accA[J], kh_, kl_, bh0, bh1, bl0, bl1);
+                            mma3(far ? farP[J] : accP[J], qh_, ql_, bh0, bh1, bl0, bl1);
+                        }
                     }
                 }
-                if (half == 0) {                               // rows 8 .. 15 of the block (the operands of rows 0 .. 7 are zero)
+                {                                              // rows 8 .. 15 of the block (the operands of rows 0 .. 7 are zero)
                     const float2 ra = *reinterpret_cast<const float2*>(mid + c), rb = *reinterpret_cast<const float2*>(mid + c + 8);
                     const float r[4] = {ra.x, ra.y, rb.x, rb.y};
                     kh_[0] = kh_[2] = kl_[0] = kl_[2] = qh_[0] = qh_[2] = ql_[0] = ql_[2] = 0u;
@@ -311,6 +330,51 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(
                     mma3(accP[3], qh_, ql_, bh0, bh1, bl0, bl1);
                 }
             }
+        }
+        float* given = reinterpret_cast<float*>(sL) + (I * I * 8 + (half ? 8 * I + 4 : 0)) * 32 + lane;    // (nothing of L is there yet)
+        if (CHANNEL) {
+#pragma unroll
+            for (int J = 0; J < 3; ++J) {
+                if (J >= I) continue;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { given[(J * 8 + e) * 32] = farA[J][e]; given[(J * 8 + 4 + e) * 32] = farP[J][e]; }
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) { given[(I * 8 + e) * 32] = accA[3][2 + e]; given[(I * 8 + 2 + e) * 32] = accP[3][2 + e]; }
+        }
+        if (CHANNEL && lane < 28) {                            // the 8 x 8 square on the diagonal that is this warp's, a pair of rows per lane
+            int ii = 1;
+            while ((ii + 1) * ii / 2 <= lane) ++ii;
+            const int i = warp * 8 + ii, j = warp * 8 + lane - ii * (ii - 1) / 2;
+            float a = 0.0f, b = 0.0f;
+#pragma unroll 4
+            for (int c = 0; c < DQ; c += 2) {
+                const float2 ki = bf2(*reinterpret_cast<const uint32_t*>(sk + i * LDR + c)), kj = bf2(*reinterpret_cast<const uint32_t*>(sk + j * LDR + c));
+                const float2 qi = bf2(*reinterpret_cast<const uint32_t*>(sq + i * LDR + c));
+                const float2 gi = *reinterpret_cast<const float2*>(sG + i * LDG + c), gj = *reinterpret_cast<const float2*>(sG + j * LDG + c);
+                const float x = kj.x * ex2_approx(gi.x - gj.x), y = kj.y * ex2_approx(gi.y - gj.y);
+                a = fmaf(ki.x, x, a); a = fmaf(ki.y, y, a);
+                b = fmaf(qi.x, x, b); b = fmaf(qi.y, y, b);
+            }
+            sD[i * LDD + (j & 15)] = s_beta[i] * s_fk[i] * s_fk[j] * a;
+            b *= s_fq[i] * s_fk[j];
+            const bf16 hi = __float2bfloat16_rn(b);
+            const int at = i * LDW + j;
+            ph[at] = hi;
+            ph[PPLANE + at] = __float2bfloat16_rn(b - __bfloat162float(hi));
+        }
+        if (CHANNEL) {
+            __syncthreads();
+            const float* got = reinterpret_cast<float*>(sL) + (I * I * 8 + (half ? 0 : 8 * I + 4)) * 32 + lane;
+#pragma unroll
+            for (int J = 0; J < 3; ++J) {
+                if (J >= I) continue;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { accA[J][e] += got[(J * 8 + e) * 32]; accP[J][e] += got[(J * 8 + 4 + e) * 32]; }
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) { accA[3][2 + e] += got[(I * 8 + e) * 32]; accP[3][2 + e] += got[(I * 8 + 2 + e) * 32]; }
+            __syncthreads();
         }
 #pragma unroll
         for (int J = 0; J < 4; ++J) {
@@ -340,27 +404,6 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(
                 *reinterpret_cast<uint32_t*>(ph + at) = hi;
                 *reinterpret_cast<uint32_t*>(ph + PPLANE + at) = lo;
             }
-        }
-        if (CHANNEL && lane < 28) {                            // the 8 x 8 square on the diagonal that is this warp's, a pair of rows per lane
-            int ii = 1;
-            while ((ii + 1) * ii / 2 <= lane) ++ii;
-            const int i = warp * 8 + ii, j = warp * 8 + lane - ii * (ii - 1) / 2;
-            float a = 0.0f, b = 0.0f;
-#pragma unroll 4
-            for (int c = 0; c < DQ; c += 2) {
-                const float2 ki = bf2(*reinterpret_cast<const uint32_t*>(sk + i * LDR + c)), kj = bf2(*reinterpret_cast<const uint32_t*>(sk + j * LDR + c));
-                const float2 qi = bf2(*reinterpret_cast<const uint32_t*>(sq + i * LDR + c));
-                const float2 gi = *reinterpret_cast<const float2*>(sG + i * LDG + c), gj = *reinterpret_cast<const float2*>(sG + j * LDG + c);
-                const float x = kj.x * ex2_approx(gi.x - gj.x), y = kj.y * ex2_approx(gi.y - gj.y);
-                a = fmaf(ki.x, x, a); a = fmaf(ki.y, y, a);
-                b = fmaf(qi.x, x, b); b = fmaf(qi.y, y, b);
-            }
-            sD[i * LDD + (j & 15)] = s_beta[i] * s_fk[i] * s_fk[j] * a;
-            b *= s_fq[i] * s_fk[j];
-            const bf16 hi = __float2bfloat16_rn(b);
-            const int at = i * LDW + j;
-            ph[at] = hi;
-            ph[PPLANE + at] = __float2bfloat16_rn(b - __bfloat162float(hi));
         }
         if (CHANNEL && tid < CH) {                             // P_ii = q_i . k_i
             const float b = s_qk[tid] * s_fq[tid] * s_fk[tid];
