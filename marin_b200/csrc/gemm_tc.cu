@@ -4,9 +4,9 @@
 // (BN = 16..256 tokens per CTA), so that a decode step with a handful of tokens still fills the 128-row
 // datapath and streams every weight exactly once.  Both operands are K-major in global memory (w is
 // [N, K], x is [T, K]) and are brought into shared memory by TMA (cp.async.bulk.tensor, 128-byte swizzle,
-// no multicast) through a ring of STAGES buffers guarded by mbarriers; one warp issues the MMAs, whose float32 accumulator
-// lives in tensor memory; four
-// warps read it back with tcgen05.ld and write out[t, n] (32 consecutive n per warp and token: coalesced).
+// no multicast) through a ring of STAGES buffers guarded by mbarriers; one warp issues the MMAs (with up to 64 tokens into two
+// accumulators in turn, which the epilogue adds), whose float32 accumulators live in tensor memory; four
+// warps read them back with tcgen05.ld and write out[t, n] (32 consecutive n per warp and token: coalesced).
 //
 // Split-K: with few tokens and few weight rows there are fewer tiles than SMs, so blockIdx.z cuts K into
 // slices.  The slices of a tile are the CTAs of one thread-block cluster and add their partial tiles through
@@ -235,11 +235,13 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
     const int kb_begin = blockIdx.z * kb_per_split;
     const int kb_end = min(total_kb, kb_begin + kb_per_split);
     const int nkb = kb_end - kb_begin;
-    // (One warp issues the MMAs.  While each cost its thread a hundred cycles, two with an accumulator each were faster up to 64 tokens; now the second is
-    // only one more that has to come to its end: a decode step of one sequence, 8 layers of the 0.6B layout, 311 us with two and 284 with one; of eight
-    // sequences, 4 layers of the 4B layout, 426 and 427.)
+    // tcgen05.mma cuts its sums off instead of rounding them, so the error of a sum grows with the additions to one accumulator.  Up to 64 tokens, where tensor
+    // memory has room for a second, even k-blocks go to one and odd ones to the other: half the error (16 tokens by 2,560 rows of 9,728 in eight slices 0.57e-6 of
+    // the sums against 64 bits, 1.20e-6 with one; by 151,936 rows of 2,560 uncut 1.27e-6 and 2.66e-6) for a second read of tensor memory (a decode step of one
+    // sequence, 8 layers of the 0.6B layout, 288 us, 285 with one; of eight sequences, 4 layers of the 4B layout, 427 and 428).
+    constexpr bool TWO = BN <= 64;
     constexpr int NSC = 64;                                           // threads that work out the per-token factors
-    constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
+    constexpr uint32_t TMEM_COLS = (TWO ? 2 * BN : BN) < 32 ? 32 : (TWO ? 2 * BN : BN);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -292,9 +294,10 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t a = smem_u32(smem + s * L::STAGE_BYTES);
             const uint64_t adesc = umma_desc(a), bdesc = umma_desc(a + L::A_BYTES);
+            const uint32_t d = tmem_d + (uint32_t)(TWO ? (i & 1) * BN : 0);
 #pragma unroll
             for (int kk = 0; kk < TC_BK / 16; ++kk)
-                umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (i > 0 || kk > 0) ? 1u : 0u, elected);
+                umma_bf16(d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (i > (TWO ? 1 : 0) || kk > 0) ? 1u : 0u, elected);
             if (i + STAGES < nkb) umma_commit(&empty[s], elected);    // only a stage that is filled again needs to be given back
         }
         umma_commit(accum, elected);
@@ -304,8 +307,8 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
         // warps 2 and 3: `tpt` threads per token (a power of two, at most 32), each adds its share of the slots in
         // slot order, up to 24 loads in flight at a time; then the shares are added in a fixed tree
         const int here = min(BN, T - t0);
-        int tpt = 32;
-        while (tpt * here > NSC && tpt > 1) tpt >>= 1;
+        int tpt = 32;                                                 // (by 32 threads up to 64 tokens whatever their number: the order of a token's sum)
+        while (tpt * here > (TWO ? 32 : NSC) && tpt > 1) tpt >>= 1;
         const int local = threadIdx.x - 64, part = local % tpt;
         const int per = (scale.slots + tpt - 1) / tpt;
         const int trips = (BN * tpt + NSC - 1) / NSC;                 // the same for every thread: shuffles below
@@ -352,6 +355,12 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
             float v[16];
             if (have) {
                 tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+                if (TWO && nkb >= 2) {                                // the odd k-blocks' accumulator
+                    float v2[16];
+                    tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(BN + c0), v2);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] += v2[j];
+                }
             }
             else {
 #pragma unroll
@@ -524,6 +533,12 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
         float v[16];
         if (have) {
             tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+            if (TWO && nkb >= 2) {
+                float v2[16];
+                tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(BN + c0), v2);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] += v2[j];
+            }
         }
         else {
 #pragma unroll

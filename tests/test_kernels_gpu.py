@@ -75,8 +75,8 @@ def test_gemm(ops, combo, T, N, K):
 
 @pytest.mark.parametrize("T", [24, 32, 16, 64])
 def test_gemm_of_a_few_tokens_many_times_back_to_back_gives_the_same_bits(ops, T):
-    """The small-batch product has two MMA issuers that share one ring of stages; launched back to back (each launch a
-    programmatic dependent of the one before, as in a decode step) its K slices start at different moments every time.
+    """The small-batch product launched back to back (each launch a
+    programmatic dependent of the one before, as in a decode step): its K slices start at different moments every time.
     Three hundred launches at a layer's real sizes must give one and the same result, the right one."""
     g = torch.Generator(device=DEV).manual_seed(40 + T)
     N, K = 2560, 9728
@@ -90,6 +90,21 @@ def test_gemm_of_a_few_tokens_many_times_back_to_back_gives_the_same_bits(ops, T
     torch.testing.assert_close(outs[0].double(), want, rtol=1e-5, atol=1e-5)
     same = (outs == outs[0]).flatten(1).all(dim=1)
     assert bool(same.all()), f"launch {int(torch.nonzero(~same)[0])} of 300 gave other bits than the first"
+
+
+@pytest.mark.parametrize("T,N,K", [(1, 2560, 2560), (16, 2560, 9728), (17, 20000, 1024), (64, 20000, 2560), (40, 4096, 4096)])
+def test_sums_of_few_tokens_go_to_two_accumulators(ops, T, N, K):
+    """An accumulator loses at most the last bit (2^-23 of itself) at each addition of 16 products.  Of positive numbers it grows evenly, so it is half its end on
+    average: with the k-blocks of a slice dealt to two, at most a quarter of the slice's K / 16 additions times 2^-23 is lost (and where up to eight slices meet
+    seven roundings of at most 2^-24, half of it and of the end on average: once 2^-23); one accumulator for all of them loses more (K / 16 times 0.38 2^-23 was seen)."""
+    g = torch.Generator(device=DEV).manual_seed(T + K)
+    x, w = torch.rand(T, K, device=DEV, generator=g).to(torch.bfloat16), torch.rand(N, K, device=DEV, generator=g).to(torch.bfloat16)
+    want = x.double() @ w.double().t()
+    for out, added in ((torch.empty(T, N, device=DEV), False), (torch.zeros(T, N, device=DEV), True)):
+        ops.gemm(x, w, out, accumulate=added)
+        per = -(-(-(-K // 64)) // ops.gemm_plan(T, N, K)[1])                            # k-blocks a slice
+        assert float(((out.double() - want).abs() / want).mean()) <= (per * 4 / 4 + 1) * 2.0 ** -23
+    ops.check_device_errors()
 
 
 @pytest.mark.parametrize("T,N,K", [(1000, 2560, 512), (2048, 2560, 4096), (777, 3000, 320), (1500, 1981, 256), (1031, 4100, 192)])
