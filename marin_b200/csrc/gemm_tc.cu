@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
                                                       const __grid_constant__ CUtensorMap map_x, void* __restrict__ out,
                                                       int mode, int T, int N, int K, int kb_per_split,
                                                       float* __restrict__ partials, int* __restrict__ counters,
-                                                      int* __restrict__ error_flag, int cluster_reduce,
+                                                      int* __restrict__ error_flag, int cluster_reduce, int accumulators,
                                                       const TcNormOut norm, const TcRowScale scale, const TcHeadsOut heads, const TcGlu glu) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ float s_scale[BN];
@@ -239,9 +239,11 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
     // memory has room for a second, even k-blocks go to one and odd ones to the other: half the error (16 tokens by 2,560 rows of 9,728 in eight slices 0.57e-6 of
     // the sums against 64 bits, 1.20e-6 with one; by 151,936 rows of 2,560 uncut 1.27e-6 and 2.66e-6) for a second read of tensor memory (a decode step of one
     // sequence, 8 layers of the 0.6B layout, 288 us, 285 with one; of eight sequences, 4 layers of the 4B layout, 427 and 428).
-    constexpr bool TWO = BN <= 64;
+    // With 128 tokens the caller says (gemm_plan: where K is cut into half the slices that there is room for).
+    constexpr bool FEW = BN <= 64;
+    const bool two = FEW || (BN == 128 && accumulators == 2);
     constexpr int NSC = 64;                                           // threads that work out the per-token factors
-    constexpr uint32_t TMEM_COLS = (TWO ? 2 * BN : BN) < 32 ? 32 : (TWO ? 2 * BN : BN);
+    const uint32_t tmem_cols = two ? (2 * BN < 32 ? 32 : 2 * BN) : BN;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -250,7 +252,7 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
     }
     if (warp == 0) {
         __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -294,10 +296,10 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t a = smem_u32(smem + s * L::STAGE_BYTES);
             const uint64_t adesc = umma_desc(a), bdesc = umma_desc(a + L::A_BYTES);
-            const uint32_t d = tmem_d + (uint32_t)(TWO ? (i & 1) * BN : 0);
+            const uint32_t d = tmem_d + (uint32_t)(two ? (i & 1) * BN : 0);
 #pragma unroll
             for (int kk = 0; kk < TC_BK / 16; ++kk)
-                umma_bf16(d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (i > (TWO ? 1 : 0) || kk > 0) ? 1u : 0u, elected);
+                umma_bf16(d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (i > (two ? 1 : 0) || kk > 0) ? 1u : 0u, elected);
             if (i + STAGES < nkb) umma_commit(&empty[s], elected);    // only a stage that is filled again needs to be given back
         }
         umma_commit(accum, elected);
@@ -308,7 +310,7 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
         // slot order, up to 24 loads in flight at a time; then the shares are added in a fixed tree
         const int here = min(BN, T - t0);
         int tpt = 32;                                                 // (by 32 threads up to 64 tokens whatever their number: the order of a token's sum)
-        while (tpt * here > (TWO ? 32 : NSC) && tpt > 1) tpt >>= 1;
+        while (tpt * here > (FEW ? 32 : NSC) && tpt > 1) tpt >>= 1;
         const int local = threadIdx.x - 64, part = local % tpt;
         const int per = (scale.slots + tpt - 1) / tpt;
         const int trips = (BN * tpt + NSC - 1) / NSC;                 // the same for every thread: shuffles below
@@ -355,7 +357,7 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
             float v[16];
             if (have) {
                 tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-                if (TWO && nkb >= 2) {                                // the odd k-blocks' accumulator
+                if (two && nkb >= 2) {                                // the odd k-blocks' accumulator
                     float v2[16];
                     tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(BN + c0), v2);
 #pragma unroll
@@ -533,7 +535,7 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
         float v[16];
         if (have) {
             tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-            if (TWO && nkb >= 2) {
+            if (two && nkb >= 2) {
                 float v2[16];
                 tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(BN + c0), v2);
 #pragma unroll
@@ -590,7 +592,7 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     }
 }
 
@@ -599,6 +601,11 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
 // TMA and runs ahead into the next tile; warp 1 issues the MMAs into one of two accumulators in tensor memory;
 // warps 2..9 drain the other accumulator (tcgen05.ld, convert, store; two warps per 32-lane quarter) meanwhile, so the tensor cores do not wait
 // for the epilogue.
+// PARTS (fewer tiles than SMs, one of 128 tokens a CTA): K is cut into two or four parts with an accumulator each, which the epilogue adds in their order: the sums, bit
+// for bit, of as many slices of K in a cluster, without the tiles' way through shared memory.  An accumulator cuts its additions off: error of 512 tokens by
+// 2,560 rows of 9,728 against 64 bits 2.5e-6 with four, as with four slices, and 10.9e-6 with one,
+// 40.7 us and 41.9 (by pairs); 512 by 4,096 rows of 1,024 9.0 and 8.7, as bfloat16 8.6 and 8.0.  (Four fill tensor memory: a CTA's next tile, if it
+// has one, waits for the epilogue.)
 // PAIR: two CTAs of a cluster work on 256 weight rows x BN tokens (cta_group::2): each loads its own 128 weight rows and half of the tokens, the
 // first one's MMA thread issues for both, each drains its own 128 rows.  A tile's tokens then lie in shared memory once for two SMs instead of twice: a third
 // less to fetch, write and read at 256 tokens, which is power, and power is the clock (2,048 tokens,
@@ -679,19 +686,33 @@ MB_API int mb_gemm_tc_probe_read(long long* host) { return (int)cudaMemcpyFromSy
 #define PROBE_OUT(slot, name)
 #endif
 
+// The same in two steps, so that several are on their way at once: nothing of v may be used before tmem_ld_wait.
+__device__ __forceinline__ void tmem_ld16_ask(uint32_t taddr, float* v) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+          "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld_wait(float* a, float* b) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) asm volatile("" : "+f"(a[i]), "+f"(b[i]));
+}
+
 template <int BN, bool PAIR>
 struct TcRing {
     static constexpr int A_BYTES = TC_BM * TC_BK * 2, B_ROWS = PAIR ? BN / 2 : BN, STAGE_BYTES = A_BYTES + B_ROWS * TC_BK * 2;
 };
 
-template <int BN, int STAGES, bool SK, bool PAIR>
+template <int BN, int STAGES, bool SK, bool PAIR, bool PARTS>
 __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                  const __grid_constant__ CUtensorMap map_x,
                                                                  void* __restrict__ out, int mode, int T, int N, int K,
                                                                  int* __restrict__ error_flag, const TcNormOut norm,
                                                                  const TcRowScale scale, const TcStreamK sk, const TcHeadsOut heads,
                                                                  const float* __restrict__ rope,
-                                                                 const __grid_constant__ CUtensorMap map_out, int reduce_out, const TcGlu glu) {
+                                                                 const __grid_constant__ CUtensorMap map_out, int reduce_out, const TcGlu glu, int parts) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ float s_pscale[2][BN];          // the per-token factors of a coupled norm, for the tile in each accumulator
     // heads finished in the epilogue: per half of the columns (its four warps), two staging buffers of sixteen tokens
@@ -710,7 +731,9 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_n = (N + CTAS * TC_BM - 1) / (CTAS * TC_BM), tiles_t = (T + BN - 1) / BN;
     const int nkb = (K + TC_BK - 1) / TC_BK;
-    constexpr uint32_t TMEM_COLS = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
+    static_assert(!PARTS || (BN == 128 && !SK && !PAIR), "four accumulators of 128 columns fill tensor memory");
+    constexpr uint32_t TMEM_COLS = PARTS ? 512 : 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
+    const int sums = PARTS ? parts : 1, sets = PARTS && sums == 4 ? 1 : 2;      // accumulators a tile; sets of them
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -761,20 +784,23 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
     } else if (role == 1 && rank == 0) {
         const uint32_t elected = elect_one(), tmem_mma = warp_same(tmem_base);
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(CTAS * TC_BM >> 4) << 24);
+        const int per = (nkb + sums - 1) / sums;                      // k-blocks an accumulator
         int it = 0, local = 0;
         bool ok = true;
         PROBE_DECL(m_full); PROBE_DECL(m_acc); PROBE_DECL(m_all);
         const long long mt_start = PROBE_T();
         TcWalk walk(sk, SK, tiles_n, tiles_t, nkb, CTAS);
         for (int tile, kb0, kb1; ok && walk.next(tile, kb0, kb1); ++local) {
-            const int buf = local & 1;
-            const uint32_t acc_phase = (local >> 1) & 1;
+            const int buf = local & (sets - 1);
+            const uint32_t acc_phase = (local >> (sets - 1)) & 1;
             const long long mt0 = PROBE_T();
             if (!mbar_wait_warp(&acc_empty[buf], acc_phase ^ 1)) { atomicExch(error_flag, 12); ok = false; break; }
             PROBE_ADD(m_acc, mt0);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t tmem_d = tmem_mma + (uint32_t)(buf * BN);
+            uint32_t tmem_d = tmem_mma + (uint32_t)(buf * sums * BN);
+            int left = per;                                           // k-blocks that the accumulator still takes
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
+                if (PARTS && left == 0) { tmem_d += BN; left = per; }
                 const int s = it % STAGES;
                 const uint32_t phase = (it / STAGES) & 1;
                 const long long mt1 = PROBE_T();
@@ -785,9 +811,10 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
                 const uint64_t adesc = umma_desc(a), bdesc = umma_desc(a + L::A_BYTES);
 #pragma unroll
                 for (int kk = 0; kk < TC_BK / 16; ++kk) {
-                    if (PAIR) umma_bf16_pair(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u, elected);
-                    else umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u, elected);
+                    if (PAIR) umma_bf16_pair(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, ((PARTS ? left < per : kb > kb0) || kk > 0) ? 1u : 0u, elected);
+                    else umma_bf16(tmem_d, adesc + 2 * kk, bdesc + 2 * kk, idesc, ((PARTS ? left < per : kb > kb0) || kk > 0) ? 1u : 0u, elected);
                 }
+                --left;
                 if (PAIR) umma_commit_pair(&empty[s], elected);
                 else umma_commit(&empty[s], elected);
             }
@@ -809,8 +836,8 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
             const bool is_head = SK && kb1 < nkb;  // the tile's first k-blocks: the next CTA's parked piece is added
             const int tile_row = tile_rows(tile, tiles_n, tiles_t) * CTAS + rank;
             const int n0 = tile_row * TC_BM, t0 = tile_tokens(tile, tiles_n, tiles_t) * BN;
-            const int buf = local & 1;
-            const uint32_t acc_phase = (local >> 1) & 1;
+            const int buf = local & (sets - 1);
+            const uint32_t acc_phase = (local >> (sets - 1)) & 1;
             if (scale.sumsq != nullptr) {
                 // while the MMAs of this tile run: each of the 256 epilogue threads adds the slots of one token, in slot
                 // order, up to 24 loads in flight; the eight warps then meet at a barrier of their own
@@ -1039,7 +1066,25 @@ __global__ void __launch_bounds__(320) gemm_tc_persistent_kernel(const __grid_co
 #pragma unroll 1
                 for (int c0 = c_begin; c0 < c_end && !beyond; c0 += 16) {
                     float v[16];
-                    tmem_ld16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c0), v);
+                    const uint32_t at = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * sums * BN + c0);
+                    if (!PARTS) {
+                        tmem_ld16(at, v);
+                    } else {
+                        float more[16];
+                        tmem_ld16_ask(at, v);
+                        tmem_ld16_ask(at + BN, more);
+                        tmem_ld_wait(v, more);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] += more[j];
+                        if (sums == 4) {
+                            float third[16];
+                            tmem_ld16_ask(at + 2 * BN, third);
+                            tmem_ld16_ask(at + 3 * BN, more);
+                            tmem_ld_wait(third, more);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) v[j] = (v[j] + third[j]) + more[j];
+                        }
+                    }
                     if (SK && is_tail) {
 #pragma unroll
                         for (int j = 0; j < 16; ++j) __stcg(parked + (size_t)(c0 + j) * TC_BM, v[j]);
@@ -1087,7 +1132,7 @@ static bool glu_fits(const TcGlu& glu, int mode, int N) {
 template <int BN, int STAGES>
 static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, void* out, int mode, int T, int N, int K, int splits,
                      int kb_per_split, float* partials, int* counters, int* error_flag, int cluster_reduce,
-                     const TcNormOut& norm, const TcRowScale& scale, const TcHeadsOut& heads, const TcGlu& glu, cudaStream_t s) {
+                     int accumulators, const TcNormOut& norm, const TcRowScale& scale, const TcHeadsOut& heads, const TcGlu& glu, cudaStream_t s) {
     constexpr int smem = STAGES * TcSmem<BN>::STAGE_BYTES + 1024 + 256;
     static_assert(STAGES * TcSmem<BN>::STAGE_BYTES >= BN * TC_BM * 4, "the cluster reduction reuses the pipeline buffers");
     static bool configured = false;
@@ -1099,7 +1144,7 @@ static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, void* out, in
     const bool clustered = cluster_reduce && splits > 1;
     return launch_kernel(gemm_tc_kernel<BN, STAGES>, dim3((N + TC_BM - 1) / TC_BM, (T + BN - 1) / BN, splits), dim3(128), smem, s,
                          clustered ? splits : 0, mw, mx, out, mode, T, N, K, kb_per_split, partials, counters, error_flag,
-                         clustered ? 1 : 0, norm, scale, heads, glu);
+                         clustered ? 1 : 0, accumulators, norm, scale, heads, glu);
 }
 
 // Tiles a launch with `bn` tokens per CTA would have (for the caller's choice of split).
@@ -1115,10 +1160,10 @@ static bool tc_reduce_out() {
     return state == 1;
 }
 
-template <int BN, int STAGES, bool SK, bool PAIR = false>
+template <int BN, int STAGES, bool SK, bool PAIR = false, bool PARTS = false>
 static int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, void* out, int mode, int T, int N, int K, int ctas,
                              int* error_flag, const TcNormOut& norm, const TcRowScale& scale, TcStreamK sk, cudaStream_t s,
-                             const TcGlu& glu, const TcHeadsOut& heads = TcHeadsOut{}, const float* rope = nullptr) {
+                             const TcGlu& glu, const TcHeadsOut& heads = TcHeadsOut{}, const float* rope = nullptr, int sums = 1) {
     // "+=" into float32 with nothing riding on it: by TMA reduction, if the rows of out can be a tensor map's
     CUtensorMap mo = mw;
     int reduce_out = 0;
@@ -1136,7 +1181,7 @@ static int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, void*
     static_assert(smem + 16384 + 8 * BN <= 227 * 1024, "the ring does not fit shared memory");
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN, STAGES, SK, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN, STAGES, SK, PAIR, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
@@ -1150,13 +1195,13 @@ static int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, void*
         sk.units_per_group = (int)((units + groups - 1) / groups);
         grid = groups * tiles_t;
     }
-    return launch_kernel(gemm_tc_persistent_kernel<BN, STAGES, SK, PAIR>, dim3(grid), dim3(320), smem, s, PAIR ? -2 : 0, mw, mx, out, mode, T, N, K,
-                         error_flag, norm, scale, sk, heads, rope, mo, reduce_out, glu);
+    return launch_kernel(gemm_tc_persistent_kernel<BN, STAGES, SK, PAIR, PARTS>, dim3(grid), dim3(320), smem, s, PAIR ? -2 : 0, mw, mx, out, mode, T, N, K,
+                         error_flag, norm, scale, sk, heads, rope, mo, reduce_out, glu, sums);
 }
 
 static int persistent_dispatch(const void* x, const void* w, void* out, int mode, int T, int N, int K, int bn, int ctas,
                                int* error_flag, const TcNormOut& norm, const TcRowScale& scale, const TcStreamK& sk, cudaStream_t s,
-                               const TcHeadsOut& heads = TcHeadsOut{}, const float* rope = nullptr, const TcGlu& glu = TC_PLAIN_GLU) {
+                               const TcHeadsOut& heads = TcHeadsOut{}, const float* rope = nullptr, const TcGlu& glu = TC_PLAIN_GLU, int sums = 1) {
     if (T <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 8 != 0 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ctas <= 0) return MB_ERR_BAD_SIZE;
     if (mode < 0 || mode >= TC_OUT_MODES || (tc_gated(mode) && N % 32 != 0) || !glu_fits(glu, mode, N)) return MB_ERR_BAD_DTYPE;
@@ -1164,6 +1209,8 @@ static int persistent_dispatch(const void* x, const void* w, void* out, int mode
     if (scale.sumsq != nullptr && (scale.slots <= 0 || scale.dim <= 0)) return MB_ERR_BAD_SIZE;
     const bool pair = bn < 0;                           // CTAs in pairs, -bn tokens a tile: nothing coupled, no stream-K
     if (pair && (norm.weight != nullptr || scale.sumsq != nullptr || sk.partials != nullptr || ctas < 2)) return MB_ERR_BAD_SIZE;
+    const int nkb = (K + TC_BK - 1) / TC_BK;
+    if ((sums != 1 && sums != 2 && sums != 4) || (sums > 1 && (sk.partials != nullptr || bn != 128 || (sums - 1) * ((nkb + sums - 1) / sums) >= nkb))) return MB_ERR_BAD_SIZE;
     CUtensorMap mw, mx;
     int rc = make_map(&mw, w, N, K, TC_BM);
     if (rc) return rc;
@@ -1177,6 +1224,7 @@ static int persistent_dispatch(const void* x, const void* w, void* out, int mode
             default: return MB_ERR_BAD_SIZE;
         }
     }
+    if (sums > 1) return launch_persistent<128, 6, false, false, true>(mw, mx, out, mode, T, N, K, ctas, error_flag, norm, scale, sk, s, glu, heads, rope, sums);
 #define PAIR_CASE(BN, STAGES) \
     case -BN: return launch_persistent<BN, STAGES, false, true>(mw, mx, out, mode, T, N, K, ctas, error_flag, norm, scale, sk, s, glu, heads, rope)
     switch (bn) {
@@ -1212,9 +1260,10 @@ static int sm_count_of_current_device() {
 }
 
 // The persistent kernel: bn tokens per tile (a multiple of 16 from 128 to 256; negative: -bn, a multiple of 32, by CTAs in pairs), `ctas` CTAs (one per SM).
-MB_API int mb_gemm_tc_persistent(const void* x, const void* w, void* out, int mode, int T, int N, int K, int bn, int ctas,
+// sums: accumulators a tile, 1 or (tiles of 128 tokens) 2 or 4.
+MB_API int mb_gemm_tc_persistent(const void* x, const void* w, void* out, int mode, int T, int N, int K, int bn, int ctas, int sums,
                                  int* error_flag, cudaStream_t s) {
-    return persistent_dispatch(x, w, out, mode, T, N, K, bn, ctas, error_flag, TcNormOut{}, TcRowScale{}, TcStreamK{}, s);
+    return persistent_dispatch(x, w, out, mode, T, N, K, bn, ctas, error_flag, TcNormOut{}, TcRowScale{}, TcStreamK{}, s, TcHeadsOut{}, nullptr, TC_PLAIN_GLU, sums);
 }
 
 // The same with the k-blocks dealt out evenly (stream-K, see TcStreamK): no last round of tiles that fills a part of
@@ -1234,25 +1283,25 @@ MB_API int mb_gemm_tc_persistent_streamk(const void* x, const void* w, void* out
 }
 
 // The same coupled with the RMS norms around it (see mb_gemm_tc_coupled; the slots are mb_gemm_tc_norm_slots(N, 1)).
-MB_API int mb_gemm_tc_persistent_coupled(const void* x, const void* w, void* out, int mode, int T, int N, int K, int bn, int ctas,
+MB_API int mb_gemm_tc_persistent_coupled(const void* x, const void* w, void* out, int mode, int T, int N, int K, int bn, int ctas, int sums,
                                          const float* norm_weight, int norm_unit_offset, void* scaled_out, float* sumsq_out,
                                          const float* scale_sumsq, int scale_slots, int scale_dim, float scale_eps,
                                          int* error_flag, cudaStream_t s) {
     TcNormOut norm{norm_weight, (bf16*)scaled_out, sumsq_out, norm_unit_offset};
     TcRowScale scale{scale_sumsq, scale_slots, scale_dim, scale_eps};
-    return persistent_dispatch(x, w, out, mode, T, N, K, bn, ctas, error_flag, norm, scale, TcStreamK{}, s);
+    return persistent_dispatch(x, w, out, mode, T, N, K, bn, ctas, error_flag, norm, scale, TcStreamK{}, s, TcHeadsOut{}, nullptr, TC_PLAIN_GLU, sums);
 }
 
 // The q|k|v product of many tokens with heads of 128 elements, each head finished in the persistent kernel's epilogue
 // (see TcHeadsOut; mb_gemm_tc_heads is the same for at most 16 tokens).  rope: [T][128] float32, cos of the 64 angles
 // then sin (mb_rope_table), or null for no rotation.
-MB_API int mb_gemm_tc_persistent_heads(const void* x, const void* w, int T, int N, int K, int bn, int ctas, void* q_out, void* k_cache,
+MB_API int mb_gemm_tc_persistent_heads(const void* x, const void* w, int T, int N, int K, int bn, int ctas, int sums, void* q_out, void* k_cache,
                                        void* v_cache, const float* q_weight, const float* k_weight, float eps, const float* rope,
                                        const int* slot_mapping, int H, int KV, int page_size, int* error_flag, cudaStream_t s) {
     if (q_out == nullptr || H <= 0 || KV < 0 || (N != H * TC_BM && N != (H + 2 * KV) * TC_BM)) return MB_ERR_BAD_SIZE;
     if (N != H * TC_BM && (k_cache == nullptr || v_cache == nullptr || slot_mapping == nullptr || page_size <= 0)) return MB_ERR_BAD_SIZE;
     TcHeadsOut heads{(bf16*)q_out, (bf16*)k_cache, (bf16*)v_cache, q_weight, k_weight, nullptr, nullptr, slot_mapping, eps, H, KV, page_size};
-    return persistent_dispatch(x, w, q_out, TC_OUT_BF16, T, N, K, bn, ctas, error_flag, TcNormOut{}, TcRowScale{}, TcStreamK{}, s, heads, rope);
+    return persistent_dispatch(x, w, q_out, TC_OUT_BF16, T, N, K, bn, ctas, error_flag, TcNormOut{}, TcRowScale{}, TcStreamK{}, s, heads, rope, TC_PLAIN_GLU, sums);
 }
 
 // x [T, K] bf16, w [N, K] bf16, out [T, N]: bf16 (mode 0), float32 (1), float32 += (2).  K must be a multiple
@@ -1260,8 +1309,9 @@ MB_API int mb_gemm_tc_persistent_heads(const void* x, const void* w, int T, int 
 // (one zeroed int per tile).  bn in {16, 32, 64, 128, 256}.
 static int gemm_tc_dispatch(const void* x, const void* w, void* out, int mode, int T, int N, int K, int bn, int splits,
                             float* partials, int* counters, int* error_flag, int cluster_reduce, const TcNormOut& norm,
-                            const TcRowScale& scale, const TcHeadsOut& heads, cudaStream_t s, const TcGlu& glu = TC_PLAIN_GLU) {
+                            const TcRowScale& scale, const TcHeadsOut& heads, cudaStream_t s, const TcGlu& glu = TC_PLAIN_GLU, int accumulators = 1) {
     if (T <= 0 || N <= 0) return 0;
+    if (accumulators != 1 && (accumulators != 2 || bn > 128)) return MB_ERR_BAD_SIZE;
     // heads are finished only where the K slices of a tile meet as a cluster
     if (heads.q_out != nullptr && (!cluster_reduce || splits < 2 || N % TC_BM != 0 || bn > 128 || T > bn)) return MB_ERR_BAD_SIZE;
     // the norm's side outputs exist for "+=" without global split-K scratch
@@ -1288,11 +1338,11 @@ static int gemm_tc_dispatch(const void* x, const void* w, void* out, int mode, i
     rc = make_map(&mx, x, T, K, bn);
     if (rc) return rc;
     switch (bn) {
-        case 16: return launch_tc<16, TC_STAGES16>(mw, mx, out, mode, T, N, K, splits, kb_per_split, partials, counters, error_flag, cluster_reduce, norm, scale, heads, glu, s);
-        case 32: return launch_tc<32, 4>(mw, mx, out, mode, T, N, K, splits, kb_per_split, partials, counters, error_flag, cluster_reduce, norm, scale, heads, glu, s);
-        case 64: return launch_tc<64, 4>(mw, mx, out, mode, T, N, K, splits, kb_per_split, partials, counters, error_flag, cluster_reduce, norm, scale, heads, glu, s);
-        case 128: return launch_tc<128, 3>(mw, mx, out, mode, T, N, K, splits, kb_per_split, partials, counters, error_flag, cluster_reduce, norm, scale, heads, glu, s);
-        case 256: return launch_tc<256, 4>(mw, mx, out, mode, T, N, K, splits, kb_per_split, partials, counters, error_flag, cluster_reduce, norm, scale, heads, glu, s);
+        case 16: return launch_tc<16, TC_STAGES16>(mw, mx, out, mode, T, N, K, splits, kb_per_split, partials, counters, error_flag, cluster_reduce, accumulators, norm, scale, heads, glu, s);
+        case 32: return launch_tc<32, 4>(mw, mx, out, mode, T, N, K, splits, kb_per_split, partials, counters, error_flag, cluster_reduce, accumulators, norm, scale, heads, glu, s);
+        case 64: return launch_tc<64, 4>(mw, mx, out, mode, T, N, K, splits, kb_per_split, partials, counters, error_flag, cluster_reduce, accumulators, norm, scale, heads, glu, s);
+        case 128: return launch_tc<128, 3>(mw, mx, out, mode, T, N, K, splits, kb_per_split, partials, counters, error_flag, cluster_reduce, accumulators, norm, scale, heads, glu, s);
+        case 256: return launch_tc<256, 4>(mw, mx, out, mode, T, N, K, splits, kb_per_split, partials, counters, error_flag, cluster_reduce, accumulators, norm, scale, heads, glu, s);
         default: return MB_ERR_BAD_SIZE;
     }
 }
@@ -1306,10 +1356,10 @@ MB_API int mb_gemm_tc(const void* x, const void* w, void* out, int mode, int T, 
 }
 
 // The same product with the K slices of a tile as one thread-block cluster (splits in {1, 2, 4, 8}): the slices
-// are added through distributed shared memory, no global scratch is touched.
-MB_API int mb_gemm_tc_cluster(const void* x, const void* w, void* out, int mode, int T, int N, int K, int bn, int splits,
+// are added through distributed shared memory, no global scratch is touched.  accumulators: 1, or with 128 tokens a tile 2 for each slice (up to 64 there are two).
+MB_API int mb_gemm_tc_cluster(const void* x, const void* w, void* out, int mode, int T, int N, int K, int bn, int splits, int accumulators,
                               int* error_flag, cudaStream_t s) {
-    return gemm_tc_dispatch(x, w, out, mode, T, N, K, bn, splits, nullptr, nullptr, error_flag, 1, TcNormOut{}, TcRowScale{}, TcHeadsOut{}, s);
+    return gemm_tc_dispatch(x, w, out, mode, T, N, K, bn, splits, nullptr, nullptr, error_flag, 1, TcNormOut{}, TcRowScale{}, TcHeadsOut{}, s, TC_PLAIN_GLU, accumulators);
 }
 
 // A gated product with its further choices (TcGlu; mode one of the gated ones): ctas 0: one CTA per tile of bn tokens; else the persistent
@@ -1336,13 +1386,13 @@ MB_API int mb_gemm_tc_norm_slots(int N, int splits) { return ((N + TC_BM - 1) / 
 //   norm_weight [N] float32, scaled_out [T, N] bf16, sumsq_out [mb_gemm_tc_norm_slots(N, splits)][T] float32: with
 //   mode 2, the updated rows times the norm weight (1 + weight with unit_offset) and their sums of squares.
 //   scale_sumsq [scale_slots][T]: token t of the product is multiplied by 1 / sqrt(sum of its slots / scale_dim + eps).
-MB_API int mb_gemm_tc_coupled(const void* x, const void* w, void* out, int mode, int T, int N, int K, int bn, int splits,
+MB_API int mb_gemm_tc_coupled(const void* x, const void* w, void* out, int mode, int T, int N, int K, int bn, int splits, int accumulators,
                               const float* norm_weight, int norm_unit_offset, void* scaled_out, float* sumsq_out,
                               const float* scale_sumsq, int scale_slots, int scale_dim, float scale_eps, int* error_flag,
                               cudaStream_t s) {
     TcNormOut norm{norm_weight, (bf16*)scaled_out, sumsq_out, norm_unit_offset};
     TcRowScale scale{scale_sumsq, scale_slots, scale_dim, scale_eps};
-    return gemm_tc_dispatch(x, w, out, mode, T, N, K, bn, splits, nullptr, nullptr, error_flag, 1, norm, scale, TcHeadsOut{}, s);
+    return gemm_tc_dispatch(x, w, out, mode, T, N, K, bn, splits, nullptr, nullptr, error_flag, 1, norm, scale, TcHeadsOut{}, s, TC_PLAIN_GLU, accumulators);
 }
 
 // The q|k|v product of at most bn tokens (16, 32, 64 or 128) with heads of 128 elements, each head finished in the

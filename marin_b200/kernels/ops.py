@@ -318,16 +318,32 @@ def check_device_errors(device=None) -> None:
 def gemm_plan(T: int, N: int, K: int):
     """Tokens per CTA and the number of K slices (1, 2, 4 or 8: the CTAs of one cluster) for the tensor-core
     kernel.  K is cut when there are fewer tiles than SMs, as far as every slice keeps at least 4 k-blocks: up to 128 tokens into as many as
-    there is room for, beyond by ``_cluster_microseconds``."""
+    there is room for (``sums_plan``), beyond into as many or half of them, by ``_cluster_microseconds``."""
     bn = 16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 else 128
-    tiles = -(-N // 128) * -(-T // bn)
+    sums = sums_plan(T, N, K)
+    if T > 128 and sums > 1:
+        tiles, nkb = -(-N // 128) * -(-T // bn), -(-K // 64)
+        return bn, min((sums, sums // 2), key=lambda s: _cluster_microseconds(tiles, nkb, s))
+    return bn, sums
+
+
+@functools.lru_cache(maxsize=4096)
+def sums_plan(T: int, N: int, K: int, most: int = 8) -> int:
+    """Into how many parts K is cut, each summed by itself (the sums are then added): 8, 4 or 2 where there are fewer tiles than SMs and two CTAs an SM find room for as
+    many slices of at least 4 k-blocks, else 1.  An accumulator in tensor memory cuts its additions off, so the error of float32 results grows with the k-blocks a
+    part has.  Whoever makes fewer slices or whole tiles (to be faster: ``gemm_plan``, ``half_round``) therefore gives each part an accumulator of its own."""
+    tiles = -(-N // 128) * -(-T // (16 if T <= 16 else 32 if T <= 32 else 64 if T <= 64 else 128))
     nkb = -(-K // 64)
     if tiles >= SM_COUNT:
-        return bn, 1
-    fits = [s for s in (8, 4, 2) if tiles * s <= 2 * SM_COUNT + 32 and -(-nkb // s) >= 4 and (s - 1) * -(-nkb // s) < nkb]
-    if T > 128:
-        return bn, min(fits + [1], key=lambda s: _cluster_microseconds(tiles, nkb, s))
-    return bn, fits[0] if fits else 1
+        return 1
+    return next((s for s in (8, 4, 2) if s <= most and tiles * s <= 2 * SM_COUNT + 32 and -(-nkb // s) >= 4 and (s - 1) * -(-nkb // s) < nkb), 1)
+
+
+def _whole_tiles(bn: int, T: int, N: int, K: int):
+    """A tile's width in the persistent kernel and its accumulators (``sums_plan``), given the width it would have with one.  Several are a round of tiles of 128, and
+    by single SMs (512 tokens by 2,560 rows of 9,728, four: 40.3 us, by pairs 42.2)."""
+    sums = sums_plan(T, N, K, 4)
+    return (128 if sums > 1 else bn), sums
 
 
 def _cluster_microseconds(tiles: int, nkb: int, splits: int) -> float:
@@ -343,8 +359,8 @@ def _cluster_microseconds(tiles: int, nkb: int, splits: int) -> float:
 def half_round(T: int, N: int, K: int) -> bool:
     """Whether a product with fewer tiles than SMs goes to the persistent kernel all the same: one round of whole tiles there is 4.9 us and 0.236 a k-block,
     without the slices' sums (B200: 6,144 rows of 1,024, 256 tokens 9.0 us for 12.2 in two slices; of 4,096 20.4 for 22.1; but 4,096 rows of 4,096 20.4
-    for 16.6 in four)."""
-    if T <= 128 or N <= 0:
+    for 16.6 in four).  Not where K has more parts than a tile has accumulators."""
+    if T <= 128 or N <= 0 or sums_plan(T, N, K) > 4:
         return False
     bn, splits = gemm_plan(T, N, K)
     nkb = -(-K // 64)
@@ -445,7 +461,8 @@ def _stream_k_width(T: int, N: int, K: int, kblock: int, fixed: float, margin: f
 
 def _persistent_product(x, w, out, mode: int, T: int, N: int, K: int, s, what: str) -> None:
     lib = _lib("mb_gemm_tc")
-    bn = stream_k_plan(T, N, K)
+    tile, sums = (paired_plan(T, N, K), 1) if mode in _GLU_MODES.values() else _whole_tiles(paired_plan(T, N, K), T, N, K)
+    bn = stream_k_plan(T, N, K) if sums == 1 else None
     if bn is not None:
         _check(lib.mb_gemm_tc_persistent_streamk(
             _ptr(x), _ptr(w), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K), _c_int(bn), _c_int(SM_COUNT),
@@ -453,7 +470,7 @@ def _persistent_product(x, w, out, mode: int, T: int, N: int, K: int, s, what: s
             what + ", stream-K")
         return
     _check(lib.mb_gemm_tc_persistent(_ptr(x), _ptr(w), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K),
-                                     _c_int(paired_plan(T, N, K)), _c_int(SM_COUNT), _ptr(s.error), _stream()), what)
+                                     _c_int(tile), _c_int(SM_COUNT), _c_int(sums), _ptr(s.error), _stream()), what)
 
 
 @functools.lru_cache(maxsize=4096)
@@ -553,8 +570,9 @@ def gemm(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, then_n
             if carried is None and scaled is None:
                 _persistent_product(x, w, out, mode, T, N, K, s, "gemm (tensor cores, persistent)")
                 return None
+            tile, sums = _whole_tiles(persistent_plan(T, N), T, N, K)
             _check(lib.mb_gemm_tc_persistent_coupled(
-                _ptr(x), _ptr(w), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K), _c_int(persistent_plan(T, N)), _c_int(SM_COUNT),
+                _ptr(x), _ptr(w), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K), _c_int(tile), _c_int(SM_COUNT), _c_int(sums),
                 _ptr(then_norm.weight) if carried is not None else None, _c_int(int(then_norm.unit_offset)) if carried is not None else _c_int(0),
                 _ptr(carried.rows) if carried is not None else None, _ptr(carried.sumsq) if carried is not None else None,
                 _ptr(scaled.sumsq) if scaled is not None else None, _c_int(scaled.slots if scaled is not None else 0),
@@ -562,6 +580,7 @@ def gemm(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, then_n
                 _ptr(s.error), _stream()), "gemm (tensor cores, persistent, coupled with a norm)")
             return carried
         bn, splits = gemm_plan(T, N, K)
+        accumulators = sums_plan(T, N, K) // splits
         s = _scratch_for(x.device)
         lib = _lib("mb_gemm_tc")
         carried = None
@@ -572,10 +591,10 @@ def gemm(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, then_n
                 carried = NormedRows(then_norm.rows, s.sumsq, slots, N, then_norm.eps)
         if carried is None and scaled is None:
             _check(lib.mb_gemm_tc_cluster(_ptr(x), _ptr(w), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K),
-                                          _c_int(bn), _c_int(splits), _ptr(s.error), _stream()), "gemm (tensor cores)")
+                                          _c_int(bn), _c_int(splits), _c_int(accumulators), _ptr(s.error), _stream()), "gemm (tensor cores)")
             return None
         _check(lib.mb_gemm_tc_coupled(
-            _ptr(x), _ptr(w), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K), _c_int(bn), _c_int(splits),
+            _ptr(x), _ptr(w), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K), _c_int(bn), _c_int(splits), _c_int(accumulators),
             _ptr(then_norm.weight) if carried is not None else None, _c_int(int(then_norm.unit_offset)) if carried is not None else _c_int(0),
             _ptr(carried.rows) if carried is not None else None, _ptr(carried.sumsq) if carried is not None else None,
             _ptr(scaled.sumsq) if scaled is not None else None, _c_int(scaled.slots if scaled is not None else 0),
@@ -678,8 +697,9 @@ def gemm_qkv_heads(x, w: torch.Tensor, q_out: torch.Tensor, q_weight, k_weight, 
         table = rope_table(ctx, positions, inv_freq) if inv_freq is not None else None
         _cost(_size(w) + _size(rows) + T * N * 2 + (_size(table) if table is not None else 0), 2.0 * T * N * Kdim)
         s = _scratch_for(rows.device)
+        tile, sums = _whole_tiles(paired_plan(T, N, Kdim), T, N, Kdim)
         _check(_lib("mb_gemm_tc").mb_gemm_tc_persistent_heads(
-            _ptr(rows), _ptr(w), _c_int(T), _c_int(N), _c_int(Kdim), _c_int(paired_plan(T, N, Kdim)), _c_int(SM_COUNT), _ptr(q_out),
+            _ptr(rows), _ptr(w), _c_int(T), _c_int(N), _c_int(Kdim), _c_int(tile), _c_int(SM_COUNT), _c_int(sums), _ptr(q_out),
             _ptr(k_cache) if write_kv else None, _ptr(v_cache) if write_kv else None, _ptr(q_weight), _ptr(k_weight), _c_float(eps),
             _ptr(table), _ptr(slot_mapping) if write_kv else None, _c_int(H), _c_int(K), _c_int(page_size), _ptr(s.error), _stream()),
             "gemm (persistent) with heads finished in the epilogue")
@@ -987,7 +1007,7 @@ def gemm_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, out: torch.Tensor,
         if scaled is not None:
             _check(_lib("mb_gemm_tc").mb_gemm_tc_persistent_coupled(
                 _ptr(x), _ptr(w_interleaved), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K), _c_int(persistent_plan(T, N)),
-                _c_int(SM_COUNT), None, _c_int(0), None, None, _ptr(scaled.sumsq), _c_int(scaled.slots), _c_int(scaled.dim),
+                _c_int(SM_COUNT), _c_int(1), None, _c_int(0), None, None, _ptr(scaled.sumsq), _c_int(scaled.slots), _c_int(scaled.dim),
                 _c_float(scaled.eps), _ptr(s.error), _stream()), "gemm+swiglu (tensor cores, persistent, coupled with a norm)")
             return
         _persistent_product(x, w_interleaved, out, mode, T, N, K, s, "gemm+swiglu (tensor cores, persistent)")
@@ -995,12 +1015,12 @@ def gemm_swiglu(x: torch.Tensor, w_interleaved: torch.Tensor, out: torch.Tensor,
     bn, _ = gemm_plan(T, N, K)
     if scaled is not None:
         _check(_lib("mb_gemm_tc").mb_gemm_tc_coupled(
-            _ptr(x), _ptr(w_interleaved), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K), _c_int(bn), _c_int(1),
+            _ptr(x), _ptr(w_interleaved), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K), _c_int(bn), _c_int(1), _c_int(1),
             None, _c_int(0), None, None, _ptr(scaled.sumsq), _c_int(scaled.slots), _c_int(scaled.dim), _c_float(scaled.eps),
             _ptr(s.error), _stream()), "gemm+swiglu (tensor cores, coupled with a norm)")
         return
     _check(_lib("mb_gemm_tc").mb_gemm_tc_cluster(_ptr(x), _ptr(w_interleaved), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K),
-                                                _c_int(bn), _c_int(1), _ptr(s.error), _stream()), "gemm+swiglu (tensor cores)")
+                                                _c_int(bn), _c_int(1), _c_int(1), _ptr(s.error), _stream()), "gemm+swiglu (tensor cores)")
 
 
 def gemm_act(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, activation: str = "relu2") -> None:

@@ -41,7 +41,7 @@ def main(argv=None) -> int:
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
 
     def run():
-        rc = lib.mb_gemm_tc_persistent(ops._ptr(x), ops._ptr(w), ops._ptr(out), 0, T, N, K, bn, ctas, ops._ptr(scratch.error), ops._stream())
+        rc = lib.mb_gemm_tc_persistent(ops._ptr(x), ops._ptr(w), ops._ptr(out), 0, T, N, K, bn, ctas, 1, ops._ptr(scratch.error), ops._stream())
         if rc:
             raise SystemExit(f"the launch was refused ({rc})")
 

@@ -972,6 +972,45 @@ def test_products_of_less_than_a_round_of_tiles(ops, T, N, K):
     ops.check_device_errors()
 
 
+@pytest.mark.parametrize("T,N,K,parts", [(512, 2560, 9728, 4), (256, 2560, 9728, 8), (256, 6144, 4096, 2), (700, 2560, 2560, 2), (130, 160, 4160, 8), (1200, 1024, 2048, 4)])
+def test_fewer_slices_or_whole_tiles_keep_as_many_sums(ops, T, N, K, parts):
+    """Of positive numbers an accumulator loses at most half of its K / 16 additions times 2^-23 (see above), K being cut into the parts there is room for; and the
+    parts' sums are rounded (once 2^-23)."""
+    g = torch.Generator(device=DEV).manual_seed(T + K)
+    x, w = torch.rand(T, K, device=DEV, generator=g).to(torch.bfloat16), torch.rand(N, K, device=DEV, generator=g).to(torch.bfloat16)
+    want = x.double() @ w.double().t()
+    for out, added in ((torch.empty(T, N, device=DEV), False), (torch.zeros(T, N, device=DEV), True)):
+        ops.gemm(x, w, out, accumulate=added)
+        assert float(((out.double() - want).abs() / want).mean()) <= (-(-(-(-K // 64)) // parts) * 4 / 2 + 1) * 2.0 ** -23
+    ops.check_device_errors()
+
+
+@pytest.mark.parametrize("T,N,K", [(512, 2560, 1032), (257, 672, 1040), (384, 3240, 520), (1200, 1000, 576), (300, 4500, 584)])
+def test_whole_tiles_with_several_accumulators_have_the_slices_bits(ops, monkeypatch, T, N, K):
+    """Two and four accumulators a tile, one set of them and two, ragged tiles and a last part that is shorter: what as many slices of a cluster give, bit for
+    bit, in every epilogue (bfloat16, float32, added to float32, squared relu)."""
+    g = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randn(T, K, device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(N, K, device=DEV, generator=g) / math.sqrt(K)).to(torch.bfloat16)
+    base = torch.randn(T, N, device=DEV, generator=g)
+    sums = ops.sums_plan(T, N, K, 4)
+    assert sums in (2, 4)
+    results = []
+    for whole in (True, False):
+        monkeypatch.setattr(ops, "half_round", lambda *a: whole)
+        monkeypatch.setattr(ops, "gemm_plan", lambda *a: (128, sums))
+        monkeypatch.setattr(ops, "sums_plan", lambda *a: sums)
+        outs = [torch.full((T, N), math.nan, device=DEV, dtype=d) for d in (torch.bfloat16, torch.float32, torch.bfloat16)] + [base.clone()]
+        ops.gemm(x, w, outs[0])
+        ops.gemm(x, w, outs[1])
+        ops.gemm(x, w, outs[2], activation="relu2")
+        ops.gemm(x, w, outs[3], accumulate=True)
+        ops.check_device_errors()
+        results.append(outs)
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("H,K,d", [(16, 8, 128), (3, 1, 64), (33, 2, 256)])
 def test_float32_heads_do_not_depend_on_how_many_share_a_block(ops, H, K, d):
     """From 256 tokens on a warp takes several heads: the bits of one token alone, and the plain formula's numbers (a sum of d squares and two products: 2^-24 d)."""
