@@ -11,8 +11,10 @@
 // 0.97e-7 (4.1; with few weight rows 1.05, 2.1), 3,072 1.1e-7 (3.6), 9,728 1.3e-7 (6.3).  With 128 k an accumulator the second stage's small
 // products meet a large sum: 5.9e-7.
 //
-// Numbers that three bf16 numbers cannot hold (not finite, above bf16's range, or so small that the last part falls below its range) are noticed on the way:
-// the outputs of a row of x that has one, and of a tile of weight rows that has one, are worked out again by plain multiply-adds over k.
+// Numbers that three bf16 numbers cannot hold (not finite, above bf16's range, or below 2^-110 with bits below its range) are noticed on the way:
+// the outputs of a row of x or of w that has one are worked out by float32 multiply-adds instead (gf_dot).
+// 333 tokens by 4,096 rows of 1,024, 33 us: 58 with one such number in x, or in w; 697 with one in every row of x.  16 by 2,560 of 9,728, 54 us: 80, 95 and 265.  (By
+// a chain of K in one thread an output, and 128 weight rows for one of them: 110, 6,730, 6,750; 2,450, 10,700, 21,400.)
 //
 // A CTA has 128 weight rows (the MMA's M) and `width` tokens (N).  Its warps fetch the next 64 k of both operands (16-byte loads, in registers
 // while the MMAs of the k ahead run), split them into the six planes of a stage in shared memory (128-byte swizzle), then add the accumulator of the
@@ -38,7 +40,7 @@ template <int BN, int STAGES>
 struct GfTile {
     static constexpr int A_PLANE = GF_BM * GF_BK * 2, B_PLANE = BN * GF_BK * 2, STAGE = 3 * (A_PLANE + B_PLANE);
     static constexpr int SUMS = GF_BM * BN;                         // numbers of one group's tile on its way to the cluster
-    static constexpr int SMEM = STAGES * STAGE + 1024 + 512;
+    static constexpr int SMEM = STAGES * STAGE + 1024;
     // Warps that fetch and split, two rows of 64 numbers a round (16 lanes of 16 bytes a row).  With two stages the last warp hands the MMAs over instead: it
     // stands where it does so while they run.  With one stage everyone waits for them.
     static constexpr int PUTTERS = STAGES > 1 ? 15 : 16;
@@ -93,10 +95,38 @@ template <int PLANE> __device__ __forceinline__ void gf_put(uint32_t at, const f
     gf_st(at + 2 * PLANE, l0, l1);
 }
 
-__device__ __noinline__ float gf_chain(const float* x, const float* w, int K) {
+// A row of x times a row of w by float32 multiply-adds, by a warp: a lane four k of every 128, the lanes' sums in a tree.  (One output at a
+// time: what a call may touch is taken from the kernel around it.  4 x 4 of them a call made the kernel 2 to 10% slower, for 340 us of the 697 above.)
+__device__ __noinline__ float gf_dot(const float* x, const float* w, int K) {
     float sum = 0.0f;
-    for (int k = 0; k < K; ++k) sum = fmaf(x[k], w[k], sum);
+#pragma unroll 4
+    for (int k = 4 * (threadIdx.x & 31); k < K; k += 128) {
+        const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
+        sum = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, sum))));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     return sum;
+}
+
+// Whether all numbers of a row split: asked by a warp.
+__device__ __noinline__ bool gf_splits(const float* row, int K) {
+    uint32_t left = 0;
+    for (int k = 4 * (threadIdx.x & 31); k < K; k += 128) {
+        const float4 v = *reinterpret_cast<const float4*>(row + k);
+        uint32_t hi, mid, lo;
+        gf_split(v.x, v.y, hi, mid, lo, left);
+        gf_split(v.z, v.w, hi, mid, lo, left);
+    }
+    return __all_sync(0xffffffffu, (left & 0xffffu) == 0);
+}
+
+// The thread's number, asked for once more: what is worked out from it behind the loop then takes no registers in the loop, which has none to spare (with the flags'
+// places from the first one 333 tokens by 4,096 rows of 1,024 took 30.6 us for 29.3).
+__device__ __forceinline__ int gf_thread() {
+    int t;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    return t;
 }
 
 __device__ __forceinline__ uint32_t gf_peer(const void* p, int rank) {
@@ -115,8 +145,9 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t full[STAGES], done[STAGES];               // a stage is filled (and its accumulator read); its MMAs are done
     __shared__ uint32_t tmem_slot;
-    __shared__ int bad_any, bad_w;                                // something is bad; a weight is (its whole tile then counts: which one follows the weights alone)
-    __shared__ uint8_t bad_x[BN];
+    __shared__ int bad_any;                                       // something is flagged
+    __shared__ uint8_t bad_x[BN], bad_w[GF_BM];                   // tokens and weight rows with a number that does not split, in this CTA's k
+    __shared__ uint8_t all_x[BN], all_w[GF_BM];                   // in all of it
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n0 = blockIdx.x * GF_BM, t0 = blockIdx.y * width, splits = gridDim.z, rank = blockIdx.z;
@@ -125,9 +156,10 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], S::PUTTERS); mbar_init(&done[s], 1); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        bad_any = bad_w = 0;
+        bad_any = 0;
     }
     if (tid < BN) bad_x[tid] = 0;
+    if (tid < GF_BM) bad_w[tid] = 0;
     if (warp == 0) tmem_alloc<false>(&tmem_slot, S::COLS);
     // A warp's rounds: two rows each, of the weights (pairs of rows 0 to 63: rounds 0 to 3 and some of 4) or of x.  No round but the last few is behind a
     // branch, so that several are worked on side by side: a pair past the last one is the last one once more (the same numbers to the same place), and a row that is
@@ -290,11 +322,13 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
         }
         for (int c = max(0, count - STAGES); c < count; ++c) add(c);
     }
+    const int tid2 = gf_thread(), warp2 = tid2 >> 5, lane2 = tid2 & 31, in2 = (warp2 & 3) * 32 + lane2;
+    auto pair2 = [&](int i) { return STAGES > 1 ? min(warp2 + S::PUTTERS * i, last_pair) : warp2 + S::PUTTERS * i; };
+    auto of_w2 = [&](int i) { return i < 4 || (STAGES > 1 && i == 4 && pair2(4) < GF_BM / 2); };
 #pragma unroll
     for (int i = 0; i < S::ROUNDS; ++i) {
         if (((i < 4 ? left_w : left[i < 4 ? 0 : i - 4]) & 0xffffu) == 0) continue;
-        if (of_w(i)) bad_w = 1;
-        else bad_x[(pair_of(i) & (GF_BM / 2 - 1)) * 2 + (lane >> 4)] = 1;
+        (of_w2(i) ? bad_w : bad_x)[(pair2(i) & (GF_BM / 2 - 1)) * 2 + (lane2 >> 4)] = 1;      // (of the weights: one of four rows)
         bad_any = 1;
     }
 #pragma unroll
@@ -308,7 +342,7 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
         } else {
 #pragma unroll
             for (int e = 0; e < STEP; ++e) {
-                float* to = sums + (c0 + i + e) * GF_BM + in;
+                float* to = sums + (c0 + i + e) * GF_BM + in2;
                 if (mine > 1) { to[0] = folded ? v[e] : cur[i + e]; to[S::SUMS] = folded ? cur[i + e] : 0.0f; }
                 else to[0] = cur[i + e];
             }
@@ -316,70 +350,99 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();                                              // tensor memory has been read, and everyone has said what was bad
-    if (warp == 0) tmem_free<false>(tmem, S::COLS);
-    if (splits == 1) {
-        const bool any = bad_any != 0;
-        if (n0 + in >= N) return;
-        float* to = out + (size_t)(t0 + c0) * N + n0 + in;
-        const int rows = min(width, T - t0) - c0;
-#pragma unroll
-        for (int i = 0; i < S::CW; i += 8) {
-            float old[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) old[e] = ACC && i + e < rows ? to[(size_t)(i + e) * N] : 0.0f;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                if (i + e >= rows) continue;
-                float v = cur[i + e];
-                if (any && (bad_w | bad_x[c0 + i + e])) v = gf_chain(x + (size_t)(t0 + c0 + i + e) * K, w + (size_t)(n0 + in) * K, K);
-                to[(size_t)(i + e) * N] = ACC ? old[e] + v : v;
-            }
-        }
+    if (warp2 == 0) tmem_free<false>(tmem, S::COLS);
+            auto store = [&](auto flagged) {
+                float* to = out + (size_t)(t0 + c0) * N + n0 + in2;
+                const int rows = min(width, T - t0) - c0;
+    #pragma unroll
+                for (int i = 0; i < S::CW; i += 8) {
+                    float old[8];
+    #pragma unroll
+                    for (int e = 0; e < 8; ++e) old[e] = ACC && i + e < rows ? to[(size_t)(i + e) * N] : 0.0f;
+    #pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        if (i + e >= rows || (decltype(flagged)::value && (all_w[in2] | all_x[c0 + i + e]))) continue;
+                        to[(size_t)(i + e) * N] = ACC ? old[e] + cur[i + e] : cur[i + e];
+                    }
+                }
+            };
+    bool any = bad_any != 0;
+    if (splits == 1 && !any) {
+        if (n0 + in2 < N) store(GfFalse());
         return;
     }
-    cluster_sync();
-    bool any = false, any_w = false;
-    for (int z = 0; z < splits; ++z) {
-        int v, u;
-        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(gf_peer(&bad_any, z)) : "memory");
-        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(u) : "r"(gf_peer(&bad_w, z)) : "memory");
-        any |= v != 0;
-        any_w |= u != 0;
+    if (any) {
+        for (int r = warp2; r < GF_BM; r += GF_THREADS / 32)
+            if (bad_w[r] != 0 && gf_splits(w + (size_t)min(n0 + r, N - 1) * K, K)) bad_w[r] = 0;
+        __syncthreads();
     }
-    for (int idx = rank * GF_THREADS + tid; idx < width * (GF_BM / 4); idx += splits * GF_THREADS) {
-        const int t = idx / (GF_BM / 4), n = idx % (GF_BM / 4) * 4;
-        if (t0 + t >= T || n0 + n >= N) continue;
-        float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (splits > 1) {
+        cluster_sync();
         for (int z = 0; z < splits; ++z) {
-            const uint32_t peer = gf_peer(sums + t * GF_BM + n, z);
-            for (int g = 0; g < mine; ++g) {
-                float4 p;
-                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w) : "r"(peer + (uint32_t)(g * S::SUMS * 4)) : "memory");
-                v[0] += p.x; v[1] += p.y; v[2] += p.z; v[3] += p.w;
-            }
-        }
-        if (any) {
-            bool bad = any_w;
-            for (int z = 0; z < splits; ++z) {
-                uint32_t u;
-                asm volatile("ld.shared::cluster.u8 %0, [%1];" : "=r"(u) : "r"(gf_peer(bad_x + t, z)) : "memory");
-                bad |= u != 0;
-            }
-            for (int e = 0; e < 4 && bad && n0 + n + e < N; ++e) v[e] = gf_chain(x + (size_t)(t0 + t) * K, w + (size_t)(n0 + n + e) * K, K);
-        }
-        float* to = out + (size_t)(t0 + t) * N + n0 + n;
-        if (n0 + n + 4 <= N && (N & 3) == 0 && ((uintptr_t)out & 15) == 0) {
-            float4 r = make_float4(v[0], v[1], v[2], v[3]);
-            if (ACC) {
-                const float4 old = *reinterpret_cast<const float4*>(to);
-                r = make_float4(old.x + v[0], old.y + v[1], old.z + v[2], old.w + v[3]);
-            }
-            *reinterpret_cast<float4*>(to) = r;
-        } else {
-            for (int e = 0; e < 4 && n0 + n + e < N; ++e) to[e] = ACC ? to[e] + v[e] : v[e];
+            int v;
+            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(gf_peer(&bad_any, z)) : "memory");
+            any |= v != 0;
         }
     }
-    cluster_sync();                                               // nobody leaves while its sums are read
+    if (any) {
+        if (tid2 < BN + GF_BM) {
+            const uint8_t* own = tid2 < BN ? bad_x + tid2 : bad_w + (tid2 - BN);
+            uint32_t all = splits == 1 ? *own : 0;
+            for (int z = 0; splits > 1 && z < splits; ++z) {
+                uint32_t u;
+                asm volatile("ld.shared::cluster.u8 %0, [%1];" : "=r"(u) : "r"(gf_peer(own, z)) : "memory");
+                all |= u;
+            }
+            (tid2 < BN ? all_x + tid2 : all_w + (tid2 - BN))[0] = (uint8_t)all;
+        }
+        __syncthreads();
+    }
+    if (splits == 1) {
+        if (n0 + in2 < N) {
+            store(GfTrue());
+        }
+    } else {
+        for (int idx = rank * GF_THREADS + tid2; idx < width * (GF_BM / 4); idx += splits * GF_THREADS) {
+            const int t = idx / (GF_BM / 4), n = idx % (GF_BM / 4) * 4;
+            if (t0 + t >= T || n0 + n >= N) continue;
+            float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (int z = 0; z < splits; ++z) {
+                const uint32_t peer = gf_peer(sums + t * GF_BM + n, z);
+                for (int g = 0; g < mine; ++g) {
+                    float4 p;
+                    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w) : "r"(peer + (uint32_t)(g * S::SUMS * 4)) : "memory");
+                    v[0] += p.x; v[1] += p.y; v[2] += p.z; v[3] += p.w;
+                }
+            }
+            float* to = out + (size_t)(t0 + t) * N + n0 + n;
+            if (!any && n0 + n + 4 <= N && (N & 3) == 0 && ((uintptr_t)out & 15) == 0) {
+                float4 r = make_float4(v[0], v[1], v[2], v[3]);
+                if (ACC) {
+                    const float4 old = *reinterpret_cast<const float4*>(to);
+                    r = make_float4(old.x + v[0], old.y + v[1], old.z + v[2], old.w + v[3]);
+                }
+                *reinterpret_cast<float4*>(to) = r;
+            } else {
+                for (int e = 0; e < 4 && n0 + n + e < N; ++e)
+                    if (!any || (all_x[t] | all_w[n + e]) == 0) to[e] = ACC ? to[e] + v[e] : v[e];
+            }
+        }
+        cluster_sync();                                           // nobody leaves while its sums are read
+    }
+    if (!any) return;
+    // the flagged ones, an output a warp (of all the tile's CTAs): tokens with all weight rows, then weight rows with the other tokens
+    const int tokens = min(width, T - t0), weights = min(GF_BM, N - n0), me = rank * (GF_THREADS / 32) + warp2, warps = splits * (GF_THREADS / 32);
+    for (int a = 0; a < tokens + weights; ++a) {
+        const bool token = a < tokens;
+        if ((token ? all_x[a] : all_w[a - tokens]) == 0) continue;
+        for (int b = me; b < (token ? weights : tokens); b += warps) {
+            const int t = token ? a : b, n = token ? b : a - tokens;
+            if (!token && all_x[t] != 0) continue;
+            const float v = gf_dot(x + (size_t)(t0 + t) * K, w + (size_t)(n0 + n) * K, K);
+            float* to = out + (size_t)(t0 + t) * N + n0 + n;
+            if (lane2 == 0) *to = ACC ? *to + v : v;
+        }
+    }
 }
 
 // Parts of K whose sums are chains of their own, by N alone (a row's result must not follow the batch): with few weight rows more CTAs share a tile.

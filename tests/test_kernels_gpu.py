@@ -1103,6 +1103,58 @@ def test_float32_product_of_numbers_that_do_not_split(ops, monkeypatch):
         assert torch.equal(torch.nan_to_num(out, 5.0), torch.nan_to_num(first, 5.0))
 
 
+@pytest.mark.parametrize("T,N,K", [(1, 300, 260), (37, 130, 68), (200, 3100, 576), (130, 257, 2052)])
+def test_float32_number_that_does_not_split_concerns_its_rows_alone(ops, monkeypatch, T, N, K):
+    """One such number in x and two in w: the other rows of both have the bits they have without, whatever the tiles; theirs are float32 sums in some order (K
+    roundings of 2^-24), added to what is there."""
+    g = torch.Generator().manual_seed(T + N)
+    x, w = torch.randn(T, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    clean = torch.empty(T, N, device=DEV)
+    ops.gemm(x, w, clean)
+    t, n1, n2 = T // 2, N // 3, N - 1
+    x[t, K // 2 + 1], w[n1, 0], w[n2, K - 1] = 1.23456e-38, -7.65432e-37, 1.1e-40
+    want, scale = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    rows = torch.ones(T, N, dtype=torch.bool, device=DEV)
+    rows[t], rows[:, n1], rows[:, n2] = False, False, False
+    first, groups = None, 8 if N <= ops.F32_FEW_ROWS else 4
+    for plan in [(16, 1), (32, groups), (48, groups // 2), (112, 1), (128, groups)]:
+        monkeypatch.setattr(ops, "f32_plan", lambda *a: plan)
+        out = torch.full((T, N), math.nan, device=DEV)
+        ops.gemm(x, w, out)
+        assert torch.equal(torch.where(rows, out, clean), torch.where(rows, clean, clean)), plan
+        assert bool(((out - want).abs() <= 2.0 ** -24 * K * scale).all())
+        first = out if first is None else first
+        assert torch.equal(out, first)
+        added = out.clone()
+        ops.gemm(x, w, added, accumulate=True)
+        assert torch.equal(added, out + out)
+        alone = torch.empty(1, N, device=DEV)
+        ops.gemm(x[t:t + 1], w, alone)
+        assert torch.equal(alone, out[t:t + 1])
+    ops.check_device_errors()
+
+
+def test_float32_number_that_does_not_split_costs_less_than_the_product(ops):
+    """It once cost 180 products: every output of 128 weight rows by a chain in one thread."""
+    T, N, K = 333, 4096, 1024
+    x, w, out = torch.randn(T, K, device=DEV), torch.randn(N, K, device=DEV), torch.empty(T, N, device=DEV)
+
+    def microseconds():
+        for _ in range(3):
+            ops.gemm(x, w, out)
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(20):
+            ops.gemm(x, w, out)
+        b.record()
+        b.synchronize()
+        return a.elapsed_time(b) * 50.0
+
+    clean = microseconds()
+    w[77, 5], x[100, 7] = 1.23456e-38, 1.23456e-38
+    assert microseconds() <= 3.0 * clean                       # (1.7 was seen)
+
+
 @pytest.mark.parametrize("activation,form", [("swiglu", None), ("relu2", None), ("glu_capped", (2.0, 1.5, 1.0))])
 @pytest.mark.parametrize("counts,h,ff,shared_ff", [((1,), 64, 64, 0), ((0, 16, 17, 0, 33, 1), 128, 192, 64), ((300, 0, 257, 256, 40), 192, 320, 128),
                                                    ((64, 65, 31, 60), 320, 64, 192), ((2,) * 100, 64, 128, 0), ((540, 3), 128, 128, 64)])
