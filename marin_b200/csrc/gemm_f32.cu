@@ -12,9 +12,10 @@
 // products meet a large sum: 5.9e-7.
 //
 // Numbers that three bf16 numbers cannot hold (not finite, above bf16's range, or below 2^-110 with bits below its range) are noticed on the way:
-// the outputs of a row of x or of w that has one are worked out by float32 multiply-adds instead (gf_dot).
-// 333 tokens by 4,096 rows of 1,024, 33 us: 58 with one such number in x, or in w; 697 with one in every row of x.  16 by 2,560 of 9,728, 54 us: 80, 95 and 265.  (By
-// a chain of K in one thread an output, and 128 weight rows for one of them: 110, 6,730, 6,750; 2,450, 10,700, 21,400.)
+// the outputs of a row of x or of w that has one are worked out by float32 multiply-adds instead (gf_dot).  So are a token's 128
+// outputs of a tile where a sum is not finite: parts of huge numbers can multiply to infinities of both signs where the numbers' products give one, or a finite sum.
+// 333 tokens by 4,096 rows of 1,024, 33 us: 58 with one such number in x, or in w; 697 with one in every row of x.  16 by 2,560 of 9,728, 54 us: 80, 95 and 265 (sums that
+// overflow everywhere cost as much as bad rows everywhere).  (By a chain of K in one thread an output, and 128 weight rows for one of them: 110, 6,730, 6,750; 2,450, 10,700, 21,400.)
 //
 // A CTA has 128 weight rows (the MMA's M) and `width` tokens (N).  Its warps fetch the next 64 k of both operands (16-byte loads, in registers
 // while the MMAs of the k ahead run), split them into the six planes of a stage in shared memory (128-byte swizzle), then add the accumulator of the
@@ -121,6 +122,8 @@ __device__ __noinline__ bool gf_splits(const float* row, int K) {
     return __all_sync(0xffffffffu, (left & 0xffffu) == 0);
 }
 
+__device__ __forceinline__ bool gf_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+
 // The thread's number, asked for once more: what is worked out from it behind the loop then takes no registers in the loop, which has none to spare (with the flags'
 // places from the first one 333 tokens by 4,096 rows of 1,024 took 30.6 us for 29.3).
 __device__ __forceinline__ int gf_thread() {
@@ -145,9 +148,9 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t full[STAGES], done[STAGES];               // a stage is filled (and its accumulator read); its MMAs are done
     __shared__ uint32_t tmem_slot;
-    __shared__ int bad_any;                                       // something is flagged
+    __shared__ int bad_any;                                       // something is flagged, or a sum is not finite
     __shared__ uint8_t bad_x[BN], bad_w[GF_BM];                   // tokens and weight rows with a number that does not split, in this CTA's k
-    __shared__ uint8_t all_x[BN], all_w[GF_BM];                   // in all of it
+    __shared__ uint8_t all_x[BN], all_w[GF_BM];                   // in all of it: 1; 2: a token of this CTA's with a sum that is not finite
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n0 = blockIdx.x * GF_BM, t0 = blockIdx.y * width, splits = gridDim.z, rank = blockIdx.z;
@@ -158,8 +161,8 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         bad_any = 0;
     }
-    if (tid < BN) bad_x[tid] = 0;
-    if (tid < GF_BM) bad_w[tid] = 0;
+    if (tid < BN) bad_x[tid] = all_x[tid] = 0;
+    if (tid < GF_BM) bad_w[tid] = all_w[tid] = 0;
     if (warp == 0) tmem_alloc<false>(&tmem_slot, S::COLS);
     // A warp's rounds: two rows each, of the weights (pairs of rows 0 to 63: rounds 0 to 3 and some of 4) or of x.  No round but the last few is behind a
     // branch, so that several are worked on side by side: a pair past the last one is the last one once more (the same numbers to the same place), and a row that is
@@ -331,6 +334,7 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
         (of_w2(i) ? bad_w : bad_x)[(pair2(i) & (GF_BM / 2 - 1)) * 2 + (lane2 >> 4)] = 1;      // (of the weights: one of four rows)
         bad_any = 1;
     }
+    bool finite = true;
 #pragma unroll
     for (int i = 0; i < S::CW; i += STEP) {
         if (c0 + i >= width) continue;
@@ -338,7 +342,10 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
         before(i, v);
         if (splits == 1) {
 #pragma unroll
-            for (int e = 0; e < STEP; ++e) cur[i + e] = v[e] + cur[i + e];
+            for (int e = 0; e < STEP; ++e) {
+                cur[i + e] = v[e] + cur[i + e];
+                finite &= gf_finite(cur[i + e]);
+            }
         } else {
 #pragma unroll
             for (int e = 0; e < STEP; ++e) {
@@ -348,6 +355,7 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
             }
         }
     }
+    if (!finite) bad_any = 1;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();                                              // tensor memory has been read, and everyone has said what was bad
     if (warp2 == 0) tmem_free<false>(tmem, S::COLS);
@@ -396,15 +404,21 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
             (tid2 < BN ? all_x + tid2 : all_w + (tid2 - BN))[0] = (uint8_t)all;
         }
         __syncthreads();
+        if (!finite && all_w[in2] == 0) {                         // (with one CTA a tile; several see the whole sum only below)
+#pragma unroll
+            for (int i = 0; i < S::CW; ++i)
+                if (c0 + i < width && !gf_finite(cur[i]) && all_x[c0 + i] == 0) all_x[c0 + i] = 2;
+        }
+        __syncthreads();
     }
     if (splits == 1) {
         if (n0 + in2 < N) {
             store(GfTrue());
         }
     } else {
+        bool odd = false;
         for (int idx = rank * GF_THREADS + tid2; idx < width * (GF_BM / 4); idx += splits * GF_THREADS) {
-            const int t = idx / (GF_BM / 4), n = idx % (GF_BM / 4) * 4;
-            if (t0 + t >= T || n0 + n >= N) continue;
+            const int t = idx / (GF_BM / 4), n = idx % (GF_BM / 4) * 4;      // (a warp a token)
             float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             for (int z = 0; z < splits; ++z) {
                 const uint32_t peer = gf_peer(sums + t * GF_BM + n, z);
@@ -414,8 +428,18 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
                     v[0] += p.x; v[1] += p.y; v[2] += p.z; v[3] += p.w;
                 }
             }
+            if (__any_sync(0xffffffffu, !(gf_finite(v[0]) && gf_finite(v[1]) && gf_finite(v[2]) && gf_finite(v[3])))) {
+                bool mine_is = false;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) mine_is |= !gf_finite(v[e]) && all_w[n + e] == 0;
+                if (__any_sync(0xffffffffu, mine_is)) {
+                    odd = true;
+                    if (all_x[t] == 0) all_x[t] = 2;
+                }
+            }
+            if (t0 + t >= T || n0 + n >= N) continue;
             float* to = out + (size_t)(t0 + t) * N + n0 + n;
-            if (!any && n0 + n + 4 <= N && (N & 3) == 0 && ((uintptr_t)out & 15) == 0) {
+            if (!any && !odd && n0 + n + 4 <= N && (N & 3) == 0 && ((uintptr_t)out & 15) == 0) {
                 float4 r = make_float4(v[0], v[1], v[2], v[3]);
                 if (ACC) {
                     const float4 old = *reinterpret_cast<const float4*>(to);
@@ -424,20 +448,23 @@ __global__ void __launch_bounds__(GF_THREADS, STAGES == 1 ? 2 : 1) gemm_f32_kern
                 *reinterpret_cast<float4*>(to) = r;
             } else {
                 for (int e = 0; e < 4 && n0 + n + e < N; ++e)
-                    if (!any || (all_x[t] | all_w[n + e]) == 0) to[e] = ACC ? to[e] + v[e] : v[e];
+                    if ((all_x[t] | all_w[n + e]) == 0) to[e] = ACC ? to[e] + v[e] : v[e];
             }
         }
         cluster_sync();                                           // nobody leaves while its sums are read
+        any = __syncthreads_or(any || odd) != 0;
     }
     if (!any) return;
-    // the flagged ones, an output a warp (of all the tile's CTAs): tokens with all weight rows, then weight rows with the other tokens
+    // The flagged ones, an output a warp of all the tile's CTAs: tokens with all weight rows, then weight rows with the other tokens.  (Tokens that this CTA alone
+    // knows of: its warps, and the flagged weight rows are among the others'.)
     const int tokens = min(width, T - t0), weights = min(GF_BM, N - n0), me = rank * (GF_THREADS / 32) + warp2, warps = splits * (GF_THREADS / 32);
     for (int a = 0; a < tokens + weights; ++a) {
         const bool token = a < tokens;
-        if ((token ? all_x[a] : all_w[a - tokens]) == 0) continue;
-        for (int b = me; b < (token ? weights : tokens); b += warps) {
+        const int flag = token ? all_x[a] : all_w[a - tokens];
+        if (flag == 0) continue;
+        for (int b = flag == 2 ? warp2 : me; b < (token ? weights : tokens); b += flag == 2 ? GF_THREADS / 32 : warps) {
             const int t = token ? a : b, n = token ? b : a - tokens;
-            if (!token && all_x[t] != 0) continue;
+            if (token ? flag == 2 && all_w[n] != 0 : all_x[t] == 1) continue;
             const float v = gf_dot(x + (size_t)(t0 + t) * K, w + (size_t)(n0 + n) * K, K);
             float* to = out + (size_t)(t0 + t) * N + n0 + n;
             if (lane2 == 0) *to = ACC ? *to + v : v;

@@ -1134,6 +1134,39 @@ def test_float32_number_that_does_not_split_concerns_its_rows_alone(ops, monkeyp
     ops.check_device_errors()
 
 
+@pytest.mark.parametrize("T,N,K", [(1, 130, 64), (40, 300, 260), (200, 3100, 512)])
+def test_float32_product_that_overflows_is_what_its_numbers_give(ops, monkeypatch, T, N, K):
+    """Numbers that split, but whose products leave float32's range or come within its last bit: infinities of the products' sign, no not-a-number of their parts, and
+    the finite sum where the parts alone would leave the range (a product of two numbers and zeros: rounded once).  Other rows keep their bits."""
+    g = torch.Generator().manual_seed(T)
+    x, w = torch.randn(T, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    clean = torch.empty(T, N, device=DEV)
+    ops.gemm(x, w, clean)
+    t = T // 2
+    x[t] = (1e22 + 3e21 * torch.rand(K, generator=g)).cuda()
+    w[N // 3] = (1e22 + 3e21 * torch.rand(K, generator=g)).cuda()
+    w[N - 1] = 0.0
+    x[0, 7], w[N - 1, 7] = 1.7012e38, 1.9990234375                                # (their first parts are 2^127 and 2, the product is below 2^128)
+    w[N // 2, 3] = 1.1e-40                                                            # (and a row that does not split, whose outputs must not be added twice)
+    rows = torch.ones(T, N, dtype=torch.bool, device=DEV)
+    rows[t], rows[0], rows[:, N // 3], rows[:, N // 2], rows[:, N - 1] = False, False, False, False, False
+    first, groups = None, 8 if N <= ops.F32_FEW_ROWS else 4
+    for plan in [(16, 1), (32, groups), (48, groups // 2), (112, 1), (128, groups)]:
+        monkeypatch.setattr(ops, "f32_plan", lambda *a: plan)
+        out = torch.full((T, N), math.nan, device=DEV)
+        ops.gemm(x, w, out)
+        assert float(out[t, N // 3]) == math.inf, plan
+        if t != 0:
+            assert float(out[0, N - 1]) == float((x[0, 7].double() * w[N - 1, 7].double()).float()) < math.inf
+        assert torch.equal(out[rows], clean[rows])
+        first = out if first is None else first
+        assert torch.equal(torch.nan_to_num(out, 5.0), torch.nan_to_num(first, 5.0))
+        added = torch.ones(T, N, device=DEV)
+        ops.gemm(x, w, added, accumulate=True)
+        assert torch.equal(torch.nan_to_num(added, 5.0), torch.nan_to_num(out + 1.0, 5.0)) and float(added[t, N // 3]) == math.inf
+    ops.check_device_errors()
+
+
 def test_float32_number_that_does_not_split_costs_less_than_the_product(ops):
     """It once cost 180 products: every output of 128 weight rows by a chain in one thread."""
     T, N, K = 333, 4096, 1024
