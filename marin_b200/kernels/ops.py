@@ -476,22 +476,22 @@ def _persistent_product(x, w, out, mode: int, T: int, N: int, K: int, s, what: s
 @functools.lru_cache(maxsize=4096)
 def f32_plan(T: int, N: int, K: int):
     """Tokens a tile and CTAs a tile of the 32-bit product on the tensor cores (neither changes a bit of the result): the least rounds of CTAs over the SMs times
-    a CTA's clocks.  Measured on B200: a stage of 64 k 1,750 + 10 a token (3,200 at 128), up to 32 tokens 2,750, or 4,500 with two CTAs an SM; 4,000 to begin
-    and end; where a cluster adds its sums 3,000 and a clock for every 16 bytes of them that a CTA reads.  Clusters of eight find room for 112 CTAs at once, of
+    a CTA's clocks.  Measured on B200: a stage of 64 k 1,750 + 10 a token (3,200 at 128), up to 32 tokens 2,750, or 4,500 with two CTAs an SM; to begin
+    and end 4,000 up to 32 tokens and 6,000 beyond (333 tokens by 48 rows of 48 by tiles of 16 4.0 us, of 48 5.7); where a cluster adds its sums 3,000 and a clock for every 16 bytes of them that a CTA reads.  Clusters of eight find room for 112 CTAs at once, of
     four for 132 (1,024 rows of 2,048 and 64 tokens: 16 clusters of eight 23.6 us, 8 of them 13.5)."""
     groups = 8 if N <= F32_FEW_ROWS else 4
     chunks = -(-K // 64)
     per = -(-chunks // groups)
     rows = -(-N // 128)
     best = None
-    for width in (16, 32) if T <= 32 else (32, 48, 64, 80, 96, 112, 128):
+    for width in (16, 32) if T <= 32 else (16, 32, 48, 64, 80, 96, 112, 128):
         for splits in (1, groups // 2, groups):
             few = width <= 32
             ctas = rows * -(-T // width) * splits
             at_once = {8: 112, 4: 132}.get(splits, SM_COUNT)
             stage = (2750 if ctas <= at_once else 4500) if few else 1750 + 10 * width + (170 if width > 112 else 0)
             adding = 3000 + width * 128 * 4 * groups // splits // 16 if splits > 1 else 0
-            cost = -(-ctas // (at_once * (2 if few else 1))) * (min(chunks, per * groups // splits) * stage + 4000 + adding)
+            cost = -(-ctas // (at_once * (2 if few else 1))) * (min(chunks, per * groups // splits) * stage + (4000 if few else 6000) + adding)
             if best is None or cost < best[0]:
                 best = (cost, width, splits)
     return best[1:]

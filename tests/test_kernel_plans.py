@@ -49,6 +49,13 @@ def test_plans_beyond_128_tokens_are_launches_the_kernels_take(T, N, K):
     assert not ops.half_round(128, N, K) and not ops.many_tokens(128, N, True)
 
 
+@pytest.mark.parametrize("T,N,K,widths", [(33, 48, 48, (16, 32)), (128, 64, 256, (16, 32)), (333, 512, 128, (16, 32)),       # 4.1 us for 5.7 by tiles of 48, 6.9 for 8.1, 5.7 for 6.7
+                                          (333, 1024, 1024, (96,)), (333, 4096, 1024, (96,)), (333, 2560, 9728, (112,)), (16, 2560, 9728, (16,))])
+def test_float32_tiles_where_they_were_measured_faster(T, N, K, widths):
+    width, splits = ops.f32_plan(T, N, K)
+    assert width in widths and splits in ((1, 4, 8) if N <= ops.F32_FEW_ROWS else (1, 2, 4))
+
+
 @pytest.mark.parametrize("E", [1, 8, 16, 32, 60, 128, 384, 512])
 @pytest.mark.parametrize("h,ff,shared_ff", [(2560, 3648, 2432), (4096, 2048, 0), (2048, 768, 768), (256, 512, 1024)])
 def test_parts_of_the_experts_last_products_cost_less_than_the_round_they_save(E, h, ff, shared_ff):
