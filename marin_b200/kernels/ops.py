@@ -435,11 +435,12 @@ def stream_k_plan(T: int, N: int, K: int) -> Optional[int]:
     """Tokens per tile if the product should run stream-K, else None.  The CTAs form groups, one CTA per token tile,
     and every group gets the same number of k-blocks of the weight-row tiles laid end to end: the time goes with
     row tiles / groups, without rounding up to whole rounds of tiles.  It needs at least one row tile per group."""
-    return _stream_k_width(T, N, K, _KBLOCK_FIXED, _STREAM_K_FIXED, _STREAM_K_MARGIN, _STREAM_K_MAX_X_BYTES) if stream_k else None
+    return _stream_k_width(T, N, K, paired_plan(T, N, K), _KBLOCK_FIXED, _STREAM_K_FIXED, _STREAM_K_MARGIN, _STREAM_K_MAX_X_BYTES) if stream_k else None
 
 
 @functools.lru_cache(maxsize=4096)
-def _stream_k_width(T: int, N: int, K: int, kblock: int, fixed: float, margin: float, most: int) -> Optional[int]:
+def _stream_k_width(T: int, N: int, K: int, tile: int, kblock: int, fixed: float, margin: float, most: int) -> Optional[int]:
+    # (tile: the width whole tiles would have, ``paired_plan``'s, which switches change)
     best = None
     rows, nkb = -(-N // 128), -(-K // 64)
     for bn in STREAM_K_TILES:
@@ -451,11 +452,10 @@ def _stream_k_width(T: int, N: int, K: int, kblock: int, fixed: float, margin: f
             best = (cost, bn)
     if best is None:
         return None
-    bn = paired_plan(T, N, K)
-    if bn > 0:
-        whole = -(-(rows * -(-T // bn)) // SM_COUNT) * (nkb * (bn + kblock) + 1600)
+    if tile > 0:
+        whole = -(-(rows * -(-T // tile)) // SM_COUNT) * (nkb * (tile + kblock) + 1600)
     else:
-        whole = 0.73 * -(-(-(-rows // 2) * -(-T // -bn)) // (SM_COUNT // 2)) * (nkb * (kblock - bn) + 2400) + 4200
+        whole = 0.73 * -(-(-(-rows // 2) * -(-T // -tile)) // (SM_COUNT // 2)) * (nkb * (kblock - tile) + 2400) + 4200
     return best[1] if best[0] < margin * whole else None
 
 

@@ -26,6 +26,17 @@ def test_stream_k_can_be_switched_off(monkeypatch):
     assert ops.stream_k_plan(2048, 2560, 9728) is None
 
 
+@pytest.mark.parametrize("T,N,K", [(436, 5120, 17408), (600, 5120, 17408), (1000, 5120, 5120)])
+def test_stream_k_follows_the_switch_of_pairs_whichever_was_asked_first(monkeypatch, T, N, K):
+    plans = {}
+    for first in (True, False):
+        ops._stream_k_width.cache_clear()
+        for pairs in (first, not first):
+            monkeypatch.setattr(ops, "pair_tiles", pairs)
+            plans[first, pairs] = ops.stream_k_plan(T, N, K)
+    assert plans[True, True] == plans[False, True] and plans[True, False] == plans[False, False]
+
+
 @pytest.mark.parametrize("T,N,K", [(1, 6144, 2560), (8, 2560, 9728), (16, 2560, 4096), (64, 151936, 2560), (128, 300, 200), (33, 1000, 72)])
 def test_few_token_plan_keeps_every_slice_in_use(T, N, K):
     bn, splits = ops.gemm_plan(T, N, K)
