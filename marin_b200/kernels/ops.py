@@ -2132,8 +2132,7 @@ def attention_pooled(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table,
     if talk is not None and ctx.num_requests > ctx.num_decode:
         blocks = _pooled_mix_blocks(ctx, window, pool)
         if (use_pooled_mix and pooled_mix_supported(q.dtype, H, K, d, dv) and page_size & (page_size - 1) == 0 and scale > 0
-                and _pooled_mix_pays(T - ctx.num_decode, ctx.num_requests - ctx.num_decode, ctx.max_query_len, blocks, K, dv,
-                                     _pooled_mix_walk(T - ctx.num_decode, ctx.num_requests - ctx.num_decode, blocks))
+                and _pooled_mix_pays(T - ctx.num_decode, ctx.num_requests - ctx.num_decode, ctx.max_query_len, blocks, K, dv)
                 and all(t is None or t.data_ptr() % 16 == 0 for t in (q, k_cache, v_cache, k_pool, v_pool, out))):
             _pooled_mix(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table, H, K, d, dv, scale, softcap or 0.0, window, pool, rows, talk, blocks)
             if ctx.num_decode == 0:
@@ -2186,18 +2185,15 @@ def _pooled_mix_tiles(tokens: int, portions: int) -> int:
     return tokens // 16 + portions
 
 
-def _pooled_mix_walk(tokens: int, portions: int, blocks: int) -> float:
-    """Blocks a CTA of the mixing kernel walks: an equal share of all tiles' (a few for its start and for a tile's)."""
-    return 4.0 + _pooled_mix_tiles(tokens, portions) * blocks / SM_COUNT
-
-
-def _pooled_mix_pays(tokens: int, portions: int, longest: int, blocks: int, K: int, dv: int, walk: Optional[float] = None) -> bool:
-    """Whether portions of so many tokens (in all) go to the kernels that mix the weights first: a portion that fills a tile, enough tokens for the blocks a CTA
-    walks (``walk``; all ``blocks`` of a tile where it is not given: with 2, 10, 19 and 35 of them from 84, 231, 291 and 335 tokens on), and mixed weights (H x 16 x 32 numbers of 16 bits a tile and block) that take no more
+def _pooled_mix_pays(tokens: int, portions: int, longest: int, blocks: int, K: int, dv: int) -> bool:
+    """Whether portions of so many tokens (in all) go to the kernels that mix the weights first: a portion that fills a tile, enough tokens for the blocks that a CTA
+    of the mixing walks (an equal share of all tiles', and a few for its start and a tile's: one portion with 2, 10, 19 and 35 blocks a tile from 175, 104, 72 and 46
+    tokens on), and mixed weights (H x 16 x 32 numbers of 16 bits a tile and block) that take no more
     memory than the heads' sums would (H x K x dv of 32 bits a token), which is what a step's working memory is planned with.  By that a window of
     1,024 passes with 8 kv heads of 128, one of 2,048 or none over more than 2,000 positions does not."""
     block, token, both = POOLED_MIX_COSTS
-    return longest >= 16 and block * (blocks if walk is None else walk) <= tokens * (token + both * blocks) and _pooled_mix_tiles(tokens, portions) * blocks * 256 <= tokens * K * dv
+    tiles = _pooled_mix_tiles(tokens, portions)
+    return longest >= 16 and block * (4.0 + tiles * blocks / SM_COUNT) <= tokens * (token + both * blocks) and tiles * blocks * 256 <= tokens * K * dv
 
 
 def pooled_mix_supported(dtype, H: int, K: int, d: int, dv: int) -> bool:
