@@ -351,7 +351,9 @@ __global__ void __launch_bounds__(256) heads_product_tc_kernel(const bf16* __res
 template <int COLS>
 static int launch_heads_tc(const void* x, int x_ld, int x_head, const void* w, void* out, int o_ld, int o_head, int tokens, int H, int N, int K, cudaStream_t s) {
     auto kernel = heads_product_tc_kernel<COLS>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HtTile<COLS>::SMEM);
+    static LaunchSmem smem;
+    const int rc = smem.allow(kernel, HtTile<COLS>::SMEM);
+    if (rc) return rc;
     const int wide = N % 8 == 0 && o_ld % 8 == 0 && o_head % 8 == 0 && (((uintptr_t)out) & 15) == 0;
     return launch_kernel(kernel, dim3(H, (N + COLS - 1) / COLS, (tokens + HT_M - 1) / HT_M), 256, HtTile<COLS>::SMEM, s, 0, (const bf16*)x, x_ld, x_head,
                          (const bf16*)w, (bf16*)out, o_ld, o_head, tokens, N, K, wide);

@@ -763,31 +763,34 @@ static int page_shift_of(int page_size) {
 
 // Requests first_req .. first_req + count - 1 of the step; which: 0 the rows' sums (lse float32 [tokens][H]), 1 the mixed weights, 2 the results (in this
 // order).  mixed: halves, (tokens / 16 + count) tiles of most_blocks blocks of H * 512; most_blocks: at least the blocks of 32 any tile of the step has.
-// q, caches, out and mixed 16-byte aligned.
+// ctas: CTAs that the mixing deals the blocks out to (one per SM).  q, caches, out and mixed 16-byte aligned.
 MB_API int mb_attn_pooled_mix(int which, const void* q, const void* k_cache, const void* v_cache, const void* k_pool, const void* v_pool, float* lse,
                               const float* talk, void* mixed, void* out, const int* block_table, int max_pages, const int* cu_tokens, const int* seq_lens,
                               int first_req, int count, int max_query_len, int page_size, float scale, float cap, int window, int pool, int pool_rows,
-                              int most_blocks, int* error_flag, cudaStream_t s) {
+                              int most_blocks, int ctas, int* error_flag, cudaStream_t s) {
     if (count <= 0 || max_query_len <= 0) return 0;
     const int shift = page_shift_of(page_size);
-    if (shift < 0 || window < 0 || pool < 0 || (pool > 0 && (k_pool == nullptr || v_pool == nullptr)) || most_blocks <= 0) return MB_ERR_BAD_SIZE;
+    if (shift < 0 || window < 0 || pool < 0 || (pool > 0 && (k_pool == nullptr || v_pool == nullptr)) || most_blocks <= 0 || ctas <= 0) return MB_ERR_BAD_SIZE;
     if (pool > 0 && pool_rows != (page_size + pool - 1) / pool) return MB_ERR_BAD_SIZE;
     if ((((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)mixed | (uintptr_t)out) & 15) != 0) return MB_ERR_BAD_SIZE;
     if (which == 0) {
-        cudaFuncSetAttribute(stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STATS_SMEM);
+        static LaunchSmem smem;
+        const int rc = smem.allow(stats_kernel, STATS_SMEM);
+        if (rc) return rc;
         return launch_kernel(stats_kernel, dim3(KH, count, (max_query_len + SQ - 1) / SQ), STATS_THREADS, STATS_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache,
                              (const bf16*)k_pool, lse, block_table, max_pages, cu_tokens, seq_lens, first_req, shift, scale, cap, window, pool, pool_rows, error_flag);
     }
     const int tiles_of = (max_query_len + NQ - 1) / NQ;
     if (which == 1) {
-        cudaFuncSetAttribute(mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MIX_SMEM);
-        int device = 0, sms = 0;
-        cudaGetDevice(&device);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        return launch_kernel(mix_kernel, dim3(sms > 0 ? sms : 1), MIX_THREADS, MIX_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache, (const bf16*)k_pool, (const float*)lse, talk,
+        static LaunchSmem smem;
+        const int rc = smem.allow(mix_kernel, MIX_SMEM);
+        if (rc) return rc;
+        return launch_kernel(mix_kernel, dim3(ctas), MIX_THREADS, MIX_SMEM, s, 0, (const bf16*)q, (const bf16*)k_cache, (const bf16*)k_pool, (const float*)lse, talk,
                              (__half*)mixed, block_table, max_pages, cu_tokens, seq_lens, first_req, count, shift, scale, cap, window, pool, pool_rows, most_blocks);
     }
-    cudaFuncSetAttribute(value_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VALUE_SMEM);
+    static LaunchSmem smem;
+    const int rc = smem.allow(value_kernel, VALUE_SMEM);
+    if (rc) return rc;
     return launch_kernel(value_kernel, dim3(KH, count, (tiles_of + VT - 1) / VT), VALUE_WORKERS + 32, VALUE_SMEM, s, 0, (const __half*)mixed, talk, (const bf16*)v_cache, (const bf16*)v_pool, (bf16*)out, block_table,
                          max_pages, cu_tokens, seq_lens, first_req, shift, window, pool, pool_rows, most_blocks, error_flag);
 }

@@ -347,15 +347,13 @@ __global__ void __launch_bounds__(4 * AT_ROWS, 2) attention_tile_kernel(
 // steps, up to 32 query heads a kv head.
 MB_API int mb_attention_tile(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table, int max_pages,
                              const int* cu_tokens, const int* seq_lens, int first_req, int count, int max_query_len, int H, int K, int d,
-                             int page_size, float scale, cudaStream_t s) {
+                             int page_size, float scale, int sms, cudaStream_t s) {
     if (count <= 0 || max_query_len <= 0) return 0;
     if (d <= 0 || d > 128 || d % 4 != 0 || K <= 0 || H % K != 0 || H / K > 32 || page_size <= 0) return MB_ERR_BAD_SIZE;
     if ((((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) & 15) != 0) return MB_ERR_BAD_SIZE;
-    int page_shift = -1, sms = 0, device = 0;
+    int page_shift = -1;
     for (int i = 0; i < 31; ++i)
         if ((1 << i) == page_size) page_shift = i;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     // 32 rows a block where that makes two blocks an SM (what a block fetches is then shared by twice the rows); a row's bits do not depend on it
     const int G = H / K, tiles = (max_query_len + 32 / G - 1) / (32 / G);
     const bool wide = G > 16 || (long long)tiles * K * count >= 2 * sms;
@@ -363,7 +361,9 @@ MB_API int mb_attention_tile(const void* q, const void* k_cache, const void* v_c
     const dim3 grid((max_query_len + per_tile - 1) / per_tile * K, count);
     const auto kernel = wide ? attention_tile_kernel<32> : attention_tile_kernel<16>;
     const int rows = wide ? 32 : 16;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM(rows));
+    static LaunchSmem smem[2];
+    const int rc = smem[wide].allow(kernel, AT_SMEM(rows));
+    if (rc) return rc;
     return launch_kernel(kernel, grid, 4 * rows, AT_SMEM(rows), s, 0, (const float*)q, (const float*)k_cache, (const float*)v_cache, (float*)out, block_table,
                          max_pages, cu_tokens, seq_lens, first_req, H, K, d, page_size, page_shift, scale);
 }

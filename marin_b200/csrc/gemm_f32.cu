@@ -480,12 +480,9 @@ template <int BN, int STAGES, bool ACC>
 static int gf_launch(const float* x, const float* w, float* out, int T, int N, int K, int width, int splits, int* error_flag, cudaStream_t s) {
     typedef GfTile<BN, STAGES> S;
     auto kernel = gemm_f32_kernel<BN, STAGES, ACC>;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static LaunchSmem smem;
+    const int rc = smem.allow(kernel, S::SMEM);
+    if (rc) return rc;
     const int groups = gf_groups(N), chunks = (K + GF_BK - 1) / GF_BK;
     const dim3 grid((N + GF_BM - 1) / GF_BM, (T + width - 1) / width, splits);
     if (grid.y > 65535) return MB_ERR_BAD_SIZE;

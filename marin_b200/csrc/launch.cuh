@@ -85,6 +85,23 @@ static inline bool pdl_enabled() {
     return state == 1;
 }
 
+// What a kernel may take of shared memory at a launch, said once per kernel and device (a static one for each kernel): a process may use several devices, each of
+// which has to be told.
+struct LaunchSmem {
+    unsigned long long told;                                          // a bit a device
+    template <typename... KArgs>
+    int allow(void (*kernel)(KArgs...), size_t bytes) {
+        int device = 0;
+        cudaError_t e = cudaGetDevice(&device);
+        if (e != cudaSuccess) return (int)e;
+        const unsigned long long bit = device < 64 ? 1ull << device : 0;
+        if ((__atomic_load_n(&told, __ATOMIC_RELAXED) & bit) != 0) return 0;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e == cudaSuccess) __atomic_fetch_or(&told, bit, __ATOMIC_RELAXED);
+        return (int)e;
+    }
+};
+
 // cluster_z > 1 launches thread-block clusters of (1, 1, cluster_z); cluster_z < -1 clusters of (-cluster_z, 1, 1).
 template <typename... KArgs, typename... Args>
 static inline int launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster_z,

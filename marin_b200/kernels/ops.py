@@ -905,7 +905,7 @@ def attention(q, k_cache, v_cache, out, ctx, block_table, H, K, d, scale, window
         _check(_lib("mb_attention_simple").mb_attention_tile(
             _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), _c_int(block_table.shape[1]), _ptr(ctx.cu_tokens), _ptr(ctx.seq_lens),
             _c_int(nd), _c_int(ctx.num_requests - nd), _c_int(ctx.max_query_len), _c_int(H), _c_int(K), _c_int(d), _c_int(page_size),
-            _c_float(scale), _stream()), "attention (tiles)")
+            _c_float(scale), _c_int(SM_COUNT), _stream()), "attention (tiles)")
         rows = nd
     if rows == 0:
         return
@@ -2244,7 +2244,7 @@ def _pooled_mix(q, k_cache, v_cache, k_pool, v_pool, out, ctx, block_table, H: i
     args = (_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(k_pool), _ptr(v_pool), _ptr(lse), _ptr(talk), _ptr(mixed), _ptr(out), _ptr(block_table),
             _c_int(block_table.shape[1]), _ptr(ctx.cu_tokens), _ptr(ctx.seq_lens), _c_int(nd), _c_int(count), _c_int(ctx.max_query_len),
             _c_int(k_cache.shape[2]), _c_float(scale), _c_float(softcap), _c_int(window), _c_int(pool), _c_int(rows), _c_int(blocks),
-            _ptr(_scratch_for(q.device).error), _stream())
+            _c_int(SM_COUNT), _ptr(_scratch_for(q.device).error), _stream())
     size = q.element_size()
     # what the algorithm needs is shared out: the queries and keys with the sums, the mixing of a pair's weights, the values and results with the last
     for which, what, nbytes, per_key, per_pair in (

@@ -1167,6 +1167,17 @@ def test_float32_product_that_overflows_is_what_its_numbers_give(ops, monkeypatc
     ops.check_device_errors()
 
 
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="one GPU")
+def test_float32_product_on_a_second_device(ops):
+    """Both tile sizes, on one device after another in one process: each device is told what shared memory the kernels take."""
+    for device in ("cuda:0", "cuda:1"):
+        for T in (8, 200):
+            with torch.cuda.device(device):
+                x, w, out = torch.randn(T, 256, device=device), torch.randn(96, 256, device=device), torch.empty(T, 96, device=device)
+                ops.gemm(x, w, out)
+                torch.testing.assert_close(out.double(), x.double() @ w.double().t(), rtol=1e-5, atol=1e-4)
+
+
 def test_float32_number_that_does_not_split_costs_less_than_the_product(ops):
     """It once cost 180 products: every output of 128 weight rows by a chain in one thread."""
     T, N, K = 333, 4096, 1024
