@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(
                 if (J < 3) { farA[J < 3 ? J : 0][e] = 0.0f; farP[J < 3 ? J : 0][e] = 0.0f; }
             }
         // a reference for the rows of this block against earlier ones: the sum at the last row before it; for its rows 8 .. 15 against
-        // its rows 0 .. 7 (worked out by the first of the two warps): the sum at its row 7
+        // its rows 0 .. 7 (each warp its half of the channels, as of all else): the sum at its row 7
         const float* ref = sG + (I > 0 ? I * 16 - 1 : 0) * LDG;
         const float* mid = sG + (I * 16 + 7) * LDG;
 #pragma unroll 1
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) prepare_kernel(
             const int j = jb * 16 + half * 8 + t2;
 #pragma unroll
             for (int rr = 0; rr < 2; ++rr) {
-                if (CHANNEL && J == 3 && rr == 0) continue;    // rows 0 .. 7 of the block's own square: pair by pair below
+                if (CHANNEL && J == 3 && rr == 0) continue;    // rows 0 .. 7 of the block's own square: pair by pair above
                 const int i = rr ? i1 : i0;
                 float a[2], b[2];
 #pragma unroll

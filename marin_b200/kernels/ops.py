@@ -380,7 +380,7 @@ def persistent_plan(T: int, N: int) -> int:
 
 #: two SMs on one tile of 256 weight rows in the persistent kernel
 pair_tiles = True
-#: from this many multiply-adds on (pairs take clusters to place and two SMs' ends to wait for; measured on B200, 36 to 2e11 multiply-adds: see ``_paired_width``)
+#: from this many multiply-adds on (pairs take clusters to place and two SMs' ends to wait for; measured on B200 over the shapes that ``_paired_width`` names)
 PAIRS_FROM = 1 << 33
 
 
@@ -638,6 +638,8 @@ def gemm_side_by_side(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> No
             gemm(x[g], w[g], out[g])
         return
     rows = G * -(-N // 128)
+    # (a round of tiles as width + 24: with the + 96 of ``_tile_by_tile`` four products of 2,560 x 2,560 and 1,000 tokens would take tiles of 208 for 144 and 65.6 us for 71.7,
+    # of 700 240 for 144 and 49.2 for 57.4, of 2,048 240 for 192 and 102.0 for 102.5; of 500, 300 and 160 the same tiles)
     tile = min(PERSISTENT_TILES, key=lambda bn: (-(-(rows * -(-T // bn)) // SM_COUNT) * (bn + 24), bn))
     _cost(_size(x) + _size(w) + _size(out), 2.0 * G * T * N * K)
     _check(_lib("mb_moe_tc").mb_moe_grouped_tc(
