@@ -1965,7 +1965,9 @@ def _expert_tile(pairs: int, E: int, shared_rows: int = 0) -> int:
     weights are then read once, and a small tile leaves room for a deep ring); equal tiles of at most 256 beyond.  A whole call by tiles of 32, 64, 128 and 256: 8
     experts of 2,560 x 3,648, two chosen, a shared one of 2,432: shares of 12 rows 111, 115, 116, 124 us; 20 122, 120, 120, 128; 25 136, 124, 122, 130; 44 199,
     134, 125, 139; 64 232, 168, 124, 137; 100 335, 238, 154, 146.  16 experts of 2,048 x 1,280, one chosen, a shared one of 1,024: 4 77, 79, 79, 84; 5 81, 78, 79,
-    84; 8 84, 80, 82, 86; 11 87, 86, 82, 89; 44 178, 122, 101, 106; 62 207, 154, 116, 111."""
+    84; 8 84, 80, 82, 86; 11 87, 86, 82, 89; 44 178, 122, 101, 106; 62 207, 154, 116, 111.  Many experts with a shared one, more than 128 tokens: 512 of 1,024 x 512, share 4
+    293, 279, 270, 279; 256 of 2,048 x 768, 5 354, 338, 328, 338; 128 of the same, 8.5 289, 279, 271, 289; 64 of 2,048 x 1,024, 8.5 211, 207, 205, 213; 32 of 2,560 x 1,408, 8.75
+    186, 182, 188, 185."""
     average = pairs / E
     if average <= 20 and shared_rows <= 128:
         return 32 if shared_rows <= 64 else 64
