@@ -459,9 +459,11 @@ def _stream_k_width(T: int, N: int, K: int, tile: int, kblock: int, fixed: float
     return best[1] if best[0] < margin * whole else None
 
 
-def _persistent_product(x, w, out, mode: int, T: int, N: int, K: int, s, what: str) -> None:
+def _persistent_product(x, w, out, mode: int, T: int, N: int, K: int, s, what: str, parts: bool = False) -> None:
+    """``parts``: a sum for every part of K (``sums_plan``), where the plan would else have cut it into slices."""
     lib = _lib("mb_gemm_tc")
-    tile, sums = (paired_plan(T, N, K), 1) if mode in _GLU_MODES.values() else _whole_tiles(paired_plan(T, N, K), T, N, K)
+    tile = paired_plan(T, N, K)
+    tile, sums = _whole_tiles(tile, T, N, K) if parts else (tile, 1)
     bn = stream_k_plan(T, N, K) if sums == 1 else None
     if bn is not None:
         _check(lib.mb_gemm_tc_persistent_streamk(
@@ -558,7 +560,8 @@ def gemm(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, then_n
             if activation != "relu2" or accumulate or out.dtype != torch.bfloat16 or then_norm is not None:
                 raise KernelError(f"gemm: activation {activation!r} goes with a plain bfloat16 output")
             mode = 4
-        if many_tokens(T, N) or half_round(T, N, K):
+        many = many_tokens(T, N)
+        if many or half_round(T, N, K):
             s = _scratch_for(x.device)
             lib = _lib("mb_gemm_tc")
             carried = None
@@ -568,9 +571,10 @@ def gemm(x, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False, then_n
                 if slots * T <= s.sumsq.numel():
                     carried = NormedRows(then_norm.rows, s.sumsq, slots, N, then_norm.eps)
             if carried is None and scaled is None:
-                _persistent_product(x, w, out, mode, T, N, K, s, "gemm (tensor cores, persistent)")
+                _persistent_product(x, w, out, mode, T, N, K, s, "gemm (tensor cores, persistent)", not many)
                 return None
-            tile, sums = _whole_tiles(persistent_plan(T, N), T, N, K)
+            tile = persistent_plan(T, N)
+            tile, sums = (tile, 1) if many else _whole_tiles(tile, T, N, K)
             _check(lib.mb_gemm_tc_persistent_coupled(
                 _ptr(x), _ptr(w), _ptr(out), _c_int(mode), _c_int(T), _c_int(N), _c_int(K), _c_int(tile), _c_int(SM_COUNT), _c_int(sums),
                 _ptr(then_norm.weight) if carried is not None else None, _c_int(int(then_norm.unit_offset)) if carried is not None else _c_int(0),
@@ -699,7 +703,11 @@ def gemm_qkv_heads(x, w: torch.Tensor, q_out: torch.Tensor, q_weight, k_weight, 
         table = rope_table(ctx, positions, inv_freq) if inv_freq is not None else None
         _cost(_size(w) + _size(rows) + T * N * 2 + (_size(table) if table is not None else 0), 2.0 * T * N * Kdim)
         s = _scratch_for(rows.device)
-        tile, sums = _whole_tiles(paired_plan(T, N, Kdim), T, N, Kdim)
+        tile, sums = paired_plan(T, N, Kdim), 1
+        if -(-N // 128) * -(-T // 128) < SM_COUNT // 2:
+            # (from half a round of tiles on heads have one sum, rounded to bfloat16 at once: a second takes 0.7 us, 300 tokens of 16 + 16 heads 12.3 for 11.6;
+            # below it K was cut into four slices while the heads had a kernel of their own, and has as many sums)
+            tile, sums = _whole_tiles(tile, T, N, Kdim)
         _check(_lib("mb_gemm_tc").mb_gemm_tc_persistent_heads(
             _ptr(rows), _ptr(w), _c_int(T), _c_int(N), _c_int(Kdim), _c_int(tile), _c_int(SM_COUNT), _c_int(sums), _ptr(q_out),
             _ptr(k_cache) if write_kv else None, _ptr(v_cache) if write_kv else None, _ptr(q_weight), _ptr(k_weight), _c_float(eps),
